@@ -22,10 +22,10 @@
 //            come pre-permuted from global memory (L1-resident weights).  The
 //            backward-data pass is the same kernel with the transposed,
 //            tap-mirrored weights and a ReLU-gate epilogue.
-//   k_wgrad  dW[tap] = X(shifted)^T dZ: one CTA per (tap, voxel slab), the
-//            chunk of X and dZ staged in shared memory and fed to the tensor
-//            cores with ldmatrix.trans; per-slab partials summed in fixed
-//            order (deterministic).
+//   k_wgrad  dW[tap] = X(shifted)^T dZ for all 27 taps at once: tiles of X
+//            (with halo) and dZ staged in shared memory and fed to the
+//            tensor cores with ldmatrix.trans; per-CTA partials summed in
+//            fixed order (deterministic).
 //   small elementwise kernels: input, pooling, upsample+concat and their
 //            backward forms, the output layer + loss, Adam, weight layouts.
 
@@ -508,111 +508,193 @@ __global__ void k_wprep_tc(const float* __restrict__ W, int cin, int cout, int t
 }  // namespace tc
 
 // ---------------------------------------------------------------------------
-// Weight gradient: part[slab][tap][ci][co] = sum over the slab's voxels v of
+// Weight gradient: part[s][tap][ci][co] = sum over CTA s's voxels v of
 // X[v + off(tap)][ci] * dZ[v][co].
+//
+// A CTA owns 16 input and CO output channels and the nine taps of one dz
+// (blockIdx.y), and a contiguous range of 8 x 16 x 2 voxel tiles.  It stages
+// a tile's X with a one-voxel halo in x and y and its dZ in shared memory
+// once for the nine taps, the next tile's copies in flight meanwhile.  Six
+// warps: one per dx and half of the output channels; a K step of the MMA is
+// the 8 x 2 (x, z) voxels of one row y.  Walking up the rows, the X fragment
+// of row Y meets the dZ fragments of rows Y + 1, Y, Y - 1 (the taps
+// dy = -1, 0, 1), of which two are still in registers, so one ldmatrix of
+// each operand feeds 3 CO / 16 MMAs: the kernel is bound by the warp-level
+// MMAs, not by shared memory.  The sums of a tap stay in registers over the
+// whole range; the partials are folded in a fixed order by k_wgrad_sum.
+// One CTA per tap, each staging both
+// operands again, took 455 us (16 -> 16) and 1097 us (48 -> 16) at 96^3; now
+// 64 and 195 us (190 TFLOP/s), with 3.2 TB/s of staging out of L2.  Nine
+// warps for all three dz of a tile staged once (fewer bytes, but three times
+// as many ranges for the same warps) took 57 and 150 us; its shorter sums
+// move the gradient of a 48 -> 16 layer by 2.2e-5 of its norm, beyond what
+// two orders of one FP32 sum should differ by.
+constexpr int kWgThreads = 192;
+constexpr int kWgX = 8, kWgY = 16, kWgZ = 2;  // tile (voxels)
+constexpr int kWgBX = kWgX + 2, kWgBY = kWgY + 2;
+constexpr int kWgBrick = kWgBX * kWgBY * kWgZ, kWgTile = kWgX * kWgY * kWgZ;
+constexpr int kWgXS = 16 * 2 + 16;  // bytes per staged X voxel (the pad keeps ldmatrix rows off each other's banks)
+__host__ __device__ constexpr int wg_zs(int co) { return co * 2 + 16; }
+__host__ __device__ constexpr int wg_stage(int co) { return kWgBrick * kWgXS + kWgTile * wg_zs(co); }
+__host__ __device__ constexpr int wg_co(int cout) { return cout < 32 ? cout : 32; }  // output channels of a CTA
+// Resident CTAs per SM: three where a layer has few channel blocks; two for
+// the wide layers (more than 32 input channels), whose partials are largest.
+constexpr int kWgCtasPerSm = 3;
+constexpr int wg_ctas_per_sm(int cin) { return cin > 32 ? 2 : kWgCtasPerSm; }
 
-constexpr int kWgChunk = 64;  // voxels staged per step
+struct WgGeom {
+    int D, H, W;
+    int cin, cout;
+    int tiles_x, tiles_y, tiles;
+};
 
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) k_wgrad(const bf16* __restrict__ X, const bf16* __restrict__ dZ,
-                                               float* __restrict__ part, int D, int H, int W, i64 slab) {
-    constexpr int MTL = CIN / 16, NTL = COUT / 8, U = MTL * NTL;
-    static_assert(U < 8 || U % 8 == 0, "tile count must be < 8 or a multiple of 8");
-    constexpr int G = U >= 8 ? 1 : (8 % U == 0 ? 8 / U : 1);  // warps sharing a tile (k split)
-    constexpr int UPW = U >= 8 ? U / 8 : 1;                   // tiles per warp
-    constexpr int XS = CIN * 2 + 16, ZS = COUT * 2 + 16;      // smem bytes per voxel row
-    constexpr int XV = CIN / 8, ZV = COUT / 8;                // 16-byte vectors per voxel
-    __shared__ __align__(16) unsigned char xs[kWgChunk * XS];
-    __shared__ __align__(16) unsigned char zs[kWgChunk * ZS];
-    __shared__ float red[8][128];
-    const int tap = blockIdx.x;
-    const int oz = tap / 9 - 1, oy = (tap / 3) % 3 - 1, ox = tap % 3 - 1;
-    const i64 V = (i64)D * H * W;
-    const i64 v0 = (i64)blockIdx.y * slab;
-    const i64 v1 = min(V, v0 + slab);
+__device__ __forceinline__ void cp16_or_zero(uint32_t dst, const void* src, bool valid) {
+    const int n = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+
+template <int CO>
+__global__ void __launch_bounds__(kWgThreads, kWgCtasPerSm)
+    k_wgrad(const bf16* __restrict__ X, const bf16* __restrict__ dZ, float* __restrict__ part, WgGeom G) {
+    constexpr int ZV = CO / 8, NT = CO / 16, ZS = wg_zs(CO);  // 16-byte vectors per dZ voxel; n-tiles of a warp
+    static_assert(NT == 1 || NT == 2, "a warp owns one or two n-tiles");
+    extern __shared__ __align__(16) unsigned char wg_smem_raw[];
+    const uint32_t base = smem_addr(wg_smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kslot = warp % G;
-    const int tile0 = U >= 8 ? warp : warp / G;
-    const bool active = U >= 8 || tile0 < U;
-    const uint32_t xb = smem_addr(xs), zb = smem_addr(zs);
-    float acc[UPW][4];
+    const int dx = warp % 3, nh = warp / 3;
+    const int dz = blockIdx.y % 3, chunk = blockIdx.y / 3;
+    const int ci0 = chunk % (G.cin / 16) * 16, co0 = chunk / (G.cin / 16) * CO;
+    const int t_lo = (int)((i64)G.tiles * blockIdx.x / gridDim.x);
+    const int t_hi = (int)((i64)G.tiles * (blockIdx.x + 1) / gridDim.x);
+    // this lane's ldmatrix rows: X voxel (lane & 7, z lane >> 4), channel half
+    // (lane >> 3) & 1; dZ voxel (lane & 7, z (lane >> 3) & 1), n-tile lane >> 4
+    // (one n-tile: the upper lanes' addresses are not used)
+    const uint32_t a_row = (((lane >> 4) * kWgBY) * kWgBX + (lane & 7) + dx) * kWgXS + ((lane >> 3) & 1) * 16;
+    const uint32_t b_row = kWgBrick * kWgXS + ((((lane >> 3) & 1) * kWgY) * kWgX + (lane & 7)) * ZS +
+                           (nh * NT + (NT == 2 ? lane >> 4 : 0)) * 16;
+    auto origin = [&](int tile, int& x0, int& y0, int& z0) {
+        const int r = tile / G.tiles_x;
+        x0 = (tile - r * G.tiles_x) * kWgX;
+        z0 = r / G.tiles_y;
+        y0 = (r - z0 * G.tiles_y) * kWgY;
+        z0 *= kWgZ;
+    };
+    auto stage = [&](int tile, int slot) {
+        int x0, y0, z0;
+        origin(tile, x0, y0, z0);
+        const uint32_t xb = base + slot * wg_stage(CO), zb = xb + kWgBrick * kWgXS;
+        for (int i = threadIdx.x; i < kWgBrick * 2; i += kWgThreads) {
+            const int hf = i & 1, v = i >> 1;
+            const int bx = v % kWgBX, q = v / kWgBX, by = q % kWgBY, bz = q / kWgBY;
+            const int gx = x0 + bx - 1, gy = y0 + by - 1, gz = z0 + bz + dz - 1;
+            const bool in = (unsigned)gx < (unsigned)G.W && (unsigned)gy < (unsigned)G.H && (unsigned)gz < (unsigned)G.D;
+            const size_t o = in ? (((size_t)gz * G.H + gy) * G.W + gx) * G.cin + ci0 + hf * 8 : 0;
+            cp16_or_zero(xb + v * kWgXS + hf * 16, X + o, in);
+        }
+        for (int i = threadIdx.x; i < kWgTile * ZV; i += kWgThreads) {
+            const int p = i % ZV, v = i / ZV;
+            const int gx = x0 + v % kWgX, q = v / kWgX, gy = y0 + q % kWgY, gz = z0 + q / kWgY;
+            const bool in = gx < G.W && gy < G.H && gz < G.D;
+            const size_t o = in ? (((size_t)gz * G.H + gy) * G.W + gx) * G.cout + co0 + p * 8 : 0;
+            cp16_or_zero(zb + v * ZS + p * 16, dZ + o, in);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[3][NT][4];
 #pragma unroll
-    for (int u = 0; u < UPW; ++u)
+    for (int t = 0; t < 3; ++t)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[u][j] = 0.f;
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[t][n][j] = 0.f;
 
-    for (i64 c0 = v0; c0 < v1; c0 += kWgChunk) {
+    if (t_lo < t_hi) stage(t_lo, 0);
+    for (int tile = t_lo; tile < t_hi; ++tile) {
+        const int slot = (tile - t_lo) & 1;
+        if (tile + 1 < t_hi) {
+            stage(tile + 1, slot ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
         __syncthreads();
-        for (int i = threadIdx.x; i < kWgChunk * (XV + ZV); i += 256) {
-            const bool isx = i < kWgChunk * XV;
-            const int j = isx ? i : i - kWgChunk * XV;
-            const int vox = isx ? j / XV : j / ZV, prt = isx ? j % XV : j % ZV;
-            const i64 v = c0 + vox;
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (v < v1) {
-                if (isx) {
-                    const int x = (int)(v % W);
-                    const i64 r = v / W;
-                    const int y = (int)(r % H), z = (int)(r / H);
-                    const int xx = x + ox, yy = y + oy, zz = z + oz;
-                    if ((unsigned)xx < (unsigned)W && (unsigned)yy < (unsigned)H && (unsigned)zz < (unsigned)D)
-                        val = __ldg(reinterpret_cast<const uint4*>(X + (((size_t)zz * H + yy) * W + xx) * CIN + prt * 8));
+        int x0, y0, z0;
+        origin(tile, x0, y0, z0);
+        const uint32_t ab = base + slot * wg_stage(CO) + a_row, bb = base + slot * wg_stage(CO) + b_row;
+        const int rows = min(kWgY, G.H - y0);  // dZ rows of the tile inside the grid
+        uint32_t b[3][NT][2];                  // dZ fragments of the last three rows, row r in b[r % 3]
+        // X row y0 - 1 + by against dZ rows by - 1 - dy; cur = by % 3
+        auto step = [&](int by, int cur, bool top, bool mid, bool low) {
+            uint32_t a[4];
+            ldsm_x4_t(a, ab + by * (kWgBX * kWgXS));
+            if (top) {
+                if (NT == 2) {
+                    uint32_t f[4];
+                    ldsm_x4_t(f, bb + by * (kWgX * ZS));
+                    b[cur][0][0] = f[0];
+                    b[cur][0][1] = f[1];
+                    b[cur][NT - 1][0] = f[2];
+                    b[cur][NT - 1][1] = f[3];
                 } else {
-                    val = __ldg(reinterpret_cast<const uint4*>(dZ + (size_t)v * COUT + prt * 8));
+                    ldsm_x2_t(b[cur][0][0], b[cur][0][1], bb + by * (kWgX * ZS));
                 }
+#pragma unroll
+                for (int n = 0; n < NT; ++n) mma_bf16(acc[0][n], a, b[cur][n][0], b[cur][n][1]);
             }
-            *reinterpret_cast<uint4*>((isx ? xs + vox * XS : zs + vox * ZS) + prt * 16) = val;
-        }
-        __syncthreads();
-        if (active) {
-            for (int ks = kslot; ks < kWgChunk / 16; ks += G) {
+            const int p1 = (cur + 2) % 3, p2 = (cur + 1) % 3;
+            if (mid) {
 #pragma unroll
-                for (int u = 0; u < UPW; ++u) {
-                    const int tile = U >= 8 ? warp + 8 * u : tile0;
-                    const int mi = tile / NTL, ni = tile % NTL;
-                    uint32_t a[4];
-                    ldsm_x4_t(a, xb + (ks * 16 + (lane >> 4) * 8 + (lane & 7)) * XS + (mi * 16 + ((lane >> 3) & 1) * 8) * 2);
-                    uint32_t b0, b1;
-                    ldsm_x2_t(b0, b1, zb + (ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * ZS + ni * 16);
-                    mma_bf16(acc[u], a, b0, b1);
-                }
+                for (int n = 0; n < NT; ++n) mma_bf16(acc[1][n], a, b[p1][n][0], b[p1][n][1]);
+            }
+            if (low) {
+#pragma unroll
+                for (int n = 0; n < NT; ++n) mma_bf16(acc[2][n], a, b[p2][n][0], b[p2][n][1]);
+            }
+        };
+        if (rows == kWgY) {  // no branch between the rows: the loads of later rows move up
+#pragma unroll
+            for (int by = 0; by < kWgY + 2; ++by) step(by, by % 3, by < kWgY, by >= 1 && by <= kWgY, by >= 2);
+        } else {
+#pragma unroll 1
+            for (int by = 0; by < rows + 2; by += 3) {
+                step(by, 0, by < rows, by >= 1 && by <= rows, by >= 2);
+                if (by + 1 < rows + 2) step(by + 1, 1, by + 1 < rows, by + 1 <= rows, by >= 1);
+                if (by + 2 < rows + 2) step(by + 2, 2, by + 2 < rows, by + 2 <= rows, true);
             }
         }
+        __syncthreads();  // this slot may be staged again
     }
-    if (G > 1) {
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < 4; ++j) red[warp][lane * 4 + j] = acc[0][j];
-        __syncthreads();
-        if (kslot != 0 || !active) return;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float s = 0.f;
-            for (int k = 0; k < G; ++k) s += red[warp + k][lane * 4 + j];
-            acc[0][j] = s;
-        }
-    }
-    if (!active) return;
-    float* out = part + ((size_t)blockIdx.y * 27 + tap) * CIN * COUT;
     const int g = lane >> 2, tq = lane & 3;
 #pragma unroll
-    for (int u = 0; u < UPW; ++u) {
-        const int tile = U >= 8 ? warp + 8 * u : tile0;
-        const int ci = (tile / NTL) * 16 + g, co = (tile % NTL) * 8 + 2 * tq;
-        out[ci * COUT + co] = acc[u][0];
-        out[ci * COUT + co + 1] = acc[u][1];
-        out[(ci + 8) * COUT + co] = acc[u][2];
-        out[(ci + 8) * COUT + co + 1] = acc[u][3];
+    for (int t = 0; t < 3; ++t) {
+        const int tap = dz * 9 + t * 3 + dx;
+        float* out = part + (((size_t)blockIdx.x * 27 + tap) * G.cin + ci0) * G.cout + co0;
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            const int co = (nh * NT + n) * 8 + 2 * tq;
+            *reinterpret_cast<float2*>(out + g * G.cout + co) = make_float2(acc[t][n][0], acc[t][n][1]);
+            *reinterpret_cast<float2*>(out + (g + 8) * G.cout + co) = make_float2(acc[t][n][2], acc[t][n][3]);
+        }
     }
 }
 
-// grad[i] += sum_s part[s][i], s in order.
-__global__ void k_wgrad_sum(const float* __restrict__ part, int S, int n, float* __restrict__ grad) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int k = 0; k < S; ++k) s += part[(size_t)k * n + i];
-        grad[i] += s;
-    }
+// grad[i] += sum_s part[s][i]: eight interleaved runs of s, each in order,
+// then the eight in order (32 outputs per block, so the reads are whole
+// 128-byte lines and S / 8 loads follow one another instead of S).
+__global__ void __launch_bounds__(256) k_wgrad_sum(const float* __restrict__ part, int S, int n,
+                                                   float* __restrict__ grad) {
+    __shared__ float sm[8][32];
+    const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;  // n is a multiple of 32
+    float s = 0.f;
+#pragma unroll 4
+    for (int k = seg; k < S; k += 8) s += __ldg(part + (size_t)k * n + i);
+    sm[seg][lane] = s;
+    __syncthreads();
+    if (seg) return;
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += sm[k][lane];
+    grad[i] += s;
 }
 
 // ---------------------------------------------------------------------------
@@ -942,7 +1024,6 @@ struct pg_unet {
     double* red = nullptr;  // reduction partials
     double* loss = nullptr;
     float* wpart = nullptr;
-    int wslabs = 0;
     double out_scale = 1.0;
     i64 adam_t = 0;
 };
@@ -1071,34 +1152,40 @@ int conv(const pg_unet* net, int lvl, int cin, int cout, const bf16* in, const u
     return bad_arg("pg_unet: no conv kernel for this channel pair");
 }
 
-template <int CIN, int COUT>
-int wgrad_t(pg_unet* net, int lvl, const bf16* X, const bf16* dZ, float* grad) {
-    const int D = net->ld[lvl], H = net->lh[lvl], W = net->lw[lvl];
-    const i64 V = net->lv[lvl];
-    int S = std::max(1, std::min(net->wslabs, ceil_div(V, kWgChunk)));
-    const i64 slab = (i64)ceil_div(ceil_div(V, S), kWgChunk) * kWgChunk;
-    S = ceil_div(V, slab);
-    const int n = 27 * CIN * COUT;
-    PG_LAUNCH(KK_UNET_WGRAD, net->stream, k_wgrad<CIN, COUT><<<dim3(27, S), 256, 0, net->stream>>>(X, dZ, net->wpart, D, H, W, slab));
-    PG_LAUNCH(KK_UNET_WGRAD, net->stream, k_wgrad_sum<<<ceil_div(n, 256), 256, 0, net->stream>>>(net->wpart, S, n, grad));
+int wg_tiles(const pg_unet* net, int lvl) {
+    return ceil_div(net->lw[lvl], kWgX) * ceil_div(net->lh[lvl], kWgY) * ceil_div(net->ld[lvl], kWgZ);
+}
+// CTAs (partial sums) per channel block of layer k's weight gradient.
+int wg_ctas(const pg_unet* net, int k) {
+    const int blocks = 3 * (kCin[k] / 16) * (kCout[k] / wg_co(kCout[k]));
+    return std::max(1, std::min(wg_tiles(net, kLevel[k]), wg_ctas_per_sm(kCin[k]) * net->num_sms / blocks));
+}
+
+template <int CO> int wgrad_t(pg_unet* net, int k, const bf16* X, const bf16* dZ) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        PG_CUDA(cudaFuncSetAttribute(k_wgrad<CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * wg_stage(CO)));
+        attr_set = true;
+    }
+    const int lvl = kLevel[k], S = wg_ctas(net, k), n = 27 * kCin[k] * kCout[k];
+    WgGeom G;
+    G.D = net->ld[lvl];
+    G.H = net->lh[lvl];
+    G.W = net->lw[lvl];
+    G.cin = kCin[k];
+    G.cout = kCout[k];
+    G.tiles_x = ceil_div(G.W, kWgX);
+    G.tiles_y = ceil_div(G.H, kWgY);
+    G.tiles = wg_tiles(net, lvl);
+    const dim3 grid(S, 3 * (kCin[k] / 16) * (kCout[k] / CO));
+    PG_LAUNCH(KK_UNET_WGRAD, net->stream, k_wgrad<CO><<<grid, kWgThreads, 2 * wg_stage(CO), net->stream>>>(X, dZ, net->wpart, G));
+    PG_LAUNCH(KK_UNET_WGRAD, net->stream, k_wgrad_sum<<<n / 32, 256, 0, net->stream>>>(net->wpart, S, n, net->grads + param_offset(k)));
     PG_CHECK_LAUNCH();
     return PG_OK;
 }
 
 int wgrad(pg_unet* net, int k, const bf16* X, const bf16* dZ) {
-    float* grad = net->grads + param_offset(k);
-    const int lvl = kLevel[k];
-#define PG_UNET_WG(A, B) \
-    if (kCin[k] == A && kCout[k] == B) return wgrad_t<A, B>(net, lvl, X, dZ, grad);
-    PG_UNET_WG(16, 16)
-    PG_UNET_WG(16, 32)
-    PG_UNET_WG(32, 32)
-    PG_UNET_WG(32, 64)
-    PG_UNET_WG(64, 64)
-    PG_UNET_WG(96, 32)
-    PG_UNET_WG(48, 16)
-#undef PG_UNET_WG
-    return bad_arg("pg_unet: no weight-gradient kernel for this layer");
+    return wg_co(kCout[k]) == 16 ? wgrad_t<16>(net, k, X, dZ) : wgrad_t<32>(net, k, X, dZ);
 }
 
 int prep_weights(pg_unet* net) {
@@ -1358,7 +1445,6 @@ int pg_unet_create(int64_t d, int64_t h, int64_t w, pg_unet** out) {
         net->lv[l] = (i64)net->ld[l] * net->lh[l] * net->lw[l];
     }
     const i64 P = num_params();
-    net->wslabs = std::max(1, 4 * net->num_sms / 27);
     // Arena layout (256-byte aligned pieces).
     std::vector<std::pair<void**, size_t>> parts;
     auto add = [&](void** p, size_t bytes) { parts.push_back({p, (bytes + 255) & ~(size_t)255}); };
@@ -1396,7 +1482,9 @@ int pg_unet_create(int64_t d, int64_t h, int64_t w, pg_unet** out) {
     add((void**)&net->scal, 32);
     add((void**)&net->red, 8 * std::max(kRedBlocks, kHeadBlocks * 17));
     add((void**)&net->loss, 8);
-    add((void**)&net->wpart, 4 * (size_t)net->wslabs * 27 * 96 * 64);
+    size_t wp = 0;
+    for (int k = 0; k < kL; ++k) wp = std::max(wp, (size_t)wg_ctas(net, k) * 27 * kCin[k] * kCout[k]);
+    add((void**)&net->wpart, 4 * wp);
     size_t total = 0;
     for (auto& p : parts) total += p.second;
     cudaError_t e = cudaMalloc(&net->arena, total);
