@@ -11,8 +11,9 @@
 //     += src[i] * low[f] + src[i + half] * high[f]; here each output gathers
 //     its contributions and adds them in the reference's (i, f) order, so
 //     the sums round the same way.
-// The level loops, the copies to the temporary and the axis orders are
-// those of fwt_1d / ifwt_1d / fwt_2d_isotropic / ifwt_2d_isotropic /
+// Lines of at least twice the filter length take the kernels of
+// pg_wavelet_pass.cuh instead (the same bits).  The level loops and the axis
+// orders are those of fwt_1d / ifwt_1d / fwt_2d_isotropic / ifwt_2d_isotropic /
 // fwt_2d_separate_isotropic / ifwt_2d_separate_isotropic /
 // fwt_2d_anisotropic (mod.rs:114-294); div_coeff_2d / inv_div_coeff_2d
 // (mod.rs:296-451) are one launch per level.  The border variants
@@ -22,6 +23,7 @@
 
 #include "pg_internal.cuh"
 #include "pg_wavelet_border.cuh"
+#include "pg_wavelet_pass.cuh"
 
 namespace pg {
 
@@ -187,14 +189,36 @@ __global__ void k_wcopy_flat(const double* __restrict__ src, double* __restrict_
 
 int wblocks(i64 n) { return (int)std::max<i64>(1, std::min<i64>((n + kWThreads - 1) / kWThreads, 4096)); }
 
-int down(cudaStream_t s, const double* src, double* dst, i64 lines, i64 len, i64 ls, i64 es, const WFilter& F) {
-    PG_LAUNCH(KK_DEC_OP, s, k_wdown<<<wblocks(lines * len), kWThreads, 0, s>>>(src, dst, lines, len, ls, es, F));
-    PG_CHECK_LAUNCH();
-    return PG_OK;
-}
-int up(cudaStream_t s, const double* src, double* dst, i64 lines, i64 len, i64 ls, i64 es, const WFilter& F) {
-    PG_LAUNCH(KK_DEC_OP, s, k_wup<<<wblocks(lines * len), kWThreads, 0, s>>>(src, dst, lines, len, ls, es, F));
-    PG_CHECK_LAUNCH();
+// One 1D pass src -> dst (distinct arrays) over a block's lines, by the pass
+// kernels of pg_wavelet_pass.cuh or, for lines shorter than twice the filter,
+// the per-sample kernels above.
+struct Pass {
+    cudaStream_t s;
+    int num_sms;
+    int run(bool down, int wavelet, const double* src, double* dst, i64 lines, i64 len, i64 ls, i64 es) const {
+        const wv::PassShape shape{lines, len, es == 1 ? ls : es, es == 1};
+        bool done = false;
+        PG_LAUNCH(KK_DEC_OP, s, done = wv::pass_run(s, num_sms, wavelet, down, src, dst, shape));
+        if (!done) {
+            const WFilter F = wv::kFilters[wavelet];
+            if (down)
+                PG_LAUNCH(KK_DEC_OP, s, k_wdown<<<wblocks(lines * len), kWThreads, 0, s>>>(src, dst, lines, len, ls, es, F));
+            else
+                PG_LAUNCH(KK_DEC_OP, s, k_wup<<<wblocks(lines * len), kWThreads, 0, s>>>(src, dst, lines, len, ls, es, F));
+        }
+        PG_CHECK_LAUNCH();
+        return PG_OK;
+    }
+    int down_x(int wl, const double* src, double* dst, i64 r, i64 c, i64 w) const { return run(true, wl, src, dst, r, c, w, 1); }
+    int down_y(int wl, const double* src, double* dst, i64 r, i64 c, i64 w) const { return run(true, wl, src, dst, c, r, 1, w); }
+    int up_x(int wl, const double* src, double* dst, i64 r, i64 c, i64 w) const { return run(false, wl, src, dst, r, c, w, 1); }
+    int up_y(int wl, const double* src, double* dst, i64 r, i64 c, i64 w) const { return run(false, wl, src, dst, c, r, 1, w); }
+};
+int make_pass(void* stream, Pass* p) {
+    p->s = (cudaStream_t)stream;
+    int dev = 0;
+    PG_CUDA(cudaGetDevice(&dev));
+    PG_CUDA(cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, dev));
     return PG_OK;
 }
 int copy(cudaStream_t s, const double* src, double* dst, i64 rows, i64 cols, i64 w) {
@@ -257,10 +281,11 @@ int pg_wavelet_fwt_1d(int wavelet, double* data, int64_t n, int levels, double* 
     if (!filter_of(wavelet, &F)) return bad_arg("pg_wavelet_fwt_1d: unknown wavelet");
     int rc;
     if ((rc = check_levels(n, levels, F))) return rc;
-    cudaStream_t s = (cudaStream_t)stream;
+    Pass p;
+    if ((rc = make_pass(stream, &p))) return rc;
     i64 size = n;
     for (int k = 0; k < levels; ++k) {  // mod.rs:114-129
-        if ((rc = copy(s, data, temp, 1, size, size)) || (rc = down(s, temp, data, 1, size, 0, 1, F))) return rc;
+        if ((rc = copy(p.s, data, temp, 1, size, size)) || (rc = p.down_x(wavelet, temp, data, 1, size, size))) return rc;
         size /= 2;
     }
     return PG_OK;
@@ -272,11 +297,12 @@ int pg_wavelet_ifwt_1d(int wavelet, double* data, int64_t n, int levels, double*
     if (!filter_of(wavelet, &F)) return bad_arg("pg_wavelet_ifwt_1d: unknown wavelet");
     int rc;
     if ((rc = check_levels(n, levels, F))) return rc;
-    cudaStream_t s = (cudaStream_t)stream;
+    Pass p;
+    if ((rc = make_pass(stream, &p))) return rc;
     i64 size = n >> levels;
     for (int k = 0; k < levels; ++k) {  // mod.rs:131-143
         size *= 2;
-        if ((rc = copy(s, data, temp, 1, size, size)) || (rc = up(s, temp, data, 1, size, 0, 1, F))) return rc;
+        if ((rc = copy(p.s, data, temp, 1, size, size)) || (rc = p.up_x(wavelet, temp, data, 1, size, size))) return rc;
     }
     return PG_OK;
 }
@@ -288,12 +314,12 @@ int pg_wavelet_fwt_2d(int mode, int wavelet_x, int wavelet_y, double* data, int6
     if (!filter_of(wavelet_x, &Fx) || !filter_of(wavelet_y, &Fy)) return bad_arg("pg_wavelet_fwt_2d: unknown wavelet");
     int rc;
     if ((rc = check_levels(h, levels, Fy)) || (rc = check_levels(w, levels, Fx))) return rc;
-    cudaStream_t s = (cudaStream_t)stream;
+    Pass p;
+    if ((rc = make_pass(stream, &p))) return rc;
     if (mode == PG_WAVELET_ISOTROPIC) {  // mod.rs:145-170, 206-231
         i64 r = h, c = w;
         for (int k = 0; k < levels; ++k) {
-            if ((rc = copy(s, data, temp, r, c, w)) || (rc = down(s, temp, data, r, c, w, 1, Fx))) return rc;
-            if ((rc = copy(s, data, temp, r, c, w)) || (rc = down(s, temp, data, c, r, 1, w, Fy))) return rc;
+            if ((rc = p.down_x(wavelet_x, data, temp, r, c, w)) || (rc = p.down_y(wavelet_y, temp, data, r, c, w))) return rc;
             r /= 2;
             c /= 2;
         }
@@ -302,13 +328,13 @@ int pg_wavelet_fwt_2d(int mode, int wavelet_x, int wavelet_y, double* data, int6
     if (mode == PG_WAVELET_ANISOTROPIC) {  // mod.rs:262-294
         i64 r = h, c = w;
         for (int k = 0; k < levels; ++k) {  // x: every row, the coarse prefix halving
-            if ((rc = copy(s, data, temp, r, c, w)) || (rc = down(s, temp, data, r, c, w, 1, Fx))) return rc;
+            if ((rc = copy(p.s, data, temp, r, c, w)) || (rc = p.down_x(wavelet_x, temp, data, r, c, w))) return rc;
             c /= 2;
         }
         r = h;
         c = w;
         for (int k = 0; k < levels; ++k) {  // y: every column, the coarse prefix halving
-            if ((rc = copy(s, data, temp, r, c, w)) || (rc = down(s, temp, data, c, r, 1, w, Fy))) return rc;
+            if ((rc = copy(p.s, data, temp, r, c, w)) || (rc = p.down_y(wavelet_y, temp, data, r, c, w))) return rc;
             r /= 2;
         }
         return PG_OK;
@@ -323,17 +349,16 @@ int pg_wavelet_ifwt_2d(int mode, int wavelet_x, int wavelet_y, double* data, int
     if (!filter_of(wavelet_x, &Fx) || !filter_of(wavelet_y, &Fy)) return bad_arg("pg_wavelet_ifwt_2d: unknown wavelet");
     int rc;
     if ((rc = check_levels(h, levels, Fy)) || (rc = check_levels(w, levels, Fx))) return rc;
-    cudaStream_t s = (cudaStream_t)stream;
+    Pass p;
+    if ((rc = make_pass(stream, &p))) return rc;
     i64 r = h >> levels, c = w >> levels;
     for (int k = 0; k < levels; ++k) {
         r *= 2;
         c *= 2;
         if (mode == PG_WAVELET_ISOTROPIC) {  // mod.rs:172-204: y, then x
-            if ((rc = copy(s, data, temp, r, c, w)) || (rc = up(s, temp, data, c, r, 1, w, Fy))) return rc;
-            if ((rc = copy(s, data, temp, r, c, w)) || (rc = up(s, temp, data, r, c, w, 1, Fx))) return rc;
+            if ((rc = p.up_y(wavelet_y, data, temp, r, c, w)) || (rc = p.up_x(wavelet_x, temp, data, r, c, w))) return rc;
         } else if (mode == PG_WAVELET_SEPARATE) {  // mod.rs:233-260: x, then y
-            if ((rc = copy(s, data, temp, r, c, w)) || (rc = up(s, temp, data, r, c, w, 1, Fx))) return rc;
-            if ((rc = copy(s, data, temp, r, c, w)) || (rc = up(s, temp, data, c, r, 1, w, Fy))) return rc;
+            if ((rc = p.up_x(wavelet_x, data, temp, r, c, w)) || (rc = p.up_y(wavelet_y, temp, data, r, c, w))) return rc;
         } else {
             return bad_arg("pg_wavelet_ifwt_2d: mode must be ISOTROPIC or SEPARATE");
         }

@@ -16,7 +16,6 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <initializer_list>
 #include <vector>
 
 #include "panopaea_gpu.h"
@@ -45,41 +44,25 @@ constexpr double kG = 0.06629126073623884;
 constexpr double kH = 0.4198446513295126;
 constexpr double kI = 0.9943689110435825;
 
+// By PG_WAVELET_*: taps, then analysis low / high and synthesis low / high.
+constexpr WFilter kFilters[5] = {
+    {2, {kS, kS}, {-kS, kS}, {kS, kS}, {kS, -kS}},
+    {6, {-kA, kA, kS, kS, kA, -kA}, {0, 0, -kS, kS, 0, 0}, {0, 0, kS, kS, 0, 0}, {-kA, -kA, kS, -kS, kA, kA}},
+    {6, {0, -kC, kB, kD, kB, -kC}, {0, kB, -kS, kB, 0, 0}, {0, kB, kS, kB, 0, 0}, {0, kC, kB, -kD, kB, kC}},
+    {10,
+     {0, kF, -kG, -kC, kH, kI, kH, -kC, -kG, kF},
+     {0, 0, 0, kB, -kS, kB, 0, 0, 0, 0},
+     {0, 0, 0, kB, kS, kB, 0, 0, 0, 0},
+     {0, -kF, -kG, kC, kH, -kI, kH, kC, -kG, -kF}},
+    {4, {-kB, kD, kD, -kB}, {-kC, kE, -kE, kC}, {kC, kE, kE, kC}, {-kB, -kD, kD, kB}},
+};
+static_assert(PG_WAVELET_HAAR == 0 && PG_WAVELET_BIOR13 == 1 && PG_WAVELET_BIOR22 == 2 && PG_WAVELET_BIOR24 == 3 &&
+                  PG_WAVELET_BIOR31 == 4,
+              "kFilters is indexed by these");
+
 inline bool filter_of(int wavelet, WFilter* out) {
-    WFilter f{};
-    auto set = [&](int n, std::initializer_list<double> ul, std::initializer_list<double> uh,
-                   std::initializer_list<double> dl, std::initializer_list<double> dh) {
-        f.n = n;
-        int k = 0;
-        for (double v : ul) f.up_low[k++] = v;
-        k = 0;
-        for (double v : uh) f.up_high[k++] = v;
-        k = 0;
-        for (double v : dl) f.down_low[k++] = v;
-        k = 0;
-        for (double v : dh) f.down_high[k++] = v;
-    };
-    switch (wavelet) {
-        case PG_WAVELET_HAAR:
-            set(2, {kS, kS}, {kS, -kS}, {kS, kS}, {-kS, kS});
-            break;
-        case PG_WAVELET_BIOR13:
-            set(6, {0, 0, kS, kS, 0, 0}, {-kA, -kA, kS, -kS, kA, kA}, {-kA, kA, kS, kS, kA, -kA}, {0, 0, -kS, kS, 0, 0});
-            break;
-        case PG_WAVELET_BIOR22:
-            set(6, {0, kB, kS, kB, 0, 0}, {0, kC, kB, -kD, kB, kC}, {0, -kC, kB, kD, kB, -kC}, {0, kB, -kS, kB, 0, 0});
-            break;
-        case PG_WAVELET_BIOR24:
-            set(10, {0, 0, 0, kB, kS, kB, 0, 0, 0, 0}, {0, -kF, -kG, kC, kH, -kI, kH, kC, -kG, -kF},
-                {0, kF, -kG, -kC, kH, kI, kH, -kC, -kG, kF}, {0, 0, 0, kB, -kS, kB, 0, 0, 0, 0});
-            break;
-        case PG_WAVELET_BIOR31:
-            set(4, {kC, kE, kE, kC}, {-kB, -kD, kD, kB}, {-kB, kD, kD, -kB}, {-kC, kE, -kE, kC});
-            break;
-        default:
-            return false;
-    }
-    *out = f;
+    if (wavelet < 0 || wavelet > 4) return false;
+    *out = kFilters[wavelet];
     return true;
 }
 
