@@ -55,8 +55,8 @@ template <class T>
 __device__ __forceinline__ void cg_init_finish(CgState* st, double* partials, double* sm, double thr, double rel_tol,
                                                i64 max_iter, double nfluid = 0.0) {
     if (!last_block(&st->counter[0])) return;
-    const double bmax = reduce_partials<true, kCgThreads>(partials, gridDim.x, sm);
-    const double sigma = reduce_partials<false, kCgThreads>(partials + kMaxBlocks, gridDim.x, sm);
+    double bmax, sigma;
+    reduce_partials_max0<kCgThreads>(partials, partials + kMaxBlocks, gridDim.x, sm, bmax, sigma);
     if (threadIdx.x == 0) {
         st->counter[0] = 0;
         // The stop test compares in T, as pcg.rs:35 / :60 do.
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_init(T* __restrict__ x, T* __
                                                           const uint8_t* __restrict__ flags, i64 n, T dt, double thr,
                                                           double rel_tol, i64 max_iter, int zero_x, CgState* st,
                                                           double* partials, double nfluid = 0.0) {
-    __shared__ double sm[32];
+    __shared__ double sm[kCgThreads + 32];
     Acc<T> sig;
     T bm = T(0);
     int bad = 0;
@@ -105,10 +105,10 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_init(T* __restrict__ x, T* __
         else sig.add(bv);  // sum(b) for the lazy projection
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&st->nan_seen, 1);
-    const double bsum = block_max<kCgThreads>((double)bm, sm);
-    const double ssum = block_sum<kCgThreads>(sig.value(), sm);
+    double ssum = sig.value();
+    block_max0_sum<kCgThreads>(bm, ssum, sm);
     if (threadIdx.x == 0) {
-        partials[blockIdx.x] = bsum;
+        partials[blockIdx.x] = (double)bm;
         partials[kMaxBlocks + blockIdx.x] = ssum;
     }
     cg_init_finish<T>(st, partials, sm, thr, rel_tol, max_iter, nfluid);
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kCgThreads)
     k_cg_init4(float4* __restrict__ x, float4* __restrict__ r, const float4* __restrict__ b, i64 n4, double thr,
                double rel_tol, i64 max_iter, int zero_x, CgState* st, double* partials, double nfluid,
                float4* __restrict__ xl) {
-    __shared__ double sm[32];
+    __shared__ double sm[kCgThreads + 32];
     float bm = 0.f;
     int bad = 0;
     float sb = 0.f;  // sum(b) for the lazy projection (feeds a small correction term)
@@ -138,10 +138,10 @@ __global__ void __launch_bounds__(kCgThreads)
         sb += (bv.x + bv.y) + (bv.z + bv.w);
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&st->nan_seen, 1);
-    const double bsum = block_max<kCgThreads>((double)bm, sm);
-    const double ssum = block_sum<kCgThreads>((double)sb, sm);
+    double ssum = (double)sb;
+    block_max0_sum<kCgThreads>(bm, ssum, sm);
     if (threadIdx.x == 0) {
-        partials[blockIdx.x] = bsum;
+        partials[blockIdx.x] = (double)bm;
         partials[kMaxBlocks + blockIdx.x] = ssum;
     }
     cg_init_finish<float>(st, partials, sm, thr, rel_tol, max_iter, nfluid);
@@ -152,16 +152,17 @@ template <class T, int ND, int PM>
 __global__ void __launch_bounds__(kCgThreads)
     k_cg_spmv(const T* __restrict__ r, const T* __restrict__ zb, T* p0, T* p1, T* __restrict__ ap,
               const uint8_t* __restrict__ flags, Dims D, T dt, CgState* st, double* partials) {
-    if (st->done) return;
-    __shared__ double sm[32];
+    __shared__ double sm[kCgThreads + 32];
     // Ping-pong by the device-side iteration count: iteration k reads
     // p[k & 1] and writes p[(k + 1) & 1] (so a CUDA graph can replay it).
-    const i64 k = *(volatile const i64*)&st->iter;
+    const CgHead H(st);
+    if (H.done) return;
+    const i64 k = H.iter;
     const T* __restrict__ p_old = (k & 1) ? p1 : p0;
     T* __restrict__ p_new = (k & 1) ? p0 : p1;
-    const int first = st->first;
-    const T beta = first ? T(0) : (T)st->beta;
-    const T zm = (PM == PM_ZBUF && st->nfluid > 0.0) ? (T)st->zmean : T(0);
+    const int first = H.first;
+    const T beta = first ? T(0) : (T)H.beta;
+    const T zm = (PM == PM_ZBUF && H.nfluid > 0.0) ? (T)H.zmean : T(0);
     const i64 n = D.nc(), w = D.w, hw = D.h * D.w;
     auto pn = [&](i64 k) -> T {
         const T z = zval<T, PM>(r, flags, zb, k, dt, zm);
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(kCgThreads)
     const double s = block_sum<kCgThreads>(acc.value(), sm);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
     if (!last_block(&st->counter[1])) return;
-    const double pap = reduce_partials<false, kCgThreads>(partials, gridDim.x, sm);
+    const double pap = reduce_partials<kCgThreads>(partials, gridDim.x, sm);
     if (threadIdx.x == 0) {
         st->counter[1] = 0;
         st->pap = pap;
@@ -220,15 +221,16 @@ __global__ void __launch_bounds__(kTX * kTY)
     k_cg_spmv3t(const T* __restrict__ r, const T* __restrict__ zb, T* p0, T* p1, T* __restrict__ ap,
                 const uint8_t* __restrict__ flags, Dims D, T dt, CgState* st, double* partials, int tiles_x,
                 int tiles_y, int zc, int nwork) {
-    if (st->done) return;
     __shared__ T S[kTY + 2][kTX + 2];
-    __shared__ double sm[32];
-    const i64 kit = *(volatile const i64*)&st->iter;
+    __shared__ double sm[kTX * kTY];
+    const CgHead H(st);
+    if (H.done) return;
+    const i64 kit = H.iter;
     const T* __restrict__ p_old = (kit & 1) ? p1 : p0;
     T* __restrict__ p_new = (kit & 1) ? p0 : p1;
-    const int first = st->first;
-    const T beta = first ? T(0) : (T)st->beta;
-    const T zm = (PM == PM_ZBUF && st->nfluid > 0.0) ? (T)st->zmean : T(0);
+    const int first = H.first;
+    const T beta = first ? T(0) : (T)H.beta;
+    const T zm = (PM == PM_ZBUF && H.nfluid > 0.0) ? (T)H.zmean : T(0);
     auto pn = [&](i64 k) -> T {
         const T z = zval<T, PM>(r, flags, zb, k, dt, zm);
         return first ? z : z + beta * p_old[k];
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(kTX * kTY)
     const double s = block_sum<kTX * kTY>(acc.value(), sm);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
     if (!last_block(&st->counter[1])) return;
-    const double pap = reduce_partials<false, kTX * kTY>(partials, gridDim.x, sm);
+    const double pap = reduce_partials<kTX * kTY>(partials, gridDim.x, sm);
     if (threadIdx.x == 0) {
         st->counter[1] = 0;
         st->pap = pap;
@@ -338,13 +340,14 @@ template <class T, int PM>
 __global__ void __launch_bounds__(kCgThreads)
     k_cg_update(T* __restrict__ x, T* __restrict__ r, const T* p0, const T* p1, const T* __restrict__ ap,
                 const uint8_t* __restrict__ flags, i64 n, T dt, CgState* st, double* partials) {
-    if (st->done) return;
-    __shared__ double sm[32];
+    __shared__ double sm[kCgThreads + 32];
     // The SpMV of this iteration wrote p[(iter + 1) & 1]; the last block
     // increments iter only after every block has read it here.
-    const i64 k = *(volatile const i64*)&st->iter;
+    const CgHead H(st);
+    if (H.done) return;
+    const i64 k = H.iter;
     const T* __restrict__ p = ((k + 1) & 1) ? p1 : p0;
-    const T alpha = (T)st->alpha, nalpha = -alpha;
+    const T alpha = (T)H.alpha, nalpha = -alpha;
     T rm = T(0);
     Acc<T> rz;
     int bad = 0;
@@ -358,15 +361,16 @@ __global__ void __launch_bounds__(kCgThreads)
         else rz.add(rv);  // sum(r) for the lazy projection
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&st->nan_seen, 1);
-    const double m = block_max<kCgThreads>((double)rm, sm);
-    const double s = block_sum<kCgThreads>(rz.value(), sm);
+    double s = rz.value();
+    block_max0_sum<kCgThreads>(rm, s, sm);
     if (threadIdx.x == 0) {
-        partials[2 * kMaxBlocks + blockIdx.x] = m;
+        partials[2 * kMaxBlocks + blockIdx.x] = (double)rm;
         partials[3 * kMaxBlocks + blockIdx.x] = s;
     }
     if (!last_block(&st->counter[2])) return;
-    const double rmax = reduce_partials<true, kCgThreads>(partials + 2 * kMaxBlocks, gridDim.x, sm);
-    const double sigma_new = reduce_partials<false, kCgThreads>(partials + 3 * kMaxBlocks, gridDim.x, sm);
+    double rmax, sigma_new;
+    reduce_partials_max0<kCgThreads>(partials + 2 * kMaxBlocks, partials + 3 * kMaxBlocks, gridDim.x, sm, rmax,
+                                     sigma_new);
     if (threadIdx.x == 0) {
         st->counter[2] = 0;
         const i64 it = st->iter + 1;
@@ -413,11 +417,12 @@ __global__ void __launch_bounds__(kCgThreads)
     k_cg_update4(float4* __restrict__ x, float4* __restrict__ r, const float4* p0, const float4* p1,
                  const float4* __restrict__ ap, i64 n4, CgState* st, double* partials, float4* __restrict__ xl,
                  const float4* __restrict__ b0) {
-    if (st->done) return;
-    __shared__ double sm[32];
-    const i64 k = *(volatile const i64*)&st->iter;
+    __shared__ double sm[kCgThreads + 32];
+    const CgHead H(st);
+    if (H.done) return;
+    const i64 k = H.iter;
     const float4* __restrict__ p = ((k + 1) & 1) ? p1 : p0;
-    const float alpha = (float)st->alpha, nalpha = -alpha;
+    const float alpha = (float)H.alpha, nalpha = -alpha;
     const bool first = b0 != nullptr && k == 0;  // uniform
     const float4* __restrict__ rin = first ? b0 : r;
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -458,15 +463,15 @@ __global__ void __launch_bounds__(kCgThreads)
     }
     if (c < n4) one(c);
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&st->nan_seen, 1);
-    const double m = block_max<kCgThreads>((double)rm, sm);
-    const double rsb = block_sum<kCgThreads>((double)rs, sm);
+    double rsb = (double)rs;
+    block_max0_sum<kCgThreads>(rm, rsb, sm);
     if (threadIdx.x == 0) {
-        partials[2 * kMaxBlocks + blockIdx.x] = m;
+        partials[2 * kMaxBlocks + blockIdx.x] = (double)rm;
         partials[3 * kMaxBlocks + blockIdx.x] = rsb;
     }
     if (!last_block(&st->counter[2])) return;
-    const double rmax = reduce_partials<true, kCgThreads>(partials + 2 * kMaxBlocks, gridDim.x, sm);
-    const double rsum = reduce_partials<false, kCgThreads>(partials + 3 * kMaxBlocks, gridDim.x, sm);
+    double rmax, rsum;
+    reduce_partials_max0<kCgThreads>(partials + 2 * kMaxBlocks, partials + 3 * kMaxBlocks, gridDim.x, sm, rmax, rsum);
     if (threadIdx.x == 0) {
         st->rsum = rsum;
         st->counter[2] = 0;
@@ -495,16 +500,17 @@ __global__ void __launch_bounds__(kCgThreads)
     k_cg_update4r(float4* __restrict__ x, float4* __restrict__ r, const float4* p0, const float4* p1,
                   const float4* __restrict__ ap, const uchar4* __restrict__ flags, i64 n4, float dt, CgState* st,
                   double* partials) {
-    if (st->done) return;
-    __shared__ double sm[32];
+    __shared__ double sm[kCgThreads + 32];
+    const CgHead H(st);
+    if (H.done) return;
     __shared__ float inv_diag[8];  // Jacobi: 1 / (n dt) for n open faces (0 for n = 0), as zof computes it
     if (PM == PM_JACOBI) {
         if (threadIdx.x < 8) inv_diag[threadIdx.x] = threadIdx.x ? __frcp_rn((float)threadIdx.x * dt) : 0.f;
         __syncthreads();
     }
-    const i64 k = *(volatile const i64*)&st->iter;
+    const i64 k = H.iter;
     const float4* __restrict__ p = ((k + 1) & 1) ? p1 : p0;
-    const float alpha = (float)st->alpha, nalpha = -alpha;
+    const float alpha = (float)H.alpha, nalpha = -alpha;
     float rm = 0.f;
     Acc<float> rz;
     int bad = 0;
@@ -546,15 +552,16 @@ __global__ void __launch_bounds__(kCgThreads)
     }
     if (c < n4) one(c);
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&st->nan_seen, 1);
-    const double m = block_max<kCgThreads>((double)rm, sm);
-    const double s = block_sum<kCgThreads>(rz.value(), sm);
+    double s = rz.value();
+    block_max0_sum<kCgThreads>(rm, s, sm);
     if (threadIdx.x == 0) {
-        partials[2 * kMaxBlocks + blockIdx.x] = m;
+        partials[2 * kMaxBlocks + blockIdx.x] = (double)rm;
         partials[3 * kMaxBlocks + blockIdx.x] = s;
     }
     if (!last_block(&st->counter[2])) return;
-    const double rmax = reduce_partials<true, kCgThreads>(partials + 2 * kMaxBlocks, gridDim.x, sm);
-    const double sigma_new = reduce_partials<false, kCgThreads>(partials + 3 * kMaxBlocks, gridDim.x, sm);
+    double rmax, sigma_new;
+    reduce_partials_max0<kCgThreads>(partials + 2 * kMaxBlocks, partials + 3 * kMaxBlocks, gridDim.x, sm, rmax,
+                                     sigma_new);
     if (threadIdx.x == 0) {
         st->counter[2] = 0;
         const i64 it = st->iter + 1;
@@ -571,6 +578,13 @@ __global__ void __launch_bounds__(kCgThreads)
             if (it >= st->max_iter) st->done = 1;  // loop bound, pcg.rs:48
         }
     }
+}
+
+// Blocks of a float4 kernel over n cells: none without a vector of its own
+// (a 64^3 update ran 1024 blocks of which 256 had work: 20 us, each block
+// adding its partials and its ticket).
+static int vec4_blocks(int nb, i64 n) {
+    return (int)std::max<i64>(1, std::min<i64>(nb, (n / 4 + kCgThreads - 1) / kCgThreads));
 }
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
@@ -627,7 +641,7 @@ static void update_launch(cudaStream_t s, int nb, T* x, T* r, const T* p0, const
     const bool vec4 = sizeof(T) == 4 && n % 4 == 0 && aligned16(x) && aligned16(r) && aligned16(p0) &&
                       aligned16(p1) && aligned16(ap) && aligned16(flags);
     if (vec4)
-        k_cg_update4r<PM><<<nb, kCgThreads, 0, s>>>((float4*)x, (float4*)r, (const float4*)p0, (const float4*)p1,
+        k_cg_update4r<PM><<<vec4_blocks(nb, n), kCgThreads, 0, s>>>((float4*)x, (float4*)r, (const float4*)p0, (const float4*)p1,
                                                     (const float4*)ap, (const uchar4*)flags, n / 4, (float)dt, st,
                                                     partials);
     else
@@ -642,17 +656,18 @@ static void launch_iter(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook
               spmv_launch<T, PM>(s, g->num_sms, buf.r, buf.z, buf.p[0], buf.p[1], buf.ap, g->flags, D, dt,
                                  g->ws.state, g->ws.partials, nb, PM == PM_ZBUF || cg_tma_enabled()));
     const i64 n = D.nc();
+    const int nb4 = vec4_blocks(nb, n);
     const bool vec4 = sizeof(T) == 4 && n % 4 == 0 && aligned16(buf.x) && aligned16(buf.r) &&
                       aligned16(buf.p[0]) && aligned16(buf.p[1]) && aligned16(buf.ap) && aligned16(g->flags);
     if (PM == PM_ZBUF && vec4 && buf.xl)
         PG_LAUNCH(KK_CG_UPDATE, s,
-                  k_cg_update4<true><<<nb, kCgThreads, 0, s>>>(
+                  k_cg_update4<true><<<nb4, kCgThreads, 0, s>>>(
                       (float4*)buf.x, (float4*)buf.r, (const float4*)buf.p[0], (const float4*)buf.p[1],
                       (const float4*)buf.ap, n / 4, g->ws.state, g->ws.partials, (float4*)buf.xl,
                       cg_fold(buf, hook) ? (const float4*)buf.b : nullptr));
     else if (PM == PM_ZBUF && vec4)
         PG_LAUNCH(KK_CG_UPDATE, s,
-                  k_cg_update4<false><<<nb, kCgThreads, 0, s>>>((float4*)buf.x, (float4*)buf.r,
+                  k_cg_update4<false><<<nb4, kCgThreads, 0, s>>>((float4*)buf.x, (float4*)buf.r,
                                                                 (const float4*)buf.p[0], (const float4*)buf.p[1],
                                                                 (const float4*)buf.ap, n / 4, g->ws.state,
                                                                 g->ws.partials, nullptr, nullptr));
@@ -779,7 +794,7 @@ static int run_cg_pm(pg_grid* g, const CgConfig& cfg, CgBuffers<T> buf, pg_pcg_s
     const bool fold = PM == PM_ZBUF && cg_fold(buf, hook);
     if (PM == PM_ZBUF && sizeof(T) == 4 && n % 4 == 0 && aligned16(buf.x) && aligned16(buf.r) && aligned16(buf.b))
         PG_LAUNCH(KK_CG_INIT, s,
-                  k_cg_init4<<<nb, kCgThreads, 0, s>>>((float4*)buf.x, fold ? nullptr : (float4*)buf.r,
+                  k_cg_init4<<<vec4_blocks(nb, n), kCgThreads, 0, s>>>((float4*)buf.x, fold ? nullptr : (float4*)buf.r,
                                                        (const float4*)buf.b, n / 4, cfg.threshold, cfg.rel_tol,
                                                        cfg.max_iter, fold ? 0 : cfg.zero_x, ws.state, ws.partials,
                                                        cfg.nfluid, (float4*)buf.xl));

@@ -93,6 +93,26 @@ int run_cg(pg_grid* g, const CgConfig& cfg, CgBuffers<T> buf, pg_pcg_stats* stat
 // PG_CG_DFX=0 turns it off (a diagnostic switch).
 bool cg_dfx_supported(const pg_grid* g, const CgBuffers<float>& buf);
 
+// What a CG kernel reads of the state, loaded together: loads behind the stop
+// test would wait for it (a second latency per kernel).  Through L1: with
+// every warp of a large launch reading them from L2 (volatile loads) the one
+// line they share took 6 us of a 31 us update.  The last block writes the
+// state only after every block has read it here.
+struct CgHead {
+    double alpha, beta, nfluid, zmean;
+    i64 iter;
+    int done, first;
+    __device__ __forceinline__ explicit CgHead(const CgState* st) {
+        done = __ldca(&st->done);
+        first = __ldca(&st->first);
+        iter = __ldca((const long long*)&st->iter);
+        alpha = __ldca(&st->alpha);
+        beta = __ldca(&st->beta);
+        nfluid = __ldca(&st->nfluid);
+        zmean = __ldca(&st->zmean);
+    }
+};
+
 // Device side: fold a freshly reduced z.r into the CG state.  Right after
 // init (iter == 0) it is sigma; afterwards beta = z.r / sigma (pcg.rs:67-68).
 // With the lazy projection on (nfluid > 0) z stands for z - m on the fluid
@@ -120,26 +140,49 @@ __device__ __forceinline__ void cg_finish_rz(CgState* st, double rz, double zsum
 }
 
 // Last-block ticket: true in every thread of the block that finished last.
-// Per-block partials must be written (by thread 0) before the call.
+// Per-block partials must be written (by thread 0, whose fence orders them)
+// before the call.
 __device__ __forceinline__ bool last_block(unsigned int* counter) {
     __shared__ bool am_last;
-    __threadfence();
     if (threadIdx.x == 0) {
-        const unsigned int t = atomicAdd(counter, 1u);
-        am_last = (t == gridDim.x - 1);
+        __threadfence();
+        am_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        __threadfence();
     }
     __syncthreads();
     return am_last;
 }
 
-// Deterministic sum (or max) of n per-block partials, by one block of NT.
-template <bool MAX, int NT> __device__ __forceinline__ double reduce_partials(const double* partials, int n, double* sm) {
+// Deterministic sum of n per-block partials, by one block of NT; two at once;
+// and a maximum (>= 0, no NaN) with a sum.  buf as in block_sum,
+// block_sum2 and block_max0_sum; valid in thread 0.
+template <int NT> __device__ __forceinline__ double reduce_partials(const double* p, int n, double* buf) {
     double v = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double pv = __ldcg(partials + i);
-        v = MAX ? fmax(v, pv) : v + pv;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += NT) v += __ldcg(p + i);
+    return block_sum<NT>(v, buf);
+}
+template <int NT>
+__device__ __forceinline__ void reduce_partials2(const double* pa, const double* pb, int n, double* buf, double& a,
+                                                 double& b) {
+    a = b = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += NT) {
+        a += __ldcg(pa + i);
+        b += __ldcg(pb + i);
     }
-    return MAX ? block_max<NT>(v, sm) : block_sum<NT>(v, sm);
+    block_sum2<NT>(a, b, buf);
+}
+template <int NT>
+__device__ __forceinline__ void reduce_partials_max0(const double* pm, const double* ps, int n, double* buf, double& m,
+                                                     double& s) {
+    m = s = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += NT) {
+        m = max0(m, __ldcg(pm + i));
+        s += __ldcg(ps + i);
+    }
+    block_max0_sum<NT>(m, s, buf);
 }
 
 }  // namespace pg

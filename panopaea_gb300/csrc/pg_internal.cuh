@@ -102,29 +102,81 @@ __host__ __device__ inline int coarse_pairs(int d, int h, int w) {
 }
 
 // ---------------------------------------------------------------------------
-// Block reductions in FP64 (deterministic for a fixed launch shape).
-template <int NT> __device__ __forceinline__ double block_sum(double v, double* sm) {
+// Block reductions in FP64 (deterministic for a fixed launch shape), valid in
+// thread 0; buf holds NT doubles per sum and is free again after the next
+// block barrier.  Every thread stores its value and one warp folds the block:
+// 12 FP64 instructions for 256 threads where a shuffle tree in every warp
+// takes 45 -- GB300 issues an FP64 warp instruction every 16 cycles per SM,
+// so the trees of 8 blocks per SM cost 3 us of a CG kernel.
+__device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sm[wid] = v;
-    __syncthreads();
-    v = (threadIdx.x < NT / 32) ? sm[threadIdx.x] : 0.0;
-    if (wid == 0)
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;  // valid in thread 0
-}
-
-template <int NT> __device__ __forceinline__ double block_max(double v, double* sm) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sm[wid] = v;
-    __syncthreads();
-    v = (threadIdx.x < NT / 32) ? sm[threadIdx.x] : 0.0;
-    if (wid == 0)
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
+}
+template <int NT> __device__ __forceinline__ double fold32(const double* buf) {  // by one warp
+    double v = buf[threadIdx.x & 31];
+#pragma unroll
+    for (int k = 32; k < NT; k += 32) v += buf[(threadIdx.x & 31) + k];
+    return warp_sum(v);
+}
+template <int NT> __device__ __forceinline__ double block_sum(double v, double* buf) {
+    __syncthreads();
+    buf[threadIdx.x] = v;
+    __syncthreads();
+    return threadIdx.x < 32 ? fold32<NT>(buf) : 0.0;
+}
+// Two sums at once, by two warps; buf: 2 NT doubles.
+template <int NT> __device__ __forceinline__ void block_sum2(double& a, double& b, double* buf) {
+    static_assert(NT >= 64, "two warps");
+    __syncthreads();
+    buf[threadIdx.x] = a;
+    buf[NT + threadIdx.x] = b;
+    __syncthreads();
+    if (threadIdx.x < 32) a = fold32<NT>(buf);
+    if (threadIdx.x >= 32 && threadIdx.x < 64) {
+        b = fold32<NT>(buf + NT);
+        if (threadIdx.x == 32) buf[NT] = b;
+    }
+    __syncthreads();
+    b = buf[NT];
+}
+// Maximum over the warp of values that are not negative and no NaN: their
+// bit patterns order as integers do, off the FP64 pipe.
+__device__ __forceinline__ float warp_max0(float v) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+__device__ __forceinline__ double warp_max0(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)__double2loint(v) : 0u);
+    return __hiloint2double((int)mh, (int)ml);
+}
+__device__ __forceinline__ float max0(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double max0(double a, double b) {  // a, b >= 0, no NaN
+    return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
+template <int NT, class T> __device__ __forceinline__ T block_max0(T v, double* buf) {
+    T* const m = (T*)buf;
+    v = warp_max0(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) m[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return threadIdx.x < 32 ? warp_max0(threadIdx.x < NT / 32 ? m[threadIdx.x] : T(0)) : T(0);
+}
+// block_max0 and block_sum at once, by two warps; buf: NT + 32 doubles.
+template <int NT, class T> __device__ __forceinline__ void block_max0_sum(T& m, double& s, double* buf) {
+    T* const mb = (T*)(buf + NT);
+    m = warp_max0(m);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) mb[threadIdx.x >> 5] = m;
+    buf[threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) s = fold32<NT>(buf);
+    if (threadIdx.x >= 32 && threadIdx.x < 64) {
+        m = warp_max0(threadIdx.x < 32 + NT / 32 ? mb[threadIdx.x - 32] : T(0));
+        if (threadIdx.x == 32) mb[0] = m;
+    }
+    __syncthreads();
+    m = mb[0];
 }
 
 // ---------------------------------------------------------------------------

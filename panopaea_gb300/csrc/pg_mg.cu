@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kMgThreads)
     k_mg_smooth(LV v, float* __restrict__ e, const float* __restrict__ f, const float* __restrict__ ec, int cw, int ch,
                 int color, CgState* st, double* partials, FastDiv fhalf, FastDiv fh) {
     if (st->done) return;
-    __shared__ double sm[32];
+    __shared__ double sm[RZ ? 2 * kMgThreads : 1];
     const int hw = v.h * v.w;
     const int half = (v.w + 1) >> 1;
     const int nrow = v.d * v.h;
@@ -262,15 +262,15 @@ __global__ void __launch_bounds__(kMgThreads)
             zs.add(e[c]);
         }
     }
-    const double s = block_sum<kMgThreads>(acc.value(), sm);
-    const double s2 = block_sum<kMgThreads>(zs.value(), sm);
+    double s = acc.value(), s2 = zs.value();
+    block_sum2<kMgThreads>(s, s2, sm);
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = s;
         partials[kMaxBlocks + blockIdx.x] = s2;
     }
     if (!last_block(&st->counter[3])) return;
-    const double rz = reduce_partials<false, kMgThreads>(partials, gridDim.x, sm);
-    const double zsum = reduce_partials<false, kMgThreads>(partials + kMaxBlocks, gridDim.x, sm);
+    double rz, zsum;
+    reduce_partials2<kMgThreads>(partials, partials + kMaxBlocks, gridDim.x, sm, rz, zsum);
     if (threadIdx.x == 0) {
         st->counter[3] = 0;
         cg_finish_rz(st, rz, zsum);
@@ -347,7 +347,6 @@ __global__ void __launch_bounds__(kPThreads, kPMinBlocks)
     constexpr int kStages = Cfg::kStages, kStageBytes = Cfg::kStageBytes;
     if (st->done) return;
     extern __shared__ unsigned char pair_smem_raw[];
-    __shared__ double sm[32];
     __shared__ float inv_tab[8];  // 1 / (n dt) for n open faces (0 for n = 0), as Cell<true>
     // 128-byte aligned by an offset (pointer arithmetic keeps every access
     // below in the shared window: LDS/STS, not generic loads)
@@ -513,15 +512,16 @@ __global__ void __launch_bounds__(kPThreads, kPMinBlocks)
         return;
     }
     if (RZ) {
-        const double s = block_sum<kPThreads>(acc.value(), sm);
-        const double s2 = block_sum<kPThreads>(zs.value(), sm);
+        double* const sm = (double*)base;  // the plane ring is free
+        double s = acc.value(), s2 = zs.value();
+        block_sum2<kPThreads>(s, s2, sm);
         if (threadIdx.x == 0) {
             partials[blockIdx.x] = s;
             partials[kMaxBlocks + blockIdx.x] = s2;
         }
         if (last_block(&st->counter[3])) {
-            const double rz = reduce_partials<false, kPThreads>(partials, gridDim.x, sm);
-            const double zsum = reduce_partials<false, kPThreads>(partials + kMaxBlocks, gridDim.x, sm);
+            double rz, zsum;
+            reduce_partials2<kPThreads>(partials, partials + kMaxBlocks, gridDim.x, sm, rz, zsum);
             if (threadIdx.x == 0) {
                 st->counter[3] = 0;
                 cg_finish_rz(st, rz, zsum);

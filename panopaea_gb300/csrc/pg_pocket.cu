@@ -119,7 +119,7 @@ int upload_pockets(const std::vector<i64>& cells, const std::vector<int>& start,
 __global__ void __launch_bounds__(kPocketThreads)
     k_pocket_sum(const float* __restrict__ a, const int* __restrict__ cells, const int* __restrict__ chunk_start,
                  int nchunk, double* __restrict__ partials) {
-    __shared__ double sm[32];
+    __shared__ double sm[kPocketThreads];
     for (int k = blockIdx.x; k < nchunk; k += gridDim.x) {
         double s = 0.0;
         for (int i = chunk_start[k] + threadIdx.x; i < chunk_start[k + 1]; i += blockDim.x) s += (double)a[cells[i]];

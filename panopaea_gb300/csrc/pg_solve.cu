@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kThreads)
         r[c] = (float)rv;
         m = fmax(m, fabs(rv));
     }
-    const double bm = block_max<kThreads>(m, sm);
+    const double bm = (double)block_max0<kThreads>(m, sm);
     __shared__ bool last;
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = bm;
@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(kThreads)
     __syncthreads();
     if (!last) return;
     double v = 0.0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v = fmax(v, __ldcg(partials + i));
-    v = block_max<kThreads>(v, sm);
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v = max0(v, __ldcg(partials + i));
+    v = block_max0<kThreads>(v, sm);
     if (threadIdx.x == 0) {
         *out = v;
         *counter = 0;
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kThreads)
         m = fmaxf(m, fabsf(rv));
         if (rv != rv) m = __int_as_float(0x7f800000);  // NaN reported as inf
     }
-    const double bm = block_max<kThreads>((double)m, sm);
+    const double bm = (double)block_max0<kThreads>(m, sm);
     __shared__ bool last;
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = bm;
@@ -193,8 +193,8 @@ __global__ void __launch_bounds__(kThreads)
     __syncthreads();
     if (!last) return;
     double v = 0.0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v = fmax(v, __ldcg(partials + i));
-    v = block_max<kThreads>(v, sm);
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v = max0(v, __ldcg(partials + i));
+    v = block_max0<kThreads>(v, sm);
     if (threadIdx.x == 0) {
         *out = v;
         *counter = 0;
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kRTX * kRTY)
             al = nl;
         }
     }
-    const double bm = block_max<kRTX * kRTY>((double)m, sm);
+    const double bm = (double)block_max0<kRTX * kRTY>(m, sm);
     __shared__ bool last;
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = bm;
@@ -297,8 +297,8 @@ __global__ void __launch_bounds__(kRTX * kRTY)
     __syncthreads();
     if (!last) return;
     double v = 0.0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v = fmax(v, __ldcg(partials + i));
-    v = block_max<kRTX * kRTY>(v, sm);
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v = max0(v, __ldcg(partials + i));
+    v = block_max0<kRTX * kRTY>(v, sm);
     if (threadIdx.x == 0) {
         *out = v;
         *counter = 0;

@@ -56,18 +56,18 @@ __global__ void __launch_bounds__(kSThreads, 2)
     k_cg_spmv3p(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUtensorMap pmap0,
                 const __grid_constant__ CUtensorMap pmap1, const __grid_constant__ CUtensorMap gmap, SpmvArgs a,
                 CgState* st, double* partials) {
-    if (st->done) return;
+    const CgHead H(st);
+    if (H.done) return;
     extern __shared__ unsigned char spmv_smem_raw[];
-    __shared__ double sm[32];
     unsigned char* const base = spmv_smem_raw + ((128u - (smem_u32(spmv_smem_raw) & 127u)) & 127u);
     float(*const S)[kSSh][kSSw] = (float(*)[kSSh][kSSw])(base + kSStages * kSStageBytes);
     uint64_t* const bars = (uint64_t*)(base + kSBarOff);
     const int tid = threadIdx.x, lane = tid & 31, ty = tid >> 5;
-    const i64 kit = *(volatile const i64*)&st->iter;
+    const i64 kit = H.iter;
     const CUtensorMap* pmap = (kit & 1) ? &pmap1 : &pmap0;  // p_old
     float* const p_new = (kit & 1) ? a.p0 : a.p1;
-    const int first = st->first;
-    const float beta = first ? 0.f : (float)st->beta;
+    const int first = H.first;
+    const float beta = first ? 0.f : (float)H.beta;
     // Jacobi: 1 / (n dt) for n open faces, computed as in zval (0 for n = 0)
     __shared__ float inv_diag[8];
     if (PM == PM_JACOBI && tid < 8) inv_diag[tid] = tid ? __frcp_rn((float)tid * a.dt) : 0.f;
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kSThreads, 2)
     };
     // p_new of cell (yl, xl) of the staged plane P (tile coordinates), with
     // z projected lazily on the fluid cells (zm = 0 when off)
-    const float zm = (PM == PM_ZBUF && st->nfluid > 0.0) ? (float)st->zmean : 0.f;
+    const float zm = (PM == PM_ZBUF && H.nfluid > 0.0) ? (float)H.zmean : 0.f;
     auto pn = [&](const unsigned char* P, int yl, int xl) -> float {
         const float z0 = Zv(P, yl + 1, xl + 4);
         float z = z0;
@@ -212,10 +212,11 @@ __global__ void __launch_bounds__(kSThreads, 2)
         }
         return;
     }
+    double* const sm = (double*)base;  // the plane ring is free
     const double s = block_sum<kSThreads>(acc.value(), sm);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
     if (!last_block(&st->counter[1])) return;
-    const double pap = reduce_partials<false, kSThreads>(partials, gridDim.x, sm);
+    const double pap = reduce_partials<kSThreads>(partials, gridDim.x, sm);
     if (threadIdx.x == 0) {
         st->counter[1] = 0;
         st->pap = pap;
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(kRThreads, 2)
         }
         m = __int_as_float(0x7fc00000);
     }
-    const double bm = block_max<kRThreads>((double)m, sm);
+    const double bm = (double)block_max0<kRThreads>(m, sm);
     __shared__ bool last;
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = bm;
@@ -397,8 +398,8 @@ __global__ void __launch_bounds__(kRThreads, 2)
     __syncthreads();
     if (!last) return;
     double v = 0.0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v = fmax(v, __ldcg(partials + i));
-    v = block_max<kRThreads>(v, sm);
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v = max0(v, __ldcg(partials + i));
+    v = block_max0<kRThreads>(v, sm);
     if (threadIdx.x == 0) {
         *out = v;
         *counter = 0;

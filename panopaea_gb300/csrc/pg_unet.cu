@@ -732,7 +732,7 @@ constexpr int kRedThreads = 256;
 constexpr int kRedBlocks = 512;
 
 __global__ void __launch_bounds__(kRedThreads) k_sumsq(const float* __restrict__ b, i64 n, double* __restrict__ part) {
-    __shared__ double sm[32];
+    __shared__ double sm[kRedThreads];
     double s = 0.0;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         const double v = b[i];
@@ -862,7 +862,7 @@ __global__ void __launch_bounds__(kHeadThreads)
            const float* __restrict__ scal, i64 n, float dt, float* __restrict__ p_out, const float* __restrict__ p_true,
            float* __restrict__ e_out, const float* __restrict__ ae, float c2, bf16* __restrict__ dZ9,
            double* __restrict__ part) {
-    __shared__ double sm[32];
+    __shared__ double sm[kHeadThreads];
     float w[16];
 #pragma unroll
     for (int c = 0; c < 16; ++c) w[c] = wh[c];
@@ -927,15 +927,14 @@ __global__ void __launch_bounds__(kHeadThreads)
 // x += alpha d, r -= alpha Ad.
 __global__ void __launch_bounds__(kRedThreads) k_dots(const float* __restrict__ d, const float* __restrict__ r,
                                                       const float* __restrict__ ad, i64 n, double* __restrict__ part) {
-    __shared__ double sm[32];
+    __shared__ double sm[2 * kRedThreads];
     double a = 0.0, b = 0.0;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         const double di = d[i];
         a += di * (double)r[i];
         b += di * (double)ad[i];
     }
-    a = block_sum<kRedThreads>(a, sm);
-    b = block_sum<kRedThreads>(b, sm);
+    block_sum2<kRedThreads>(a, b, sm);
     if (threadIdx.x == 0) {
         part[2 * blockIdx.x] = a;
         part[2 * blockIdx.x + 1] = b;
@@ -1347,7 +1346,7 @@ __global__ void __launch_bounds__(kRedThreads)
     k_lp_fold(const float* __restrict__ z, const float* __restrict__ r, const float* __restrict__ ap, i64 n,
               CgState* st, double* partials) {
     if (st->done) return;
-    __shared__ double sm[32];
+    __shared__ double sm[2 * kRedThreads];
     Acc<float> zr, zap;
     const bool first = st->iter == 0;
     for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (i64)gridDim.x * blockDim.x) {
@@ -1355,15 +1354,15 @@ __global__ void __launch_bounds__(kRedThreads)
         zr.add(zv * r[v]);
         if (!first) zap.add(zv * ap[v]);
     }
-    const double s1 = block_sum<kRedThreads>(zr.value(), sm);
-    const double s2 = block_sum<kRedThreads>(zap.value(), sm);
+    double s1 = zr.value(), s2 = zap.value();
+    block_sum2<kRedThreads>(s1, s2, sm);
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = s1;
         partials[kMaxBlocks + blockIdx.x] = s2;
     }
     if (!last_block(&st->counter[3])) return;
-    const double rz = reduce_partials<false, kRedThreads>(partials, gridDim.x, sm);
-    const double za = reduce_partials<false, kRedThreads>(partials + kMaxBlocks, gridDim.x, sm);
+    double rz, za;
+    reduce_partials2<kRedThreads>(partials, partials + kMaxBlocks, gridDim.x, sm, rz, za);
     if (threadIdx.x == 0) {
         st->counter[3] = 0;
         if (!isfinite(rz) || !isfinite(za)) {
