@@ -15,8 +15,10 @@
 // (red, black) and after (black, red) the coarse correction, so the V-cycle
 // is a symmetric operator and CG stays valid.  The coarsest level (at most
 // kCoarseMax cells) is solved by one block in shared memory with symmetric
-// sweeps (coarse_pairs of its shape).  Every level of at most kTailCells
-// cells runs inside one single-block kernel (k_mg_tail).
+// sweeps (coarse_pairs of its shape).  The small levels (in 2D up to the whole
+// V-cycle) run in one thread-block cluster (k_mg_ctail); hierarchies without
+// a level for it run their levels of at most kTailCells cells inside one
+// single-block kernel (k_mg_tail).
 //
 // Fusions: the first pre-smoothing red half-sweep starts from e = 0, so red
 // values are f*invd and the black half-sweep computes them on the fly; the
@@ -48,6 +50,7 @@ struct MgLevel {
     float* wy = nullptr;
     float* wz = nullptr;
     float* invd = nullptr;
+    float4* wp = nullptr;  // the cluster tail's packed weights (levels it runs, from 1)
     float* e = nullptr;  // correction (levels >= 1)
     float* f = nullptr;  // right-hand side (levels >= 1)
 };
@@ -64,10 +67,11 @@ struct MgHierarchy {
     Pockets pockets;  // fluid components (empty when the fluid is connected)
     int tail = 0;     // first level handled by the single-block tail kernel (nlev: none)
     float* cinv = nullptr;  // coarsest level of at most kCinvCells cells: its pseudo-inverse (row-major)
-    int ct_lt = 0;    // cluster tail (3D): first level (0: not used), first rank-0 level, ranks
+    int ct_lt = 0;    // cluster tail: first level, first rank-0 level, ranks (0: not used)
     int ct_ls = 0;
     int ct_ranks = 0;
     size_t ct_smem = 0;
+    void* ct_mem = nullptr;  // its packed weights
     double nfluid = 0;  // cells with an open face (the lazy projection's count)
     // fine level of 3D grids: fused red-black pairs (k_mg_pair) ping-pong
     // between z and e0b; tensor maps of the flags and of the vectors met
@@ -1061,41 +1065,70 @@ __global__ void __launch_bounds__(kTailThreads) k_mg_tail(TailArgs A, CgState* s
 }
 
 // ---------------------------------------------------------------------------
-// Cluster tail (3D): the levels from the first one of at most kCtCells cells
-// down to the coarsest, in ONE thread-block cluster of R blocks (16 where the
-// device allows it, else 8).  Levels larger than kCtLocal cells are cut into
-// z slabs of ppc = ceil(d / R) planes, one per rank, each rank holding its
-// slab of wx, wy, wz, 1/diag, e and f in shared memory; a rank updates its own
-// cells and reads the neighbouring planes of other ranks through distributed
-// shared memory, with a cluster barrier between half-sweeps.  Smaller levels
-// live in rank 0 alone and run the single-block tail's phases with block
-// barriers.  Every cell is computed by the same formula, in the same order of
+// Cluster tail: the levels from the first one that fits down to the coarsest,
+// in ONE thread-block cluster of R blocks (16 where the device allows it, else
+// 8); in 2D that can be the whole V-cycle.  What bounds it is latency: a few
+// thousand cells per half-sweep, eight half-sweeps per level one after
+// another.  So everything a half-sweep waits for is kept near:
+//   - levels of more than kCtLocal cells are cut into slabs of ppc planes (z;
+//     rows in 2D), one per rank; smaller ones live in rank 0 alone, with block
+//     barriers instead of cluster barriers;
+//   - a thread owns up to kCtPairs x-pairs (one red and one black cell each)
+//     and holds their weights, 1/diag and right-hand side in registers for
+//     all half-sweeps of the level (two 16-byte loads per cell from a packed
+//     copy); only the correction e is in shared memory;
+//   - e is stored colour by colour (pair k of row y, plane z at
+//     (z h + y) half + k): a half-sweep reads one colour and writes the other
+//     at stride 1, without bank conflicts; a missing neighbour has weight 0
+//     and a finite value (e starts as zeros), so a cell is six loads and six
+//     multiply-adds without a branch -- 32 warps issue every instruction of a
+//     half-sweep 8 times per scheduler, and that was most of its time;
+//   - a slab carries a halo plane on either side, and a rank PUSHES its
+//     boundary planes into its neighbours' halos as it computes them: remote
+//     stores complete behind the cluster barrier, where remote loads made
+//     every half-sweep wait 2000 to 4000 cycles;
+//   - slabs of a level are twice those of the next distributed one, so a
+//     plane's children and its parent's halo are on the same rank; the last
+//     distributed level sends its residual terms to rank 0.
+// Every cell is computed by the same formula, in the same order of
 // operations, as k_mg_smooth / k_mg_restrict8 / the single-block tail, so the
-// V-cycle is bit-identical to the per-level kernels plus k_mg_tail.
+// V-cycle is bit-identical to the per-level kernels plus k_mg_tail (z.r of a
+// whole V-cycle is summed in another order).  2D levels run as (h, 1, w):
+// their y weights in the place of the z weights, the same order of terms.
+// Measured (ncu): the levels below 64^3 33 us (remote loads and weights in
+// shared memory: 37.5), a whole 256^2 V-cycle 62 us (18 launches and the
+// single-block tail: 107).  A half-sweep of 32^3 takes about 1350 cycles, 1000
+// of them the cluster barrier.
 
-constexpr int kCtThreads = 1024;
-constexpr int kCtCells = 32768;  // first level of the cluster tail: at most this many cells
-constexpr int kCtLocal = 512;    // levels at most this large live in rank 0 alone
+constexpr int kCtThreads = 512;
+constexpr int kCtPairs = 4;      // x-pairs per thread: a slab of a level has at most 2048
+constexpr int kCtLocal = 2048;   // levels at most this large live in rank 0 alone (4096 cells' weights take one SM 2 x 5000 cycles to load)
 constexpr int kCtMaxRanks = 16;
 constexpr int kCtSmemMax = 200 * 1024;
 
 struct CtLevel {
-    int d, h, w;
-    int ppc;  // planes per rank (d: the level lives in rank 0)
-    int off;  // offset (floats) of the level's block [wx | wy | wz | invd | e | f] in shared memory
-    int P;    // floats per array of the block: ppc * h * w
-    FastDiv fhalf, fh, fw, fhw, fppc;  // invariant divisors (w + 1) / 2, h, w, h * w, ppc
-    const float* wx;
-    const float* wy;
-    const float* wz;
-    const float* invd;
+    int d, h, w, half;  // half = (w + 1) / 2 pairs per row
+    int ps;             // pairs per plane: h * half
+    int ppc;            // planes per rank (d: the level lives in rank 0)
+    int P;              // (ppc + 2) * ps: one colour of e, own planes from 1
+    int eoff, foff;     // floats: e (2 P), f (2 ppc ps, own planes from 0)
+    FastDiv fhalf, fh, fhw, fw;
+    const float4* wp;   // packed weights, 2 per cell: {xl, xh, yl, yh}, {zl, zh, 1/diag, 0}
+    const uint8_t* flags;  // level 0 of the grid: weights from the flags
 };
 
 struct CtArgs {
     int lt, ls, nl, nsmooth, ranks;
-    float* e_out;       // global e of level lt
-    const float* f_in;  // global f of level lt
+    int nd;
+    int zero4;          // float4s of shared memory that start as zeros (e and f of every level)
+    int toff;           // residual terms of one slab
+    int coff, cP;       // the first local level's e around the rank's own planes; one colour of it
+    int zoff;           // the coarsest level's [wx | wy | wz | invd | e | f] (rank 0)
+    float dt;
+    float* e_out;       // global e of level lt (z when lt = 0)
+    const float* f_in;  // global f of level lt (r when lt = 0)
     const float* cinv;  // the coarsest level's pseudo-inverse, or null
+    const float *zwx, *zwy, *zwz, *zinvd;  // the coarsest level's weights (zwy null in 2D)
     CtLevel L[kMaxLevels];
 };
 
@@ -1114,233 +1147,402 @@ __device__ __forceinline__ float* ct_map(float* p, unsigned rank) {
 __device__ __forceinline__ void ct_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-
-// Array 0 (wx) of level L at plane z, on the rank that owns it.
-__device__ __forceinline__ float* ct_plane(float* const* peer, const CtLevel& L, int z) {
-    int zl;
-    const int r = split(z, L.ppc, L.fppc, zl);
-    return peer[r] + L.off + zl * L.h * L.w;
+__device__ __forceinline__ void ct_barrier(bool dist) {
+    if (dist)
+        ct_sync();
+    else
+        __syncthreads();
 }
 
-// Neighbour value of the smoother at the cell whose array-0 entry is q
-// (z, y, x): e, f / diag (first half-sweep from e = 0) or e + the coarse
-// correction of its parent (first post-smoothing half-sweep).
-template <int MODE>
-__device__ __forceinline__ float ct_nb(float* const* peer, const float* q, int P, const CtLevel* Lc, int z, int y,
-                                       int x) {
-    if (MODE == NB_FIRST) return q[5 * P] * q[3 * P];
-    if (MODE == NB_PROLONG) {
-        const float* pc = ct_plane(peer, *Lc, z >> 1) + 4 * Lc->P + (y >> 1) * Lc->w + (x >> 1);
-        return q[4 * P] + *pc;
+struct CtCell {  // all zero where an odd row has no such cell
+    float xl, xh, yl, yh, zl, zh, inv, f;
+};
+
+// The pairs of the calling thread on one level.
+struct CtPairs {
+    CtCell c[kCtPairs][2];  // [pair][colour]
+    int ib[kCtPairs];       // index in a colour of e (0: no pair)
+    int s[kCtPairs];        // (y + z) & 1: the red cell is 2 k + s
+    unsigned push;          // bit 2 j: a neighbour below holds the pair's plane as a halo; 2 j + 1: above
+};
+
+struct CtTeam {
+    float* csm;
+    uint32_t lo, hi;  // shared-window addresses of the same memory in rank - 1 and rank + 1
+    int rank;
+};
+__device__ __forceinline__ uint32_t ct_addr(const float* p, unsigned rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void ct_store(uint32_t base, int i, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(base + 4u * (uint32_t)i), "f"(v) : "memory");
+}
+
+// First plane and number of planes of the calling rank's slab.
+__device__ __forceinline__ int ct_z0(const CtLevel& L, int rank, bool dist) { return dist ? rank * L.ppc : 0; }
+__device__ __forceinline__ int ct_nz(const CtLevel& L, int rank, bool dist) {
+    return dist ? max(0, min(L.ppc, L.d - rank * L.ppc)) : L.d;
+}
+
+// Plane (of the slab), row and pair of pair i.
+__device__ __forceinline__ void ct_pos(const CtLevel& L, int i, int& zl, int& y, int& k) {
+    const int row = split(i, L.half, L.fhalf, k);
+    zl = split(row, L.h, L.fh, y);
+}
+
+// Weights and 1/diag of the thread's pairs into registers (and, on the first
+// level, f from global memory; elsewhere ct_load_f takes it from shared
+// memory once the restriction has written it).
+__device__ __forceinline__ void ct_load(const CtArgs& A, int l, int rank, CtPairs& P) {
+    const CtLevel& L = A.L[l];
+    const bool dist = l < A.ls;
+    const int z0 = ct_z0(L, rank, dist), total = ct_nz(L, rank, dist) * L.ps;
+    P.push = 0;
+#pragma unroll
+    for (int j = 0; j < kCtPairs; ++j) {
+        const int i = (int)threadIdx.x + j * kCtThreads;
+        P.ib[j] = 0;
+        if (i >= total) continue;
+        int zl, y, k;
+        ct_pos(L, i, zl, y, k);
+        const int z = z0 + zl, s = (y + z) & 1;
+        P.ib[j] = i + L.ps;
+        P.s[j] = s;
+        if (dist && zl == 0 && z > 0) P.push |= 1u << (2 * j);
+        if (dist && zl == L.ppc - 1 && z + 1 < L.d) P.push |= 2u << (2 * j);
+        const int g0 = (z * L.h + y) * L.w + 2 * k;
+#pragma unroll
+        for (int col = 0; col < 2; ++col) {
+            const int u = s ^ col, g = g0 + u;
+            CtCell& C = P.c[j][col];
+            C = CtCell{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (2 * k + u >= L.w) continue;
+            if (L.flags) {  // as Cell<true>; 2D only
+                const unsigned fl = L.flags[g];
+                C.xl = (fl & XLO) ? A.dt : 0.f;
+                C.xh = (fl & XHI) ? A.dt : 0.f;
+                C.zl = (fl & YLO) ? A.dt : 0.f;
+                C.zh = (fl & YHI) ? A.dt : 0.f;
+                const int n = __popc(fl);
+                C.inv = n ? __frcp_rn((float)n * A.dt) : 0.f;
+            } else {
+                const float4 a = L.wp[2 * g], b = L.wp[2 * g + 1];
+                C.xl = a.x;
+                C.xh = a.y;
+                C.yl = a.z;
+                C.yh = a.w;
+                C.zl = b.x;
+                C.zh = b.y;
+                C.inv = b.z;
+            }
+            if (l == A.lt) C.f = A.f_in[g];
+        }
     }
-    return q[4 * P];
+}
+__device__ __forceinline__ void ct_load_f(const CtTeam& T, const CtLevel& L, CtPairs& P) {
+    const int step = L.ppc * L.ps;  // (f starts as zeros: an odd row's missing cell keeps 0)
+#pragma unroll
+    for (int j = 0; j < kCtPairs; ++j)
+        if (P.ib[j]) {
+            const float* f = T.csm + L.foff + P.ib[j] - L.ps;
+            P.c[j][0].f = f[0];
+            P.c[j][1].f = f[step];
+        }
 }
 
-// One half-sweep of a distributed level over the calling rank's planes.
-// Every value a cell may need is loaded before any is used (a missing
-// neighbour's offset is clamped to the cell itself and its value ignored),
-// so a cell waits for one round of shared and distributed-shared loads.
-template <int MODE>
-__device__ void ct_smooth(float* const* peer, const CtLevel& L, const CtLevel* Lc, int rank, int color) {
-    const int h = L.h, w = L.w, P = L.P;
-    const int z0 = rank * L.ppc, nz = max(0, min(L.ppc, L.d - z0));
-    const int half = (w + 1) >> 1, total = nz * h * half;
-    float* B = peer[rank] + L.off;
-    for (int i = threadIdx.x; i < total; i += blockDim.x) {
-        int k2, y;
-        const int row = split(i, half, L.fhalf, k2);
-        const int zl = split(row, h, L.fh, y), z = z0 + zl;
-        const int x = 2 * k2 + ((y + z + color) & 1);
-        if (x >= w) continue;
-        const int c = row * w + x;
-        const float* q = B + c;
-        const bool hx = x + 1 < w, hy = y + 1 < h, hz = z + 1 < L.d;
-        const int ox0 = x > 0 ? -1 : 0, ox1 = hx ? 1 : 0, oy0 = y > 0 ? -w : 0, oy1 = hy ? w : 0;
-        const float* qd = z > 0 ? (zl > 0 ? q - h * w : ct_plane(peer, L, z - 1) + y * w + x) : q;
-        const float* qu = hz ? (zl + 1 < L.ppc ? q + h * w : ct_plane(peer, L, z + 1) + y * w + x) : q;
-        const float wxl = q[0], wxh_ = q[ox1], wyl = q[P], wyh_ = q[P + oy1], wzl = q[2 * P], wzh_ = qu[2 * P];
-        const float inv = q[3 * P];
-        float s = q[5 * P];
-        if (MODE == NB_SELF) {
-            B[4 * P + c] = s * inv;
+// e = v at index i of the slab's shared memory (pair j), and in the
+// neighbours' halos where that is a boundary plane.
+__device__ __forceinline__ void ct_put(const CtTeam& T, int slab, unsigned push, int j, int i, float v) {
+    T.csm[i] = v;
+    if (push >> (2 * j) & 1u) ct_store(T.lo, i + slab, v);
+    if (push >> (2 * j) & 2u) ct_store(T.hi, i - slab, v);
+}
+
+// The coarse correction onto the red cells of the slab and its halos, ahead of
+// the first post-smoothing half-sweep (over black): cb is the coarse level's e
+// (plane Z at (Z - Zb) cps, cP floats per colour).
+__device__ __forceinline__ void ct_correct(const CtTeam& T, const CtLevel& L, const CtLevel& Lc, const float* cb,
+                                           int Zb, int cP, int z0, int nz) {
+    const int za = max(z0 - 1, 0), n = (min(z0 + nz + 1, L.d) - za) * L.ps;
+    float* e = T.csm + L.eoff + (za - z0 + 1) * L.ps;
+    for (int i = threadIdx.x; i < n; i += kCtThreads) {
+        int zp, y, k;
+        ct_pos(L, i, zp, y, k);
+        const int Z = (za + zp) >> 1, Y = y >> 1;  // the red cell 2 k + s has the parent column k
+        e[i] += cb[((k + Y + Z) & 1 ? cP : 0) + (Z - Zb) * Lc.ps + Y * Lc.half + (k >> 1)];
+    }
+}
+
+// One half-sweep over a colour.
+template <int COL>
+__device__ __forceinline__ void ct_sweep(const CtTeam& T, const CtLevel& L, const CtPairs& P) {
+    const int own = L.eoff + COL * L.P, half = L.half, ps = L.ps, slab = L.ppc * ps;
+    const float* e = T.csm + L.eoff + (1 - COL) * L.P;  // the other colour
+#pragma unroll
+    for (int j = 0; j < kCtPairs; ++j) {
+        if (!P.ib[j]) continue;
+        const CtCell& C = P.c[j][COL];
+        const int u = P.s[j] ^ COL;  // x = 2 k + u
+        const float* q = e + P.ib[j];
+        const float n0 = q[u - 1], n1 = q[u], n2 = q[-half], n3 = q[half], n4 = q[-ps], n5 = q[ps];
+        float s = C.f;
+        s += C.xl * n0;
+        s += C.xh * n1;
+        s += C.yl * n2;
+        s += C.yh * n3;
+        s += C.zl * n4;
+        s += C.zh * n5;
+        ct_put(T, slab, P.push, j, own + P.ib[j], s * C.inv);
+    }
+}
+
+// Residual terms of the slab, colour by colour like f: into this rank's
+// shared memory, or (to0) into rank 0's at the planes' place in the level.
+__device__ __forceinline__ void ct_terms(const CtTeam& T, const CtArgs& A, const CtLevel& L, const CtPairs& P,
+                                         bool to0) {
+    const int half = L.half, ps = L.ps, tP = (to0 ? L.d : L.ppc) * ps;
+    const int at = A.toff - ps + (to0 ? T.rank * L.ppc * ps : 0);
+    const uint32_t dst = ct_addr(T.csm, 0u);
+#pragma unroll
+    for (int j = 0; j < kCtPairs; ++j) {
+        if (!P.ib[j]) continue;
+#pragma unroll
+        for (int col = 0; col < 2; ++col) {
+            const CtCell& C = P.c[j][col];
+            const int u = P.s[j] ^ col;
+            const float* q = T.csm + L.eoff + (1 - col) * L.P + P.ib[j];
+            const float ecv = T.csm[L.eoff + col * L.P + P.ib[j]];
+            const float n0 = q[u - 1], n1 = q[u], n2 = q[-half], n3 = q[half], n4 = q[-ps], n5 = q[ps];
+            float a = 0.f;
+            a += C.xl * (ecv - n0);
+            a += C.xh * (ecv - n1);
+            a += C.yl * (ecv - n2);
+            a += C.yh * (ecv - n3);
+            a += C.zl * (ecv - n4);
+            a += C.zh * (ecv - n5);
+            if (to0)
+                ct_store(dst, at + col * tP + P.ib[j], C.f - a);
+            else
+                T.csm[at + col * tP + P.ib[j]] = C.f - a;
+        }
+    }
+}
+
+// The terms summed over children into the next level's f, in (z, y, x) order
+// as k_mg_restrict8 does, over nz planes from the even plane z0 (tP terms per
+// colour, from plane z0); the next level's red cells start from e = f / diag
+// (its first half-sweep).  The next level is this rank's own planes of a
+// distributed level, or rank 0's (this rank).
+__device__ __forceinline__ void ct_sum(const CtTeam& T, const CtArgs& A, int l, int z0, int nz, int tP) {
+    const CtLevel &L = A.L[l], &Lc = A.L[l + 1];
+    const bool cdist = l + 1 < A.ls, coarsest = l + 2 == A.nl;
+    const int Z0 = z0 >> 1, chw = Lc.h * Lc.w, total = ((nz + 1) >> 1) * chw, half = L.half, ps = L.ps;
+    const float* t = T.csm + A.toff;
+    for (int i = threadIdx.x; i < total; i += kCtThreads) {
+        int YX, X;
+        const int Zl = split(i, chw, Lc.fhw, YX), Z = Z0 + Zl;
+        const float inv = coarsest ? 0.f : Lc.wp[2 * (Z * chw + YX) + 1].z;
+        const int Y = split(YX, Lc.w, Lc.fw, X);
+        // children (z, y, 2 X) and (z, y, 2 X + 1): pair X of row y, the red
+        // one first where y + z is even; a row's missing cell has term 0
+        const bool y1 = 2 * Y + 1 < L.h, z1 = 2 * Zl + 1 < nz;
+        const float* q = t + 2 * Zl * ps + 2 * Y * half + X;
+        const float* qy = q + (y1 ? half : 0);
+        const float* qz = q + (z1 ? ps : 0);
+        const float* qyz = qz + (y1 ? half : 0);
+        const float a0 = q[0], a1 = q[tP], b0 = qy[tP], b1 = qy[0], c0 = qz[tP], c1 = qz[0], d0 = qyz[0],
+                    d1 = qyz[tP];
+        float sum = a0 + a1;
+        if (y1) {
+            sum += b0;
+            sum += b1;
+        }
+        if (z1) {
+            sum += c0;
+            sum += c1;
+            if (y1) {
+                sum += d0;
+                sum += d1;
+            }
+        }
+        if (coarsest) {
+            T.csm[A.zoff + 5 * Lc.d * chw + Z * chw + YX] = sum;
             continue;
         }
-        const float n0 = ct_nb<MODE>(peer, q + ox0, P, Lc, z, y, x + (x > 0 ? -1 : 0));
-        const float n1 = ct_nb<MODE>(peer, q + ox1, P, Lc, z, y, x + ox1);
-        const float n2 = ct_nb<MODE>(peer, q + oy0, P, Lc, z, y + (y > 0 ? -1 : 0), x);
-        const float n3 = ct_nb<MODE>(peer, q + oy1, P, Lc, z, y + (hy ? 1 : 0), x);
-        const float n4 = ct_nb<MODE>(peer, qd, P, Lc, z > 0 ? z - 1 : z, y, x);
-        const float n5 = ct_nb<MODE>(peer, qu, P, Lc, hz ? z + 1 : z, y, x);
-        const float wxh = hx ? wxh_ : 0.f, wyh = hy ? wyh_ : 0.f, wzh = hz ? wzh_ : 0.f;
-        if (wxl != 0.f) s += wxl * n0;
-        if (wxh != 0.f) s += wxh * n1;
-        if (wyl != 0.f) s += wyl * n2;
-        if (wyh != 0.f) s += wyh * n3;
-        if (wzl != 0.f) s += wzl * n4;
-        if (wzh != 0.f) s += wzh * n5;
-        B[4 * P + c] = s * inv;
+        const int Zo = cdist ? Zl : Z;  // plane within the next level's slab
+        const int col = (X + Y + Z) & 1, c = Zo * Lc.ps + Y * Lc.half + (X >> 1);
+        T.csm[Lc.foff + col * Lc.ppc * Lc.ps + c] = sum;
+        if (col == 0) {
+            const float ev = sum * inv;
+            const int ei = Lc.eoff + c + Lc.ps;
+            T.csm[ei] = ev;
+            if (cdist && Zl == 0 && Z > 0) ct_store(T.lo, ei + Lc.ppc * Lc.ps, ev);
+            if (cdist && Zl == Lc.ppc - 1 && Z + 1 < Lc.d) ct_store(T.hi, ei - Lc.ppc * Lc.ps, ev);
+        }
     }
 }
 
-// Residual of distributed level L summed over children into f of level Lc,
-// one thread per child (eight lanes per coarse cell, summed by the first in
-// (z, y, x) order as k_mg_restrict8 does).  Coarse plane Z is computed by the
-// rank owning fine plane 2Z.
-__device__ void ct_restrict(float* const* peer, const CtLevel& L, const CtLevel& Lc, int rank) {
-    const int h = L.h, w = L.w, P = L.P;
-    const int ch = Lc.h, cw = Lc.w, chw = ch * cw;
-    // coarse planes Z with 2Z in [rank * ppc, (rank + 1) * ppc)
-    const int Z0 = (rank * L.ppc + 1) / 2, Z1 = min(Lc.d, ((rank + 1) * L.ppc + 1) / 2);
-    const int total = max(0, Z1 - Z0) * chw;
-    const unsigned lane = threadIdx.x & 31, grp = lane & ~7u;
-    const int n8 = (total * 8 + 31) & ~31;  // whole warps: every lane runs the same trips
-    for (int t = threadIdx.x; t < n8; t += blockDim.x) {
-        const int i = t >> 3, j = t & 7;
-        int YX, X;
-        const int Z = Z0 + split(i, chw, Lc.fhw, YX);
-        const int Y = split(YX, cw, Lc.fw, X);
-        const int z = 2 * Z + (j >> 2), y = 2 * Y + ((j >> 1) & 1), x = 2 * X + (j & 1);
-        const bool has = i < total && z < L.d && y < h && x < w;
-        float term = 0.f;
-        if (has) {
-            const int k = y * w + x;
-            const float* q = ct_plane(peer, L, z) + k;
-            const bool hx = x + 1 < w, hy = y + 1 < h, hz = z + 1 < L.d;
-            const int ox0 = x > 0 ? -1 : 0, ox1 = hx ? 1 : 0, oy0 = y > 0 ? -w : 0, oy1 = hy ? w : 0;
-            const float* pd = z > 0 ? ct_plane(peer, L, z - 1) + k : q;
-            const float* pu = hz ? ct_plane(peer, L, z + 1) + k : q;
-            const float wxl = q[0], wxh_ = q[ox1], wyl = q[P], wyh_ = q[P + oy1], wzl = q[2 * P], wzh_ = pu[2 * P];
-            const float ecv = q[4 * P], e0 = q[4 * P + ox0], e1 = q[4 * P + ox1], e2 = q[4 * P + oy0],
-                        e3 = q[4 * P + oy1], e4 = pd[4 * P], e5 = pu[4 * P], fv = q[5 * P];
-            const float wxh = hx ? wxh_ : 0.f, wyh = hy ? wyh_ : 0.f, wzh = hz ? wzh_ : 0.f;
-            float a = 0.f;
-            if (wxl != 0.f) a += wxl * (ecv - e0);
-            if (wxh != 0.f) a += wxh * (ecv - e1);
-            if (wyl != 0.f) a += wyl * (ecv - e2);
-            if (wyh != 0.f) a += wyh * (ecv - e3);
-            if (wzl != 0.f) a += wzl * (ecv - e4);
-            if (wzh != 0.f) a += wzh * (ecv - e5);
-            term = fv - a;
-        }
-        const unsigned valid = __ballot_sync(0xffffffffu, has);
-        float sum = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float tk = __shfl_sync(0xffffffffu, term, grp + k);
-            if ((valid >> (grp + k)) & 1u) sum += tk;
-        }
-        if (j == 0 && i < total) ct_plane(peer, Lc, Z)[5 * Lc.P + YX] = sum;
-    }
-}
-
-__global__ void __launch_bounds__(kCtThreads) k_mg_ctail(CtArgs A, CgState* st) {
+__global__ void __launch_bounds__(kCtThreads) k_mg_ctail(const __grid_constant__ CtArgs A, CgState* st) {
     if (st->done) return;  // the same value in every block of the cluster
     extern __shared__ float csm[];
-    __shared__ float* peer[kCtMaxRanks];
-    const int rank = (int)ct_rank();
-    if (threadIdx.x < A.ranks) peer[threadIdx.x] = ct_map(csm, threadIdx.x);
-    __syncthreads();
+    __shared__ double sums[kCtMaxRanks][2];
+    CtTeam T;
+    T.csm = csm;
+    T.rank = (int)ct_rank();
+    T.lo = ct_addr(csm, (unsigned)max(T.rank - 1, 0));
+    T.hi = ct_addr(csm, (unsigned)min(T.rank + 1, A.ranks - 1));
     const int lt = A.lt, ls = A.ls, nl = A.nl, ns = A.nsmooth;
-    // load: the distributed levels' slabs, and rank 0's levels
-    for (int l = lt; l < nl; ++l) {
+    CtPairs P;
+    ct_load(A, lt, T.rank, P);
+    for (int i = threadIdx.x; i < A.zero4; i += kCtThreads) ((float4*)csm)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    ct_sync();  // every block runs and has zeroed its e: remote stores from here on
+    // the first level's red cells: e = f / diag
+#pragma unroll
+    for (int j = 0; j < kCtPairs; ++j)
+        if (P.ib[j])
+            ct_put(T, A.L[lt].ppc * A.L[lt].ps, P.push, j, A.L[lt].eoff + P.ib[j], P.c[j][0].f * P.c[j][0].inv);
+    // Down the levels lt .. nl - 2, the coarsest, and up again, every level
+    // through the same code: a half-sweep is a few hundred instructions that
+    // run once per level, and code of its own for each level and direction
+    // would be fetched from L2 each time.
+    const int down = nl - 1 - lt;
+    for (int t = 0; t <= 2 * down; ++t) {
+        const bool up = t > down;
+        const int l = lt + (up ? 2 * down - t : t);
+        const bool dist = l < ls;
+        if (!dist && T.rank != 0) continue;
         const CtLevel& L = A.L[l];
-        const int z0 = l < ls ? rank * L.ppc : 0;
-        const int nz = l < ls ? max(0, min(L.ppc, L.d - z0)) : (rank == 0 ? L.d : 0);
-        const int n = nz * L.h * L.w, g0 = z0 * L.h * L.w;
-        float* B = csm + L.off;
-        for (int c = threadIdx.x; c < n; c += blockDim.x) {
-            B[c] = L.wx[g0 + c];
-            B[L.P + c] = L.wy[g0 + c];
-            B[2 * L.P + c] = L.wz[g0 + c];
-            B[3 * L.P + c] = L.invd[g0 + c];
-            if (l == lt) B[5 * L.P + c] = A.f_in[g0 + c];
-        }
-    }
-    ct_sync();
-    // down through the distributed levels
-    for (int l = lt; l < ls; ++l) {
-        const CtLevel& L = A.L[l];
-        ct_smooth<NB_FIRST>(peer, L, nullptr, rank, 1);
-        ct_sync();
-        if (ns == 1) {
-            ct_smooth<NB_SELF>(peer, L, nullptr, rank, 0);
-            ct_sync();
-        }
-        for (int k = 1; k < ns; ++k) {
-            ct_smooth<NB_PLAIN>(peer, L, nullptr, rank, 0);
-            ct_sync();
-            ct_smooth<NB_PLAIN>(peer, L, nullptr, rank, 1);
-            ct_sync();
-        }
-        ct_restrict(peer, L, A.L[l + 1], rank);
-        ct_sync();
-    }
-    // rank 0: levels [ls, nl) as in the single-block tail
-    if (rank == 0) {
-        auto lv = [&](int l) -> LV {
-            const CtLevel& T = A.L[l];
-            float* p = csm + T.off;
+        if (t == down) {  // rank 0: the coarsest level
+            const int n = L.d * L.h * L.w;
+            float* B = csm + A.zoff;
+            if (!A.cinv) {
+                for (int c = threadIdx.x; c < n; c += kCtThreads) {
+                    B[c] = A.zwx[c];
+                    B[n + c] = A.zwy ? A.zwy[c] : 0.f;
+                    B[2 * n + c] = A.zwz[c];
+                    B[3 * n + c] = A.zinvd[c];
+                }
+                __syncthreads();
+            }
             LV v;
             v.nd = 3;
-            v.d = T.d;
-            v.h = T.h;
-            v.w = T.w;
+            v.d = L.d;
+            v.h = L.h;
+            v.w = L.w;
             v.flags = nullptr;
-            v.wx = p;
-            v.wy = p + T.P;
-            v.wz = p + 2 * T.P;
-            v.invd = p + 3 * T.P;
+            v.wx = B;
+            v.wy = B + n;
+            v.wz = B + 2 * n;
+            v.invd = B + 3 * n;
             v.dt = 0.f;
-            return v;
-        };
-        auto E = [&](int l) -> float* { return csm + A.L[l].off + 4 * A.L[l].P; };
-        auto F = [&](int l) -> float* { return csm + A.L[l].off + 5 * A.L[l].P; };
-        for (int l = ls; l + 1 < nl; ++l) {
-            const CtLevel& c = A.L[l + 1];
-            const LV v = lv(l);
-            float* e = E(l);
-            const float* f = F(l);
-            tail_smooth<NB_FIRST>(v, e, f, nullptr, c.w, c.h, 1);
-            if (ns == 1) tail_smooth<NB_SELF>(v, e, f, nullptr, c.w, c.h, 0);
-            for (int k = 1; k < ns; ++k) {
-                tail_smooth<NB_PLAIN>(v, e, f, nullptr, c.w, c.h, 0);
-                tail_smooth<NB_PLAIN>(v, e, f, nullptr, c.w, c.h, 1);
+            tail_coarsest(v, B + 4 * n, B + 5 * n, A.cinv);
+            // colour by colour, as the levels above read it
+            for (int i = threadIdx.x; i < n; i += kCtThreads) {
+                int yx, x;
+                const int z = split(i, L.h * L.w, L.fhw, yx), y = split(yx, L.w, L.fw, x);
+                csm[L.eoff + ((x + y + z) & 1) * L.P + (z + 1) * L.ps + y * L.half + (x >> 1)] = B[4 * n + i];
             }
-            tail_restrict(v, e, f, F(l + 1), c.d, c.h, c.w);
-        }
-        tail_coarsest(lv(nl - 1), E(nl - 1), F(nl - 1), A.cinv);
-        for (int l = nl - 2; l >= ls; --l) {
-            const CtLevel& c = A.L[l + 1];
-            const LV v = lv(l);
-            float* e = E(l);
-            const float* f = F(l);
-            tail_smooth<NB_PROLONG>(v, e, f, E(l + 1), c.w, c.h, 1);
-            for (int k = 0; k < ns; ++k) {
-                if (k > 0) tail_smooth<NB_PLAIN>(v, e, f, nullptr, c.w, c.h, 1);
-                tail_smooth<NB_PLAIN>(v, e, f, nullptr, c.w, c.h, 0);
+            __syncthreads();
+        } else {
+            const CtLevel& Lc = A.L[l + 1];
+            const int z0 = ct_z0(L, T.rank, dist), nz = ct_nz(L, T.rank, dist);
+            const bool last = l + 1 == ls;  // the last distributed level
+            if (t > 0) ct_load(A, l, T.rank, P);
+            // what the level reads is complete: its first red cells, the
+            // restriction into it, or rank 0's part of the correction below
+            if (dist && (!up || last)) ct_sync();
+            if (l > lt) ct_load_f(T, L, P);
+            if (up) {
+                ct_correct(T, L, Lc, csm + (last ? A.coff : Lc.eoff), dist ? (z0 - 1) >> 1 : -1, last ? A.cP : Lc.P,
+                           z0, nz);
+                __syncthreads();
+            }
+            const int sweeps = up ? 2 * ns : 2 * ns - 1;  // black first, then in turn
+            for (int k = 0; k < sweeps; ++k) {
+                if (k & 1)
+                    ct_sweep<0>(T, L, P);
+                else
+                    ct_sweep<1>(T, L, P);
+                ct_barrier(dist);
+            }
+            if (!up) {
+                ct_terms(T, A, L, P, last);
+                ct_barrier(last);
+                if (!last) {
+                    ct_sum(T, A, l, z0, nz, L.ppc * L.ps);
+                } else if (T.rank == 0) {
+                    ct_sum(T, A, l, 0, L.d, L.d * L.ps);
+                }
+                __syncthreads();
             }
         }
+        if (l == ls && t >= down) {
+            // the correction to the ranks: the parents of each one's planes
+            // and halos, from plane (r ppc - 1) >> 1
+            const int ppc = A.L[ls - 1].ppc, n = (ppc / 2 + 2) * L.ps;
+            for (int i = threadIdx.x; i < 2 * n; i += kCtThreads) {
+                const int col = i >= n, c = i - col * n;
+                const int src = L.eoff + col * L.P + c + L.ps, at = A.coff + col * A.cP + c;
+                for (int r = 0; r < A.ranks; ++r) {
+                    const int o = ((r * ppc - 1) >> 1) * L.ps;  // (plane -1: the halo's zeros)
+                    if (c + o < L.d * L.ps) ct_store(ct_addr(csm, (unsigned)r), at, csm[src + o]);
+                }
+            }
+        }
+    }
+    // the first level's correction to global memory (own planes) and, for a
+    // whole V-cycle, z.r and sum(z)
+    const CtLevel& L = A.L[lt];
+    const int z0 = T.rank * L.ppc;
+    Acc<float> acc, zs;
+#pragma unroll
+    for (int j = 0; j < kCtPairs; ++j) {
+        if (!P.ib[j]) continue;
+        int zl, y, k;
+        ct_pos(L, (int)threadIdx.x + j * kCtThreads, zl, y, k);
+        const int g = ((z0 + zl) * L.h + y) * L.w + 2 * k;
+#pragma unroll
+        for (int col = 0; col < 2; ++col) {
+            const int u = P.s[j] ^ col;
+            if (2 * k + u >= L.w) continue;
+            const float ev = csm[L.eoff + col * L.P + P.ib[j]];
+            A.e_out[g + u] = ev;
+            if (lt == 0) {
+                acc.add(ev * P.c[j][col].f);
+                zs.add(ev);
+            }
+        }
+    }
+    if (lt > 0) return;
+    double a = acc.value(), c = zs.value();
+    block_sum2<kCtThreads>(a, c, (double*)csm);  // (starts with a barrier: e has been read)
+    if (threadIdx.x == 0) {
+        double* d = (double*)ct_map((float*)&sums[T.rank][0], 0u);
+        d[0] = a;
+        d[1] = c;
     }
     ct_sync();
-    // up through the distributed levels
-    for (int l = ls - 1; l >= lt; --l) {
-        const CtLevel& L = A.L[l];
-        ct_smooth<NB_PROLONG>(peer, L, &A.L[l + 1], rank, 1);
-        ct_sync();
-        for (int k = 0; k < ns; ++k) {
-            if (k > 0) {
-                ct_smooth<NB_PLAIN>(peer, L, nullptr, rank, 1);
-                ct_sync();
-            }
-            ct_smooth<NB_PLAIN>(peer, L, nullptr, rank, 0);
-            ct_sync();
+    if (T.rank == 0 && threadIdx.x == 0) {
+        double rz = 0.0, zsum = 0.0;
+        for (int r = 0; r < A.ranks; ++r) {
+            rz += sums[r][0];
+            zsum += sums[r][1];
         }
+        cg_finish_rz(st, rz, zsum);
     }
-    // level lt's correction to global memory (own slab, own shared memory)
-    const CtLevel& L = A.L[lt];
-    const int z0 = rank * L.ppc, nz = max(0, min(L.ppc, L.d - z0));
-    const float* Eo = csm + L.off + 4 * L.P;
-    for (int c = threadIdx.x; c < nz * L.h * L.w; c += blockDim.x) A.e_out[z0 * L.h * L.w + c] = Eo[c];
+}
+
+// Packed weights of a level for the cluster tail (wy null: 2D, whose y
+// weights stand for z).
+__global__ void k_mg_pack(float4* __restrict__ wp, const float* __restrict__ wx, const float* __restrict__ wy,
+                          const float* __restrict__ wz, const float* __restrict__ invd, int d, int h, int w) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d * h * w; c += gridDim.x * blockDim.x) {
+        const int x = c % w, zy = c / w, y = zy % h, z = zy / h;
+        wp[2 * c] = make_float4(wx[c], x + 1 < w ? wx[c + 1] : 0.f, wy ? wy[c] : 0.f, wy && y + 1 < h ? wy[c + w] : 0.f);
+        wp[2 * c + 1] = make_float4(wz[c], z + 1 < d ? wz[c + h * w] : 0.f, invd[c], 0.f);
+    }
 }
 
 // Coarse face weights: half the sum of the fine weights on the coarse face.
@@ -1408,6 +1610,7 @@ void release_mg(Extras* ex) {
         release_pockets(&ex->mg->pockets);
         cudaFree(ex->mg->mem);
         cudaFree(ex->mg->e0b);
+        cudaFree(ex->mg->ct_mem);
         cudaFree(ex->mg->cinv);
         delete ex->mg;
         ex->mg = nullptr;
@@ -1620,6 +1823,23 @@ static int ensure_mg(pg_grid* g, double dt, MgHierarchy** out) {
         const LV cv = view(*H, l + 1);
         PG_LAUNCH(KK_MG_SETUP, s, k_mg_invd<<<blocks_for(g, nc), kMgThreads, 0, s>>>(cv, C.invd));
     }
+    if (H->ct_ranks > 0) {
+        const bool d3 = g->dims.nd == 3;
+        size_t cells = 0;
+        for (int l = std::max(1, H->ct_lt); l + 1 < nl; ++l) cells += (size_t)H->lv[l].D.nc();
+        err = cudaMalloc(&H->ct_mem, std::max<size_t>(cells, 1) * 2 * sizeof(float4));
+        if (err != cudaSuccess) return cuda_fail(err, "cudaMalloc(mg packed weights)");
+        float4* q = (float4*)H->ct_mem;
+        for (int l = std::max(1, H->ct_lt); l + 1 < nl; ++l) {
+            MgLevel& L = H->lv[l];
+            L.wp = q;
+            q += 2 * (size_t)L.D.nc();
+            PG_LAUNCH(KK_MG_SETUP, s,
+                      k_mg_pack<<<blocks_for(g, L.D.nc()), kMgThreads, 0, s>>>(
+                          L.wp, L.wx, d3 ? L.wy : nullptr, d3 ? L.wz : L.wy, L.invd, d3 ? (int)L.D.d : (int)L.D.h,
+                          d3 ? (int)L.D.h : 1, (int)L.D.w));
+        }
+    }
     PG_CHECK_LAUNCH();
     if (const int crc = coarsest_pinv(g, H)) return crc;
     *out = H;
@@ -1799,30 +2019,67 @@ static int launch_tail(pg_grid* g, const MgHierarchy& H, int nsmooth) {
     return PG_OK;
 }
 
-// Shared-memory layout of the cluster tail with R ranks; 0 when it does not
-// fit.
+// Shapes and shared-memory layout of the cluster tail for levels [lt, ls)
+// distributed over R ranks and [ls, nl) in rank 0; 0 when it does not fit.
 static size_t ctail_layout(const MgHierarchy& H, int lt, int ls, int R, CtArgs* A) {
-    size_t off = 0;
+    size_t off = 0, terms = 0;
+    const bool d3 = H.D0.nd == 3;
+    const auto depth = [&](int l) { return d3 ? H.lv[l].D.d : H.lv[l].D.h; };
+    A->lt = lt;
+    A->ls = ls;
+    A->nl = H.nlev;
+    A->nd = H.D0.nd;
+    A->dt = (float)H.dt;
+    A->ranks = R;
+    // planes per rank: doubled from the last distributed level on
+    i64 ppc = (depth(ls - 1) + R - 1) / R;
+    for (int l = ls - 1; l > lt; --l) ppc *= 2;
     for (int l = lt; l < H.nlev; ++l) {
         const Dims& D = H.lv[l].D;
         CtLevel& L = A->L[l];
-        L.d = (int)D.d;
-        L.h = (int)D.h;
+        L.d = (int)depth(l);
+        L.h = d3 ? (int)D.h : 1;
         L.w = (int)D.w;
-        L.ppc = l < ls ? (int)((D.d + R - 1) / R) : (int)D.d;
-        L.P = (int)(((size_t)L.ppc * D.h * D.w + 3) & ~(size_t)3);
-        L.fhalf = fast_div((unsigned)((D.w + 1) / 2));
-        L.fh = fast_div((unsigned)D.h);
-        L.fw = fast_div((unsigned)D.w);
-        L.fhw = fast_div((unsigned)(D.h * D.w));
-        L.fppc = fast_div((unsigned)L.ppc);
-        L.off = (int)off;
-        L.wx = H.lv[l].wx;
-        L.wy = H.lv[l].wy;
-        L.wz = H.lv[l].wz;
-        L.invd = H.lv[l].invd;
-        off += 6 * (size_t)L.P;
+        L.half = (L.w + 1) / 2;
+        L.ps = L.h * L.half;
+        L.ppc = l < ls ? (int)ppc : L.d;
+        if (l < ls) ppc /= 2;
+        L.fhalf = fast_div((unsigned)L.half);
+        L.fh = fast_div((unsigned)L.h);
+        L.fw = fast_div((unsigned)L.w);
+        L.fhw = fast_div((unsigned)(L.h * L.w));
+        L.flags = l == 0 ? H.flags : nullptr;
+        L.wp = H.lv[l].wp;
+        const i64 own = std::min<i64>(L.ppc, L.d);
+        if (l + 1 < H.nlev && own * L.ps > kCtPairs * kCtThreads) return 0;
+        const size_t P = (size_t)(L.ppc + 2) * L.ps, F = (size_t)L.ppc * L.ps;
+        if (2 * (P + F) > (size_t)kCtSmemMax) return 0;  // (keeps the offsets in range)
+        L.P = (int)P;
+        L.eoff = (int)off;
+        off += 2 * P;
+        L.foff = (int)off;
+        off += 2 * F;
+        // the last distributed level's terms all go to rank 0
+        terms = std::max(terms, l == ls - 1 ? 2 * (size_t)L.d * L.ps : 2 * F);
+        if (off > (size_t)kCtSmemMax) return 0;
     }
+    const CtLevel& S = A->L[ls];
+    const CtLevel& Z = A->L[H.nlev - 1];
+    off = (off + 3) & ~(size_t)3;
+    A->zero4 = (int)(off / 4);
+    A->toff = (int)off;
+    off += terms;
+    A->coff = (int)off;
+    A->cP = (A->L[ls - 1].ppc / 2 + 2) * S.ps;
+    off += 2 * (size_t)A->cP;
+    A->zoff = (int)off;
+    off += 6 * (size_t)Z.d * Z.h * Z.w;
+    off = std::max(off, (size_t)2 * 2 * kCtThreads);  // the final sums' doubles
+    const MgLevel& C = H.lv[H.nlev - 1];
+    A->zwx = C.wx;
+    A->zwy = d3 ? C.wy : nullptr;
+    A->zwz = d3 ? C.wz : C.wy;
+    A->zinvd = C.invd;
     const size_t bytes = off * sizeof(float);
     return bytes <= (size_t)kCtSmemMax ? bytes : 0;
 }
@@ -1842,63 +2099,60 @@ static cudaLaunchConfig_t ctail_config(int R, size_t smem, cudaStream_t s, cudaL
     return cfg;
 }
 
-// Cluster tail for 3D hierarchies: a level of at most kCtCells cells above
-// the rank-0 levels, 16 or 8 ranks that fit and can be resident together;
+// Cluster tail: from the first level whose slabs fit 16 (or 8) ranks that can
+// be resident together, at least one level above the rank-0 levels.  3D
+// hierarchies keep their fine level out of it (its pair kernels use the whole
+// chip); 2D ones take it in where it fits, as the whole V-cycle.
 // PG_MG_CTAIL=0 keeps the per-level kernels and the single-block tail (a
 // diagnostic switch read per build).
 static void ctail_setup(MgHierarchy* H) {
-    H->ct_lt = 0;
+    H->ct_ranks = 0;
     const char* env = getenv("PG_MG_CTAIL");
-    if ((env && env[0] == '0') || H->D0.nd != 3) return;
+    if (env && env[0] == '0') return;
     const int nl = H->nlev;
-    int lt = 0, ls = 0;
-    for (int l = 1; l < nl; ++l)
-        if (H->lv[l].D.nc() <= kCtCells) {
-            lt = l;
-            break;
+    for (int R : {16, 8})
+        for (int lt = H->D0.nd == 3 ? 1 : 0; lt + 1 < nl; ++lt) {
+            // a rank-0 level: small enough, and its pairs (rows of odd width
+            // have one more) within a block's
+            const auto local = [&](int l) {
+                const Dims& D = H->lv[l].D;
+                return D.nc() <= kCtLocal && (l == nl - 1 || D.d * D.h * ((D.w + 1) / 2) <= kCtPairs * kCtThreads);
+            };
+            int ls = lt + 1;
+            while (ls < nl - 1 && !local(ls)) ++ls;
+            if (local(lt) || !local(ls)) continue;
+            CtArgs A{};
+            const size_t smem = ctail_layout(*H, lt, ls, R, &A);
+            if (smem == 0) continue;
+            if (cudaFuncSetAttribute(k_mg_ctail, cudaFuncAttributeMaxDynamicSharedMemorySize, kCtSmemMax) !=
+                    cudaSuccess ||
+                (R > 8 && cudaFuncSetAttribute(k_mg_ctail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                              cudaSuccess)) {
+                cudaGetLastError();
+                break;
+            }
+            cudaLaunchAttribute at[1];
+            const cudaLaunchConfig_t cfg = ctail_config(R, smem, nullptr, at);
+            int nclusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&nclusters, k_mg_ctail, &cfg) != cudaSuccess || nclusters < 1) {
+                cudaGetLastError();
+                continue;
+            }
+            H->ct_lt = lt;
+            H->ct_ls = ls;
+            H->ct_ranks = R;
+            H->ct_smem = smem;
+            return;
         }
-    if (lt == 0) return;
-    for (int l = lt; l < nl; ++l)
-        if (H->lv[l].D.nc() <= kCtLocal) {
-            ls = l;
-            break;
-        }
-    if (ls <= lt || ls > nl - 1) return;
-    for (int R : {16, 8}) {
-        CtArgs A{};
-        const size_t smem = ctail_layout(*H, lt, ls, R, &A);
-        if (smem == 0) continue;
-        if (cudaFuncSetAttribute(k_mg_ctail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            (R > 8 && cudaFuncSetAttribute(k_mg_ctail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                          cudaSuccess)) {
-            cudaGetLastError();
-            continue;
-        }
-        cudaLaunchAttribute at[1];
-        const cudaLaunchConfig_t cfg = ctail_config(R, smem, nullptr, at);
-        int nclusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&nclusters, k_mg_ctail, &cfg) != cudaSuccess || nclusters < 1) {
-            cudaGetLastError();
-            continue;
-        }
-        H->ct_lt = lt;
-        H->ct_ls = ls;
-        H->ct_ranks = R;
-        H->ct_smem = smem;
-        return;
-    }
 }
 
-static int launch_ctail(pg_grid* g, const MgHierarchy& H, int nsmooth) {
+// e, f: of the cluster tail's first level.
+static int launch_ctail(pg_grid* g, const MgHierarchy& H, int nsmooth, float* e, const float* f) {
     CtArgs A{};
     ctail_layout(H, H.ct_lt, H.ct_ls, H.ct_ranks, &A);
-    A.lt = H.ct_lt;
-    A.ls = H.ct_ls;
-    A.nl = H.nlev;
     A.nsmooth = nsmooth;
-    A.ranks = H.ct_ranks;
-    A.e_out = H.lv[H.ct_lt].e;
-    A.f_in = H.lv[H.ct_lt].f;
+    A.e_out = e;
+    A.f_in = f;
     A.cinv = H.cinv;
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = ctail_config(H.ct_ranks, H.ct_smem, g->stream, at);
@@ -1978,7 +2232,7 @@ static int vcycle(pg_grid* g, const MgHierarchy& H, const float* r, float* z, in
     }
     // levels [0, top) run as per-level kernels; [top, nl) in the tail kernel
     // (or, without a tail, the coarsest level alone in k_mg_coarse)
-    const bool ctail = H.ct_lt > 0;
+    const bool ctail = H.ct_ranks > 0 && l0 <= H.ct_lt;
     const bool tail = ctail || H.tail < nl;
     const int top = ctail ? H.ct_lt : tail ? H.tail : nl - 1;
     // Fine level of 3D grids as fused pairs: 2 * nsmooth of them alternate
@@ -2030,7 +2284,7 @@ static int vcycle(pg_grid* g, const MgHierarchy& H, const float* r, float* z, in
         }
     }
     if (tail) {
-        const int rc = ctail ? launch_ctail(g, H, nsmooth) : launch_tail(g, H, nsmooth);
+        const int rc = ctail ? launch_ctail(g, H, nsmooth, E(top), F(top)) : launch_tail(g, H, nsmooth);
         if (rc) return rc;
     } else {
         const LV v = view(H, nl - 1);
