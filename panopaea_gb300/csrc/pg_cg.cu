@@ -10,7 +10,9 @@
 // The scalars (sigma, alpha, beta, the stop test) live in a device-side
 // CgState written by the last block of each reduction kernel, so the host
 // polls a pinned copy every few iterations and never sits between kernels.
-// Once the stop test fires every later kernel returns at entry.
+// Once the stop test fires every later kernel returns at entry.  Small double
+// grids run the identity / Jacobi CG as one cooperative kernel instead
+// (pg_cg_coop.cu).
 //
 // GB300 runs FP64 at 1/64 of the FP32 rate, so no per-cell work is FP64:
 // each thread accumulates a compensated FP32 partial (float fields) and
@@ -777,20 +779,15 @@ static int get_graph(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook* h
     return PG_OK;
 }
 
+// The init kernel and the loop of two kernels per iteration (plus the outer
+// preconditioner's): a graph launch (*out), or polled by the host.
 template <class T, int PM>
-static int run_cg_pm(pg_grid* g, const CgConfig& cfg, CgBuffers<T> buf, pg_pcg_stats* stats, ZHook* hook) {
-    int rc = ensure_workspace(g);
-    if (rc) return rc;
-    const Dims& D = g->dims;
-    const i64 n = D.nc();
+static int run_loop(pg_grid* g, const CgConfig& cfg, const CgBuffers<T>& buf, ZHook* hook, int nb, CgGraph** out) {
+    const i64 n = g->dims.nc();
     const T dt = (T)cfg.dt;
-    const int nb = grid_blocks(g, n, kCgThreads, 8);
     Workspace& ws = g->ws;
     cudaStream_t s = g->stream;
-    // The double-float iterate exists only in the float4 kernels.
-    if (buf.xl && (PM != PM_ZBUF || !cg_dfx_ok(buf, n, g->flags)))
-        return bad_arg("run_cg: a double-float iterate needs the float4 MG path");
-    PG_CUDA(cudaMemsetAsync(ws.state, 0, sizeof(CgState), s));
+    int rc;
     const bool fold = PM == PM_ZBUF && cg_fold(buf, hook);
     if (PM == PM_ZBUF && sizeof(T) == 4 && n % 4 == 0 && aligned16(buf.x) && aligned16(buf.r) && aligned16(buf.b))
         PG_LAUNCH(KK_CG_INIT, s,
@@ -807,7 +804,7 @@ static int run_cg_pm(pg_grid* g, const CgConfig& cfg, CgBuffers<T> buf, pg_pcg_s
     if (PM == PM_ZBUF) hook->bind(buf.ap);
     if (PM == PM_ZBUF && (rc = hook->apply(g, fold ? (const void*)buf.b : (const void*)buf.r, buf.z))) return rc;
     // Device-side loop: one graph launch runs every iteration.
-    CgGraph* G = nullptr;
+    CgGraph*& G = *out;
     if (graphs_enabled() && cfg.max_iter > 0) {
         if ((rc = get_graph<T, PM>(g, buf, dt, nb, hook, &G))) return rc;
         PG_CUDA(cudaGraphLaunch(G->exec, s));
@@ -837,6 +834,29 @@ static int run_cg_pm(pg_grid* g, const CgConfig& cfg, CgBuffers<T> buf, pg_pcg_s
         pending = slot;
         slot ^= 1;
     }
+    return PG_OK;
+}
+
+template <class T, int PM>
+static int run_cg_pm(pg_grid* g, const CgConfig& cfg, CgBuffers<T> buf, pg_pcg_stats* stats, ZHook* hook) {
+    int rc = ensure_workspace(g);
+    if (rc) return rc;
+    const Dims& D = g->dims;
+    const i64 n = D.nc();
+    const T dt = (T)cfg.dt;
+    const int nb = grid_blocks(g, n, kCgThreads, 8);
+    Workspace& ws = g->ws;
+    cudaStream_t s = g->stream;
+    // The double-float iterate exists only in the float4 kernels.
+    if (buf.xl && (PM != PM_ZBUF || !cg_dfx_ok(buf, n, g->flags)))
+        return bad_arg("run_cg: a double-float iterate needs the float4 MG path");
+    PG_CUDA(cudaMemsetAsync(ws.state, 0, sizeof(CgState), s));
+    bool coop = false;
+    if (sizeof(T) == 8 && PM != PM_ZBUF &&
+        (rc = cg_coop_run(g, cfg, reinterpret_cast<const CgBuffers<double>&>(buf), PM, &coop)))
+        return rc;
+    CgGraph* G = nullptr;
+    if (!coop && (rc = run_loop<T, PM>(g, cfg, buf, hook, nb, &G))) return rc;
     static_assert(sizeof(CgState) % 4 == 0, "CgState words");
     k_words_out<<<1, 64, 0, s>>>((const unsigned*)ws.state, (unsigned*)(ws.state_host + 2),
                                  (int)(sizeof(CgState) / 4));

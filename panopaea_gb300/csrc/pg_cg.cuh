@@ -88,6 +88,11 @@ struct ZHook {
 template <class T>
 int run_cg(pg_grid* g, const CgConfig& cfg, CgBuffers<T> buf, pg_pcg_stats* stats, ZHook* hook = nullptr);
 
+// The whole identity / Jacobi solve of a small double grid as one cooperative
+// kernel (pg_cg_coop.cu); *done: it was launched and leaves the final state.
+int cg_coop_run(pg_grid* g, const CgConfig& cfg, const CgBuffers<double>& buf, int pm, bool* done);
+size_t cg_coop_bytes();  // its exchange slots (Workspace::coop)
+
 // Whether run_cg with MG preconditioning can carry x as the double-float pair
 // (buf.x, buf.xl): float4-aligned buffers and flags, cells a multiple of 4.
 // PG_CG_DFX=0 turns it off (a diagnostic switch).

@@ -3,6 +3,7 @@
 #include <cstring>
 #include <vector>
 
+#include "pg_cg.cuh"
 #include "pg_internal.cuh"
 
 namespace pg {
@@ -30,6 +31,7 @@ int ensure_workspace(pg_grid* g) {
     PG_CUDA(cudaMalloc(&ws.partials, sizeof(double) * 4 * kMaxBlocks));
     PG_CUDA(cudaMalloc(&ws.state, sizeof(CgState)));
     PG_CUDA(cudaMemset(ws.state, 0, sizeof(CgState)));
+    PG_CUDA(cudaMalloc(&ws.coop, cg_coop_bytes()));
     // slots 0, 1: the host-polled loop; slot 2: the final state; then one
     // double (a reduction result read back by the host)
     PG_CUDA(cudaMallocHost(&ws.state_host, 3 * sizeof(CgState) + sizeof(double)));
@@ -158,6 +160,7 @@ int pg_grid_destroy(pg_grid* g) {
     cudaFree(g->ws.state);
     cudaFreeHost(g->ws.state_host);
     cudaFree(g->ws.vec);
+    cudaFree(g->ws.coop);
     if (g->ws.ev[0]) cudaEventDestroy(g->ws.ev[0]);
     if (g->ws.ev[1]) cudaEventDestroy(g->ws.ev[1]);
     release_extras(g);

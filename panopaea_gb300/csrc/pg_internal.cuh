@@ -213,6 +213,7 @@ struct Workspace {
     size_t vec_bytes = 0;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     void* graphs = nullptr;      // cached CG-loop graphs (pg_cg.cu)
+    void* coop = nullptr;        // exchange slots of the cooperative CG (pg_cg_coop.cu)
 };
 
 constexpr int kMaxBlocks = 4096;

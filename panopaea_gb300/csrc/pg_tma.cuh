@@ -81,7 +81,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
     return false;
 }
 
-// Host: the stage-wait poll budget of pg_spmv.cu's and pg_mg.cu's kernels.
+// Host: the stage-wait poll budget of pg_spmv.cu's and pg_mg.cu's kernels, and
+// that of pg_cg_coop.cu's exchanges.
+int set_stage_wait_polls_coop(unsigned polls);
 int set_stage_wait_polls_spmv(unsigned polls);
 int set_stage_wait_polls_mg(unsigned polls);
 
