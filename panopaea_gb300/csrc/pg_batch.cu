@@ -152,14 +152,12 @@ __global__ void k_b_project(float* __restrict__ vel, const float* __restrict__ p
 // ---------------------------------------------------------------------------
 // CG over all grids (pcg.rs:14-82 per grid)
 
-// PM_ZBUF: r is the MG z buffer, used as z - zm on the fluid cells.
 template <int PM> __device__ __forceinline__ float bz(const float* __restrict__ r, const uint8_t* __restrict__ flags,
-                                                      i64 k, float dt, float zm = 0.f) {
+                                                      i64 k, float dt) {
     if (PM == PM_JACOBI) {
         const int n = __popc((unsigned)flags[k]);
         return n ? r[k] * __frcp_rn((float)n * dt) : 0.f;
     }
-    if (PM == PM_ZBUF) return flags[k] ? r[k] - zm : r[k];
     return r[k];
 }
 
@@ -195,17 +193,18 @@ __global__ void k_b_cg_init(float* __restrict__ x, float* __restrict__ r, const 
 // One block per grid: fold the grid's tile partials (fixed order).
 // stage 0: after init; 1: after the SpMV (p.Ap); 2: after the update.
 // zbuf (stage 2): z comes from an outer preconditioner after the update,
-// so beta and sigma are set later (bmg_rz_finalize).
+// so beta and sigma are set later (bmg_rz_finalize).  range: the partials
+// of each grid where they are not one per tile.
 template <int STAGE>
 __global__ void k_b_finalize(const GInfo* __restrict__ gi, BState* __restrict__ st, const double* __restrict__ partials,
                              int n, double rel_tol, double thr_abs, int max_iter, int* active, int zbuf = 0,
-                             const double* __restrict__ nfluid = nullptr) {
+                             const double* __restrict__ nfluid = nullptr, const int2* __restrict__ range = nullptr) {
     __shared__ double sm[32];
     const int g = blockIdx.x;
     if (g >= n) return;
     BState& S = st[g];
     if (STAGE != 0 && S.done) return;
-    const int t0 = gi[g].t0, t1 = gi[g].t1;
+    const int t0 = range ? range[g].x : gi[g].t0, t1 = range ? range[g].y : gi[g].t1;
     double a = 0.0, bb = 0.0;
     for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
         const double pa = partials[2 * (i64)t], pb = partials[2 * (i64)t + 1];
@@ -293,14 +292,11 @@ __global__ void k_b_spmv(const float* __restrict__ r, float* p0, float* p1, floa
         const GInfo G = gi[t.grid];
         const int it = S.iter, first = S.first;
         const float beta = first ? 0.f : S.fbeta;
-        const float zm = PM == PM_ZBUF ? S.fzm : 0.f;
         const float* p_old = (it & 1) ? p1 : p0;
         float* p_new = (it & 1) ? p0 : p1;
-        // p_new of cell k; `fluid`: k has an open face (a neighbour behind an
-        // open face always has), the cells the projected z applies to
-        auto pn = [&](i64 k, bool fluid) -> float {
+        auto pn = [&](i64 k) -> float {  // p_new of cell k
             if (!FUSED) return p_new[k];
-            const float z = PM == PM_ZBUF ? (fluid ? r[k] - zm : r[k]) : bz<PM>(r, flags, k, dt);
+            const float z = bz<PM>(r, flags, k, dt);
             return first ? z : z + beta * p_old[k];
         };
         const int xx = t.x0 + (int)threadIdx.x % tx, yy = t.y0 + (int)threadIdx.x / tx;
@@ -308,12 +304,12 @@ __global__ void k_b_spmv(const float* __restrict__ r, float* p0, float* p1, floa
         if (xx < G.w && yy < G.h) {
             const i64 c = G.coff + (i64)yy * G.w + xx;
             const uint8_t f = flags[c];
-            const float pc = pn(c, f != 0);
+            const float pc = pn(c);
             if (FUSED) p_new[c] = pc;
-            const float gy_lo = (f & YLO) ? -sub_rn(pc, pn(c - G.w, true)) : 0.f;
-            const float gy_hi = (f & YHI) ? -sub_rn(pn(c + G.w, true), pc) : 0.f;
-            const float gx_lo = (f & XLO) ? sub_rn(pn(c - 1, true), pc) : 0.f;
-            const float gx_hi = (f & XHI) ? sub_rn(pc, pn(c + 1, true)) : 0.f;
+            const float gy_lo = (f & YLO) ? -sub_rn(pc, pn(c - G.w)) : 0.f;
+            const float gy_hi = (f & YHI) ? -sub_rn(pn(c + G.w), pc) : 0.f;
+            const float gx_lo = (f & XLO) ? sub_rn(pn(c - 1), pc) : 0.f;
+            const float gx_hi = (f & XHI) ? sub_rn(pc, pn(c + 1)) : 0.f;
             const float a = mul_rn(add_rn(sub_rn(sub_rn(gy_hi, gy_lo), gx_lo), gx_hi), dt);
             ap[c] = a;
             acc.add(pc * a);
@@ -341,7 +337,7 @@ __global__ void k_b_pupdate(const float* __restrict__ r, float* p0, float* p1, c
             const i64 c = G.coff + (i64)yy * G.w + xx;
             const float* p_old = (S.iter & 1) ? p1 : p0;
             float* p_new = (S.iter & 1) ? p0 : p1;
-            const float z = bz<PM>(r, flags, c, dt, PM == PM_ZBUF ? S.fzm : 0.f);
+            const float z = bz<PM>(r, flags, c, dt);
             p_new[c] = S.first ? z : z + S.fbeta * p_old[c];
         }
     }
@@ -374,8 +370,7 @@ __global__ void k_b_update(float* __restrict__ x, float* __restrict__ r, const f
                 const int nn = __popc((unsigned)flags[c]);
                 z = nn ? rv * __frcp_rn((float)nn * dt) : 0.f;
             }
-            if (PM == PM_ZBUF) rz.add(rv);  // sum(r) for the lazy projection
-            else rz.add(z * rv);
+            rz.add(z * rv);
         }
         double m, s;
         tmaxsum(rm, f2_of(rz), sm, &m, &s);
@@ -436,30 +431,17 @@ static int bblocks(const pg_batch* B, int ntiles) {
 }
 
 // One CG iteration over all grids.  PM_ZBUF: z = V(r) by the batched
-// multigrid; the SpMV and update run in their identity-preconditioner form
-// with z in place of r.
+// multigrid, which brings its own SpMV and update.
 template <int PM> static void b_iter(pg_batch* B, cudaStream_t s, float dt, float* x, int nsmooth = 2) {
     if (PM == PM_ZBUF) {
-        const int nt = B->tx * B->ty, nb = bblocks(B, B->ntiles);
-        if (B->fused) {
-            PG_LAUNCH(KK_CG_SPMV, s,
-                      k_b_spmv<PM_ZBUF, 1><<<nb, nt, 0, s>>>(B->z, B->p0, B->p1, B->ap, B->flags, B->ginfo, B->tiles,
-                                                             B->ntiles, B->tx, B->ty, dt, B->state, B->partials));
-        } else {
-            PG_LAUNCH(KK_CG_SPMV, s,
-                      k_b_pupdate<PM_ZBUF><<<nb, nt, 0, s>>>(B->z, B->p0, B->p1, B->flags, B->ginfo, B->tiles, B->ntiles,
-                                                             B->tx, B->ty, dt, B->state));
-            PG_LAUNCH(KK_CG_SPMV, s,
-                      k_b_spmv<PM_ZBUF, 0><<<nb, nt, 0, s>>>(B->z, B->p0, B->p1, B->ap, B->flags, B->ginfo, B->tiles,
-                                                             B->ntiles, B->tx, B->ty, dt, B->state, B->partials));
-        }
+        bmg_spmv(B, s, dt);
         PG_LAUNCH(KK_STEP_MISC, s,
-                  k_b_finalize<1><<<B->n, 128, 0, s>>>(B->ginfo, B->state, B->partials, B->n, 0.0, 0.0, 0, B->active));
-        PG_LAUNCH(KK_CG_UPDATE, s,
-                  k_b_update<PM_ZBUF><<<nb, nt, 0, s>>>(x, B->r, B->p0, B->p1, B->ap, B->flags, B->ginfo, B->tiles,
-                                                        B->ntiles, B->tx, B->ty, dt, B->state, B->partials));
+                  k_b_finalize<1><<<B->n, 128, 0, s>>>(B->ginfo, B->state, bmg_partials(B), B->n, 0.0, 0.0, 0, B->active,
+                                                       0, nullptr, bmg_spmv_range(B)));
+        bmg_update(B, s, x);
         PG_LAUNCH(KK_STEP_MISC, s,
-                  k_b_finalize<2><<<B->n, 128, 0, s>>>(B->ginfo, B->state, B->partials, B->n, 0.0, 0.0, 0, B->active, 1));
+                  k_b_finalize<2><<<B->n, 128, 0, s>>>(B->ginfo, B->state, bmg_partials(B), B->n, 0.0, 0.0, 0, B->active,
+                                                       1, nullptr, bmg_update_range(B)));
         bmg_vcycle(B, s, nsmooth);
         bmg_rz_finalize(B, s, 0);
         return;

@@ -9,15 +9,19 @@
 // the children's residuals, prolongation adds the parent's correction;
 // red-black Gauss-Seidel, `nsmooth` sweeps (red, black) before and (black,
 // red) after, so the V-cycle is symmetric; the coarsest level is solved in
-// shared memory by symmetric sweeps.  Grids have different depths:
-// level l of the batch packs level l of every grid deep enough, each stage
-// is ONE launch over a tile list of that level (smoothing tiles of 64 x 8
-// cells on level 0, 64 x 32 above, one cell of the colour per row and
-// thread; restriction tiles of 32 x 8 coarse cells), and the coarsest solve
-// is one launch with one block per grid, each at its own coarsest level.  Tiles of grids whose CG has
-// converged return at once.  The last fine half-sweep writes one z.r
-// partial per tile; a per-grid block folds them in a fixed order.
+// shared memory by symmetric sweeps.  Grids have different depths: level l
+// of the batch packs level l of every grid that has it.
+//
+// The large levels are smoothed by warps that march down strips of 64
+// columns (k_bmg_pair: both half-sweeps of a pair from one read of the
+// level, restriction and z.r on the way), one launch for all grids; the
+// rest of a grid's hierarchy, from its first level of kBmgTailCells cells or
+// fewer in all, is one block's work in shared memory (k_bmg_tail), one
+// launch as well.  The CG kernels around the V-cycle march likewise.  Grids
+// whose CG has converged return at once.  Every warp writes one partial
+// sum; a per-grid block folds them in a fixed order.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "pg_batch.cuh"
@@ -26,31 +30,28 @@ namespace pg {
 
 constexpr int kBmgMaxLevels = 16;
 constexpr int kBmgCoarseMax = 2048;
-constexpr int kBmgCoarseThreads = 512;
-constexpr int kSmTX = 32, kSmTY = 8;  // smoothing block: 256 threads, 32 x 8
-// rows per thread (kSmTY apart) on level 0 and on the coarser levels: a
-// smoothing tile is 64 x (8 sm_rows) cells
-constexpr int kSmRows0 = 1, kSmRows = 4;
-__host__ __device__ constexpr int sm_rows(bool l0) { return l0 ? kSmRows0 : kSmRows; }
-constexpr int kRtX = 32, kRtY = 8;    // restriction tile: 32 x 8 coarse cells
+constexpr int kRtX = 32, kRtY = 8;  // setup tile: 32 x 8 coarse cells
+constexpr int kMarchThreads = 128;  // four strips per block
+// Cells (of all its levels together, 20 bytes each) that a block keeps in
+// shared memory, two blocks per SM: 64 x 64 and the levels below it are 5456.
+constexpr int kBmgTailCells = 5600;
+constexpr int kBmgTailThreads = 512;
+constexpr int kUpdateCells = 2048;  // cells per warp of the CG update
 
 struct BLevel {
     int h, w;     // this grid's dims at this level
     i64 off;      // its first cell in the level's packed arrays (level 0: the batch offset)
     int coarse;   // the grid's coarsest level
-    int t0, t1;   // its smoothing tiles (level 0)
+    int tail;     // its first level of k_bmg_tail
+    int t0, t1;   // its smoothing strips (level 0)
     int ch, cw;   // dims at the next level (0 if none)
     i64 coff;     // first cell at the next level
 };
 
-struct CoarseInfo {
-    const float* wx;
-    const float* wy;
-    const float* invd;
-    float* e;
-    const float* f;
-    int h, w, level;
-    i64 off;
+// Cells [c0, c1) of a grid in the packed fields.
+struct Chunk {
+    int grid, pad;
+    i64 c0, c1;
 };
 
 struct BatchMg {
@@ -60,18 +61,25 @@ struct BatchMg {
     uint64_t id = 0;
     std::vector<void*> allocs;
     BLevel* info[kBmgMaxLevels] = {};
-    Tile* stiles[kBmgMaxLevels] = {};
+    Strip* strips[kBmgMaxLevels] = {};
     int nst[kBmgMaxLevels] = {};
-    int nsmoothing[kBmgMaxLevels] = {};  // grids smoothing at this level
+    int nsmoothing[kBmgMaxLevels] = {};  // grids smoothing at this level by k_bmg_pair
     Tile* rtiles[kBmgMaxLevels] = {};
     int nrt[kBmgMaxLevels] = {};
     float* wx[kBmgMaxLevels] = {};
     float* wy[kBmgMaxLevels] = {};
     float* invd[kBmgMaxLevels] = {};
     float* e[kBmgMaxLevels] = {};
+    float* e2[kBmgMaxLevels] = {};  // k_bmg_pair writes e and e2 in turn (level 0: z and ap)
     float* f[kBmgMaxLevels] = {};
-    CoarseInfo* coarse = nullptr;
-    double* partials = nullptr;
+    int tail_cells = 0;             // of the grid with the largest tail
+    Strip* cg_strips = nullptr;     // the SpMV's: 64 columns each, no overlap
+    int ncg = 0;
+    int2* cg_range = nullptr;
+    Chunk* chunks = nullptr;        // the CG update's
+    int nchunk = 0;
+    int2* chunk_range = nullptr;
+    double* partials = nullptr;     // 2 per strip or chunk
     Pockets pockets;  // fluid components of the grids with more than one
 };
 
@@ -81,10 +89,10 @@ struct BLv {
     const float* wx;
     const float* wy;
     const float* invd;
-    float* e;
     const float* f;
     const uint8_t* flags;  // level 0
     const float* ec;       // next level's correction (prolongation)
+    float* fc;             // next level's right-hand side (restriction)
     float dt;
     int level;
 };
@@ -110,226 +118,654 @@ template <bool L0> struct BCell {
     }
 };
 
-enum { BNB_PLAIN = 0, BNB_FIRST = 1, BNB_PROLONG = 2, BNB_SELF = 3 };
+enum { BP_PLAIN = 0, BP_SELF = 1, BP_PROLONG = 2 };
 
-template <bool L0, int MODE>
-__device__ __forceinline__ float bnb(const BLv& v, const BLevel& L, i64 k, int y, int x) {
-    if (MODE == BNB_FIRST) {
-        if (L0) {
-            const int n = __popc((unsigned)v.flags[k]);
-            return n ? v.f[k] * __frcp_rn((float)n * v.dt) : 0.f;
-        }
-        return v.f[k] * v.invd[k];
-    }
-    if (MODE == BNB_PROLONG) return v.e[k] + v.ec[L.coff + (i64)(y >> 1) * L.cw + (x >> 1)];
-    return v.e[k];
+// s + weight * neighbour over a cell's open faces (x-, x+, y-, y+).
+__device__ __forceinline__ float nb_sum(float s, float wl, float wr, float wu, float wd, float nl, float nr, float nu,
+                                        float nd) {
+    if (wl != 0.f) s = fmaf(wl, nl, s);
+    if (wr != 0.f) s = fmaf(wr, nr, s);
+    if (wu != 0.f) s = fmaf(wu, nu, s);
+    if (wd != 0.f) s = fmaf(wd, nd, s);
+    return s;
 }
 
-// What one red-black update of cell c = (y, x) reads, loaded before any of
-// it is used: a neighbour outside the grid is read at the cell itself (the
-// weight of a boundary face is 0, so it is never added), so a thread's
-// loads for all its rows issue together instead of waiting on the flags.
-template <bool L0, int MODE> struct BUpd {
-    float f, inv, w[4], n[4];
-    __device__ __forceinline__ void load(const BLv& v, const BLevel& L, i64 c, int y, int x) {
-        const int h = L.h, wd = L.w;
-        const bool xl = x > 0, xh = x + 1 < wd, yl = y > 0, yh = y + 1 < h;
-        f = v.f[c];
-        if (L0) {
-            const unsigned fl = v.flags[c];
-            w[0] = (fl & XLO) ? v.dt : 0.f;
-            w[1] = (fl & XHI) ? v.dt : 0.f;
-            w[2] = (fl & YLO) ? v.dt : 0.f;
-            w[3] = (fl & YHI) ? v.dt : 0.f;
-            const int nn = __popc(fl);
-            inv = nn ? __frcp_rn((float)nn * v.dt) : 0.f;
-        } else {
-            const float wxh = v.wx[xh ? c + 1 : c], wyh = v.wy[yh ? c + wd : c];
-            w[0] = v.wx[c];
-            w[1] = xh ? wxh : 0.f;
-            w[2] = v.wy[c];
-            w[3] = yh ? wyh : 0.f;
-            inv = v.invd[c];
+// What a lane holds of a row: e and f of its two cells, and their flags
+// (level 0) or weights and 1 / diagonal (coarser levels).
+template <bool L0> struct BRow {
+    float2 e, f;
+    Flag2 raw;  // as loaded; fl: both
+    unsigned fl;
+    float2 wx, wy, inv;
+    float wr;   // the second cell's x+ weight, from the next lane
+    float ec;   // as loaded: the correction to prolong
+};
+
+// One red-black pair over a strip: the first colour of row y (from the old
+// values of the rows around it), then the second colour of row y - 1 (from
+// the new ones), which finishes that row; with REST the residual of row y - 2
+// follows and is summed to the next level, with RZ the finished row's z.r and
+// sum(z).  C1: the parity of x + y of the first colour.  FA: the first
+// colour in this row is the lane's first cell.
+template <bool L0, int MODE, int C1, bool RZ, bool REST, bool VEC> struct March {
+    const BLv& v;
+    const BLevel& L;
+    const float* __restrict__ ein;
+    float* __restrict__ eout;
+    int lane, x, y0, y1;
+    bool va, vb, own, ownb;
+    float tab;  // lane f: 1 / diagonal of a cell with face-open bits f (level 0)
+    i64 at;     // index of the lane's first cell in the next row to fetch
+    int next;   // that row
+    int stop;   // the last row needed
+    BRow<L0> r[5];  // rows y - 3 .. y + 1
+    float rsum = 0.f;
+    Acc<float> acc, zs;
+
+    __device__ __forceinline__ March(const BLv& v_, const BLevel& L_, const Strip& S, const float* ein_, float* eout_)
+        : v(v_), L(L_), ein(ein_), eout(eout_) {
+        lane = threadIdx.x & 31;
+        x = S.x0 + 2 * lane;
+        y0 = S.y0;
+        y1 = S.y1;
+        va = x < L.w;
+        vb = x + 1 < L.w;
+        const int lo = S.x0 ? S.x0 + 4 : 0, hi = S.x0 + 64 >= L.w ? L.w : S.x0 + 60;
+        own = x >= lo && x < hi;
+        ownb = own && vb;
+        const int n = __popc(lane & 15);
+        tab = L0 && n ? __frcp_rn((float)n * v.dt) : 0.f;
+    }
+
+    // Row `next` (zeros outside the grid, so that no weight points there).
+    __device__ __forceinline__ BRow<L0> fetch() {
+        BRow<L0> q;
+        q.e = q.f = q.wx = q.wy = q.inv = make_float2(0.f, 0.f);
+        q.fl = q.raw.a = q.raw.b = 0;
+        q.wr = q.ec = 0.f;
+        if (next >= 0 && next <= stop) {  // uniform per warp
+            q.f = ld2<VEC>(v.f + at, va, vb);
+            if (L0) {
+                q.raw.template load<VEC>(v.flags + at, va, vb);
+            } else {
+                q.wx = ld2<VEC>(v.wx + at, va, vb);
+                q.wy = ld2<VEC>(v.wy + at, va, vb);
+                q.inv = ld2<VEC>(v.invd + at, va, vb);
+            }
+            if (MODE != BP_SELF) q.e = ld2<VEC>(ein + at, va, vb);
+            if (MODE == BP_PROLONG && va) q.ec = v.ec[L.coff + (i64)(next >> 1) * L.cw + (x >> 1)];
         }
-        if (MODE != BNB_SELF) {
-            n[0] = bnb<L0, MODE>(v, L, xl ? c - 1 : c, y, xl ? x - 1 : x);
-            n[1] = bnb<L0, MODE>(v, L, xh ? c + 1 : c, y, xh ? x + 1 : x);
-            n[2] = bnb<L0, MODE>(v, L, yl ? c - wd : c, yl ? y - 1 : y, x);
-            n[3] = bnb<L0, MODE>(v, L, yh ? c + wd : c, yh ? y + 1 : y, x);
+        ++next;
+        at += L.w;
+        return q;
+    }
+
+    __device__ __forceinline__ void push(const BRow<L0>& q) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r[k] = r[k + 1];
+        r[4] = q;
+        if (MODE == BP_PROLONG) {
+            r[4].e.x += q.ec;
+            r[4].e.y += q.ec;
+        }
+        if (L0) {
+            r[4].fl = q.raw.template both<VEC>();
+        } else {
+            const float n = __shfl_down_sync(0xffffffffu, q.wx.x, 1);
+            r[4].wr = lane < 31 ? n : 0.f;
         }
     }
-    // f + sum over the open faces of weight * neighbour, times 1 / diagonal
-    __device__ __forceinline__ float value() const {
-        float s = f;
-        if (MODE != BNB_SELF) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (w[j] != 0.f) s += w[j] * n[j];
+
+    // Weights of the first (A) or second cell of row k.
+    template <bool A> __device__ __forceinline__ void weights(int k, float& wl, float& wr, float& wu, float& wd) const {
+        if (L0) {
+            const unsigned f = A ? r[k].fl : r[k].fl >> 8;
+            wl = (f & XLO) ? v.dt : 0.f;
+            wr = (f & XHI) ? v.dt : 0.f;
+            wu = (f & YLO) ? v.dt : 0.f;
+            wd = (f & YHI) ? v.dt : 0.f;
+        } else {
+            wl = A ? r[k].wx.x : r[k].wx.y;
+            wr = A ? r[k].wx.y : r[k].wr;
+            wu = A ? r[k].wy.x : r[k].wy.y;
+            wd = A ? r[k + 1].wy.x : r[k + 1].wy.y;
         }
-        return s * inv;
+    }
+    template <bool A> __device__ __forceinline__ float inv(int k) const {
+        if (L0) return __shfl_sync(0xffffffffu, tab, A ? r[k].fl : r[k].fl >> 8);
+        return A ? r[k].inv.x : r[k].inv.y;
+    }
+    // The four neighbours' values.
+    template <bool A> __device__ __forceinline__ void around(int k, float& nl, float& nr, float& nu, float& nd) const {
+        if (A) {
+            nl = __shfl_up_sync(0xffffffffu, r[k].e.y, 1);
+            nr = r[k].e.y;
+        } else {
+            nl = r[k].e.x;
+            nr = __shfl_down_sync(0xffffffffu, r[k].e.x, 1);
+        }
+        nu = A ? r[k - 1].e.x : r[k - 1].e.y;
+        nd = A ? r[k + 1].e.x : r[k + 1].e.y;
+    }
+    template <bool A> __device__ __forceinline__ float updated(int k) const {
+        float wl, wr, wu, wd, nl, nr, nu, nd;
+        weights<A>(k, wl, wr, wu, wd);
+        around<A>(k, nl, nr, nu, nd);
+        return nb_sum(A ? r[k].f.x : r[k].f.y, wl, wr, wu, wd, nl, nr, nu, nd) * inv<A>(k);
+    }
+    template <bool A> __device__ __forceinline__ float residual(int k) const {
+        float wl, wr, wu, wd, nl, nr, nu, nd;
+        weights<A>(k, wl, wr, wu, wd);
+        around<A>(k, nl, nr, nu, nd);
+        const float c = A ? r[k].e.x : r[k].e.y;
+        return (A ? r[k].f.x : r[k].f.y) - nb_sum(0.f, wl, wr, wu, wd, c - nl, c - nr, c - nu, c - nd);
+    }
+
+    template <bool FA> __device__ __forceinline__ void step(int y) {
+        float n;
+        if (MODE == BP_SELF) {
+            const float i = inv<FA>(3), f = FA ? r[3].f.x : r[3].f.y;
+            n = i != 0.f ? f * i : 0.f;
+        } else {
+            n = updated<FA>(3);
+        }
+        (FA ? r[3].e.x : r[3].e.y) = n;
+        const float m = updated<FA>(2);  // (the colours swap cells from row to row)
+        (FA ? r[2].e.x : r[2].e.y) = m;
+        if (y - 1 >= y0 && y - 1 < y1) {  // uniform per warp
+            st2<VEC>(eout + (at - 5 * (i64)L.w), r[2].e, own, ownb);  // (fetched: rows up to y + 3)
+            if (RZ) {
+                if (own) {
+                    acc.add(r[2].e.x * r[2].f.x);
+                    zs.add(r[2].e.x);
+                }
+                if (ownb) {
+                    acc.add(r[2].e.y * r[2].f.y);
+                    zs.add(r[2].e.y);
+                }
+            }
+        }
+        if (REST && y - 2 >= y0) {
+            const float a = residual<true>(1), b = residual<false>(1);
+            if ((y & 1) == 0) rsum = a + b;
+            else {
+                rsum += a;
+                rsum += b;
+                const int Y = (y - 2) >> 1;
+                if (Y < L.ch && 2 * Y < y1 && own) v.fc[L.coff + (i64)Y * L.cw + (x >> 1)] = rsum;
+            }
+        }
+    }
+
+    __device__ __forceinline__ void run() {
+        int y = y0 - (REST ? 2 : 1);
+        const int last = y0 + ((y1 - y0 + 1) & ~1) + (REST ? 1 : 0);
+        constexpr bool FA = REST ? C1 == 0 : C1 == 1;
+        next = y - 1;
+        stop = min(L.h - 1, last + 1);
+        at = L.off + (i64)next * L.w + x;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            r[k].e = r[k].f = r[k].wx = r[k].wy = r[k].inv = make_float2(0.f, 0.f);
+            r[k].fl = r[k].raw.a = r[k].raw.b = 0;
+            r[k].wr = r[k].ec = 0.f;
+        }
+        push(fetch());
+        push(fetch());
+        BRow<L0> q0 = fetch(), q1 = fetch();  // two rows ahead
+        for (; y < last; y += 2) {
+            push(q0);
+            q0 = fetch();
+            step<FA>(y);
+            push(q1);
+            q1 = fetch();
+            step<!FA>(y + 1);
+        }
     }
 };
 
-// One red-black half-sweep of colour `color` at one level of every grid
-// that smooths there; with RZ (level 0, last) also the per-tile z.r and
-// sum(z).  A thread updates one cell of the colour in each of sm_rows(L0)
-// rows (kSmTY apart): loads of all rows first, then the updates, then
-// the stores.
-template <bool L0, int MODE, bool RZ>
-__global__ void __launch_bounds__(kSmTX * kSmTY, L0 ? 8 : 3)
-    k_bmg_smooth(BLv v, const Tile* __restrict__ tiles, int ntiles, int color, const BState* __restrict__ st,
-                 double* __restrict__ partials) {
-    __shared__ F2 sm[64];
-    FOR_TILES(tiles, ntiles) {
-        const Tile t = tiles[ti];
-        if (st[t.grid].done) continue;  // uniform per block
-        const BLevel L = v.info[t.grid];
-        const bool upd = L.coarse > v.level;
-        if (!upd && !RZ) continue;
-        const int iy = threadIdx.x / kSmTX, ix = threadIdx.x % kSmTX;
-        Acc<float> acc, zs;  // z.r and sum(z) (RZ)
-        constexpr int R = sm_rows(L0);
-        BUpd<L0, MODE> u[R];
-        float ev[R], eo[R], fo[R];  // the colour's new values; the other colour's e, f (RZ)
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int y = t.y0 + iy + r * kSmTY;
-            const int x = t.x0 + 2 * ix + ((y + color) & 1);
-            if (y < L.h && x < L.w) {
-                const i64 c = L.off + (i64)y * L.w + x;
-                if (upd) u[r].load(v, L, c, y, x);
-                else if (RZ) {
-                    u[r].f = v.f[c];
-                    ev[r] = v.e[c];
-                }
-            }
-            // the other colour is not written by this launch: read it now
-            const int xo = t.x0 + 2 * ix + ((y + color + 1) & 1);
-            if (RZ && y < L.h && xo < L.w) {
-                const i64 c = L.off + (i64)y * L.w + xo;
-                eo[r] = v.e[c];
-                fo[r] = v.f[c];
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int y = t.y0 + iy + r * kSmTY;
-            const int x = t.x0 + 2 * ix + ((y + color) & 1);
-            if (y < L.h && x < L.w) {
-                if (upd) {
-                    ev[r] = u[r].value();
-                    v.e[L.off + (i64)y * L.w + x] = ev[r];
-                }
-                if (RZ) {
-                    acc.add(ev[r] * u[r].f);
-                    zs.add(ev[r]);
-                }
-            }
-            const int xo = t.x0 + 2 * ix + ((y + color + 1) & 1);
-            if (RZ && y < L.h && xo < L.w) {
-                acc.add(eo[r] * fo[r]);
-                zs.add(eo[r]);
-            }
-        }
-        if (RZ) {
-            double a, b;
-            tsum2(f2_of(acc), f2_of(zs), sm, &a, &b);
-            if (threadIdx.x == 0) {
-                partials[2 * (i64)ti] = a;
-                partials[2 * (i64)ti + 1] = b;
-            }
-        }
-    }
-}
-
-// Residual of level l restricted (summed over children) to level l+1.
-template <bool L0>
-__global__ void __launch_bounds__(kRtX * kRtY)
-    k_bmg_restrict(BLv v, float* __restrict__ fc, const Tile* __restrict__ tiles, int ntiles,
-                   const BState* __restrict__ st) {
-    FOR_TILES(tiles, ntiles) {
-        const Tile t = tiles[ti];
-        if (st[t.grid].done) continue;
-        const BLevel L = v.info[t.grid];
-        const int Y = t.y0 + (int)threadIdx.x / kRtX, X = t.x0 + (int)threadIdx.x % kRtX;
-        if (Y >= L.ch || X >= L.cw) continue;
-        // the (up to) four children's loads first, then their residuals in
-        // row-major order
-        BUpd<L0, BNB_PLAIN> u[4];
-        float ec[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int y = 2 * Y + (k >> 1), x = 2 * X + (k & 1);
-            if (y < L.h && x < L.w) {
-                const i64 c = L.off + (i64)y * L.w + x;
-                u[k].load(v, L, c, y, x);
-                ec[k] = v.e[c];
-            }
-        }
-        float sum = 0.f;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int y = 2 * Y + (k >> 1), x = 2 * X + (k & 1);
-            if (y < L.h && x < L.w) {
-                float a = 0.f;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (u[k].w[j] != 0.f) a += u[k].w[j] * (ec[k] - u[k].n[j]);
-                sum += u[k].f - a;
-            }
-        }
-        fc[L.coff + (i64)Y * L.cw + X] = sum;
-    }
-}
-
-// Each grid's coarsest level: one block per grid, shared memory, symmetric
-// red-black sweeps from e = 0 (coarse_pairs of its shape).  A grid too small to
-// coarsen is solved this way on level 0 (weights from its flags).
-__global__ void __launch_bounds__(kBmgCoarseThreads)
-    k_bmg_coarse(const CoarseInfo* __restrict__ ci, const BState* __restrict__ st, float* __restrict__ z,
-                 const float* __restrict__ r, const uint8_t* __restrict__ flags, float dt) {
-    __shared__ float se[kBmgCoarseMax], sf[kBmgCoarseMax], sx[kBmgCoarseMax], sy[kBmgCoarseMax], si[kBmgCoarseMax];
-    const int g = blockIdx.x;
-    if (st[g].done) return;
-    const CoarseInfo C = ci[g];
-    const int n = C.h * C.w;
-    for (int c = threadIdx.x; c < n; c += blockDim.x) {
-        se[c] = 0.f;
-        if (C.level == 0) {
-            const uint8_t fl = flags[C.off + c];
-            sf[c] = r[C.off + c];
-            sx[c] = (fl & XLO) ? dt : 0.f;
-            sy[c] = (fl & YLO) ? dt : 0.f;
-            const int k = __popc((unsigned)fl);
-            si[c] = k ? __frcp_rn((float)k * dt) : 0.f;
+// A smoothing pair at one level of every grid that smooths there, from ein
+// to eout.  RZ (level 0, last): also z.r and sum(z) per strip, for grids
+// that don't smooth on level 0 as well (z, left by k_bmg_tail, is in eout).
+//
+// Bound by memory: a pair reads f, flags and e and writes e, 13 bytes per
+// cell on level 0, where two half-sweeps of a launch each read all of it and
+// wrote half, 8 launches and a restriction per V-cycle.  In a strip the rows
+// are read once (registers hold them while they are neighbours), x neighbours
+// come by shuffle; two lanes at an inner edge of a strip and two or three
+// rows at its ends are recomputed: the pair needs two cells beyond its own,
+// the residual three.  256 grids of 21 M cells, all running: 47 us the first
+// pair, 80 with the restriction (issue bound at 0.74 per cycle), 62 with the
+// prolongation, 67 with z.r (loads in flight: 28 warps of 70 registers), where
+// the eight half-sweeps took 75 to 141 each and the restriction 98.
+template <bool L0, int MODE, int C1, bool RZ, bool REST>
+__global__ void __launch_bounds__(kMarchThreads, L0 ? (RZ || REST ? 7 : 8) : 5)
+    k_bmg_pair(BLv v, const float* __restrict__ ein, float* __restrict__ eout, const Strip* __restrict__ strips, int n,
+               const BState* __restrict__ st, double* __restrict__ partials) {
+    const int i = blockIdx.x * (kMarchThreads / 32) + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const Strip S = strips[i];
+    if (st[S.grid].done) return;
+    const BLevel L = v.info[S.grid];
+    F2 a{0.f, 0.f}, b{0.f, 0.f};
+    if (L.tail > v.level) {
+        if (((L.off | (i64)L.w) & 1) == 0) {
+            March<L0, MODE, C1, RZ, REST, true> m(v, L, S, ein, eout);
+            m.run();
+            a = f2_of(m.acc);
+            b = f2_of(m.zs);
         } else {
-            sf[c] = C.f[c];
-            sx[c] = C.wx[c];
-            sy[c] = C.wy[c];
-            si[c] = C.invd[c];
+            March<L0, MODE, C1, RZ, REST, false> m(v, L, S, ein, eout);
+            m.run();
+            a = f2_of(m.acc);
+            b = f2_of(m.zs);
+        }
+    } else if (RZ) {
+        const int lo = S.x0 ? S.x0 + 4 : 0, hi = S.x0 + 64 >= L.w ? L.w : S.x0 + 60;
+        Acc<float> acc, zs;
+        for (int y = S.y0; y < S.y1; ++y)
+            for (int x = lo + (threadIdx.x & 31); x < hi; x += 32) {
+                const i64 c = L.off + (i64)y * L.w + x;
+                acc.add(eout[c] * v.f[c]);
+                zs.add(eout[c]);
+            }
+        a = f2_of(acc);
+        b = f2_of(zs);
+    }
+    if (RZ) {
+        a = f2_warp(a);
+        b = f2_warp(b);
+        if ((threadIdx.x & 31) == 0) {
+            partials[2 * (i64)i] = (double)a.hi + (double)a.lo;
+            partials[2 * (i64)i + 1] = (double)b.hi + (double)b.lo;
+        }
+    }
+}
+
+// Device view of the levels of k_bmg_tail.
+struct BTail {
+    const BLevel* info[kBmgMaxLevels];
+    const float* wx[kBmgMaxLevels];
+    const float* wy[kBmgMaxLevels];
+    const float* invd[kBmgMaxLevels];
+    const float* f[kBmgMaxLevels];
+    float* e[kBmgMaxLevels];
+    const uint8_t* flags;
+    float dt;
+    int nsmooth;
+};
+
+// One level in shared memory: n cells each of e, f, wx, wy, 1 / diagonal.
+struct TailLevel {
+    float* e;
+    int h, w, n;
+    unsigned magic;  // i / w = umulhi(i, magic) (w >= 2)
+    __device__ __forceinline__ TailLevel(float* at, int h_, int w_) : e(at), h(h_), w(w_), n(h_ * w_) {
+        magic = 0xffffffffu / (unsigned)w + 1u;
+    }
+    __device__ __forceinline__ float* f() const { return e + n; }
+    __device__ __forceinline__ float* wx() const { return e + 2 * n; }
+    __device__ __forceinline__ float* wy() const { return e + 3 * n; }
+    __device__ __forceinline__ float* inv() const { return e + 4 * n; }
+    // Cell i of a colour, in row-major order: of the pair 2i, 2i + 1 one cell
+    // has the colour (rows of odd length: always the same one).  It may be n.
+    __device__ __forceinline__ int cell(int i, int color) const {
+        return 2 * i + ((w & 1) ? color : (((int)__umulhi(2u * (unsigned)i, magic) + color) & 1));
+    }
+};
+
+// One half-sweep; C: the next level, whose correction the neighbours get
+// (PROLONG).  A neighbour behind a closed face is not added, outside the grid
+// the cell itself is read.
+template <bool PROLONG>
+__device__ __forceinline__ void tail_sweep(const TailLevel& T, const TailLevel& C, int color, int t, int nt) {
+    const int items = (T.n + 1) >> 1;
+#pragma unroll 2
+    for (int i = t; i < items; i += nt) {
+        const int c = T.cell(i, color);
+        if (c >= T.n) continue;
+        const int y = (int)__umulhi((unsigned)c, T.magic), x = c - y * T.w;
+        const bool xl = x > 0, xh = x + 1 < T.w, yl = y > 0, yh = y + 1 < T.h;
+        const int l = xl ? c - 1 : c, r = xh ? c + 1 : c, u = yl ? c - T.w : c, d = yh ? c + T.w : c;
+        const float wl = T.wx()[c], wr = xh ? T.wx()[r] : 0.f, wu = T.wy()[c], wd = yh ? T.wy()[d] : 0.f;
+        float nl = T.e[l], nr = T.e[r], nu = T.e[u], nd = T.e[d];
+        if (PROLONG) {
+            const float* row = C.e + (y >> 1) * C.w;
+            nl += row[(xl ? x - 1 : x) >> 1];
+            nr += row[(xh ? x + 1 : x) >> 1];
+            nu += C.e[((yl ? y - 1 : y) >> 1) * C.w + (x >> 1)];
+            nd += C.e[((yh ? y + 1 : y) >> 1) * C.w + (x >> 1)];
+        }
+        T.e[c] = nb_sum(T.f()[c], wl, wr, wu, wd, nl, nr, nu, nd) * T.inv()[c];
+    }
+}
+
+// The rest of a grid's V-cycle, one block per grid: from level L.tail (its
+// right-hand side restricted there by k_bmg_pair, or r itself) down to the
+// coarsest level, solved by symmetric sweeps from e = 0, and up again; the
+// correction of level L.tail (or z) is written out.
+//
+// Bound by latency: a half-sweep of 64 x 64 cells is four cells per thread,
+// and each launch that it was cost 6 to 8 us.  A coarsest level of up to 64
+// cells is one warp's work, a cell of each colour per lane, neighbours by
+// shuffle (512 threads took 38 us for the 128 half-sweeps, nearly all of it
+// at barriers).  37 us for 256 grids at once, 15 for a few, where the launches
+// of these levels took 250.
+__global__ void __launch_bounds__(kBmgTailThreads, 2) k_bmg_tail(BTail v, const BState* __restrict__ st) {
+    extern __shared__ float smem[];
+    const int g = blockIdx.x, tid = threadIdx.x, nt = kBmgTailThreads;
+    if (st[g].done) return;
+    const int lt = v.info[0][g].tail, lc = v.info[0][g].coarse;
+    {
+        float* at = smem;
+        for (int l = lt; l <= lc; ++l) {
+            const BLevel L = v.info[l][g];
+            const TailLevel T(at, L.h, L.w);
+#pragma unroll 4
+            for (int c = tid; c < T.n; c += nt) {
+                float inv, wx, wy;
+                if (l == 0) {
+                    const unsigned fl = v.flags[L.off + c];
+                    wx = (fl & XLO) ? v.dt : 0.f;
+                    wy = (fl & YLO) ? v.dt : 0.f;
+                    const int k = __popc(fl);
+                    inv = k ? __frcp_rn((float)k * v.dt) : 0.f;
+                } else {
+                    wx = v.wx[l][L.off + c];
+                    wy = v.wy[l][L.off + c];
+                    inv = v.invd[l][L.off + c];
+                }
+                const float f = l == lt ? v.f[l][L.off + c] : 0.f;
+                T.wx()[c] = wx;
+                T.wy()[c] = wy;
+                T.inv()[c] = inv;
+                if (l == lt) {
+                    T.f()[c] = f;
+                    T.e[c] = inv != 0.f ? f * inv : 0.f;  // the first half-sweep (the other colour is not read)
+                }
+            }
+            at += 5 * T.n;
         }
     }
     __syncthreads();
-    const int pairs = coarse_pairs(1, C.h, C.w);
-    for (int it = 0; it < 4 * pairs; ++it) {
-        const int color = it < 2 * pairs ? (it & 1) : ((it & 1) ^ 1);
-        for (int c = threadIdx.x; c < n; c += blockDim.x) {
-            const int y = c / C.w, x = c - y * C.w;
-            if (((x + y) & 1) != color) continue;
-            float s = sf[c];
-            if (x > 0) s += sx[c] * se[c - 1];
-            if (x + 1 < C.w) s += sx[c + 1] * se[c + 1];
-            if (y > 0) s += sy[c] * se[c - C.w];
-            if (y + 1 < C.h) s += sy[c + C.w] * se[c + C.w];
-            se[c] = s * si[c];
+    float* at = smem;
+    for (int l = lt; l < lc; ++l) {
+        const BLevel L = v.info[l][g];
+        const TailLevel T(at, L.h, L.w), C(at + 5 * T.n, L.ch, L.cw);
+        tail_sweep<false>(T, T, 1, tid, nt);
+        __syncthreads();
+        for (int k = 1; k < v.nsmooth; ++k) {
+            tail_sweep<false>(T, T, 0, tid, nt);
+            __syncthreads();
+            tail_sweep<false>(T, T, 1, tid, nt);
+            __syncthreads();
         }
+        for (int c = tid; c < C.n; c += nt) {
+            const int Y = (int)__umulhi((unsigned)c, C.magic), X = c - Y * C.w;
+            float sum = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int y = 2 * Y + (k >> 1), x = 2 * X + (k & 1);
+                if (y >= T.h || x >= T.w) continue;
+                const int i = y * T.w + x;
+                const bool xh = x + 1 < T.w, yh = y + 1 < T.h;
+                const float wl = T.wx()[i], wr = xh ? T.wx()[i + 1] : 0.f, wu = T.wy()[i],
+                            wd = yh ? T.wy()[i + T.w] : 0.f;
+                const float e = T.e[i];
+                sum += T.f()[i] - nb_sum(0.f, wl, wr, wu, wd, e - T.e[x > 0 ? i - 1 : i], e - T.e[xh ? i + 1 : i],
+                                         e - T.e[y > 0 ? i - T.w : i], e - T.e[yh ? i + T.w : i]);
+            }
+            C.f()[c] = sum;
+            const float inv = C.inv()[c];
+            C.e[c] = l + 1 < lc && inv != 0.f ? sum * inv : 0.f;
+        }
+        at += 5 * T.n;
         __syncthreads();
     }
-    for (int c = threadIdx.x; c < n; c += blockDim.x) {
-        if (C.level == 0)
-            z[C.off + c] = se[c];
-        else
-            C.e[c] = se[c];
+    {
+        const BLevel L = v.info[lc][g];
+        const TailLevel T(at, L.h, L.w);
+        if (lt == lc) {
+            for (int c = tid; c < T.n; c += nt) T.e[c] = 0.f;
+            __syncthreads();
+        }
+        const int pairs = coarse_pairs(1, L.h, L.w);
+        if (T.n <= 64) {
+            if (tid < 32) {
+                // per colour: the lane's cell, its weights (0 at closed faces and
+                // past the grid) and the lanes that hold its neighbours
+                float f[2], inv[2], w[2][4], e[2] = {0.f, 0.f};
+                int nb[2][4];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int c = T.cell(tid, q);
+                    const bool in = c < T.n;
+                    const int y = (int)__umulhi((unsigned)c, T.magic), x = c - y * T.w;
+                    f[q] = in ? T.f()[c] : 0.f;
+                    inv[q] = in ? T.inv()[c] : 0.f;
+                    const bool face[4] = {in && x > 0, in && x + 1 < T.w, in && y > 0, in && y + 1 < T.h};
+                    const int to[4] = {c - 1, c + 1, c - T.w, c + T.w};
+                    const float* from[4] = {T.wx() + c, T.wx() + to[1], T.wy() + c, T.wy() + to[3]};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        nb[q][j] = face[j] ? to[j] >> 1 : tid;
+                        w[q][j] = face[j] ? *from[j] : 0.f;
+                    }
+                }
+                auto sweep = [&](auto colour) {
+                    constexpr int q = decltype(colour)::value;
+                    float n[4], s = f[q];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) n[j] = __shfl_sync(0xffffffffu, e[1 - q], nb[q][j]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s = fmaf(w[q][j], n[j], s);
+                    e[q] = s * inv[q];
+                };
+                using Zero = std::integral_constant<int, 0>;
+                using One = std::integral_constant<int, 1>;
+                for (int p = 0; p < pairs; ++p) {
+                    sweep(Zero{});
+                    sweep(One{});
+                }
+                for (int p = 0; p < pairs; ++p) {
+                    sweep(One{});
+                    sweep(Zero{});
+                }
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int c = T.cell(tid, q);
+                    if (c < T.n) T.e[c] = e[q];
+                }
+            }
+            __syncthreads();
+        } else {
+            for (int it = 0; it < 4 * pairs; ++it) {
+                tail_sweep<false>(T, T, it < 2 * pairs ? (it & 1) : ((it & 1) ^ 1), tid, nt);
+                __syncthreads();
+            }
+        }
+    }
+    for (int l = lc - 1; l >= lt; --l) {
+        const BLevel L = v.info[l][g];
+        const TailLevel C(at, L.ch, L.cw);
+        at -= 5 * L.h * L.w;
+        const TailLevel T(at, L.h, L.w);
+        tail_sweep<true>(T, C, 1, tid, nt);
+        __syncthreads();
+        for (int k = 0; k < v.nsmooth; ++k) {
+            if (k > 0) {
+                tail_sweep<false>(T, T, 1, tid, nt);
+                __syncthreads();
+            }
+            tail_sweep<false>(T, T, 0, tid, nt);
+            __syncthreads();
+        }
+    }
+    const BLevel L = v.info[lt][g];
+    for (int c = tid; c < L.h * L.w; c += nt) v.e[lt][L.off + c] = smem[c];
+}
+
+// p = z + beta p (z - zmean on fluid cells; ping-pong by the grid's iteration
+// count), A p and p.Ap over strips of 64 columns, 17 bytes per cell.  The
+// cells beside a strip are read by its edge lanes, the rows above and below
+// once more by the strips there.  72 us for 21 M cells (54 at the copy rate)
+// where a block per tile of 256 cells, its state and tile loaded and its sum
+// folded for each, took 211.
+template <bool VEC>
+__device__ __forceinline__ F2 bmg_spmv_strip(const BLevel& L, const Strip& S, const BState& st, const float* z, float* p0,
+                                             float* p1, float* ap, const uint8_t* flags, float dt) {
+    const int lane = threadIdx.x & 31, x = S.x0 + 2 * lane;
+    const bool va = x < L.w, vb = x + 1 < L.w;
+    const bool first = st.first != 0;
+    const float beta = st.fbeta, zm = st.fzm;
+    const float* __restrict__ p_old = (st.iter & 1) ? p1 : p0;
+    float* __restrict__ p_new = (st.iter & 1) ? p0 : p1;
+    // the cell beside the strip: left of lane 0, right of lane 31
+    const int dx = lane == 0 ? -1 : 2;
+    const bool edge = (lane == 0 && S.x0 > 0) || (lane == 31 && S.x0 + 64 < L.w);
+    struct Row {
+        float2 z, p;
+        Flag2 fl;
+        float ez, ep;
+    };
+    i64 at = L.off + (i64)(S.y0 - 1) * L.w + x;
+    int next = S.y0 - 1;
+    auto fetch = [&]() {
+        Row q;
+        q.z = q.p = make_float2(0.f, 0.f);
+        q.fl.a = q.fl.b = 0;
+        q.ez = q.ep = 0.f;
+        if (next >= 0 && next < L.h && next <= S.y1) {
+            q.z = ld2<VEC>(z + at, va, vb);
+            q.fl.template load<VEC>(flags + at, va, vb);
+            if (edge) q.ez = z[at + dx];
+            if (!first) {
+                q.p = ld2<VEC>(p_old + at, va, vb);
+                if (edge) q.ep = p_old[at + dx];
+            }
+        }
+        ++next;
+        at += L.w;
+        return q;
+    };
+    // p_new; the projected z applies to cells with an open face (a neighbour
+    // behind an open face always has one)
+    auto pn = [&](float zv, float pv, bool fluid) {
+        const float zz = fluid ? zv - zm : zv;
+        return first ? zz : fmaf(beta, pv, zz);
+    };
+    auto of = [&](const Row& q) {
+        const unsigned f = q.fl.template both<VEC>();
+        return make_float2(pn(q.z.x, q.p.x, (f & 0xffu) != 0), pn(q.z.y, q.p.y, (f >> 8) != 0));
+    };
+    Row q0 = fetch(), q1 = fetch(), q2 = fetch();
+    float2 up = of(q0), cur = of(q1);
+    unsigned fl = q1.fl.template both<VEC>();
+    float ext = pn(q1.ez, q1.ep, true);
+    q0 = q2;
+    q1 = fetch();
+    Acc<float> acc;
+    i64 out = L.off + (i64)S.y0 * L.w + x;
+#pragma unroll 2
+    for (int y = S.y0; y < S.y1; ++y, out += L.w) {
+        const Row q = q0;  // row y + 1
+        q0 = q1;
+        q1 = fetch();
+        const float2 dn = of(q);
+        float l = __shfl_up_sync(0xffffffffu, cur.y, 1), r = __shfl_down_sync(0xffffffffu, cur.x, 1);
+        l = lane == 0 ? ext : l;
+        r = lane == 31 ? ext : r;
+        auto apply = [&](unsigned f, float pc, float pl, float pr, float pu, float pd) {
+            const float gy_lo = (f & YLO) ? -sub_rn(pc, pu) : 0.f;
+            const float gy_hi = (f & YHI) ? -sub_rn(pd, pc) : 0.f;
+            const float gx_lo = (f & XLO) ? sub_rn(pl, pc) : 0.f;
+            const float gx_hi = (f & XHI) ? sub_rn(pc, pr) : 0.f;
+            return mul_rn(add_rn(sub_rn(sub_rn(gy_hi, gy_lo), gx_lo), gx_hi), dt);
+        };
+        const float2 a = make_float2(apply(fl, cur.x, l, cur.y, up.x, dn.x), apply(fl >> 8, cur.y, cur.x, r, up.y, dn.y));
+        st2<VEC>(p_new + out, cur, va, vb);
+        st2<VEC>(ap + out, a, va, vb);
+        if (va) acc.add(cur.x * a.x);
+        if (vb) acc.add(cur.y * a.y);
+        up = cur;
+        cur = dn;
+        fl = q.fl.template both<VEC>();
+        ext = pn(q.ez, q.ep, true);
+    }
+    return f2_of(acc);
+}
+
+__global__ void __launch_bounds__(kMarchThreads, 7)
+    k_bmg_spmv(const BLevel* __restrict__ info, const Strip* __restrict__ strips, int n, const BState* __restrict__ st,
+               const float* __restrict__ z, float* p0, float* p1, float* __restrict__ ap,
+               const uint8_t* __restrict__ flags, float dt, double* __restrict__ partials) {
+    const int i = blockIdx.x * (kMarchThreads / 32) + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const Strip S = strips[i];
+    const BState& B = st[S.grid];
+    if (B.done) return;
+    const BLevel L = info[S.grid];
+    F2 a = ((L.off | (i64)L.w) & 1) == 0 ? bmg_spmv_strip<true>(L, S, B, z, p0, p1, ap, flags, dt)
+                                         : bmg_spmv_strip<false>(L, S, B, z, p0, p1, ap, flags, dt);
+    a = f2_warp(a);
+    if ((threadIdx.x & 31) == 0) {
+        partials[2 * (i64)i] = (double)a.hi + (double)a.lo;
+        partials[2 * (i64)i + 1] = 0.0;
+    }
+}
+
+// x += alpha p, r -= alpha Ap, max|r| and sum(r), one warp per chunk of a
+// grid's cells, four at a time where the fields' 16-byte groups allow it; 24
+// bytes per cell.  71 us for 21 M cells (76 at the copy rate, part of it in
+// L2), 181 with a block per tile.
+__global__ void __launch_bounds__(256)
+    k_bmg_update(const Chunk* __restrict__ chunks, int n, const BState* __restrict__ st, float* __restrict__ x,
+                 float* __restrict__ r, const float* p0, const float* p1, const float* __restrict__ ap, int vec,
+                 double* __restrict__ partials) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const Chunk C = chunks[i];
+    const BState& S = st[C.grid];
+    if (S.done) return;
+    const float* __restrict__ p = ((S.iter + 1) & 1) ? p1 : p0;
+    const float al = S.falpha, nal = -al;
+    float rm = 0.f;
+    Acc<float> sum;
+    auto one = [&](float& xv, float& rv, float pv, float av) {
+        xv = fmaf(al, pv, xv);
+        rv = fmaf(nal, av, rv);
+        rm = fmaxf(rm, isfinite(rv) ? fabsf(rv) : __int_as_float(0x7f800000));
+        sum.add(rv);  // for the lazy projection
+    };
+    auto single = [&](i64 c) {
+        float xv = x[c], rv = r[c];
+        one(xv, rv, p[c], ap[c]);
+        x[c] = xv;
+        r[c] = rv;
+    };
+    // the whole groups of four between c0 and c1, the cells around them one by one
+    const i64 g0 = vec ? (C.c0 + 3) / 4 * 4 : C.c1, g1 = vec ? C.c1 / 4 * 4 : C.c1;
+    if (g0 < g1) {
+        for (i64 c = g0 + 4 * lane; c < g1; c += 128) {
+            float4 xv = *reinterpret_cast<const float4*>(x + c), rv = *reinterpret_cast<const float4*>(r + c);
+            const float4 pv = *reinterpret_cast<const float4*>(p + c), av = *reinterpret_cast<const float4*>(ap + c);
+            one(xv.x, rv.x, pv.x, av.x);
+            one(xv.y, rv.y, pv.y, av.y);
+            one(xv.z, rv.z, pv.z, av.z);
+            one(xv.w, rv.w, pv.w, av.w);
+            *reinterpret_cast<float4*>(x + c) = xv;
+            *reinterpret_cast<float4*>(r + c) = rv;
+        }
+        if (C.c0 + lane < g0) single(C.c0 + lane);
+        if (g1 + lane < C.c1) single(g1 + lane);
+    } else {
+        for (i64 c = C.c0 + lane; c < C.c1; c += 32) single(c);
+    }
+    for (int o = 16; o > 0; o >>= 1) rm = fmaxf(rm, __shfl_xor_sync(0xffffffffu, rm, o));
+    const F2 t = f2_warp(f2_of(sum));
+    if (lane == 0) {
+        partials[2 * (i64)i] = (double)rm;
+        partials[2 * (i64)i + 1] = (double)t.hi + (double)t.lo;
     }
 }
 
@@ -372,7 +808,7 @@ __global__ void k_bmg_invd(BLv v, float* __restrict__ invd, const Tile* __restri
     }
 }
 
-// Per grid: z.r = sum of its level-0 tile partials (fixed order).
+// Per grid: z.r = sum of its level-0 strips' partials (fixed order).
 // first: sigma = z.r; else beta = z.r / sigma, sigma = z.r.
 __global__ void k_bmg_rz_finalize(const BLevel* __restrict__ info0, BState* __restrict__ st,
                                   const double* __restrict__ partials, int n, int first) {
@@ -435,10 +871,10 @@ static BLv view(const pg_batch* B, int l) {
     v.wx = M.wx[l];
     v.wy = M.wy[l];
     v.invd = M.invd[l];
-    v.e = l == 0 ? B->z : M.e[l];
     v.f = l == 0 ? B->r : M.f[l];
     v.flags = B->flags;
     v.ec = l + 1 < M.nlev ? M.e[l + 1] : nullptr;
+    v.fc = l + 1 < M.nlev ? M.f[l + 1] : nullptr;
     v.dt = M.dt;
     v.level = l;
     return v;
@@ -499,7 +935,7 @@ static int bmg_build(pg_batch* B, float dt) {
             L.h = hs[g][l];
             L.w = wsz[g][l];
             L.off = l == 0 ? B->coff[g] : lvcells[l];
-            if (l > 0) lvcells[l] += (i64)L.h * L.w;
+            if (l > 0) lvcells[l] += ((i64)L.h * L.w + 1) & ~(i64)1;  // (even: rows of pairs stay aligned)
         }
     lvcells[0] = B->ncells;
     for (int l = 0; l < nlev; ++l)
@@ -509,6 +945,38 @@ static int bmg_build(pg_batch* B, float dt) {
                 info[l][g].cw = wsz[g][l + 1];
                 info[l][g].coff = info[l + 1][g].off;
             }
+    for (int g = 0; g < n; ++g) {
+        int t = coarse[g];
+        i64 cells = (i64)hs[g][t] * wsz[g][t];
+        while (t > 0 && cells + (i64)hs[g][t - 1] * wsz[g][t - 1] <= kBmgTailCells) {
+            --t;
+            cells += (i64)hs[g][t] * wsz[g][t];
+        }
+        M->tail_cells = std::max(M->tail_cells, (int)cells);
+        for (int l = 0; l < nlev; ++l) info[l][g].tail = t;
+    }
+    // strips of a level: `step` columns apart, chunks of up to `rows` rows (an
+    // even number; fewer where the strips would not fill the chip)
+    auto make_strips = [&](int l, bool all, int step, std::vector<Strip>& st) {
+        for (int rows = 32; rows >= 8; rows /= 2) {
+            st.clear();
+            for (int g = 0; g < n; ++g) {
+                BLevel& L = info[l][g];
+                const int t0 = (int)st.size();
+                if (all || l < L.tail) {
+                    const int per = (L.h + rows - 1) / rows, rc = ((L.h + per - 1) / per + 1) & ~1;
+                    for (int y0 = 0; y0 < L.h; y0 += rc)
+                        for (int x0 = 0;; x0 += step) {
+                            st.push_back(Strip{g, y0, std::min(y0 + rc, L.h), x0});
+                            if (x0 + 64 >= L.w) break;
+                        }
+                }
+                L.t0 = t0;
+                L.t1 = (int)st.size();
+            }
+            if ((i64)st.size() >= (i64)B->num_sms * 24) break;
+        }
+    };
     auto dalloc = [&](void** p, size_t bytes) -> int {
         cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(batch mg)");
@@ -516,63 +984,73 @@ static int bmg_build(pg_batch* B, float dt) {
         return PG_OK;
     };
     int rc;
-    for (int l = 0; l < nlev; ++l) {
-        std::vector<Tile> st, rt;
+    auto upload = [&](void** p, const void* src, size_t bytes) -> int {
+        const int e = dalloc(p, bytes);
+        if (e) return e;
+        if (bytes) PG_CUDA(cudaMemcpy(*p, src, bytes, cudaMemcpyHostToDevice));
+        return PG_OK;
+    };
+    {  // the CG kernels' work lists
+        std::vector<Strip> st;
+        std::vector<Chunk> ch;
+        std::vector<int2> sr(n), cr(n);
+        make_strips(0, true, 64, st);
         for (int g = 0; g < n; ++g) {
-            BLevel& L = info[l][g];
-            if (l == 0) L.t0 = (int)st.size();
-            if (l == 0 || l < coarse[g]) {
-                for (int y0 = 0; y0 < L.h; y0 += kSmTY * sm_rows(l == 0))
-                    for (int x0 = 0; x0 < L.w; x0 += 2 * kSmTX) st.push_back(Tile{g, y0, x0});
-                if (l < coarse[g]) M->nsmoothing[l] += 1;
-            }
-            if (l == 0) L.t1 = (int)st.size();
+            sr[g] = make_int2(info[0][g].t0, info[0][g].t1);
+            cr[g].x = (int)ch.size();
+            for (i64 c = B->coff[g]; c < B->coff[g + 1]; c += kUpdateCells)
+                ch.push_back(Chunk{g, 0, c, std::min(c + kUpdateCells, B->coff[g + 1])});
+            cr[g].y = (int)ch.size();
+        }
+        M->ncg = (int)st.size();
+        M->nchunk = (int)ch.size();
+        if ((rc = upload((void**)&M->cg_strips, st.data(), sizeof(Strip) * st.size())) ||
+            (rc = upload((void**)&M->cg_range, sr.data(), sizeof(int2) * n)) ||
+            (rc = upload((void**)&M->chunks, ch.data(), sizeof(Chunk) * ch.size())) ||
+            (rc = upload((void**)&M->chunk_range, cr.data(), sizeof(int2) * n)))
+            return rc;
+    }
+    for (int l = 0; l < nlev; ++l) {
+        std::vector<Strip> st;
+        std::vector<Tile> rt;
+        make_strips(l, l == 0, 56, st);  // (every grid on level 0: z.r)
+        for (int g = 0; g < n; ++g) {
+            const BLevel& L = info[l][g];
+            M->nsmoothing[l] += l < L.tail;
             if (l < coarse[g])
                 for (int y0 = 0; y0 < L.ch; y0 += kRtY)
                     for (int x0 = 0; x0 < L.cw; x0 += kRtX) rt.push_back(Tile{g, y0, x0});
         }
         M->nst[l] = (int)st.size();
         M->nrt[l] = (int)rt.size();
-        if ((rc = dalloc((void**)&M->info[l], sizeof(BLevel) * n)) ||
-            (rc = dalloc((void**)&M->stiles[l], sizeof(Tile) * st.size())) ||
-            (rc = dalloc((void**)&M->rtiles[l], sizeof(Tile) * rt.size())))
+        if ((rc = upload((void**)&M->info[l], info[l].data(), sizeof(BLevel) * n)) ||
+            (rc = upload((void**)&M->strips[l], st.data(), sizeof(Strip) * st.size())) ||
+            (rc = upload((void**)&M->rtiles[l], rt.data(), sizeof(Tile) * rt.size())))
             return rc;
-        PG_CUDA(cudaMemcpy(M->info[l], info[l].data(), sizeof(BLevel) * n, cudaMemcpyHostToDevice));
-        if (!st.empty()) PG_CUDA(cudaMemcpy(M->stiles[l], st.data(), sizeof(Tile) * st.size(), cudaMemcpyHostToDevice));
-        if (!rt.empty()) PG_CUDA(cudaMemcpy(M->rtiles[l], rt.data(), sizeof(Tile) * rt.size(), cudaMemcpyHostToDevice));
         if (l >= 1) {
             const size_t b = sizeof(float) * (size_t)lvcells[l];
             if ((rc = dalloc((void**)&M->wx[l], b)) || (rc = dalloc((void**)&M->wy[l], b)) ||
                 (rc = dalloc((void**)&M->invd[l], b)) || (rc = dalloc((void**)&M->e[l], b)) ||
                 (rc = dalloc((void**)&M->f[l], b)))
                 return rc;
+            if (M->nsmoothing[l] && (rc = dalloc((void**)&M->e2[l], b))) return rc;
         }
-        if (l == 0 && (rc = dalloc((void**)&M->partials, 2 * sizeof(double) * st.size()))) return rc;
     }
-    std::vector<CoarseInfo> ci(n);
-    for (int g = 0; g < n; ++g) {
-        const int c = coarse[g];
-        const BLevel& L = info[c][g];
-        ci[g] = CoarseInfo{M->wx[c] ? M->wx[c] + L.off : nullptr,
-                           M->wy[c] ? M->wy[c] + L.off : nullptr,
-                           M->invd[c] ? M->invd[c] + L.off : nullptr,
-                           M->e[c] ? M->e[c] + L.off : nullptr,
-                           M->f[c] ? M->f[c] + L.off : nullptr,
-                           L.h, L.w, c, L.off};
-        if (c == 0) ci[g].off = B->coff[g];
-    }
+    if ((rc = dalloc((void**)&M->partials, 2 * sizeof(double) * std::max({M->nst[0], M->ncg, M->nchunk})))) return rc;
+    PG_CUDA(cudaFuncSetAttribute(k_bmg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(5 * sizeof(float)) * kBmgTailCells));
     // fluid components of every grid with more than one (host labelling, once per mask)
     {
         std::vector<uint8_t> hf((size_t)B->ncells);
         PG_CUDA(cudaMemcpy(hf.data(), B->flags, hf.size(), cudaMemcpyDeviceToHost));
         std::vector<i64> cells;
-        std::vector<int> start;
-        for (int g = 0; g < n; ++g)
+        std::vector<int> start, owner;
+        for (int g = 0; g < n; ++g) {
             find_pockets(hf.data() + B->coff[g], 2, 1, B->h[g], B->w[g], B->coff[g], cells, start);
-        if ((rc = upload_pockets(cells, start, &M->pockets))) return rc;
+            owner.resize(start.empty() ? 0 : start.size() - 1, g);
+        }
+        if ((rc = upload_pockets(cells, start, &M->pockets, owner))) return rc;
     }
-    if ((rc = dalloc((void**)&M->coarse, sizeof(CoarseInfo) * n))) return rc;
-    PG_CUDA(cudaMemcpy(M->coarse, ci.data(), sizeof(CoarseInfo) * n, cudaMemcpyHostToDevice));
     // coarse operators
     cudaStream_t s = B->stream;
     for (int l = 0; l + 1 < nlev; ++l) {
@@ -590,27 +1068,43 @@ static int bmg_build(pg_batch* B, float dt) {
     return PG_OK;
 }
 
-template <bool L0, int MODE, bool RZ>
-static void bsmooth(pg_batch* B, cudaStream_t s, int l, int color) {
+static int march_blocks(int n) { return (n + kMarchThreads / 32 - 1) / (kMarchThreads / 32); }
+
+template <bool L0, int MODE, int C1, bool RZ, bool REST>
+static void bpair(pg_batch* B, cudaStream_t s, int l, const float* ein, float* eout) {
     BatchMg& M = *B->mg;
     const BLv v = view(B, l);
     PG_LAUNCH(l == 0 ? KK_MG_SMOOTH : KK_MG_SMOOTH_C, s,
-              k_bmg_smooth<L0, MODE, RZ><<<bmg_blocks(B, M.nst[l]), kSmTX * kSmTY, 0, s>>>(v, M.stiles[l], M.nst[l],
-                                                                                           color, B->state, M.partials));
+              k_bmg_pair<L0, MODE, C1, RZ, REST><<<march_blocks(M.nst[l]), kMarchThreads, 0, s>>>(
+                  v, ein, eout, M.strips[l], M.nst[l], B->state, M.partials));
 }
 
-static void bsmooth_any(pg_batch* B, cudaStream_t s, int l, int color, int mode, bool rz = false) {
-    if (l == 0) {
-        if (mode == BNB_FIRST) bsmooth<true, BNB_FIRST, false>(B, s, l, color);
-        else if (mode == BNB_SELF) bsmooth<true, BNB_SELF, false>(B, s, l, color);
-        else if (mode == BNB_PROLONG) bsmooth<true, BNB_PROLONG, false>(B, s, l, color);
-        else if (rz) bsmooth<true, BNB_PLAIN, true>(B, s, l, color);
-        else bsmooth<true, BNB_PLAIN, false>(B, s, l, color);
-    } else {
-        if (mode == BNB_FIRST) bsmooth<false, BNB_FIRST, false>(B, s, l, color);
-        else if (mode == BNB_SELF) bsmooth<false, BNB_SELF, false>(B, s, l, color);
-        else if (mode == BNB_PROLONG) bsmooth<false, BNB_PROLONG, false>(B, s, l, color);
-        else bsmooth<false, BNB_PLAIN, false>(B, s, l, color);
+// The pairs before (and the restriction) or after the coarser levels; they
+// write e and its twin in turn, so that the last one leaves it in e.
+template <bool L0> static void bmg_down(pg_batch* B, cudaStream_t s, int l, int nsmooth) {
+    float *to = L0 ? B->ap : B->mg->e2[l], *other = L0 ? B->z : B->mg->e[l];  // (A p is dead here)
+    if (nsmooth == 1) {
+        bpair<L0, BP_SELF, 0, false, true>(B, s, l, nullptr, to);
+        return;
+    }
+    bpair<L0, BP_SELF, 0, false, false>(B, s, l, nullptr, to);
+    for (int k = 1; k < nsmooth; ++k, std::swap(to, other)) {
+        if (k == nsmooth - 1) bpair<L0, BP_PLAIN, 0, false, true>(B, s, l, to, other);
+        else bpair<L0, BP_PLAIN, 0, false, false>(B, s, l, to, other);
+    }
+}
+
+template <bool L0> static void bmg_up(pg_batch* B, cudaStream_t s, int l, int nsmooth) {
+    float *to = L0 ? B->ap : B->mg->e2[l], *other = L0 ? B->z : B->mg->e[l];
+    if (nsmooth & 1) std::swap(to, other);  // (where bmg_down ended: `other`)
+    if (nsmooth == 1) {
+        bpair<L0, BP_PROLONG, 1, L0, false>(B, s, l, other, to);
+        return;
+    }
+    bpair<L0, BP_PROLONG, 1, false, false>(B, s, l, other, to);
+    for (int k = 1; k < nsmooth; ++k, std::swap(to, other)) {
+        if (k == nsmooth - 1) bpair<L0, BP_PLAIN, 1, L0, false>(B, s, l, to, other);
+        else bpair<L0, BP_PLAIN, 1, false, false>(B, s, l, to, other);
     }
 }
 
@@ -618,40 +1112,54 @@ static void bsmooth_any(pg_batch* B, cudaStream_t s, int l, int color, int mode,
 // with more than one (r in place).
 void bmg_vcycle(pg_batch* B, cudaStream_t s, int nsmooth) {
     BatchMg& M = *B->mg;
-    pocket_project(s, B->r, M.pockets);
-    for (int l = 0; l + 1 < M.nlev; ++l) {
-        if (!M.nsmoothing[l]) continue;
-        bsmooth_any(B, s, l, 1, BNB_FIRST);
-        if (nsmooth == 1) bsmooth_any(B, s, l, 0, BNB_SELF);
-        for (int k = 1; k < nsmooth; ++k) {
-            bsmooth_any(B, s, l, 0, BNB_PLAIN);
-            bsmooth_any(B, s, l, 1, BNB_PLAIN);
-        }
-        const BLv v = view(B, l);
-        const int nb = bmg_blocks(B, M.nrt[l]);
-        if (l == 0)
-            PG_LAUNCH(KK_MG_RESTRICT, s, k_bmg_restrict<true><<<nb, kRtX * kRtY, 0, s>>>(v, M.f[1], M.rtiles[0], M.nrt[0], B->state));
-        else
-            PG_LAUNCH(KK_MG_RESTRICT_C, s, k_bmg_restrict<false><<<nb, kRtX * kRtY, 0, s>>>(v, M.f[l + 1], M.rtiles[l], M.nrt[l], B->state));
+    pocket_project(s, B->r, M.pockets, &B->state[0].done, sizeof(BState));
+    int deepest = 0;  // levels [0, deepest) have grids that smooth there
+    while (deepest < M.nlev && M.nsmoothing[deepest]) ++deepest;
+    for (int l = 0; l < deepest; ++l) {
+        if (l == 0) bmg_down<true>(B, s, l, nsmooth);
+        else bmg_down<false>(B, s, l, nsmooth);
     }
+    BTail v;
+    for (int l = 0; l < kBmgMaxLevels; ++l) {
+        v.info[l] = M.info[l];
+        v.wx[l] = M.wx[l];
+        v.wy[l] = M.wy[l];
+        v.invd[l] = M.invd[l];
+        v.f[l] = l == 0 ? B->r : M.f[l];
+        v.e[l] = l == 0 ? B->z : M.e[l];
+    }
+    v.flags = B->flags;
+    v.dt = M.dt;
+    v.nsmooth = nsmooth;
     PG_LAUNCH(KK_MG_COARSE, s,
-              k_bmg_coarse<<<B->n, kBmgCoarseThreads, 0, s>>>(M.coarse, B->state, B->z, B->r, B->flags, M.dt));
-    bool rz_done = false;
-    for (int l = M.nlev - 2; l >= 0; --l) {
-        if (!M.nsmoothing[l]) continue;
-        bsmooth_any(B, s, l, 1, BNB_PROLONG);
-        for (int k = 0; k < nsmooth; ++k) {
-            if (k > 0) bsmooth_any(B, s, l, 1, BNB_PLAIN);
-            const bool rz = l == 0 && k == nsmooth - 1;
-            bsmooth_any(B, s, l, 0, BNB_PLAIN, rz);
-            rz_done = rz_done || rz;
-        }
+              k_bmg_tail<<<B->n, kBmgTailThreads, 5 * sizeof(float) * M.tail_cells, s>>>(v, B->state));
+    for (int l = deepest - 1; l >= 0; --l) {
+        if (l == 0) bmg_up<true>(B, s, l, nsmooth);
+        else bmg_up<false>(B, s, l, nsmooth);
     }
-    // No grid smooths on level 0 (every grid too small to coarsen): the
-    // z.r partials alone.
-    if (!rz_done) bsmooth<true, BNB_PLAIN, true>(B, s, 0, 0);
-    pocket_project(s, B->z, M.pockets);
+    // No grid smooths on level 0 (all are small): the z.r partials alone.
+    if (deepest == 0) bpair<true, BP_PLAIN, 1, true, false>(B, s, 0, B->ap, B->z);
+    pocket_project(s, B->z, M.pockets, &B->state[0].done, sizeof(BState));
 }
+
+void bmg_spmv(pg_batch* B, cudaStream_t s, float dt) {
+    BatchMg& M = *B->mg;
+    PG_LAUNCH(KK_CG_SPMV, s,
+              k_bmg_spmv<<<march_blocks(M.ncg), kMarchThreads, 0, s>>>(M.info[0], M.cg_strips, M.ncg, B->state, B->z, B->p0,
+                                                                       B->p1, B->ap, B->flags, dt, M.partials));
+}
+
+void bmg_update(pg_batch* B, cudaStream_t s, float* x) {
+    BatchMg& M = *B->mg;
+    const int vec = ((uintptr_t)x & 15) == 0;  // (the batch's own fields are)
+    PG_LAUNCH(KK_CG_UPDATE, s,
+              k_bmg_update<<<(M.nchunk + 7) / 8, 256, 0, s>>>(M.chunks, M.nchunk, B->state, x, B->r, B->p0, B->p1, B->ap,
+                                                              vec, M.partials));
+}
+
+const double* bmg_partials(const pg_batch* B) { return B->mg->partials; }
+const int2* bmg_spmv_range(const pg_batch* B) { return B->mg->cg_range; }
+const int2* bmg_update_range(const pg_batch* B) { return B->mg->chunk_range; }
 
 void bmg_rz_finalize(pg_batch* B, cudaStream_t s, int first) {
     BatchMg& M = *B->mg;

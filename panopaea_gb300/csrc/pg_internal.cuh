@@ -307,16 +307,22 @@ struct Pockets {
     int* start = nullptr;        // ncomp + 1 offsets into cells
     int* chunk_start = nullptr;  // nchunk + 1 offsets into cells
     int* chunk_comp = nullptr;   // component of each chunk
+    int* chunk_owner = nullptr;  // grid of each chunk (batches)
     int* comp_chunk = nullptr;   // ncomp + 1 offsets into the chunks
     double* partials = nullptr;  // nchunk partial sums, then ncomp means
     int ncomp = 0, nchunk = 0;
+    int max_chunks = 0;          // of a component
 };
 void find_pockets(const uint8_t* flags, int nd, i64 d, i64 h, i64 w, i64 base, std::vector<i64>& cells,
                   std::vector<int>& start);
-int upload_pockets(const std::vector<i64>& cells, const std::vector<int>& start, Pockets* pk);
+// comp_owner: the grid of each component (batches).
+int upload_pockets(const std::vector<i64>& cells, const std::vector<int>& start, Pockets* pk,
+                   const std::vector<int>& comp_owner = {});
 void release_pockets(Pockets* pk);
-// a -= its mean over each component (stream-ordered; nothing for connected fluid)
-void pocket_project(cudaStream_t s, float* a, const Pockets& pk);
+// a -= its mean over each component (stream-ordered; nothing for connected
+// fluid).  done (batches): grid g is left alone where the int at
+// done + g * stride bytes is set.
+void pocket_project(cudaStream_t s, float* a, const Pockets& pk, const int* done = nullptr, size_t stride = 0);
 
 int ensure_workspace(pg_grid* g);
 
