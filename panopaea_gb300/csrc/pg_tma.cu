@@ -41,6 +41,18 @@ bool encode_map_3d(CUtensorMap* map, const void* base, int elem, i64 w, i64 h, i
     return r == CUDA_SUCCESS;
 }
 
+bool encode_map_voxels_bf16(CUtensorMap* map, const void* base, int c, int w, int h, int d, int bx, int by, int bz) {
+    auto fn = encode_fn();
+    if (!fn || !base || ((uintptr_t)base & 15) || c % 16) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)d};
+    const cuuint64_t strides[3] = {2 * (cuuint64_t)c, 2 * (cuuint64_t)c * w, 2 * (cuuint64_t)c * w * h};
+    const cuuint32_t box[4] = {16, (cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace pg
 
 extern "C" int pg_debug_set_stage_wait_polls(uint32_t polls) {

@@ -41,6 +41,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
                  : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
     unsigned ok;
     asm volatile(
@@ -93,6 +97,16 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
         "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        : "memory");
+}
+
+// 4D tiled load of the box at (c, x, y, z), completing on bar.
+__device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap* map, uint64_t* bar, int c, int x, int y,
+                                            int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+        "l"((uint64_t)map), "r"(c), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
 
@@ -155,5 +169,9 @@ inline int zwalk_blocks(int ntiles, i64 d, int cap) {
 // elements with box (bx, by, 1); false when the CUDA driver rejects it (base,
 // stride or box alignment) -- callers then use their non-TMA path.
 bool encode_map_3d(CUtensorMap* map, const void* base, int elem, i64 w, i64 h, i64 d, int bx, int by);
+// Map of a channels-last BF16 field [d][h][w][c] (c a multiple of 16), loads of
+// 16 channels of bx x by x bz voxels, 32 bytes each, in the 32-byte swizzle.
+bool encode_map_voxels_bf16(CUtensorMap* map, const void* base, int c, int w, int h, int d, int bx, int by, int bz);
+
 
 }  // namespace pg

@@ -15,7 +15,8 @@
 // Every conv is 3x3x3, zero padded, followed by ReLU.
 //
 // Kernels:
-//   k_conv   implicit-GEMM conv: M = voxels of a CTA tile, N = C_out,
+//   tc::k_conv_tc  implicit-GEMM conv on tcgen05.mma (below)
+//   k_conv   the same on mma.sync: M = voxels of a CTA tile, N = C_out,
 //            K = 27 taps x C_in.  The input brick (tile + 1-voxel halo, one
 //            16-channel chunk at a time) is staged in shared memory with a
 //            48-byte voxel stride (conflict-free ldmatrix rows); B fragments
@@ -204,25 +205,41 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const bf16* __restrict__ 
 // (kind::f16, BF16 operands, FP32 accumulators in tensor memory), issued by
 // one thread, operands described in shared memory.
 //
-// GEMM per CTA: M = 128 output voxels (an 8 x 16 x-y tile of one z plane),
-// N = C_out, K = 27 taps x C_in; TZ consecutive z planes per CTA, each with
+// GEMM per tile: M = 128 output voxels (an 8 x 16 x-y tile of one z plane),
+// N = C_out, K = 27 taps x C_in; TZ consecutive z planes per tile, each with
 // its own 128 x N accumulator in tensor memory.  The input brick (tile plus
-// a one-voxel halo, TZ + 2 planes) is staged per 16-channel chunk in a
-// chunk-planar layout: [8-channel half][bz][by][bx] x 16 bytes.  In that
-// layout the A operand of every tap is a plain K-major, no-swizzle operand
-// inside the brick -- core matrices of 8 consecutive x voxels x 16 bytes
-// (contiguous 128 B), 8-row groups one brick row (BX x 16 B) apart, the two
-// 8-channel halves one plane apart -- so a tap is only a different start
-// address: no im2col copy.  The weights of a chunk arrive pre-laid-out as
-// [tap][8-channel half][n][8] (B operand, K-major: n rows 16 B apart, 8-row
-// groups 128 B apart, halves N x 16 B apart).
+// a one-voxel halo, TZ + 2 planes) is staged per 16-channel chunk as
+// [bz][by][bx] x 32 bytes in the 32-byte swizzle (the halves of a voxel change
+// places where bit 7 of its address is set), by one TMA load that also fills
+// in the zeros outside the grid.  In that layout the A operand of every tap
+// is a K-major operand inside the brick -- 8 consecutive x voxels, 8-row
+// groups one brick row (BX x 32 B) apart -- so a tap is only a different
+// start address: no im2col copy.  The weights of a chunk arrive pre-laid-out
+// as [tap][8-channel half][n][8] (B operand, K-major, no swizzle: n rows 16 B
+// apart, 8-row groups 128 B apart, halves N x 16 B apart).
+//
+// A CTA walks over tiles and keeps the tensor cores fed: three stages of
+// bricks and two sets of accumulators, so that while the MMAs of one (tile,
+// chunk) run, the bricks of the next two are on their way and eight warps
+// write out the tile before.  A ninth warp issues the MMAs: it is held up
+// while the tensor cores' queue is full, for about as long as they compute.
+// The weights stay in shared memory where all of a layer's fit beside the
+// bricks, else a chunk's travel with its brick.  An MMA of N = 48 takes 42
+// cycles where its 4 KB A operand alone takes 32 to read; a 16 -> 16 tile is
+// 54 of them, 33 us of a layer at 128^3, which takes 42 (48 -> 16: 131).  One
+// CTA per tile, loading, multiplying and storing in turn, took 83 (182); with
+// this walk but the bricks loaded by the eight warps (9 loads and stores of 16
+// bytes per thread, 1200 to 2300 cycles of every 3800) 58 (141).
 namespace tc {
 
 constexpr int TX = 8, TY = 16, BX = TX + 2, BY = TY + 2;
-constexpr int kThreads = 256;
+constexpr int kVox = 32;  // bytes of a voxel's 16 channels
+constexpr int kWorkers = 256, kThreads = kWorkers + 32;  // copy and write out; issue the MMAs
 
 // Shared-memory matrix descriptor, no swizzle (start, leading- and
-// stride-dimension byte offsets in 16-byte units; descriptor version 1).
+// stride-dimension byte offsets in 16-byte units; descriptor version 1), and
+// the 32-byte swizzle's bits to add (patterns start at multiples of 256 B).
+constexpr uint64_t kSwizzle32 = 6ull << 61;
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
@@ -245,34 +262,63 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+// 1 in one lane of the (converged) warp.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p;
+}
+// Called by a whole warp, issued by its elected lane: with every operand
+// uniform over the warp an MMA takes a few instructions to issue; from a
+// divergent thread each operand's way into the uniform registers made it 93
+// cycles, more than the tensor cores need for N <= 96.
+__device__ __forceinline__ void mma(uint32_t leader, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                    uint32_t acc) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc), "r"(leader)
         : "memory");
 }
-// One arrival on bar once every tcgen05.mma this thread issued has completed.
-__device__ __forceinline__ void commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
+// One arrival on bar once every tcgen05.mma the elected lane issued has completed.
+__device__ __forceinline__ void commit(uint32_t leader, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+        "r"(leader)
+        : "memory");
 }
-// Zero 8 consecutive 32-bit columns of this thread's lane.
-__device__ __forceinline__ void st8_zero(uint32_t taddr) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(0u)
-                 : "memory");
+// Zero 16 consecutive 32-bit columns of this thread's lane.
+__device__ __forceinline__ void st16_zero(uint32_t taddr) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+        "r"(0u)
+        : "memory");
 }
 
-// 8 consecutive 32-bit columns of this thread's lane.
-__device__ __forceinline__ void ld8(uint32_t taddr, float (&v)[8]) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
+// 16 consecutive 32-bit columns of this thread's lane.
+__device__ __forceinline__ void ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Contiguous copy by the bulk-copy engine, completing on bar.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void st_shared(uint32_t at, uint4 v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
 // Small output channel counts merge the three z taps into one MMA: an input
@@ -285,179 +331,265 @@ __device__ __forceinline__ void ld8(uint32_t taddr, float (&v)[8]) {
 // loop, for the layers whose MMA is bound by that shared-memory traffic.
 __host__ __device__ constexpr bool merge_dz(int n) { return n <= 32; }
 
-template <int COUT> struct Cfg {
+template <int CIN, int COUT, int TZ_> struct Cfg {
     static constexpr bool kMerge = merge_dz(COUT);
-    static constexpr int TZ = COUT >= 96 ? 2 : 4;
+    static constexpr int KC = CIN / 16;
+    static constexpr int TZ = TZ_;
     static constexpr int BZ = TZ + 2;
-    static constexpr int kPlane = BX * BY * BZ * 16;      // one 8-channel half of the brick
-    static constexpr int kBrick = 2 * kPlane;             // one 16-channel chunk
+    static constexpr int kBrick = BX * BY * BZ * kVox;    // one 16-channel chunk
     static constexpr int kWTap = 2 * COUT * 16;           // one tap of one chunk
     static constexpr int kWTap9 = 3 * kWTap;              // merged: the three z taps of one (dx, dy)
     static constexpr int kWChunk = 27 * kWTap;
-    static constexpr int kBrickOff = 128, kWOff = kBrickOff + kBrick;
-    static constexpr size_t kSmem = 128 + (size_t)kBrick + kWChunk;
+    // Stages: three where they fit; all of the weights beside them or, where
+    // those don't fit even with two, a chunk with each brick.
+    static constexpr int kBrickOff = 256, kFree = 227 * 1024 - kBrickOff - 256;
+    static constexpr bool kResident = 2 * kBrick + KC * kWChunk <= kFree;
+    static constexpr int NS = (kResident ? 3 * kBrick + KC * kWChunk : 3 * (kBrick + kWChunk)) <= kFree ? 3 : 2;
+    static constexpr int kWOff = kBrickOff + NS * kBrick;
+    static constexpr size_t kSmem = kWOff + (size_t)(kResident ? KC : NS) * kWChunk;
     static constexpr int kAccCols = kMerge ? (TZ + 4) * COUT : TZ * COUT;
-    static constexpr int kCols = kAccCols <= 32 ? 32 : (kAccCols <= 64 ? 64 : (kAccCols <= 128 ? 128 : (kAccCols <= 256 ? 256 : 512)));
-    static_assert(kAccCols <= 512, "accumulators must fit in tensor memory");
-    static_assert(kPlane % 16 == 0 && kBrick % 128 == 0, "operand alignment");
+    static constexpr int kCols = kAccCols <= 32 ? 64 : (kAccCols <= 64 ? 128 : (kAccCols <= 128 ? 256 : 512));  // two sets
+    static_assert(kAccCols <= 256, "two sets of accumulators must fit in tensor memory");
+    static_assert(kSmem + 256 <= 227 * 1024, "bricks and weights must fit in shared memory");
+    static_assert(kBrick % 256 == 0 && kWChunk % 128 == 0, "operand alignment");
     // tensor-memory column of output plane t's accumulator
     __host__ __device__ static constexpr int col(int t) { return kMerge ? (TZ + 1 - t) * COUT : t * COUT; }
 };
 
 struct Geom {
     int D, H, W;
-    int tiles_x, tiles_y;
+    int tiles_x, tiles_y, tiles;
 };
 
-// wtc: [chunk][tap][half][n][8] BF16 (see above); err: set when a wait for
-// the tensor cores gave up (the result is then not to be trusted).
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads) k_conv_tc(const bf16* __restrict__ in, const bf16* __restrict__ wtc,
-                                                      bf16* __restrict__ out, const bf16* __restrict__ gate, Geom G,
-                                                      int epi, int* err) {
-    typedef Cfg<COUT> C;
-    constexpr int KC = CIN / 16, TZ = C::TZ;
+// vox: the input's map.  wtc: [chunk][tap][half][n][8] BF16 (see above).
+// CA > 0: the input is the concatenation [up's voxel at half the coordinates
+// (CA channels) | vox] that k_upcat would write.  err: set when a wait for the tensor cores gave
+// up (the result is then not to be trusted).
+template <int CIN, int COUT, int TZ_, int CA>
+__global__ void __launch_bounds__(kThreads)
+    k_conv_tc(const __grid_constant__ CUtensorMap vox, const bf16* __restrict__ up, const bf16* __restrict__ wtc,
+              bf16* __restrict__ out, const bf16* __restrict__ gate, Geom G, int epi, int* err) {
+    typedef Cfg<CIN, COUT, TZ_> C;
+    constexpr int KC = C::KC, TZ = C::TZ;
     constexpr uint32_t kIdesc = idesc_bf16(128, COUT);
     extern __shared__ __align__(128) unsigned char tc_smem_raw[];
-    unsigned char* const base = tc_smem_raw + ((128u - (smem_u32(tc_smem_raw) & 127u)) & 127u);
-    uint64_t* const bar = (uint64_t*)base;
-    uint32_t* const tslot = (uint32_t*)(base + 8);
-    unsigned char* const brick = base + C::kBrickOff;
-    unsigned char* const wsm = base + C::kWOff;
+    unsigned char* const base = tc_smem_raw + ((256u - (smem_u32(tc_smem_raw) & 255u)) & 255u);
+    constexpr int NS = C::NS;
+    uint64_t* const full = (uint64_t*)base;  // per stage, items in turn: the warps are ready for the item's MMAs
+    uint64_t* const cfull = full + NS;       // what is copied for it (brick, weights) is in shared memory
+    uint64_t* const bar = cfull + NS;        // its MMAs are done
+    uint32_t* const tslot = (uint32_t*)(base + 128);
+    const uint32_t bricks = smem_u32(base + C::kBrickOff), wsm = smem_u32(base + C::kWOff);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int t = blockIdx.x;
-    const int x0 = (t % G.tiles_x) * TX;
-    t /= G.tiles_x;
-    const int y0 = (t % G.tiles_y) * TY;
-    const int z0 = (t / G.tiles_y) * TZ;
+    const int q = warp & 3, half = warp >> 2;  // this warp's TMEM lanes 32 q .. +31, and every second accumulator
     if (warp == 0) tmem_alloc(tslot, C::kCols);
     if (tid == 0) {
-        mbar_init(bar, 1);
+        for (int k = 0; k < NS; ++k) {
+            mbar_init(full + k, kWorkers / 32);
+            mbar_init(cfull + k, 1);
+            mbar_init(bar + k, 1);
+        }
         mbar_fence_init();
     }
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tslot;
-    if (C::kMerge) {  // every merged MMA accumulates: start the accumulators at zero
-        if (warp < 4) {
-            for (int c = 0; c < C::kAccCols; c += 8) st8_zero(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c);
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16);
+    constexpr int kUnits = TZ * COUT / 16;  // 128 x 16 pieces of a tile's accumulators
+    if (C::kMerge && warp < kWorkers / 32) {  // every merged MMA accumulates: start the accumulators at zero
+        for (int u = half; u < 2 * kUnits; u += 2) {
+            const int v = u % kUnits;
+            st16_zero(tlane + (uint32_t)((u / kUnits) * (C::kCols / 2) + C::col(v / (COUT / 16)) + v % (COUT / 16) * 16));
         }
-        fence_before();
-        __syncthreads();
-        fence_after();
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
-    bool ok = true;  // block-uniform
-    int committed = -1;
-    for (int kc = 0; kc < KC; ++kc) {
-        if (kc > 0) {  // the previous chunk's MMAs have read the brick and the weights
-            bool w = true;
-            if (tid == 0) w = mbar_wait(bar, (kc - 1) & 1);
-            ok = !__syncthreads_or(!w);
-            if (!ok) break;
+    auto origin = [&](int tile, int& x0, int& y0, int& z0) {
+        const int r = tile / G.tiles_x;
+        x0 = (tile - r * G.tiles_x) * TX;
+        z0 = r / G.tiles_y;
+        y0 = (r - z0 * G.tiles_y) * TY;
+        z0 *= TZ;
+    };
+    // item i: chunk i % KC of the CTA's tile i / KC
+    const int items = ((G.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * KC;
+    auto tile_of = [&](int i) { return (int)blockIdx.x + i / KC * (int)gridDim.x; };
+    // What item i needs copied, started by one thread.
+    auto brick_copied = [&](int i) { return CA == 0 || i % KC * 16 >= CA; };
+    auto weights_copied = [&](int i) { return !C::kResident || i < KC; };
+    auto copy = [&](int i) {
+        const int kc = i % KC, s = i % NS;
+        if (!brick_copied(i) && !weights_copied(i)) {
+            mbar_arrive(cfull + s);
+            return;
         }
-        // brick of this chunk: voxel (bx, by, bz) half hf at brick + hf * plane + voxel * 16
-        constexpr int nvox = BX * BY * C::BZ;
-        for (int i = tid; i < 2 * nvox; i += kThreads) {
-            const int hf = i & 1, v = i >> 1;
-            const int bx = v % BX, r = v / BX, by = r % BY, bz = r / BY;
-            const int gx = x0 + bx - 1, gy = y0 + by - 1, gz = z0 + bz - 1;
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if ((unsigned)gx < (unsigned)G.W && (unsigned)gy < (unsigned)G.H && (unsigned)gz < (unsigned)G.D)
-                val = __ldg(reinterpret_cast<const uint4*>(in + (((size_t)gz * G.H + gy) * G.W + gx) * CIN + kc * 16 +
-                                                           hf * 8));
-            *reinterpret_cast<uint4*>(brick + hf * C::kPlane + v * 16) = val;
+        mbar_expect_tx(cfull + s, (brick_copied(i) ? C::kBrick : 0) + (weights_copied(i) ? C::kWChunk : 0));
+        if (brick_copied(i)) {
+            int x0, y0, z0;
+            origin(tile_of(i), x0, y0, z0);
+            tma_load_4d(bricks + (uint32_t)(s * C::kBrick), &vox, cfull + s, kc * 16 - CA, x0 - 1, y0 - 1, z0 - 1);
         }
-        // weights of this chunk (contiguous)
-        {
-            const uint4* src = reinterpret_cast<const uint4*>(wtc + (size_t)kc * (C::kWChunk / 2));
-            uint4* dst = reinterpret_cast<uint4*>(wsm);
-            for (int i = tid; i < C::kWChunk / 16; i += kThreads) dst[i] = __ldg(src + i);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> tensor-core reads
-        __syncthreads();
-        if (tid == 0) {
-            fence_after();
-            const uint32_t bs = smem_u32(brick), ws = smem_u32(wsm);
-            if (C::kMerge) {
-                constexpr uint32_t kIdesc3 = idesc_bf16(128, 3 * COUT);
-#pragma unroll 1
-                for (int tap9 = 0; tap9 < 9; ++tap9) {
-                    const int dy = tap9 / 3, dx = tap9 % 3;
-                    const uint64_t bdesc = sdesc(ws + tap9 * C::kWTap9, 3 * COUT * 16, 128);
+        if (weights_copied(i))
+            bulk_load(wsm + (uint32_t)((C::kResident ? kc : s) * C::kWChunk),
+                      reinterpret_cast<const unsigned char*>(wtc) + (size_t)kc * C::kWChunk, C::kWChunk, cfull + s);
+    };
+    // A brick of the upsampled channels: every voxel of `up` that its parents
+    // cover is loaded once, 16 bytes per lane, and stored to its children.
+    constexpr int UX = BX / 2 + 1, UY = BY / 2 + 1, UZ = C::BZ / 2 + 1, kUp = 2 * UX * UY * UZ;
+    constexpr int NU = CA > 0 ? (kUp + kWorkers - 1) / kWorkers : 1;
+    uint4 piece[NU];
+    auto fetch_up = [&](int i) {
+        int x0, y0, z0;
+        origin(tile_of(i), x0, y0, z0);
 #pragma unroll
-                    for (int pz = 0; pz < C::BZ; ++pz) {
-                        const uint32_t a = bs + (uint32_t)(((pz * BY + dy) * BX + dx) * 16);
-                        mma(tmem + (uint32_t)C::col(pz), sdesc(a, C::kPlane, BX * 16), bdesc, kIdesc3, 1u);
-                    }
-                }
-            } else {
-#pragma unroll 1
-                for (int tap = 0; tap < 27; ++tap) {
-                    const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-                    const uint64_t bdesc = sdesc(ws + tap * C::kWTap, COUT * 16, 128);
+        for (int k = 0; k < NU; ++k) {
+            const int j = tid + k * kWorkers, v = j >> 1;
+            const int X = x0 / 2 - 1 + v % UX, Y = y0 / 2 - 1 + v / UX % UY, Z = z0 / 2 - 1 + v / (UX * UY);
+            piece[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (j < kUp && (unsigned)X < (unsigned)(G.W / 2) && (unsigned)Y < (unsigned)(G.H / 2) &&
+                (unsigned)Z < (unsigned)(G.D / 2))
+                piece[k] = __ldg(reinterpret_cast<const uint4*>(
+                    up + (((i64)Z * (G.H / 2) + Y) * (G.W / 2) + X) * CA + i % KC * 16 + (j & 1) * 8));
+        }
+    };
+    auto fill_up = [&](int i) {
+        const uint32_t brick = bricks + (uint32_t)(i % NS * C::kBrick);
 #pragma unroll
-                    for (int tz = 0; tz < TZ; ++tz) {
-                        const uint32_t a = bs + (uint32_t)((((tz + dz) * BY + dy) * BX + dx) * 16);
-                        mma(tmem + (uint32_t)(tz * COUT), sdesc(a, C::kPlane, BX * 16), bdesc, kIdesc,
-                            (kc > 0 || tap > 0) ? 1u : 0u);
-                    }
-                }
+        for (int k = 0; k < NU; ++k) {
+            const int j = tid + k * kWorkers, v = j >> 1;
+            const int bx = 2 * (v % UX) - 1, by = 2 * (v / UX % UY) - 1, bz = 2 * (v / (UX * UY)) - 1;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const int x = bx + (c & 1), y = by + (c >> 1 & 1), z = bz + (c >> 2);
+                const uint32_t at = brick + (uint32_t)(((z * BY + y) * BX + x) * kVox);
+                if (j < kUp && (unsigned)x < BX && (unsigned)y < BY && (unsigned)z < C::BZ)
+                    st_shared(at + (((uint32_t)j ^ at >> 7) & 1u) * 16, piece[k]);
             }
-            commit(bar);
         }
-        committed = kc;
-    }
-    // every MMA has completed before the accumulators are read
-    if (ok) {
-        bool w = true;
-        if (tid == 0) w = mbar_wait(bar, (KC - 1) & 1);
-        ok = !__syncthreads_or(!w);
-    }
-    if (!ok) {
-        // a wait gave up: flag it, wait once more (bounded) for the tensor
-        // cores' last committed group, and leave the accumulators unread
-        if (tid == 0) {
-            atomicExch(err, 1);
-            if (committed >= 0) mbar_wait(bar, committed & 1);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // stored brick -> tensor-core reads
+    };
+    auto multiply = [&](uint32_t leader, int i) {
+        const int kc = i % KC;
+        const uint32_t acc = tmem + (uint32_t)((i / KC & 1) * (C::kCols / 2));
+        // (start addresses count in 16 bytes)
+        const uint64_t a0 = sdesc(bricks + (uint32_t)(i % NS * C::kBrick), 16, BX * kVox) | kSwizzle32;
+        const uint64_t b0 =
+            sdesc(wsm + (uint32_t)((C::kResident ? kc : i % NS) * C::kWChunk), (C::kMerge ? 3 : 1) * COUT * 16, 128);
+        if (C::kMerge) {
+            constexpr uint32_t kIdesc3 = idesc_bf16(128, 3 * COUT);
+#pragma unroll
+            for (int tap9 = 0; tap9 < 9; ++tap9) {
+                const int dy = tap9 / 3, dx = tap9 % 3;
+#pragma unroll
+                for (int pz = 0; pz < C::BZ; ++pz)
+                    mma(leader, acc + (uint32_t)C::col(pz), a0 + (uint64_t)(((pz * BY + dy) * BX + dx) * (kVox / 16)),
+                        b0 + (uint64_t)(tap9 * C::kWTap9 / 16), kIdesc3, 1u);
+            }
+        } else {
+#pragma unroll
+            for (int tap = 0; tap < 27; ++tap) {
+                const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
+#pragma unroll
+                for (int tz = 0; tz < TZ; ++tz)
+                    mma(leader, acc + (uint32_t)(tz * COUT), a0 + (uint64_t)((((tz + dz) * BY + dy) * BX + dx) * (kVox / 16)),
+                        b0 + (uint64_t)(tap * C::kWTap / 16), kIdesc, (kc > 0 || tap > 0) ? 1u : 0u);
+            }
         }
-        __syncthreads();
-    } else {
-        fence_after();
-        // warp w reads lanes 32 (w % 4) .. +31 (rows of the tile) of the planes of its half
-        const int q = warp & 3, half = warp >> 2;
+        commit(leader, bar + i % NS);
+    };
+    // The accumulators of the tile that ended with item i, written out (and zeroed).
+    auto finish = [&](int i) {
+        int x0, y0, z0;
+        origin(tile_of(i), x0, y0, z0);
+        const uint32_t acc = tlane + (uint32_t)((i / KC & 1) * (C::kCols / 2));
         const int m = q * 32 + lane;
         const int x = x0 + (m & 7), y = y0 + (m >> 3);
-        constexpr int PZ = TZ / 2;
 #pragma unroll 1
-        for (int tz = half * PZ; tz < (half + 1) * PZ; ++tz) {
-            const int z = z0 + tz;
+        for (int u = half; u < kUnits; u += 2) {
+            const int tz = u / (COUT / 16), cg = u % (COUT / 16), z = z0 + tz;
             const bool in_grid = x < G.W && y < G.H && z < G.D;
-            const size_t o = (((size_t)z * G.H + y) * G.W + x) * COUT;
-#pragma unroll 1
-            for (int cg = 0; cg < COUT / 8; ++cg) {
-                float v[8];
-                ld8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(C::col(tz) + cg * 8), v);
-                if (!in_grid) continue;
-                if (epi == EPI_RELU) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) v[i] = v[i] > 0.f ? v[i] : 0.f;
-                } else if (epi == EPI_GATE) {
-                    const uint4 gv = *reinterpret_cast<const uint4*>(gate + o + cg * 8);
-                    const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        __nv_bfloat162 pr;
-                        memcpy(&pr, &gw[i], 4);
-                        if (!(__bfloat162float(pr.x) > 0.f)) v[2 * i] = 0.f;
-                        if (!(__bfloat162float(pr.y) > 0.f)) v[2 * i + 1] = 0.f;
-                    }
-                }
-                *reinterpret_cast<uint4*>(out + o + cg * 8) =
-                    make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
-                               pack_bf16(v[6], v[7]));
+            const size_t o = (((size_t)z * G.H + y) * G.W + x) * COUT + cg * 16;
+            uint4 gv[2] = {};
+            if (epi == EPI_GATE && in_grid) {
+                gv[0] = *reinterpret_cast<const uint4*>(gate + o);
+                gv[1] = *reinterpret_cast<const uint4*>(gate + o + 8);
             }
+            const uint32_t at = acc + (uint32_t)(C::col(tz) + cg * 16);
+            float v[16];
+            ld16(at, v);
+            if (C::kMerge) st16_zero(at);
+            if (!in_grid) continue;
+            if (epi == EPI_RELU) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = v[j] > 0.f ? v[j] : 0.f;
+            } else if (epi == EPI_GATE) {
+                const uint32_t gw[8] = {gv[0].x, gv[0].y, gv[0].z, gv[0].w, gv[1].x, gv[1].y, gv[1].z, gv[1].w};
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    __nv_bfloat162 pr;
+                    memcpy(&pr, &gw[j], 4);
+                    if (!(__bfloat162float(pr.x) > 0.f)) v[2 * j] = 0.f;
+                    if (!(__bfloat162float(pr.y) > 0.f)) v[2 * j + 1] = 0.f;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                *reinterpret_cast<uint4*>(out + o + 8 * j) =
+                    make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
+                               pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7]));
+        }
+        if (C::kMerge) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    };
+    // A wait that gives up ends the warp's work and flags the result; the
+    // others' waits then complete or give up as well.
+    if (warp < kWorkers / 32) {
+        auto done = [&](int i) {  // item i's MMAs (uniform per warp)
+            const bool w = lane != 0 || mbar_wait(bar + i % NS, (unsigned)(i / NS) & 1u);
+            const bool ok = __all_sync(0xffffffffu, w);
+            fence_after();
+            return ok;
+        };
+        bool ok = true;
+        int last = -1;  // the last item whose copies were started
+        auto load = [&](int i) {  // item i into its stage; then the pieces of the next
+            if (i < items) {
+                if (tid == 0) copy(i);
+                if (CA > 0 && !brick_copied(i)) fill_up(i);
+                last = i;
+            }
+            if (CA > 0 && i + 1 < items && !brick_copied(i + 1)) fetch_up(i + 1);
+        };
+        if (CA > 0) fetch_up(0);
+        for (int i = 0; i < NS - 1; ++i) load(i);
+        for (int i = 0; i < items; ++i) {
+            fence_before();  // (accumulators read and zeroed)
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full + i % NS);
+            if (i > 0 && !(ok = done(i - 1))) break;  // the item before has read its operands
+            load(i + NS - 1);
+            if (i > 0 && i % KC == 0) finish(i - 1);
+        }
+        if (ok && (ok = done(items - 1))) finish(items - 1);
+        if (!ok && lane == 0) {
+            atomicExch(err, 1);
+            if (tid == 0)  // (bounded) for the copies in flight
+                for (int i = max(0, last - NS + 1); i <= last; ++i)
+                    mbar_wait(cfull + i % NS, (unsigned)(i / NS) & 1u);
+        }
+    } else {
+        const uint32_t leader = elect_one();
+        for (int i = 0; i < items; ++i) {
+            const unsigned parity = (unsigned)(i / NS) & 1u;
+            if (!__all_sync(0xffffffffu, mbar_wait(full + i % NS, parity) && mbar_wait(cfull + i % NS, parity))) {
+                // flag it and wait (bounded) for the last committed group
+                if (leader) {
+                    atomicExch(err, 1);
+                    if (i > 0) mbar_wait(bar + (i - 1) % NS, (unsigned)((i - 1) / NS) & 1u);
+                }
+                break;
+            }
+            fence_after();
+            multiply(leader, i);
         }
     }
     fence_before();
@@ -1074,38 +1206,62 @@ int conv_t(const pg_unet* net, int lvl, const bf16* in, const uint2* w, bf16* ou
     return PG_OK;
 }
 
-// The tensor-core convolution: one CTA per 8 x 16 x TZ output tile; the
-// launch's dynamic shared memory also caps the CTAs per SM so that their
-// tensor-memory columns fit in the SM's 512.
-template <int CIN, int COUT>
-int conv_tc_t(const pg_unet* net, int lvl, const bf16* in, const bf16* wtc, bf16* out, const bf16* gate, int epi) {
-    typedef tc::Cfg<COUT> Cf;
-    static size_t smem = 0;
-    if (!smem) {
-        size_t s = Cf::kSmem + 128;
-        PG_CUDA(cudaFuncSetAttribute(tc::k_conv_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     227 * 1024));
+// The tensor-core convolution: CTAs that walk over the 8 x 16 x TZ output
+// tiles; the launch's dynamic shared memory also caps the CTAs per SM so that
+// their tensor-memory columns fit in the SM's 512.
+template <int CIN, int COUT, int TZ, int CA>
+int conv_tc_z(const pg_unet* net, int lvl, const bf16* in, const bf16* up, const bf16* wtc, bf16* out, const bf16* gate,
+              int epi) {
+    typedef tc::Cfg<CIN, COUT, TZ> Cf;
+    const auto kernel = tc::k_conv_tc<CIN, COUT, TZ, CA>;
+    struct Shape {
+        size_t smem = Cf::kSmem + 256;
+        int per_sm = 0;
+        cudaError_t e;
+    };
+    static const Shape shape = [&] {
+        Shape r;
         const int maxb = 512 / Cf::kCols;
-        int bps = 0;
-        PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, tc::k_conv_tc<CIN, COUT>, tc::kThreads, s));
-        if (bps > maxb) {
-            s = std::max(s, (size_t)(228 * 1024 / (maxb + 1) - 1024 + 128));
-            PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, tc::k_conv_tc<CIN, COUT>, tc::kThreads, s));
+        if ((r.e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)) ||
+            (r.e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_sm, kernel, tc::kThreads, r.smem)))
+            return r;
+        if (r.per_sm > maxb) {
+            r.smem = std::max(r.smem, (size_t)(228 * 1024 / (maxb + 1) - 1024 + 128));
+            r.e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_sm, kernel, tc::kThreads, r.smem);
         }
-        if (bps < 1 || bps > maxb) return bad_arg("pg_unet: tensor-core conv does not fit an SM");
-        smem = s;
-    }
+        if (!r.e && r.per_sm > maxb) r.per_sm = 0;
+        return r;
+    }();
+    PG_CUDA(shape.e);
+    if (shape.per_sm < 1) return bad_arg("pg_unet: tensor-core conv does not fit an SM");
     tc::Geom G;
     G.D = net->ld[lvl];
     G.H = net->lh[lvl];
     G.W = net->lw[lvl];
     G.tiles_x = ceil_div(G.W, tc::TX);
     G.tiles_y = ceil_div(G.H, tc::TY);
-    const int nb = G.tiles_x * G.tiles_y * ceil_div(G.D, Cf::TZ);
+    G.tiles = G.tiles_x * G.tiles_y * ceil_div(G.D, TZ);
+    CUtensorMap vox;
+    if (!encode_map_voxels_bf16(&vox, in, CIN - CA, G.W, G.H, G.D, tc::BX, tc::BY, Cf::BZ)) {
+        set_error("pg_unet: no tensor map for a layer's input");
+        return PG_CUDA_ERROR;
+    }
+    const int nb = std::min(G.tiles, shape.per_sm * net->num_sms);
     PG_LAUNCH(KK_UNET_CONV, net->stream,
-              tc::k_conv_tc<CIN, COUT><<<nb, tc::kThreads, smem, net->stream>>>(in, wtc, out, gate, G, epi, net->err));
+              kernel<<<nb, tc::kThreads, shape.smem, net->stream>>>(vox, up, wtc, out, gate, G, epi, net->err));
     PG_CHECK_LAUNCH();
     return PG_OK;
+}
+
+// Planes per tile: four (two for 96 channels, whose weights fill shared
+// memory); two where tiles of four leave SMs without work.
+template <int CIN, int COUT, int CA = 0>
+int conv_tc_t(const pg_unet* net, int lvl, const bf16* in, const bf16* wtc, bf16* out, const bf16* gate, int epi,
+              const bf16* up = nullptr) {
+    constexpr int TZ = COUT >= 96 ? 2 : 4;
+    const int tiles = ceil_div(net->lw[lvl], tc::TX) * ceil_div(net->lh[lvl], tc::TY) * ceil_div(net->ld[lvl], TZ);
+    if (TZ == 4 && tiles < net->num_sms) return conv_tc_z<CIN, COUT, 2, CA>(net, lvl, in, up, wtc, out, gate, epi);
+    return conv_tc_z<CIN, COUT, TZ, CA>(net, lvl, in, up, wtc, out, gate, epi);
 }
 
 // The tensor-core path unless PG_UNET_TC=0 (a diagnostic switch: the legacy
@@ -1227,8 +1383,12 @@ int check_grid(const pg_unet* net, const pg_grid* g) {
 }
 
 // Normalise b, run the encoder/decoder; Y[9] holds the last features.
-int forward(pg_unet* net, const pg_grid* g, const float* b, double dt) {
+// train: a backward pass follows, which reads the concatenations C0 and C1;
+// otherwise the convolutions read their two inputs where they are (k_upcat
+// took 99 us at 128^3, more than it saves them).
+int forward(pg_unet* net, const pg_grid* g, const float* b, double dt, bool train = false) {
     int rc;
+    const bool cat = train || !tc_enabled();
     if ((rc = prep_weights(net))) return rc;
     const i64 V0 = net->lv[0];
     cudaStream_t s = net->stream;
@@ -1244,10 +1404,20 @@ int forward(pg_unet* net, const pg_grid* g, const float* b, double dt) {
     if ((rc = C(2, net->P0)) || (rc = C(3, net->Y[2]))) return rc;
     PG_LAUNCH(KK_UNET_MISC, s, k_pool<<<blocks_for(net, net->lv[2] * 32), 256, 0, s>>>(net->Y[3], 32, net->ld[1], net->lh[1], net->lw[1], net->P1));
     if ((rc = C(4, net->P1)) || (rc = C(5, net->Y[4]))) return rc;
-    PG_LAUNCH(KK_UNET_MISC, s, k_upcat<<<blocks_for(net, net->lv[1] * 12), 256, 0, s>>>(net->Y[5], 64, net->Y[3], 32, net->ld[1], net->lh[1], net->lw[1], net->C1));
-    if ((rc = C(6, net->C1)) || (rc = C(7, net->Y[6]))) return rc;
-    PG_LAUNCH(KK_UNET_MISC, s, k_upcat<<<blocks_for(net, net->lv[0] * 6), 256, 0, s>>>(net->Y[7], 32, net->Y[1], 16, net->ld[0], net->lh[0], net->lw[0], net->C0));
-    if ((rc = C(8, net->C0)) || (rc = C(9, net->Y[8]))) return rc;
+    if (cat) {
+        PG_LAUNCH(KK_UNET_MISC, s, k_upcat<<<blocks_for(net, net->lv[1] * 12), 256, 0, s>>>(net->Y[5], 64, net->Y[3], 32, net->ld[1], net->lh[1], net->lw[1], net->C1));
+        rc = C(6, net->C1);
+    } else {
+        rc = conv_tc_t<96, 32, 64>(net, 1, net->Y[3], net->tcf[6], net->Y[6], nullptr, EPI_RELU, net->Y[5]);
+    }
+    if (rc || (rc = C(7, net->Y[6]))) return rc;
+    if (cat) {
+        PG_LAUNCH(KK_UNET_MISC, s, k_upcat<<<blocks_for(net, net->lv[0] * 6), 256, 0, s>>>(net->Y[7], 32, net->Y[1], 16, net->ld[0], net->lh[0], net->lw[0], net->C0));
+        rc = C(8, net->C0);
+    } else {
+        rc = conv_tc_t<48, 16, 32>(net, 0, net->Y[1], net->tcf[8], net->Y[8], nullptr, EPI_RELU, net->Y[7]);
+    }
+    if (rc || (rc = C(9, net->Y[8]))) return rc;
     PG_CHECK_LAUNCH();
     return PG_OK;
 }
@@ -1559,7 +1729,7 @@ int pg_unet_accumulate_f32(pg_unet* net, const pg_grid* g, const float* b, const
     if (!(dt > 0.0)) return bad_arg("pg_unet_accumulate_f32: dt must be > 0");
     int rc;
     if ((rc = check_grid(net, g))) return rc;
-    if ((rc = forward(net, g, b, dt)) || (rc = head(net, g, dt, nullptr, p_true)) || (rc = backward(net))) return rc;
+    if ((rc = forward(net, g, b, dt, true)) || (rc = head(net, g, dt, nullptr, p_true)) || (rc = backward(net))) return rc;
     if (loss) {
         PG_CUDA(cudaMemcpyAsync(loss, net->loss, sizeof(double), cudaMemcpyDeviceToHost, net->stream));
         PG_CUDA(cudaStreamSynchronize(net->stream));
