@@ -55,6 +55,7 @@ constexpr int kL = 10;
 constexpr int kCin[kL] = {16, 16, 16, 32, 32, 64, 96, 32, 48, 16};
 constexpr int kCout[kL] = {16, 16, 32, 32, 64, 64, 32, 32, 16, 16};
 constexpr int kLevel[kL] = {0, 0, 1, 1, 2, 2, 1, 1, 0, 0};
+constexpr int kSkip[kL] = {0, 0, 0, 0, 0, 0, 3, 0, 1, 0};  // decoder layers 6, 8: the layer concatenated
 
 inline i64 param_offset(int k) {
     i64 o = 0;
@@ -606,7 +607,18 @@ __global__ void __launch_bounds__(kThreads)
 // tap-mirrored) W[26 - tap][n][k] of the forward layer.
 // With merge_dz(N) the three z taps of one (dx, dy) are stacked along N:
 // wtc[chunk][dy 3 + dx][half][dz N + n][8].
-__global__ void k_wprep_tc(const float* __restrict__ W, int cin, int cout, int transposed, bf16* __restrict__ wtc) {
+// blockIdx.y: layer, forward then backward-data (one launch: 19 of 3 us each
+// were launch latency).
+struct PrepArgs {
+    const float* W[2 * kL];
+    bf16* wtc[2 * kL];  // null: no such layout
+    int cin[kL], cout[kL];
+};
+__global__ void k_wprep_tc(PrepArgs A) {
+    const int layer = blockIdx.y >> 1, transposed = blockIdx.y & 1, cin = A.cin[layer], cout = A.cout[layer];
+    const float* __restrict__ W = A.W[blockIdx.y];
+    bf16* __restrict__ wtc = A.wtc[blockIdx.y];
+    if (!wtc) return;
     const int K = transposed ? cout : cin, N = transposed ? cin : cout;
     const bool merged = merge_dz(N);
     const int n_all = 27 * K * N;
@@ -677,6 +689,7 @@ constexpr int wg_ctas_per_sm(int cin) { return cin > 32 ? 2 : kWgCtasPerSm; }
 struct WgGeom {
     int D, H, W;
     int cin, cout;
+    int ca;  // > 0: the first ca input channels come from `up`, at half the coordinates (X has the others)
     int tiles_x, tiles_y, tiles;
 };
 
@@ -687,7 +700,8 @@ __device__ __forceinline__ void cp16_or_zero(uint32_t dst, const void* src, bool
 
 template <int CO>
 __global__ void __launch_bounds__(kWgThreads, kWgCtasPerSm)
-    k_wgrad(const bf16* __restrict__ X, const bf16* __restrict__ dZ, float* __restrict__ part, WgGeom G) {
+    k_wgrad(const bf16* __restrict__ X, const bf16* __restrict__ up, const bf16* __restrict__ dZ,
+            float* __restrict__ part, WgGeom G) {
     constexpr int ZV = CO / 8, NT = CO / 16, ZS = wg_zs(CO);  // 16-byte vectors per dZ voxel; n-tiles of a warp
     static_assert(NT == 1 || NT == 2, "a warp owns one or two n-tiles");
     extern __shared__ __align__(16) unsigned char wg_smem_raw[];
@@ -720,8 +734,12 @@ __global__ void __launch_bounds__(kWgThreads, kWgCtasPerSm)
             const int bx = v % kWgBX, q = v / kWgBX, by = q % kWgBY, bz = q / kWgBY;
             const int gx = x0 + bx - 1, gy = y0 + by - 1, gz = z0 + bz + dz - 1;
             const bool in = (unsigned)gx < (unsigned)G.W && (unsigned)gy < (unsigned)G.H && (unsigned)gz < (unsigned)G.D;
-            const size_t o = in ? (((size_t)gz * G.H + gy) * G.W + gx) * G.cin + ci0 + hf * 8 : 0;
-            cp16_or_zero(xb + v * kWgXS + hf * 16, X + o, in);
+            const bf16* src = X;
+            if (in && ci0 < G.ca)
+                src = up + (((size_t)(gz >> 1) * (G.H >> 1) + (gy >> 1)) * (G.W >> 1) + (gx >> 1)) * G.ca + ci0 + hf * 8;
+            else if (in)
+                src = X + (((size_t)gz * G.H + gy) * G.W + gx) * (G.cin - G.ca) + ci0 - G.ca + hf * 8;
+            cp16_or_zero(xb + v * kWgXS + hf * 16, src, in);
         }
         for (int i = threadIdx.x; i < kWgTile * ZV; i += kWgThreads) {
             const int p = i % ZV, v = i / ZV;
@@ -813,11 +831,21 @@ __global__ void __launch_bounds__(kWgThreads, kWgCtasPerSm)
 // grad[i] += sum_s part[s][i]: eight interleaved runs of s, each in order,
 // then the eight in order (32 outputs per block, so the reads are whole
 // 128-byte lines and S / 8 loads follow one another instead of S).
-__global__ void __launch_bounds__(256) k_wgrad_sum(const float* __restrict__ part, int S, int n,
-                                                   float* __restrict__ grad) {
+// All layers in one launch (ten of 7 us each were launch latency).
+struct WgSumArgs {
+    const float* part[kL];
+    float* grad[kL];
+    int S[kL], n[kL], block0[kL];  // block0: a layer's first block
+};
+__global__ void __launch_bounds__(256) k_wgrad_sum(WgSumArgs A) {
     __shared__ float sm[8][32];
     const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + lane;  // n is a multiple of 32
+    int layer = kL - 1;
+    while (blockIdx.x < (unsigned)A.block0[layer]) --layer;
+    const float* __restrict__ part = A.part[layer];
+    float* __restrict__ grad = A.grad[layer];
+    const int S = A.S[layer], n = A.n[layer];
+    const int i = (blockIdx.x - A.block0[layer]) * 32 + lane;  // n is a multiple of 32
     float s = 0.f;
 #pragma unroll 4
     for (int k = seg; k < S; k += 8) s += __ldg(part + (size_t)k * n + i);
@@ -874,12 +902,19 @@ __global__ void __launch_bounds__(kRedThreads) k_sumsq(const float* __restrict__
     if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
+// The sum of a stride-spaced column of partials, by one warp (a thread alone
+// takes 60 cycles per addition: 33 us for 512).
+__device__ __forceinline__ double warp_fold(const double* __restrict__ part, int n, int stride) {
+    double s = 0.0;
+    for (int i = threadIdx.x & 31; i < n; i += 32) s += part[(size_t)i * stride];
+    return warp_sum(s);
+}
+
 // scal = {s, 1/s, s * out_scale, dt / (s * out_scale)}
 __global__ void k_scalars(const double* __restrict__ part, int nparts, i64 n, float out_scale, float dt,
                           float* __restrict__ scal) {
+    const double ss = warp_fold(part, nparts, 1);
     if (threadIdx.x != 0) return;
-    double ss = 0.0;
-    for (int i = 0; i < nparts; ++i) ss += part[i];
     const float s = (float)sqrt(ss / (double)n);
     const float scale = __fmul_rn(s, out_scale);
     scal[0] = s;
@@ -894,32 +929,100 @@ __global__ void k_input(const float* __restrict__ b, const uint8_t* __restrict__
     for (i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (i64)gridDim.x * blockDim.x) {
         const float c0 = __fmul_rn(b[v], inv_s);
         const float c1 = __fmul_rn((float)__popc(flags[v] & 63u), 1.0f / 6.0f);
-        uint4 lo = make_uint4(pack_bf16(c0, c1), 0u, 0u, 0u);
-        uint4* o = reinterpret_cast<uint4*>(X0 + v * 16);
-        o[0] = lo;
-        o[1] = make_uint4(0u, 0u, 0u, 0u);
+        // (channels 8 to 15 are zero from the start)
+        *reinterpret_cast<uint4*>(X0 + v * 16) = make_uint4(pack_bf16(c0, c1), 0u, 0u, 0u);
     }
 }
 
 // ---------------------------------------------------------------------------
 // Pooling and upsampling (fine level dims D, H, W; coarse = half).
 
-// out[u][c] = bf16(0.125 * sum of the 8 children, in (dz, dy, dx) order)
-__global__ void k_pool(const bf16* __restrict__ in, int C, int D, int H, int W, bf16* __restrict__ out) {
-    const int cd = D / 2, ch = H / 2, cw = W / 2;
-    const i64 n = (i64)cd * ch * cw * C;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        const i64 u = i / C;
-        const int x = (int)(u % cw), y = (int)((u / cw) % ch), z = (int)(u / ((i64)cw * ch));
-        float s = 0.f;
+// The kernels below move 8 channels (16 bytes) per thread: blockIdx.y walks over
+// the z planes, a plane's index is split with multiplications.  One channel
+// per thread and 64-bit divisions took 54, 47 and 107 us (pooling at 128^3,
+// the two backward forms at 96^3).
+struct Vec8 {
+    float v[8];
+};
+__device__ __forceinline__ Vec8 load8(const bf16* p) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    Vec8 r;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int fz = 2 * z + (k >> 2), fy = 2 * y + ((k >> 1) & 1), fx = 2 * x + (k & 1);
-            s = __fadd_rn(s, __bfloat162float(in[(((size_t)fz * H + fy) * W + fx) * C + c]));
-        }
-        out[i] = __float2bfloat16_rn(__fmul_rn(0.125f, s));
+    for (int k = 0; k < 4; ++k) {
+        __nv_bfloat162 h;
+        memcpy(&h, &w[k], 4);
+        r.v[2 * k] = __bfloat162float(h.x);
+        r.v[2 * k + 1] = __bfloat162float(h.y);
     }
+    return r;
+}
+__device__ __forceinline__ void store8(bf16* p, const Vec8& a) {
+    *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16(a.v[0], a.v[1]), pack_bf16(a.v[2], a.v[3]),
+                                              pack_bf16(a.v[4], a.v[5]), pack_bf16(a.v[6], a.v[7]));
+}
+// The sum of the 8 children of coarse voxel (z, y, x), in (dz, dy, dx) order;
+// voxels of ct channels, the first at c.
+__device__ __forceinline__ Vec8 sum_children(const bf16* __restrict__ in, int ct, int c, int H, int W, int z, int y, int x) {
+    Vec8 s = {};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int fz = 2 * z + (k >> 2), fy = 2 * y + ((k >> 1) & 1), fx = 2 * x + (k & 1);
+        const Vec8 a = load8(in + (((size_t)fz * H + fy) * W + fx) * ct + c);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s.v[j] = __fadd_rn(s.v[j], a.v[j]);
+    }
+    return s;
+}
+
+// out[u][c] = bf16(0.125 * sum of the 8 children)
+__global__ void k_pool(const bf16* __restrict__ in, int C, int D, int H, int W, FastDiv fv, FastDiv fw,
+                       bf16* __restrict__ out) {
+    const int ch = H / 2, cw = W / 2, nv = C / 8;
+    for (int z = blockIdx.y; z < D / 2; z += gridDim.y)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ch * cw * nv; i += gridDim.x * blockDim.x) {
+            int c, x;
+            const int y = split(split(i, nv, fv, c), cw, fw, x);
+            Vec8 s = sum_children(in, C, 8 * c, H, W, z, y, x);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s.v[j] = __fmul_rn(0.125f, s.v[j]);
+            store8(out + (((size_t)z * ch + y) * cw + x) * C + 8 * c, s);
+        }
+}
+
+// dz[u][c] = y[u][c] > 0 ? bf16(sum_children dcat[child][c]) : 0, c < ca
+__global__ void k_upback_gate(const bf16* __restrict__ dcat, int ct, int ca, const bf16* __restrict__ y, int D, int H,
+                              int W, FastDiv fv, FastDiv fw, bf16* __restrict__ dz) {
+    const int ch = H / 2, cw = W / 2, nv = ca / 8;
+    for (int z = blockIdx.y; z < D / 2; z += gridDim.y)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ch * cw * nv; i += gridDim.x * blockDim.x) {
+            int c, x;
+            const int yy = split(split(i, nv, fv, c), cw, fw, x);
+            const size_t o = (((size_t)z * ch + yy) * cw + x) * ca + 8 * c;
+            const Vec8 g = load8(y + o);
+            Vec8 s = sum_children(dcat, ct, 8 * c, H, W, z, yy, x);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s.v[j] = g.v[j] > 0.f ? s.v[j] : 0.f;
+            store8(dz + o, s);
+        }
+}
+
+// dz[v][c] = y[v][c] > 0 ? bf16(dcat[v][off + c] + 0.125 * dp[parent(v)][c]) : 0
+__global__ void k_poolback_gate(const bf16* __restrict__ dcat, int ct, int off, const bf16* __restrict__ dp, int C,
+                                const bf16* __restrict__ y, int D, int H, int W, FastDiv fv, FastDiv fw,
+                                bf16* __restrict__ dz) {
+    const int nv = C / 8;
+    for (int z = blockIdx.y; z < D; z += gridDim.y)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < H * W * nv; i += gridDim.x * blockDim.x) {
+            int c, x;
+            const int yy = split(split(i, nv, fv, c), W, fw, x);
+            const size_t v = ((size_t)z * H + yy) * W + x, u = ((size_t)(z / 2) * (H / 2) + yy / 2) * (W / 2) + x / 2;
+            const Vec8 a = load8(dcat + v * ct + off + 8 * c), b = load8(dp + u * C + 8 * c), g = load8(y + v * C + 8 * c);
+            Vec8 s;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s.v[j] = g.v[j] > 0.f ? __fadd_rn(a.v[j], __fmul_rn(0.125f, b.v[j])) : 0.f;
+            store8(dz + v * C + 8 * c, s);
+        }
 }
 
 // out[v] = [coarse[parent(v)] (ca channels) | skip[v] (cb channels)], 8-channel vectors
@@ -940,40 +1043,6 @@ __global__ void k_upcat(const bf16* __restrict__ coarse, int ca, const bf16* __r
             val = *reinterpret_cast<const uint4*>(skip + v * cb + (k * 8 - ca));
         }
         *reinterpret_cast<uint4*>(out + v * ct + k * 8) = val;
-    }
-}
-
-// dz[u][c] = y[u][c] > 0 ? bf16(sum_children dcat[child][c]) : 0, c < ca
-__global__ void k_upback_gate(const bf16* __restrict__ dcat, int ct, int ca, const bf16* __restrict__ y, int D, int H,
-                              int W, bf16* __restrict__ dz) {
-    const int cd = D / 2, ch = H / 2, cw = W / 2;
-    const i64 n = (i64)cd * ch * cw * ca;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        const int c = (int)(i % ca);
-        const i64 u = i / ca;
-        const int x = (int)(u % cw), yy = (int)((u / cw) % ch), z = (int)(u / ((i64)cw * ch));
-        float s = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int fz = 2 * z + (k >> 2), fy = 2 * yy + ((k >> 1) & 1), fx = 2 * x + (k & 1);
-            s = __fadd_rn(s, __bfloat162float(dcat[(((size_t)fz * H + fy) * W + fx) * ct + c]));
-        }
-        dz[i] = __bfloat162float(y[i]) > 0.f ? __float2bfloat16_rn(s) : __float2bfloat16_rn(0.f);
-    }
-}
-
-// dz[v][c] = y[v][c] > 0 ? bf16(dcat[v][off + c] + 0.125 * dp[parent(v)][c]) : 0
-__global__ void k_poolback_gate(const bf16* __restrict__ dcat, int ct, int off, const bf16* __restrict__ dp, int C,
-                                const bf16* __restrict__ y, int D, int H, int W, bf16* __restrict__ dz) {
-    const i64 n = (i64)D * H * W * C;
-    const int ch = H / 2, cw = W / 2;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        const i64 v = i / C;
-        const int x = (int)(v % W), yy = (int)((v / W) % H), z = (int)(v / ((i64)W * H));
-        const i64 u = ((i64)(z / 2) * ch + yy / 2) * cw + x / 2;
-        const float s = __fadd_rn(__bfloat162float(dcat[v * ct + off + c]), __fmul_rn(0.125f, __bfloat162float(dp[u * C + c])));
-        dz[i] = __bfloat162float(y[i]) > 0.f ? __float2bfloat16_rn(s) : __float2bfloat16_rn(0.f);
     }
 }
 
@@ -1074,12 +1143,8 @@ __global__ void __launch_bounds__(kRedThreads) k_dots(const float* __restrict__ 
 }
 
 __global__ void k_alpha(const double* __restrict__ part, int nb, float* __restrict__ alpha) {
+    const double a = warp_fold(part, nb, 2), b = warp_fold(part + 1, nb, 2);
     if (threadIdx.x != 0) return;
-    double a = 0.0, b = 0.0;
-    for (int i = 0; i < nb; ++i) {
-        a += part[2 * i];
-        b += part[2 * i + 1];
-    }
     *alpha = (b > 0.0 && isfinite(a / b)) ? (float)(a / b) : 0.f;
 }
 
@@ -1092,13 +1157,12 @@ __global__ void k_step(float* __restrict__ x, float* __restrict__ r, const float
     }
 }
 
-// grad_wh[c] += sum_blocks part[c]; loss_out = sum part[16] / n
+// grad_wh[c] += sum_blocks part[c]; loss_out = sum part[16] / n; a warp each
 __global__ void k_head_sum(const double* __restrict__ part, int nb, i64 n, float* __restrict__ grad_wh,
                            double* __restrict__ loss_out) {
-    const int c = threadIdx.x;
-    if (c > 16) return;
-    double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += part[b * 17 + c];
+    const int c = threadIdx.x >> 5;
+    const double s = warp_fold(part + c, nb, 17);
+    if (threadIdx.x & 31) return;
     if (c < 16)
         grad_wh[c] += (float)s;
     else
@@ -1143,7 +1207,7 @@ struct pg_unet {
     bf16* tcf[kL] = {};  // tensor-core (tcgen05) weight layouts: forward
     bf16* tct[kL] = {};  // and backward-data
     int* err = nullptr;  // set by a kernel whose bounded wait gave up
-    bool wdirty = true;
+    bool wdirty = true, wdirty_mma = true;  // the layouts' weights are older than the parameters
     bf16 *X0 = nullptr, *Y[kL] = {}, *P0 = nullptr, *P1 = nullptr, *C1 = nullptr, *C0 = nullptr;
     bf16 *G0a = nullptr, *G0b = nullptr, *dC0 = nullptr, *G1a = nullptr, *G1b = nullptr, *dC1 = nullptr,
          *dP0 = nullptr, *G2a = nullptr, *G2b = nullptr, *dP1 = nullptr;
@@ -1154,7 +1218,7 @@ struct pg_unet {
     float* scal = nullptr;  // 4 floats
     double* red = nullptr;  // reduction partials
     double* loss = nullptr;
-    float* wpart = nullptr;
+    float* wpart[kL] = {};  // weight-gradient partials
     double out_scale = 1.0;
     i64 adam_t = 0;
 };
@@ -1167,6 +1231,9 @@ int pow2_floor(int x) {
     while (p * 2 <= x) p *= 2;
     return p;
 }
+
+// Grid of the plane-walking kernels: d planes of n threads.
+dim3 plane_grid(i64 n, int d) { return dim3((unsigned)((n + 255) / 256), (unsigned)std::min(d, 65535)); }
 
 int blocks_for(const pg_unet* net, i64 n, int threads = 256) {
     i64 b = (n + threads - 1) / threads;
@@ -1316,51 +1383,79 @@ int wg_ctas(const pg_unet* net, int k) {
     return std::max(1, std::min(wg_tiles(net, kLevel[k]), wg_ctas_per_sm(kCin[k]) * net->num_sms / blocks));
 }
 
-template <int CO> int wgrad_t(pg_unet* net, int k, const bf16* X, const bf16* dZ) {
+template <int CO> int wgrad_t(pg_unet* net, int k, const bf16* X, const bf16* up, const bf16* dZ) {
     static bool attr_set = false;
     if (!attr_set) {
         PG_CUDA(cudaFuncSetAttribute(k_wgrad<CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * wg_stage(CO)));
         attr_set = true;
     }
-    const int lvl = kLevel[k], S = wg_ctas(net, k), n = 27 * kCin[k] * kCout[k];
+    const int lvl = kLevel[k], S = wg_ctas(net, k);
     WgGeom G;
     G.D = net->ld[lvl];
     G.H = net->lh[lvl];
     G.W = net->lw[lvl];
     G.cin = kCin[k];
     G.cout = kCout[k];
+    G.ca = up ? kCin[k] - kCout[kSkip[k]] : 0;
     G.tiles_x = ceil_div(G.W, kWgX);
     G.tiles_y = ceil_div(G.H, kWgY);
     G.tiles = wg_tiles(net, lvl);
     const dim3 grid(S, 3 * (kCin[k] / 16) * (kCout[k] / CO));
-    PG_LAUNCH(KK_UNET_WGRAD, net->stream, k_wgrad<CO><<<grid, kWgThreads, 2 * wg_stage(CO), net->stream>>>(X, dZ, net->wpart, G));
-    PG_LAUNCH(KK_UNET_WGRAD, net->stream, k_wgrad_sum<<<n / 32, 256, 0, net->stream>>>(net->wpart, S, n, net->grads + param_offset(k)));
+    PG_LAUNCH(KK_UNET_WGRAD, net->stream, k_wgrad<CO><<<grid, kWgThreads, 2 * wg_stage(CO), net->stream>>>(X, up, dZ, net->wpart[k], G));
     PG_CHECK_LAUNCH();
     return PG_OK;
 }
 
-int wgrad(pg_unet* net, int k, const bf16* X, const bf16* dZ) {
-    return wg_co(kCout[k]) == 16 ? wgrad_t<16>(net, k, X, dZ) : wgrad_t<32>(net, k, X, dZ);
+// The partials of layer k's weight gradient; X, and up with a decoder's
+// concatenation [up | X].
+int wgrad(pg_unet* net, int k, const bf16* X, const bf16* dZ, const bf16* up = nullptr) {
+    return wg_co(kCout[k]) == 16 ? wgrad_t<16>(net, k, X, up, dZ) : wgrad_t<32>(net, k, X, up, dZ);
+}
+
+// Every layer's partials folded into its gradient.
+int wgrad_sums(pg_unet* net) {
+    WgSumArgs A;
+    int blocks = 0;
+    for (int k = 0; k < kL; ++k) {
+        A.part[k] = net->wpart[k];
+        A.grad[k] = net->grads + param_offset(k);
+        A.S[k] = wg_ctas(net, k);
+        A.n[k] = 27 * kCin[k] * kCout[k];
+        A.block0[k] = blocks;
+        blocks += A.n[k] / 32;
+    }
+    PG_LAUNCH(KK_UNET_WGRAD, net->stream, k_wgrad_sum<<<blocks, 256, 0, net->stream>>>(A));
+    PG_CHECK_LAUNCH();
+    return PG_OK;
 }
 
 int prep_weights(pg_unet* net) {
-    if (!net->wdirty) return PG_OK;
+    if (tc_enabled() ? !net->wdirty : !net->wdirty_mma) return PG_OK;
+    if (tc_enabled()) {
+        tc::PrepArgs A = {};
+        int most = 0;
+        for (int k = 0; k < kL; ++k) {
+            A.cin[k] = kCin[k];
+            A.cout[k] = kCout[k];
+            A.W[2 * k] = A.W[2 * k + 1] = net->params + param_offset(k);
+            A.wtc[2 * k] = net->tcf[k];
+            A.wtc[2 * k + 1] = k ? net->tct[k] : nullptr;
+            most = std::max(most, 27 * kCin[k] * kCout[k]);
+        }
+        PG_LAUNCH(KK_UNET_MISC, net->stream,
+                  tc::k_wprep_tc<<<dim3(ceil_div(most, 1024), 2 * kL), 256, 0, net->stream>>>(A));
+        PG_CHECK_LAUNCH();
+        net->wdirty = false;
+        return PG_OK;
+    }
     for (int k = 0; k < kL; ++k) {
         const int n = 27 * kCin[k] * kCout[k] / 2;  // both layouts: 2 x (27 * cin/16 * cout/8 * 32)
         PG_LAUNCH(KK_UNET_MISC, net->stream,
                   k_wprep<<<ceil_div(n, 256), 256, 0, net->stream>>>(net->params + param_offset(k), kCin[k], kCout[k],
                                                                       net->wf[k], k ? net->wt[k] : nullptr));
-        const int nt = 27 * kCin[k] * kCout[k];
-        PG_LAUNCH(KK_UNET_MISC, net->stream,
-                  tc::k_wprep_tc<<<ceil_div(nt, 256), 256, 0, net->stream>>>(net->params + param_offset(k), kCin[k],
-                                                                              kCout[k], 0, net->tcf[k]));
-        if (k)
-            PG_LAUNCH(KK_UNET_MISC, net->stream,
-                      tc::k_wprep_tc<<<ceil_div(nt, 256), 256, 0, net->stream>>>(net->params + param_offset(k), kCin[k],
-                                                                                  kCout[k], 1, net->tct[k]));
     }
     PG_CHECK_LAUNCH();
-    net->wdirty = false;
+    net->wdirty_mma = false;
     return PG_OK;
 }
 
@@ -1382,13 +1477,13 @@ int check_grid(const pg_unet* net, const pg_grid* g) {
     return PG_OK;
 }
 
-// Normalise b, run the encoder/decoder; Y[9] holds the last features.
-// train: a backward pass follows, which reads the concatenations C0 and C1;
-// otherwise the convolutions read their two inputs where they are (k_upcat
-// took 99 us at 128^3, more than it saves them).
-int forward(pg_unet* net, const pg_grid* g, const float* b, double dt, bool train = false) {
+// Normalise b, run the encoder/decoder; Y[9] holds the last features.  The
+// decoder's convolutions and weight gradients read their two inputs where
+// they are; only the mma.sync convolutions need them written side by side
+// (k_upcat: 99 us at 128^3).
+int forward(pg_unet* net, const pg_grid* g, const float* b, double dt) {
     int rc;
-    const bool cat = train || !tc_enabled();
+    const bool cat = !tc_enabled();
     if ((rc = prep_weights(net))) return rc;
     const i64 V0 = net->lv[0];
     cudaStream_t s = net->stream;
@@ -1400,9 +1495,9 @@ int forward(pg_unet* net, const pg_grid* g, const float* b, double dt, bool trai
         return conv(net, kLevel[k], kCin[k], kCout[k], in, net->wf[k], net->tcf[k], net->Y[k], nullptr, EPI_RELU);
     };
     if ((rc = C(0, net->X0)) || (rc = C(1, net->Y[0]))) return rc;
-    PG_LAUNCH(KK_UNET_MISC, s, k_pool<<<blocks_for(net, net->lv[1] * 16), 256, 0, s>>>(net->Y[1], 16, net->ld[0], net->lh[0], net->lw[0], net->P0));
+    PG_LAUNCH(KK_UNET_MISC, s, k_pool<<<plane_grid((i64)net->lh[1] * net->lw[1] * 2, net->ld[1]), 256, 0, s>>>(net->Y[1], 16, net->ld[0], net->lh[0], net->lw[0], fast_div(2), fast_div(net->lw[1]), net->P0));
     if ((rc = C(2, net->P0)) || (rc = C(3, net->Y[2]))) return rc;
-    PG_LAUNCH(KK_UNET_MISC, s, k_pool<<<blocks_for(net, net->lv[2] * 32), 256, 0, s>>>(net->Y[3], 32, net->ld[1], net->lh[1], net->lw[1], net->P1));
+    PG_LAUNCH(KK_UNET_MISC, s, k_pool<<<plane_grid((i64)net->lh[2] * net->lw[2] * 4, net->ld[2]), 256, 0, s>>>(net->Y[3], 32, net->ld[1], net->lh[1], net->lw[1], fast_div(4), fast_div(net->lw[2]), net->P1));
     if ((rc = C(4, net->P1)) || (rc = C(5, net->Y[4]))) return rc;
     if (cat) {
         PG_LAUNCH(KK_UNET_MISC, s, k_upcat<<<blocks_for(net, net->lv[1] * 12), 256, 0, s>>>(net->Y[5], 64, net->Y[3], 32, net->ld[1], net->lh[1], net->lw[1], net->C1));
@@ -1432,28 +1527,28 @@ int backward(pg_unet* net) {
     };
     // level 0 decoder: dZ9 = G0a (from k_head)
     if ((rc = wgrad(net, 9, net->Y[8], net->G0a)) || (rc = BD(9, net->G0a, net->G0b, net->Y[8], EPI_GATE))) return rc;
-    if ((rc = wgrad(net, 8, net->C0, net->G0b)) || (rc = BD(8, net->G0b, net->dC0, nullptr, EPI_NONE))) return rc;
-    PG_LAUNCH(KK_UNET_MISC, s, k_upback_gate<<<blocks_for(net, net->lv[1] * 32), 256, 0, s>>>(net->dC0, 48, 32, net->Y[7], d0, h0, w0, net->G1a));
+    if ((rc = wgrad(net, 8, net->Y[1], net->G0b, net->Y[7])) || (rc = BD(8, net->G0b, net->dC0, nullptr, EPI_NONE))) return rc;
+    PG_LAUNCH(KK_UNET_MISC, s, k_upback_gate<<<plane_grid((i64)h1 * w1 * 4, d1), 256, 0, s>>>(net->dC0, 48, 32, net->Y[7], d0, h0, w0, fast_div(4), fast_div(w1), net->G1a));
     // level 1 decoder
     if ((rc = wgrad(net, 7, net->Y[6], net->G1a)) || (rc = BD(7, net->G1a, net->G1b, net->Y[6], EPI_GATE))) return rc;
-    if ((rc = wgrad(net, 6, net->C1, net->G1b)) || (rc = BD(6, net->G1b, net->dC1, nullptr, EPI_NONE))) return rc;
-    PG_LAUNCH(KK_UNET_MISC, s, k_upback_gate<<<blocks_for(net, net->lv[2] * 64), 256, 0, s>>>(net->dC1, 96, 64, net->Y[5], d1, h1, w1, net->G2a));
+    if ((rc = wgrad(net, 6, net->Y[3], net->G1b, net->Y[5])) || (rc = BD(6, net->G1b, net->dC1, nullptr, EPI_NONE))) return rc;
+    PG_LAUNCH(KK_UNET_MISC, s, k_upback_gate<<<plane_grid((i64)net->lh[2] * net->lw[2] * 8, net->ld[2]), 256, 0, s>>>(net->dC1, 96, 64, net->Y[5], d1, h1, w1, fast_div(8), fast_div(net->lw[2]), net->G2a));
     // level 2
     if ((rc = wgrad(net, 5, net->Y[4], net->G2a)) || (rc = BD(5, net->G2a, net->G2b, net->Y[4], EPI_GATE))) return rc;
     if ((rc = wgrad(net, 4, net->P1, net->G2b)) || (rc = BD(4, net->G2b, net->dP1, nullptr, EPI_NONE))) return rc;
-    PG_LAUNCH(KK_UNET_MISC, s, k_poolback_gate<<<blocks_for(net, net->lv[1] * 32), 256, 0, s>>>(net->dC1, 96, 64, net->dP1, 32, net->Y[3], d1, h1, w1, net->G1a));
+    PG_LAUNCH(KK_UNET_MISC, s, k_poolback_gate<<<plane_grid((i64)h1 * w1 * 4, d1), 256, 0, s>>>(net->dC1, 96, 64, net->dP1, 32, net->Y[3], d1, h1, w1, fast_div(4), fast_div(w1), net->G1a));
     // level 1 encoder
     if ((rc = wgrad(net, 3, net->Y[2], net->G1a)) || (rc = BD(3, net->G1a, net->G1b, net->Y[2], EPI_GATE))) return rc;
     if ((rc = wgrad(net, 2, net->P0, net->G1b)) || (rc = BD(2, net->G1b, net->dP0, nullptr, EPI_NONE))) return rc;
-    PG_LAUNCH(KK_UNET_MISC, s, k_poolback_gate<<<blocks_for(net, net->lv[0] * 16), 256, 0, s>>>(net->dC0, 48, 32, net->dP0, 16, net->Y[1], d0, h0, w0, net->G0a));
+    PG_LAUNCH(KK_UNET_MISC, s, k_poolback_gate<<<plane_grid((i64)h0 * w0 * 2, d0), 256, 0, s>>>(net->dC0, 48, 32, net->dP0, 16, net->Y[1], d0, h0, w0, fast_div(2), fast_div(w0), net->G0a));
     // level 0 encoder
     if ((rc = wgrad(net, 1, net->Y[0], net->G0a)) || (rc = BD(1, net->G0a, net->G0b, net->Y[0], EPI_GATE))) return rc;
-    if ((rc = wgrad(net, 0, net->X0, net->G0b))) return rc;
+    if ((rc = wgrad(net, 0, net->X0, net->G0b)) || (rc = wgrad_sums(net))) return rc;
     PG_CHECK_LAUNCH();
     return PG_OK;
 }
 
-constexpr int kHeadBlocks = 256;
+constexpr int kHeadBlocks = 608;  // (training: its FP64 sums are the bound, so every SM gets as many)
 
 // out = A in on the network's stream (A = dt * the grid's masked Laplacian).
 int apply_a(pg_unet* net, const pg_grid* g, float* out, const float* in, double dt) {
@@ -1470,18 +1565,19 @@ int head(pg_unet* net, const pg_grid* g, double dt, float* p_out, const float* p
     const float c2 = 2.0f / (float)V0;
     cudaStream_t s = net->stream;
     const int nb = (int)std::min<i64>(kHeadBlocks, std::max<i64>(1, (V0 + kHeadThreads - 1) / kHeadThreads));
+    const int nw = blocks_for(net, V0, kHeadThreads);  // without sums
     const float* wh = net->params + param_offset(kL);
     const float* ae = nullptr;
     if (p_true && net->loss_kind == 1) {
         // e = q - t, then A1 e (dt = 1) into the scratch ad
-        PG_LAUNCH(KK_UNET_MISC, s, k_head<<<nb, kHeadThreads, 0, s>>>(net->Y[9], g->flags, wh, net->scal, V0, (float)dt, nullptr, p_true, net->r, nullptr, c2, net->G0a, net->red));
+        PG_LAUNCH(KK_UNET_MISC, s, k_head<<<nw, kHeadThreads, 0, s>>>(net->Y[9], g->flags, wh, net->scal, V0, (float)dt, nullptr, p_true, net->r, nullptr, c2, net->G0a, net->red));
         int rc;
         if ((rc = apply_a(net, g, net->ad, net->r, 1.0))) return rc;
         ae = net->ad;
     }
-    PG_LAUNCH(KK_UNET_MISC, s, k_head<<<nb, kHeadThreads, 0, s>>>(net->Y[9], g->flags, wh, net->scal, V0, (float)dt, p_out, p_true, nullptr, ae, c2, net->G0a, net->red));
+    PG_LAUNCH(KK_UNET_MISC, s, k_head<<<p_true ? nb : nw, kHeadThreads, 0, s>>>(net->Y[9], g->flags, wh, net->scal, V0, (float)dt, p_out, p_true, nullptr, ae, c2, net->G0a, net->red));
     if (p_true)
-        PG_LAUNCH(KK_UNET_MISC, s, k_head_sum<<<1, 32, 0, s>>>(net->red, nb, V0, net->grads + param_offset(kL), net->loss));
+        PG_LAUNCH(KK_UNET_MISC, s, k_head_sum<<<1, 17 * 32, 0, s>>>(net->red, nb, V0, net->grads + param_offset(kL), net->loss));
     PG_CHECK_LAUNCH();
     return PG_OK;
 }
@@ -1651,9 +1747,7 @@ int pg_unet_create(int64_t d, int64_t h, int64_t w, pg_unet** out) {
     add((void**)&net->scal, 32);
     add((void**)&net->red, 8 * std::max(kRedBlocks, kHeadBlocks * 17));
     add((void**)&net->loss, 8);
-    size_t wp = 0;
-    for (int k = 0; k < kL; ++k) wp = std::max(wp, (size_t)wg_ctas(net, k) * 27 * kCin[k] * kCout[k]);
-    add((void**)&net->wpart, 4 * wp);
+    for (int k = 0; k < kL; ++k) add((void**)&net->wpart[k], 4 * (size_t)wg_ctas(net, k) * 27 * kCin[k] * kCout[k]);
     size_t total = 0;
     for (auto& p : parts) total += p.second;
     cudaError_t e = cudaMalloc(&net->arena, total);
@@ -1696,7 +1790,7 @@ int pg_unet_set_params(pg_unet* net, const float* host, double out_scale) {
     PG_CUDA(cudaStreamSynchronize(net->stream));
     net->out_scale = out_scale;
     net->adam_t = 0;
-    net->wdirty = true;
+    net->wdirty = net->wdirty_mma = true;
     return PG_OK;
 }
 
@@ -1729,7 +1823,7 @@ int pg_unet_accumulate_f32(pg_unet* net, const pg_grid* g, const float* b, const
     if (!(dt > 0.0)) return bad_arg("pg_unet_accumulate_f32: dt must be > 0");
     int rc;
     if ((rc = check_grid(net, g))) return rc;
-    if ((rc = forward(net, g, b, dt, true)) || (rc = head(net, g, dt, nullptr, p_true)) || (rc = backward(net))) return rc;
+    if ((rc = forward(net, g, b, dt)) || (rc = head(net, g, dt, nullptr, p_true)) || (rc = backward(net))) return rc;
     if (loss) {
         PG_CUDA(cudaMemcpyAsync(loss, net->loss, sizeof(double), cudaMemcpyDeviceToHost, net->stream));
         PG_CUDA(cudaStreamSynchronize(net->stream));
@@ -1756,7 +1850,7 @@ int pg_unet_adam_step(pg_unet* net, const pg_adam_params* a) {
                                                                   (float)a->eps, (float)a->grad_scale, (float)c1,
                                                                   (float)c2));
     PG_CHECK_LAUNCH();
-    net->wdirty = true;
+    net->wdirty = net->wdirty_mma = true;
     return PG_OK;
 }
 
