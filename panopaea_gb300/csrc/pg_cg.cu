@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(kCgThreads)
     __shared__ double sm[kCgThreads + 32];
     // Ping-pong by the device-side iteration count: iteration k reads
     // p[k & 1] and writes p[(k + 1) & 1] (so a CUDA graph can replay it).
+    grid_dep();
     const CgHead H(st);
     if (H.done) return;
     const i64 k = H.iter;
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(kTX * kTY)
                 int tiles_y, int zc, int nwork) {
     __shared__ T S[kTY + 2][kTX + 2];
     __shared__ double sm[kTX * kTY];
+    grid_dep();
     const CgHead H(st);
     if (H.done) return;
     const i64 kit = H.iter;
@@ -331,10 +333,10 @@ static void spmv_launch(cudaStream_t s, int num_sms, const T* r, const T* zb, T*
         const int zc = (int)std::max<i64>(4, (D.d + want_chunks - 1) / want_chunks);
         const int nwork = tiles_x * tiles_y * (int)((D.d + zc - 1) / zc);
         const int nb = std::max(1, std::min(nwork, cap));
-        k_cg_spmv3t<T, PM><<<nb, kTX * kTY, 0, s>>>(r, zb, p0, p1, ap, flags, D, dt, st, partials, tiles_x, tiles_y,
-                                                    zc, nwork);
+        launch_dep(D.nc(), k_cg_spmv3t<T, PM>, nb, kTX * kTY, 0, s, r, zb, p0, p1, ap, flags, D, dt, st, partials, tiles_x, tiles_y, zc,
+                   nwork);
     } else {
-        k_cg_spmv<T, 2, PM><<<nb_flat, kCgThreads, 0, s>>>(r, zb, p0, p1, ap, flags, D, dt, st, partials);
+        launch_dep(D.nc(), k_cg_spmv<T, 2, PM>, nb_flat, kCgThreads, 0, s, r, zb, p0, p1, ap, flags, D, dt, st, partials);
     }
 }
 
@@ -345,6 +347,7 @@ __global__ void __launch_bounds__(kCgThreads)
     __shared__ double sm[kCgThreads + 32];
     // The SpMV of this iteration wrote p[(iter + 1) & 1]; the last block
     // increments iter only after every block has read it here.
+    grid_dep();
     const CgHead H(st);
     if (H.done) return;
     const i64 k = H.iter;
@@ -420,6 +423,7 @@ __global__ void __launch_bounds__(kCgThreads)
                  const float4* __restrict__ ap, i64 n4, CgState* st, double* partials, float4* __restrict__ xl,
                  const float4* __restrict__ b0) {
     __shared__ double sm[kCgThreads + 32];
+    grid_dep();
     const CgHead H(st);
     if (H.done) return;
     const i64 k = H.iter;
@@ -503,6 +507,7 @@ __global__ void __launch_bounds__(kCgThreads)
                   const float4* __restrict__ ap, const uchar4* __restrict__ flags, i64 n4, float dt, CgState* st,
                   double* partials) {
     __shared__ double sm[kCgThreads + 32];
+    grid_dep();
     const CgHead H(st);
     if (H.done) return;
     __shared__ float inv_diag[8];  // Jacobi: 1 / (n dt) for n open faces (0 for n = 0), as zof computes it
@@ -643,11 +648,10 @@ static void update_launch(cudaStream_t s, int nb, T* x, T* r, const T* p0, const
     const bool vec4 = sizeof(T) == 4 && n % 4 == 0 && aligned16(x) && aligned16(r) && aligned16(p0) &&
                       aligned16(p1) && aligned16(ap) && aligned16(flags);
     if (vec4)
-        k_cg_update4r<PM><<<vec4_blocks(nb, n), kCgThreads, 0, s>>>((float4*)x, (float4*)r, (const float4*)p0, (const float4*)p1,
-                                                    (const float4*)ap, (const uchar4*)flags, n / 4, (float)dt, st,
-                                                    partials);
+        launch_dep(n, k_cg_update4r<PM>, vec4_blocks(nb, n), kCgThreads, 0, s, (float4*)x, (float4*)r, (const float4*)p0,
+                   (const float4*)p1, (const float4*)ap, (const uchar4*)flags, n / 4, (float)dt, st, partials);
     else
-        k_cg_update<T, PM><<<nb, kCgThreads, 0, s>>>(x, r, p0, p1, ap, flags, n, dt, st, partials);
+        launch_dep(n, k_cg_update<T, PM>, nb, kCgThreads, 0, s, x, r, p0, p1, ap, flags, n, dt, st, partials);
 }
 
 template <class T, int PM>
@@ -663,24 +667,24 @@ static void launch_iter(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook
                       aligned16(buf.p[0]) && aligned16(buf.p[1]) && aligned16(buf.ap) && aligned16(g->flags);
     if (PM == PM_ZBUF && vec4 && buf.xl)
         PG_LAUNCH(KK_CG_UPDATE, s,
-                  k_cg_update4<true><<<nb4, kCgThreads, 0, s>>>(
+                  launch_dep(n, k_cg_update4<true>, nb4, kCgThreads, 0, s,
                       (float4*)buf.x, (float4*)buf.r, (const float4*)buf.p[0], (const float4*)buf.p[1],
                       (const float4*)buf.ap, n / 4, g->ws.state, g->ws.partials, (float4*)buf.xl,
                       cg_fold(buf, hook) ? (const float4*)buf.b : nullptr));
     else if (PM == PM_ZBUF && vec4)
         PG_LAUNCH(KK_CG_UPDATE, s,
-                  k_cg_update4<false><<<nb4, kCgThreads, 0, s>>>((float4*)buf.x, (float4*)buf.r,
+                  launch_dep(n, k_cg_update4<false>, nb4, kCgThreads, 0, s, (float4*)buf.x, (float4*)buf.r,
                                                                 (const float4*)buf.p[0], (const float4*)buf.p[1],
                                                                 (const float4*)buf.ap, n / 4, g->ws.state,
-                                                                g->ws.partials, nullptr, nullptr));
+                                                                g->ws.partials, (float4*)nullptr, (const float4*)nullptr));
     else if (PM != PM_ZBUF)
         PG_LAUNCH(KK_CG_UPDATE, s,
                   update_launch<T, PM>(s, nb, buf.x, buf.r, buf.p[0], buf.p[1], buf.ap, g->flags, n, dt, g->ws.state,
                                        g->ws.partials));
     else
         PG_LAUNCH(KK_CG_UPDATE, s,
-                  k_cg_update<T, PM><<<nb, kCgThreads, 0, s>>>(buf.x, buf.r, buf.p[0], buf.p[1], buf.ap, g->flags, n,
-                                                               dt, g->ws.state, g->ws.partials));
+                  launch_dep(n, k_cg_update<T, PM>, nb, kCgThreads, 0, s, buf.x, buf.r, buf.p[0], buf.p[1], buf.ap, g->flags, n,
+                             dt, g->ws.state, g->ws.partials));
     if (PM == PM_ZBUF) hook->apply(g, buf.r, buf.z);
 }
 
@@ -690,6 +694,7 @@ static void launch_iter(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook
 // one-thread kernel that clears the condition once the device-side stop
 // test has fired.  No host round trip and no launch past convergence.
 __global__ void k_cg_cond(const CgState* st, cudaGraphConditionalHandle h) {
+    grid_dep();
     cudaGraphSetConditional(h, st->done ? 0u : 1u);
 }
 
@@ -757,7 +762,7 @@ static int get_graph(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook* h
     cudaError_t err = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (err == cudaSuccess) {
         launch_iter<T, PM>(g, buf, dt, nb, hook);
-        k_cg_cond<<<1, 1, 0, cs>>>(g->ws.state, h);
+        launch_dep(g->dims.nc(), k_cg_cond, 1, 1, 0, cs, (const CgState*)g->ws.state, h);
         cudaGraph_t captured = nullptr;
         err = cudaStreamEndCapture(cs, &captured);
     }

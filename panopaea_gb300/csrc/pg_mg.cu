@@ -172,6 +172,7 @@ template <bool L0, int MODE, bool RZ>
 __global__ void __launch_bounds__(kMgThreads)
     k_mg_smooth(LV v, float* __restrict__ e, const float* __restrict__ f, const float* __restrict__ ec, int cw, int ch,
                 int color, CgState* st, double* partials, FastDiv fhalf, FastDiv fh) {
+    grid_dep();
     if (st->done) return;
     __shared__ double sm[RZ ? 2 * kMgThreads : 1];
     const int hw = v.h * v.w;
@@ -349,7 +350,6 @@ __global__ void __launch_bounds__(kPThreads, kPMinBlocks)
               CgState* st, double* partials) {
     typedef PairCfg<M1> Cfg;
     constexpr int kStages = Cfg::kStages, kStageBytes = Cfg::kStageBytes;
-    if (st->done) return;
     extern __shared__ unsigned char pair_smem_raw[];
     __shared__ float inv_tab[8];  // 1 / (n dt) for n open faces (0 for n = 0), as Cell<true>
     // 128-byte aligned by an offset (pointer arithmetic keeps every access
@@ -368,6 +368,8 @@ __global__ void __launch_bounds__(kPThreads, kPMinBlocks)
         tma_prefetch_map(&gmap);
     }
     if (tid < 8) inv_tab[tid] = tid ? __frcp_rn((float)tid * dt) : 0.f;
+    grid_dep();
+    if (st->done) return;
     __syncthreads();
     const int h = a.h, w = a.w, d = a.d;
     const int per_plane = a.tiles_x * a.tiles_y;
@@ -566,7 +568,6 @@ struct RestrictArgs {
 __global__ void __launch_bounds__(kQThreads)
     k_mg_restrict3p(const __grid_constant__ CUtensorMap emap, const __grid_constant__ CUtensorMap fmap,
                     const __grid_constant__ CUtensorMap gmap, RestrictArgs a, CgState* st) {
-    if (st->done) return;
     extern __shared__ unsigned char rs_smem_raw[];
     unsigned char* const base = rs_smem_raw + ((128u - (smem_u32(rs_smem_raw) & 127u)) & 127u);
     uint64_t* const bars = (uint64_t*)(base + kQBarOff);
@@ -578,6 +579,8 @@ __global__ void __launch_bounds__(kQThreads)
         tma_prefetch_map(&fmap);
         tma_prefetch_map(&gmap);
     }
+    grid_dep();
+    if (st->done) return;
     __syncthreads();
     const float dt = a.dt;
     const int d = a.d;
@@ -719,6 +722,7 @@ template <bool L0>
 __global__ void __launch_bounds__(kMgThreads)
     k_mg_restrict(LV v, const float* __restrict__ e, const float* __restrict__ f, float* __restrict__ fc, int cd,
                   int ch, int cw, CgState* st, FastDiv fcw, FastDiv fch) {
+    grid_dep();
     if (st->done) return;
     const int nc = cd * ch * cw;
     for (int C = blockIdx.x * blockDim.x + threadIdx.x; C < nc; C += gridDim.x * blockDim.x) {
@@ -742,6 +746,7 @@ template <bool L0>
 __global__ void __launch_bounds__(kMgThreads)
     k_mg_restrict8(LV v, const float* __restrict__ e, const float* __restrict__ f, float* __restrict__ fc, int cd,
                    int ch, int cw, CgState* st, FastDiv fcw, FastDiv fch) {
+    grid_dep();
     if (st->done) return;
     const int nc = cd * ch * cw;
     const unsigned lane = threadIdx.x & 31, grp = lane & ~7u;
@@ -1237,7 +1242,23 @@ __device__ __forceinline__ void ct_load(const CtArgs& A, int l, int rank, CtPair
                 C.zh = b.y;
                 C.inv = b.z;
             }
-            if (l == A.lt) C.f = A.f_in[g];
+        }
+    }
+}
+// f of the first level, from global memory.
+__device__ __forceinline__ void ct_load_first(const CtArgs& A, int rank, CtPairs& P) {
+    const CtLevel& L = A.L[A.lt];
+    const int z0 = ct_z0(L, rank, A.lt < A.ls);
+#pragma unroll
+    for (int j = 0; j < kCtPairs; ++j) {
+        if (!P.ib[j]) continue;
+        int zl, y, k;
+        ct_pos(L, P.ib[j] - L.ps, zl, y, k);
+        const int g0 = ((z0 + zl) * L.h + y) * L.w + 2 * k;
+#pragma unroll
+        for (int col = 0; col < 2; ++col) {
+            const int u = P.s[j] ^ col;
+            if (2 * k + u < L.w) P.c[j][col].f = A.f_in[g0 + u];
         }
     }
 }
@@ -1385,7 +1406,6 @@ __device__ __forceinline__ void ct_sum(const CtTeam& T, const CtArgs& A, int l, 
 }
 
 __global__ void __launch_bounds__(kCtThreads) k_mg_ctail(const __grid_constant__ CtArgs A, CgState* st) {
-    if (st->done) return;  // the same value in every block of the cluster
     extern __shared__ float csm[];
     __shared__ double sums[kCtMaxRanks][2];
     CtTeam T;
@@ -1395,8 +1415,13 @@ __global__ void __launch_bounds__(kCtThreads) k_mg_ctail(const __grid_constant__
     T.hi = ct_addr(csm, (unsigned)min(T.rank + 1, A.ranks - 1));
     const int lt = A.lt, ls = A.ls, nl = A.nl, ns = A.nsmooth;
     CtPairs P;
+    // the first level's weights (no kernel of the solve writes them) before the
+    // wait for the kernels ahead
     ct_load(A, lt, T.rank, P);
     for (int i = threadIdx.x; i < A.zero4; i += kCtThreads) ((float4*)csm)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    grid_dep();
+    if (st->done) return;  // the same value in every block of the cluster
+    ct_load_first(A, T.rank, P);
     ct_sync();  // every block runs and has zeroed its e: remote stores from here on
     // the first level's red cells: e = f / diag
 #pragma unroll
@@ -1449,7 +1474,10 @@ __global__ void __launch_bounds__(kCtThreads) k_mg_ctail(const __grid_constant__
             const CtLevel& Lc = A.L[l + 1];
             const int z0 = ct_z0(L, T.rank, dist), nz = ct_nz(L, T.rank, dist);
             const bool last = l + 1 == ls;  // the last distributed level
-            if (t > 0) ct_load(A, l, T.rank, P);
+            if (t > 0) {
+                ct_load(A, l, T.rank, P);
+                if (l == lt) ct_load_first(A, T.rank, P);
+            }
             // what the level reads is complete: its first red cells, the
             // restriction into it, or rank 0's part of the correction below
             if (dist && (!up || last)) ct_sync();
@@ -1937,8 +1965,8 @@ static void pair_t(pg_grid* g, const MgHierarchy& H, const CUtensorMap* em, cons
     cudaStream_t s = g->stream;
     const int nb = M1 == PR_PROLONG ? P.nb_prolong : P.nb_plain;
     PG_LAUNCH(KK_MG_PAIR, s,
-              k_mg_pair<M1, RZ><<<nb, kPThreads, PairCfg<M1>::kSmem, s>>>(*em, *P.fm, H.gmap, H.cmap, a,
-                                                                          g->ws.state, g->ws.partials));
+              launch_dep(g->dims.nc(), k_mg_pair<M1, RZ>, nb, kPThreads, PairCfg<M1>::kSmem, s, *em, *P.fm, H.gmap, H.cmap, a, g->ws.state,
+                         g->ws.partials));
 }
 
 // One fused pair: first half-sweep over colour c1 in `mode` from ein
@@ -1977,7 +2005,7 @@ static bool restrict_tma(pg_grid* g, const MgHierarchy& H, const float* e, const
     a.tiles_y = (a.h + kQY - 1) / kQY;
     const int nb = zwalk_blocks(a.tiles_x * a.tiles_y, a.d / 2, restrict_cap(g));
     cudaStream_t s = g->stream;
-    PG_LAUNCH(KK_MG_RESTRICT, s, k_mg_restrict3p<<<nb, kQThreads, kQSmem, s>>>(*em, *fm, H.rgmap, a, g->ws.state));
+    PG_LAUNCH(KK_MG_RESTRICT, s, launch_dep(g->dims.nc(), k_mg_restrict3p, nb, kQThreads, kQSmem, s, *em, *fm, H.rgmap, a, g->ws.state));
     return true;
 }
 
@@ -2154,8 +2182,11 @@ static int launch_ctail(pg_grid* g, const MgHierarchy& H, int nsmooth, float* e,
     A.e_out = e;
     A.f_in = f;
     A.cinv = H.cinv;
-    cudaLaunchAttribute at[1];
-    const cudaLaunchConfig_t cfg = ctail_config(H.ct_ranks, H.ct_smem, g->stream, at);
+    cudaLaunchAttribute at[2] = {};
+    cudaLaunchConfig_t cfg = ctail_config(H.ct_ranks, H.ct_smem, g->stream, at);
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = g->dims.nc() <= kDepCells ? 2 : 1;
     cudaError_t err = cudaSuccess;
     PG_LAUNCH(KK_MG_COARSE, g->stream, err = cudaLaunchKernelEx(&cfg, k_mg_ctail, A, g->ws.state));
     if (err != cudaSuccess) return cuda_fail(err, "cluster tail launch");
@@ -2174,9 +2205,8 @@ static void smooth(pg_grid* g, const MgHierarchy& H, int l, float* e, const floa
     }
     cudaStream_t s = g->stream;
     PG_LAUNCH(l == 0 ? KK_MG_SMOOTH : KK_MG_SMOOTH_C, s,
-              k_mg_smooth<L0, MODE, RZ><<<blocks_for(g, n), kMgThreads, 0, s>>>(
-                  v, e, f, ec, cw, ch, color, g->ws.state, g->ws.partials, fast_div((unsigned)((v.w + 1) >> 1)),
-                  fast_div((unsigned)v.h)));
+              launch_dep(g->dims.nc(), k_mg_smooth<L0, MODE, RZ>, blocks_for(g, n), kMgThreads, 0, s, v, e, f, ec, cw, ch, color,
+                         g->ws.state, g->ws.partials, fast_div((unsigned)((v.w + 1) >> 1)), fast_div((unsigned)v.h)));
 }
 
 template <bool L0>
@@ -2272,14 +2302,14 @@ static int vcycle(pg_grid* g, const MgHierarchy& H, const float* r, float* z, in
             cudaStream_t ss = s;
             if (nc <= kRestrictPerChild) {
                 if (l == 0)
-                    PG_LAUNCH(kind, ss, k_mg_restrict8<true><<<blocks_for(g, 8 * nc), kMgThreads, 0, ss>>>(v, e, f, C.f, cd, ch, cw, g->ws.state, fcw, fch));
+                    PG_LAUNCH(kind, ss, launch_dep(g->dims.nc(), k_mg_restrict8<true>, blocks_for(g, 8 * nc), kMgThreads, 0, ss, v, e, f, C.f, cd, ch, cw, g->ws.state, fcw, fch));
                 else
-                    PG_LAUNCH(kind, ss, k_mg_restrict8<false><<<blocks_for(g, 8 * nc), kMgThreads, 0, ss>>>(v, e, f, C.f, cd, ch, cw, g->ws.state, fcw, fch));
+                    PG_LAUNCH(kind, ss, launch_dep(g->dims.nc(), k_mg_restrict8<false>, blocks_for(g, 8 * nc), kMgThreads, 0, ss, v, e, f, C.f, cd, ch, cw, g->ws.state, fcw, fch));
             } else {
                 if (l == 0)
-                    PG_LAUNCH(kind, ss, k_mg_restrict<true><<<blocks_for(g, nc), kMgThreads, 0, ss>>>(v, e, f, C.f, cd, ch, cw, g->ws.state, fcw, fch));
+                    PG_LAUNCH(kind, ss, launch_dep(g->dims.nc(), k_mg_restrict<true>, blocks_for(g, nc), kMgThreads, 0, ss, v, e, f, C.f, cd, ch, cw, g->ws.state, fcw, fch));
                 else
-                    PG_LAUNCH(kind, ss, k_mg_restrict<false><<<blocks_for(g, nc), kMgThreads, 0, ss>>>(v, e, f, C.f, cd, ch, cw, g->ws.state, fcw, fch));
+                    PG_LAUNCH(kind, ss, launch_dep(g->dims.nc(), k_mg_restrict<false>, blocks_for(g, nc), kMgThreads, 0, ss, v, e, f, C.f, cd, ch, cw, g->ws.state, fcw, fch));
             }
         }
     }

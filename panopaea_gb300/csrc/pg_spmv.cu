@@ -56,18 +56,11 @@ __global__ void __launch_bounds__(kSThreads, 2)
     k_cg_spmv3p(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUtensorMap pmap0,
                 const __grid_constant__ CUtensorMap pmap1, const __grid_constant__ CUtensorMap gmap, SpmvArgs a,
                 CgState* st, double* partials) {
-    const CgHead H(st);
-    if (H.done) return;
     extern __shared__ unsigned char spmv_smem_raw[];
     unsigned char* const base = spmv_smem_raw + ((128u - (smem_u32(spmv_smem_raw) & 127u)) & 127u);
     float(*const S)[kSSh][kSSw] = (float(*)[kSSh][kSSw])(base + kSStages * kSStageBytes);
     uint64_t* const bars = (uint64_t*)(base + kSBarOff);
     const int tid = threadIdx.x, lane = tid & 31, ty = tid >> 5;
-    const i64 kit = H.iter;
-    const CUtensorMap* pmap = (kit & 1) ? &pmap1 : &pmap0;  // p_old
-    float* const p_new = (kit & 1) ? a.p0 : a.p1;
-    const int first = H.first;
-    const float beta = first ? 0.f : (float)H.beta;
     // Jacobi: 1 / (n dt) for n open faces, computed as in zval (0 for n = 0)
     __shared__ float inv_diag[8];
     if (PM == PM_JACOBI && tid < 8) inv_diag[tid] = tid ? __frcp_rn((float)tid * a.dt) : 0.f;
@@ -75,9 +68,18 @@ __global__ void __launch_bounds__(kSThreads, 2)
         for (int s = 0; s < kSStages; ++s) mbar_init(&bars[s], 1);
         mbar_fence_init();
         tma_prefetch_map(&zmap);
-        tma_prefetch_map(pmap);
+        tma_prefetch_map(&pmap0);
+        tma_prefetch_map(&pmap1);
         tma_prefetch_map(&gmap);
     }
+    grid_dep();
+    const CgHead H(st);
+    if (H.done) return;
+    const i64 kit = H.iter;
+    const CUtensorMap* pmap = (kit & 1) ? &pmap1 : &pmap0;  // p_old
+    float* const p_new = (kit & 1) ? a.p0 : a.p1;
+    const int first = H.first;
+    const float beta = first ? 0.f : (float)H.beta;
     __syncthreads();
     const float dt = a.dt;
     const int h = a.h, w = a.w, d = a.d;
@@ -489,11 +491,11 @@ bool spmv_tma_launch(cudaStream_t s, int num_sms, int pm, const float* zb, float
     a.tiles_y = (a.h + kSY - 1) / kSY;
     const int nb = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, cap);
     if (pm == PM_ZBUF)
-        k_cg_spmv3p<PM_ZBUF><<<nb, kSThreads, kSSmem, s>>>(zm, pm0, pm1, gm, a, st, partials);
+        launch_dep(D.nc(), k_cg_spmv3p<PM_ZBUF>, nb, kSThreads, kSSmem, s, zm, pm0, pm1, gm, a, st, partials);
     else if (pm == PM_JACOBI)
-        k_cg_spmv3p<PM_JACOBI><<<nb, kSThreads, kSSmem, s>>>(zm, pm0, pm1, gm, a, st, partials);
+        launch_dep(D.nc(), k_cg_spmv3p<PM_JACOBI>, nb, kSThreads, kSSmem, s, zm, pm0, pm1, gm, a, st, partials);
     else
-        k_cg_spmv3p<PM_NONE><<<nb, kSThreads, kSSmem, s>>>(zm, pm0, pm1, gm, a, st, partials);
+        launch_dep(D.nc(), k_cg_spmv3p<PM_NONE>, nb, kSThreads, kSSmem, s, zm, pm0, pm1, gm, a, st, partials);
     return true;
 }
 
