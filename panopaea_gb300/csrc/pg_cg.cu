@@ -217,6 +217,12 @@ __global__ void __launch_bounds__(kCgThreads)
 // registers of the planes below and above.  Work items (tile, z chunk) are
 // handed out grid-stride, so the block count (and the reduction partials)
 // stays bounded for any grid size.  Same arithmetic as k_cg_spmv.
+//
+// Bound by latency: with 64 warps per SM a plane is about 1300 issue cycles, as
+// long as one trip to L2, so everything a plane needs is loaded a plane (the
+// cells themselves two planes) ahead and combined where it is used, and two
+// tiles in turn need one barrier per plane.  Loading the halo and the flags
+// where they are used took 56 us at 150 x 170 x 131.
 constexpr int kTX = 32, kTY = 8;
 
 template <class T, int PM>
@@ -224,7 +230,7 @@ __global__ void __launch_bounds__(kTX * kTY)
     k_cg_spmv3t(const T* __restrict__ r, const T* __restrict__ zb, T* p0, T* p1, T* __restrict__ ap,
                 const uint8_t* __restrict__ flags, Dims D, T dt, CgState* st, double* partials, int tiles_x,
                 int tiles_y, int zc, int nwork) {
-    __shared__ T S[kTY + 2][kTX + 2];
+    __shared__ T S2[2][kTY + 2][kTX + 2];
     __shared__ double sm[kTX * kTY];
     grid_dep();
     const CgHead H(st);
@@ -235,46 +241,63 @@ __global__ void __launch_bounds__(kTX * kTY)
     const int first = H.first;
     const T beta = first ? T(0) : (T)H.beta;
     const T zm = (PM == PM_ZBUF && H.nfluid > 0.0) ? (T)H.zmean : T(0);
-    auto pn = [&](i64 k) -> T {
-        const T z = zval<T, PM>(r, flags, zb, k, dt, zm);
-        return first ? z : z + beta * p_old[k];
+    // what p_new of a cell is made of, as loaded
+    struct Raw {
+        T z, p;
+        unsigned f;
+    };
+    auto load = [&](i64 k, bool ok, bool with_flags) {
+        Raw q{T(0), T(0), 0u};
+        if (ok) {
+            q.z = PM == PM_ZBUF ? zb[k] : r[k];
+            if (with_flags) q.f = flags[k];
+            if (!first) q.p = p_old[k];
+        }
+        return q;
+    };
+    auto pn = [&](const Raw& q) -> T {  // (z as zval)
+        T z = q.z;
+        if (PM == PM_JACOBI) {
+            const int n = __popc(q.f);
+            z = n ? z * rcp_rn<T>((T)n * dt) : T(0);
+        }
+        if (PM == PM_ZBUF && q.f) z -= zm;
+        return first ? z : z + beta * q.p;
     };
     const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;
     const int w = (int)D.w, h = (int)D.h, d = (int)D.d;
     const i64 hw = (i64)h * w;
     const int per_plane = tiles_x * tiles_y;
+    const int dx = tx == 0 ? -1 : 1, dy = ty == 0 ? -1 : 1;  // this thread's halo cells, if any
     Acc<T> acc;
+    int buf = 0;
     for (int item = blockIdx.x; item < nwork; item += gridDim.x) {
         const int tz = item / per_plane, t2 = item - tz * per_plane;
         const int x = (t2 % tiles_x) * kTX + tx, y = (t2 / tiles_x) * kTY + ty;
         const int z0 = tz * zc, z1 = min(z0 + zc, d);
         const bool inside = x < w && y < h;
+        const bool halo_x = inside && ((tx == 0 && x > 0) || (tx == kTX - 1 && x + 1 < w));
+        const bool halo_y = inside && ((ty == 0 && y > 0) || (ty == kTY - 1 && y + 1 < h));
         const i64 col = (i64)y * w + x;
-        T below = T(0), cur = T(0), above = T(0);
-        if (inside) {
-            if (z0 > 0) below = pn((i64)(z0 - 1) * hw + col);
-            cur = pn((i64)z0 * hw + col);
-            if (z0 + 1 < d) above = pn((i64)(z0 + 1) * hw + col);
-        }
-        for (int z = z0; z < z1; ++z) {
-            const i64 c = (i64)z * hw + col;
-            // Loads for plane z + 2 are issued here and combined only after
-            // this plane's stencil, so their latency overlaps the step.
-            T rz = T(0), rp = T(0);
-            if (inside && z + 2 < d && z + 1 < z1) {
-                rz = zval<T, PM>(r, flags, zb, c + 2 * hw, dt, zm);
-                if (!first) rp = p_old[c + 2 * hw];
-            }
+        i64 c = (i64)z0 * hw + col;
+        const Raw r0 = load(c - hw, inside && z0 > 0, true), r1 = load(c, inside, true);
+        Raw next = load(c + hw, inside && z0 + 1 < d, true);
+        Raw hx = load(c + dx, halo_x, PM != PM_NONE), hy = load(c + dy * (i64)w, halo_y, PM != PM_NONE);
+        T below = pn(r0), cur = pn(r1);
+        unsigned f = r1.f;
+        for (int z = z0; z < z1; ++z, c += hw, buf ^= 1) {
+            T(*const S)[kTX + 2] = S2[buf];
+            const bool more = z + 1 < z1;
+            const T above = pn(next);
+            const unsigned f_above = next.f;
             S[ty + 1][tx + 1] = cur;
-            if (inside) {
-                if (tx == 0 && x > 0) S[ty + 1][0] = pn(c - 1);
-                if (tx == kTX - 1 && x + 1 < w) S[ty + 1][kTX + 1] = pn(c + 1);
-                if (ty == 0 && y > 0) S[0][tx + 1] = pn(c - w);
-                if (ty == kTY - 1 && y + 1 < h) S[kTY + 1][tx + 1] = pn(c + w);
-            }
+            if (halo_x) S[ty + 1][tx + 1 + dx] = pn(hx);
+            if (halo_y) S[ty + 1 + dy][tx + 1] = pn(hy);
+            next = load(c + 2 * hw, inside && more && z + 2 < d, true);
+            hx = load(c + hw + dx, halo_x && more, PM != PM_NONE);
+            hy = load(c + hw + dy * (i64)w, halo_y && more, PM != PM_NONE);
             __syncthreads();
             if (inside) {
-                const uint8_t f = flags[c];
                 const T pc = cur;
                 const T gy_lo = (f & YLO) ? -sub_rn(pc, S[ty][tx + 1]) : T(0);
                 const T gy_hi = (f & YHI) ? -sub_rn(S[ty + 2][tx + 1], pc) : T(0);
@@ -289,10 +312,9 @@ __global__ void __launch_bounds__(kTX * kTY)
                 ap[c] = a;
                 acc.add(pc * a);
             }
-            __syncthreads();
             below = cur;
             cur = above;
-            above = first ? rz : rz + beta * rp;
+            f = f_above;
         }
     }
     const double s = block_sum<kTX * kTY>(acc.value(), sm);
