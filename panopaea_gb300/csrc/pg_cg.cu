@@ -362,16 +362,33 @@ static void spmv_launch(cudaStream_t s, int num_sms, const T* r, const T* zb, T*
     }
 }
 
+// The WHILE node that repeats an iteration (graph form; off outside of it):
+// the update kernel ends it, as it is where a solve ends, so that no kernel
+// has to be launched to look.  What another kernel ended (or the init), the
+// update finds at its start.
+struct LoopCond {
+    cudaGraphConditionalHandle h = 0;
+    int on = 0;
+    __device__ __forceinline__ void end() const {
+        if (on && threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
+    }
+    // at a kernel's start; done: nothing is left to do
+    __device__ __forceinline__ bool over(int done) const {
+        if (done && blockIdx.x == 0) end();
+        return done != 0;
+    }
+};
+
 template <class T, int PM>
 __global__ void __launch_bounds__(kCgThreads)
     k_cg_update(T* __restrict__ x, T* __restrict__ r, const T* p0, const T* p1, const T* __restrict__ ap,
-                const uint8_t* __restrict__ flags, i64 n, T dt, CgState* st, double* partials) {
+                const uint8_t* __restrict__ flags, i64 n, T dt, CgState* st, double* partials, LoopCond loop = {}) {
     __shared__ double sm[kCgThreads + 32];
     // The SpMV of this iteration wrote p[(iter + 1) & 1]; the last block
     // increments iter only after every block has read it here.
     grid_dep();
     const CgHead H(st);
-    if (H.done) return;
+    if (loop.over(H.done)) return;
     const i64 k = H.iter;
     const T* __restrict__ p = ((k + 1) & 1) ? p1 : p0;
     const T alpha = (T)H.alpha, nalpha = -alpha;
@@ -414,6 +431,7 @@ __global__ void __launch_bounds__(kCgThreads)
             else st->rsum = sigma_new;
             if (it >= st->max_iter) st->done = 1;          // loop bound, pcg.rs:48
         }
+        if (st->done) loop.end();
     }
 }
 
@@ -443,11 +461,11 @@ template <bool DFX>
 __global__ void __launch_bounds__(kCgThreads)
     k_cg_update4(float4* __restrict__ x, float4* __restrict__ r, const float4* p0, const float4* p1,
                  const float4* __restrict__ ap, i64 n4, CgState* st, double* partials, float4* __restrict__ xl,
-                 const float4* __restrict__ b0) {
+                 const float4* __restrict__ b0, LoopCond loop) {
     __shared__ double sm[kCgThreads + 32];
     grid_dep();
     const CgHead H(st);
-    if (H.done) return;
+    if (loop.over(H.done)) return;
     const i64 k = H.iter;
     const float4* __restrict__ p = ((k + 1) & 1) ? p1 : p0;
     const float alpha = (float)H.alpha, nalpha = -alpha;
@@ -515,6 +533,7 @@ __global__ void __launch_bounds__(kCgThreads)
         } else if (it >= st->max_iter) {  // loop bound, pcg.rs:48
             st->done = 1;
         }
+        if (st->done) loop.end();
     }
 }
 
@@ -527,11 +546,11 @@ template <int PM>
 __global__ void __launch_bounds__(kCgThreads)
     k_cg_update4r(float4* __restrict__ x, float4* __restrict__ r, const float4* p0, const float4* p1,
                   const float4* __restrict__ ap, const uchar4* __restrict__ flags, i64 n4, float dt, CgState* st,
-                  double* partials) {
+                  double* partials, LoopCond loop) {
     __shared__ double sm[kCgThreads + 32];
     grid_dep();
     const CgHead H(st);
-    if (H.done) return;
+    if (loop.over(H.done)) return;
     __shared__ float inv_diag[8];  // Jacobi: 1 / (n dt) for n open faces (0 for n = 0), as zof computes it
     if (PM == PM_JACOBI) {
         if (threadIdx.x < 8) inv_diag[threadIdx.x] = threadIdx.x ? __frcp_rn((float)threadIdx.x * dt) : 0.f;
@@ -606,6 +625,7 @@ __global__ void __launch_bounds__(kCgThreads)
             cg_finish_rz(st, sigma_new);            // pcg.rs:65-68
             if (it >= st->max_iter) st->done = 1;  // loop bound, pcg.rs:48
         }
+        if (st->done) loop.end();
     }
 }
 
@@ -666,18 +686,18 @@ static bool cg_tma_enabled() {
 // update here, so they compute the same iterates on the same buffers.
 template <class T, int PM>
 static void update_launch(cudaStream_t s, int nb, T* x, T* r, const T* p0, const T* p1, const T* ap,
-                          const uint8_t* flags, i64 n, T dt, CgState* st, double* partials) {
+                          const uint8_t* flags, i64 n, T dt, CgState* st, double* partials, LoopCond loop = {}) {
     const bool vec4 = sizeof(T) == 4 && n % 4 == 0 && aligned16(x) && aligned16(r) && aligned16(p0) &&
                       aligned16(p1) && aligned16(ap) && aligned16(flags);
     if (vec4)
         launch_dep(n, k_cg_update4r<PM>, vec4_blocks(nb, n), kCgThreads, 0, s, (float4*)x, (float4*)r, (const float4*)p0,
-                   (const float4*)p1, (const float4*)ap, (const uchar4*)flags, n / 4, (float)dt, st, partials);
+                   (const float4*)p1, (const float4*)ap, (const uchar4*)flags, n / 4, (float)dt, st, partials, loop);
     else
-        launch_dep(n, k_cg_update<T, PM>, nb, kCgThreads, 0, s, x, r, p0, p1, ap, flags, n, dt, st, partials);
+        launch_dep(n, k_cg_update<T, PM>, nb, kCgThreads, 0, s, x, r, p0, p1, ap, flags, n, dt, st, partials, loop);
 }
 
 template <class T, int PM>
-static void launch_iter(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook* hook) {
+static void launch_iter(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook* hook, LoopCond loop = {}) {
     const Dims& D = g->dims;
     cudaStream_t s = g->stream;
     PG_LAUNCH(KK_CG_SPMV, s,
@@ -692,34 +712,29 @@ static void launch_iter(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook
                   launch_dep(n, k_cg_update4<true>, nb4, kCgThreads, 0, s,
                       (float4*)buf.x, (float4*)buf.r, (const float4*)buf.p[0], (const float4*)buf.p[1],
                       (const float4*)buf.ap, n / 4, g->ws.state, g->ws.partials, (float4*)buf.xl,
-                      cg_fold(buf, hook) ? (const float4*)buf.b : nullptr));
+                      cg_fold(buf, hook) ? (const float4*)buf.b : nullptr, loop));
     else if (PM == PM_ZBUF && vec4)
         PG_LAUNCH(KK_CG_UPDATE, s,
                   launch_dep(n, k_cg_update4<false>, nb4, kCgThreads, 0, s, (float4*)buf.x, (float4*)buf.r,
                                                                 (const float4*)buf.p[0], (const float4*)buf.p[1],
                                                                 (const float4*)buf.ap, n / 4, g->ws.state,
-                                                                g->ws.partials, (float4*)nullptr, (const float4*)nullptr));
+                                                                g->ws.partials, (float4*)nullptr, (const float4*)nullptr, loop));
     else if (PM != PM_ZBUF)
         PG_LAUNCH(KK_CG_UPDATE, s,
                   update_launch<T, PM>(s, nb, buf.x, buf.r, buf.p[0], buf.p[1], buf.ap, g->flags, n, dt, g->ws.state,
-                                       g->ws.partials));
+                                       g->ws.partials, loop));
     else
         PG_LAUNCH(KK_CG_UPDATE, s,
                   launch_dep(n, k_cg_update<T, PM>, nb, kCgThreads, 0, s, buf.x, buf.r, buf.p[0], buf.p[1], buf.ap, g->flags, n,
-                             dt, g->ws.state, g->ws.partials));
+                             dt, g->ws.state, g->ws.partials, loop));
     if (PM == PM_ZBUF) hook->apply(g, buf.r, buf.z);
 }
 
 // ---------------------------------------------------------------------------
 // CUDA-graph form of the iteration loop: a WHILE conditional node whose body
-// is one iteration (SpMV, update, the outer preconditioner's kernels) and a
-// one-thread kernel that clears the condition once the device-side stop
-// test has fired.  No host round trip and no launch past convergence.
-__global__ void k_cg_cond(const CgState* st, cudaGraphConditionalHandle h) {
-    grid_dep();
-    cudaGraphSetConditional(h, st->done ? 0u : 1u);
-}
-
+// is one iteration (SpMV, update, the outer preconditioner's kernels); the
+// update clears the condition once the device-side stop test has fired.  No
+// host round trip and no launch past convergence.
 struct CgGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -783,12 +798,11 @@ static int get_graph(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook* h
     const int64_t before = prof_capture_begin();
     cudaError_t err = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (err == cudaSuccess) {
-        launch_iter<T, PM>(g, buf, dt, nb, hook);
-        launch_dep(g->dims.nc(), k_cg_cond, 1, 1, 0, cs, (const CgState*)g->ws.state, h);
+        launch_iter<T, PM>(g, buf, dt, nb, hook, LoopCond{h, 1});
         cudaGraph_t captured = nullptr;
         err = cudaStreamEndCapture(cs, &captured);
     }
-    E.body_kernels = (int)(prof_capture_end() - before) + 1;
+    E.body_kernels = (int)(prof_capture_end() - before);
     g->stream = saved;
     cudaStreamDestroy(cs);
     if (err != cudaSuccess) {
