@@ -1955,8 +1955,8 @@ static bool pair_plan(const MgHierarchy& H, const float* r, const float* z, Pair
     a.tiles_y = (a.h + kPY - 1) / kPY;
     a.l2keep = H.l2keep;
     // every resident block, each with an equal share of the plane-tiles
-    P->nb_plain = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, H.pair_cap_plain);
-    P->nb_prolong = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, H.pair_cap);
+    P->nb_plain = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, H.pair_cap_plain, kZMinPlanesMg);
+    P->nb_prolong = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, H.pair_cap, kZMinPlanesMg);
     return true;
 }
 
@@ -2003,7 +2003,7 @@ static bool restrict_tma(pg_grid* g, const MgHierarchy& H, const float* e, const
     a.fc = fc;
     a.tiles_x = (a.w + kQX - 1) / kQX;
     a.tiles_y = (a.h + kQY - 1) / kQY;
-    const int nb = zwalk_blocks(a.tiles_x * a.tiles_y, a.d / 2, restrict_cap(g));
+    const int nb = zwalk_blocks(a.tiles_x * a.tiles_y, a.d / 2, restrict_cap(g), kZMinPlanesMg);
     cudaStream_t s = g->stream;
     PG_LAUNCH(KK_MG_RESTRICT, s, launch_dep(g->dims.nc(), k_mg_restrict3p, nb, kQThreads, kQSmem, s, *em, *fm, H.rgmap, a, g->ws.state));
     return true;

@@ -489,7 +489,7 @@ bool spmv_tma_launch(cudaStream_t s, int num_sms, int pm, const float* zb, float
     a.ap = ap;
     a.tiles_x = (a.w + kSX - 1) / kSX;
     a.tiles_y = (a.h + kSY - 1) / kSY;
-    const int nb = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, cap);
+    const int nb = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, cap, pm == PM_ZBUF ? kZMinPlanesMg : kZMinPlanes);
     if (pm == PM_ZBUF)
         launch_dep(D.nc(), k_cg_spmv3p<PM_ZBUF>, nb, kSThreads, kSSmem, s, zm, pm0, pm1, gm, a, st, partials);
     else if (pm == PM_JACOBI)
@@ -526,7 +526,7 @@ bool residual_df_tma_launch(cudaStream_t s, int num_sms, const float* b, const f
     a.r = r;
     a.tiles_x = (a.w + kRX - 1) / kRX;
     a.tiles_y = (a.h + kRY - 1) / kRY;
-    const int nb = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, cap);
+    const int nb = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, cap, kZMinPlanesMg);
     k_residual_df3p<<<nb, kRThreads, kRSmem, s>>>(hm, lm, bm, gm, a, partials, counter, out, st);
     return true;
 }

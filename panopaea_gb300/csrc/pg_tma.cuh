@@ -158,9 +158,15 @@ struct ZWalk {
 // Blocks of a z-marching launch: every resident block (cap), but no fewer
 // than kZMinPlanes planes per block.
 constexpr int kZMinPlanes = 8;
-inline int zwalk_blocks(int ntiles, i64 d, int cap) {
+// The multigrid solve's kernels: on a small grid more blocks are worth the
+// planes computed twice (64^3 has 256 plane-tiles: 32 blocks of 8 leave 120
+// SMs idle): its room step takes 895 us with 8 planes and 685 with 2, a pair
+// 11 to 17 us, 8 to 13 with 4 and 6.6 to 12 with 2.  Plain and Jacobi CG keep 8,
+// and with it the order of their sums.
+constexpr int kZMinPlanesMg = 2;
+inline int zwalk_blocks(int ntiles, i64 d, int cap, int min_planes = kZMinPlanes) {
     const i64 total = (i64)ntiles * d;
-    i64 nb = total / kZMinPlanes;
+    i64 nb = total / min_planes;
     if (nb > cap) nb = cap;
     return nb < 1 ? 1 : (int)nb;
 }
