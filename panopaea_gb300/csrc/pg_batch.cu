@@ -178,8 +178,7 @@ __global__ void k_b_cg_init(float* __restrict__ x, float* __restrict__ r, const 
             x[c] = 0.f;
             r[c] = bv;
             bm = isfinite(bv) ? fabsf(bv) : __int_as_float(0x7f800000);
-            if (PM == PM_ZBUF) sig.add(bv);  // sum(b) for the lazy projection
-            else sig.add(bz<PM>(b, flags, c, dt) * bv);
+            sig.add(bz<PM>(b, flags, c, dt) * bv);
         }
         double m, s;
         tmaxsum(bm, f2_of(sig), sm, &m, &s);
@@ -433,7 +432,7 @@ static int bblocks(const pg_batch* B, int ntiles) {
 // One CG iteration over all grids.  PM_ZBUF: z = V(r) by the batched
 // multigrid, which brings its own SpMV and update.
 template <int PM> static void b_iter(pg_batch* B, cudaStream_t s, float dt, float* x, int nsmooth = 2) {
-    if (PM == PM_ZBUF) {
+    if constexpr (PM == PM_ZBUF) {
         bmg_spmv(B, s, dt);
         PG_LAUNCH(KK_STEP_MISC, s,
                   k_b_finalize<1><<<B->n, 128, 0, s>>>(B->ginfo, B->state, bmg_partials(B), B->n, 0.0, 0.0, 0, B->active,
@@ -520,14 +519,18 @@ static int b_solve(pg_batch* B, const pg_solver_params* prm, float dt, float* x,
     const int nsmooth = prm->mg_smooth > 0 ? prm->mg_smooth : 2;
     // init: r = b (PM_ZBUF: z comes from the V-cycle; sum(b) for the lazy projection)
     PG_CUDA(cudaMemsetAsync(B->active, 0, sizeof(int), s));
-    PG_LAUNCH(KK_CG_INIT, s,
-              k_b_cg_init<PM><<<nb, nt, 0, s>>>(x, B->r, B->b, B->flags, B->ginfo, B->tiles, B->ntiles, B->tx, B->ty,
-                                                dt, B->partials));
+    if constexpr (PM == PM_ZBUF)
+        bmg_init(B, s, x);
+    else
+        PG_LAUNCH(KK_CG_INIT, s,
+                  k_b_cg_init<PM><<<nb, nt, 0, s>>>(x, B->r, B->b, B->flags, B->ginfo, B->tiles, B->ntiles, B->tx, B->ty,
+                                                    dt, B->partials));
     PG_LAUNCH(KK_STEP_MISC, s,
-              k_b_finalize<0><<<B->n, 128, 0, s>>>(B->ginfo, B->state, B->partials, B->n,
+              k_b_finalize<0><<<B->n, 128, 0, s>>>(B->ginfo, B->state, PM == PM_ZBUF ? bmg_partials(B) : B->partials, B->n,
                                                    prm->rel_stop ? prm->rel_tol : 0.0, prm->threshold,
                                                    (int)std::min<i64>(prm->max_iter, 1 << 30), B->active, 0,
-                                                   PM == PM_ZBUF ? B->nfluid : nullptr));
+                                                   PM == PM_ZBUF ? B->nfluid : nullptr,
+                                                   PM == PM_ZBUF ? bmg_update_range(B) : nullptr));
     if (PM == PM_ZBUF) {
         bmg_vcycle(B, s, nsmooth);
         bmg_rz_finalize(B, s, 1);

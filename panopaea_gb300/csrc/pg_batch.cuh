@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "pg_cg.cuh"
+#include "pg_march2d.cuh"
 #include "pg_ops2d.cuh"
 
 namespace pg {
@@ -194,50 +195,6 @@ __device__ __forceinline__ void tmaxsum(float m, F2 v, F2* sm, double* om, doubl
 
 #define FOR_TILES(list, count) for (int ti = blockIdx.x; ti < (count); ti += gridDim.x)
 
-// A strip: up to 64 columns of one grid from the even column x0 on, marched
-// down rows [y0, y1) by one warp that holds two neighbouring columns per lane.
-struct Strip {
-    int grid, y0, y1, x0;
-};
-
-// Two neighbouring values of a row; VEC: the pair is 8-byte aligned and whole.
-template <bool VEC> __device__ __forceinline__ float2 ld2(const float* p, bool a, bool b) {
-    float2 v = make_float2(0.f, 0.f);
-    if (VEC) {
-        if (a) v = *reinterpret_cast<const float2*>(p);
-    } else {
-        if (a) v.x = p[0];
-        if (b) v.y = p[1];
-    }
-    return v;
-}
-
-template <bool VEC> __device__ __forceinline__ void st2(float* p, float2 v, bool a, bool b) {
-    if (VEC) {
-        if (a) *reinterpret_cast<float2*>(p) = v;
-    } else {
-        if (a) p[0] = v.x;
-        if (b) p[1] = v.y;
-    }
-}
-
-// Two flag bytes, kept apart until they are used (a load must not be waited
-// for where it is issued).
-struct Flag2 {
-    unsigned a, b;
-    template <bool VEC> __device__ __forceinline__ void load(const uint8_t* p, bool va, bool vb) {
-        a = b = 0;
-        if (VEC) {
-            if (va) a = *reinterpret_cast<const unsigned short*>(p);
-        } else {
-            if (va) a = p[0];
-            if (vb) b = p[1];
-        }
-    }
-    // the second cell's in bits 8 and up
-    template <bool VEC> __device__ __forceinline__ unsigned both() const { return VEC ? a : a | b << 8; }
-};
-
 // Batched multigrid (pg_batch_mg.cu).
 // (Re)build the hierarchy of every grid for the batch's mask and dt.
 int bmg_ensure(pg_batch* B, float dt);
@@ -250,6 +207,8 @@ void bmg_rz_finalize(pg_batch* B, cudaStream_t s, int first);
 // and the max|r|, sum(r) partials; one partial pair per strip / chunk.
 void bmg_spmv(pg_batch* B, cudaStream_t s, float dt);
 void bmg_update(pg_batch* B, cudaStream_t s, float* x);
+// x = 0, r = b, the max|b|, sum(b) partials (ranges as the update's).
+void bmg_init(pg_batch* B, cudaStream_t s, float* x);
 const double* bmg_partials(const pg_batch* B);
 const int2* bmg_spmv_range(const pg_batch* B);    // per grid: its strips
 const int2* bmg_update_range(const pg_batch* B);  // per grid: its chunks

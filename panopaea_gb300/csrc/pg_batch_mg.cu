@@ -31,21 +31,17 @@ namespace pg {
 constexpr int kBmgMaxLevels = 16;
 constexpr int kBmgCoarseMax = 2048;
 constexpr int kRtX = 32, kRtY = 8;  // setup tile: 32 x 8 coarse cells
-constexpr int kMarchThreads = 128;  // four strips per block
 // Cells (of all its levels together, 20 bytes each) that a block keeps in
 // shared memory, two blocks per SM: 64 x 64 and the levels below it are 5456.
 constexpr int kBmgTailCells = 5600;
 constexpr int kBmgTailThreads = 512;
 constexpr int kUpdateCells = 2048;  // cells per warp of the CG update
 
-struct BLevel {
-    int h, w;     // this grid's dims at this level
-    i64 off;      // its first cell in the level's packed arrays (level 0: the batch offset)
+// A grid at a level (off: in the level's packed arrays; level 0: the batch's).
+struct BLevel : MarchLevel {
     int coarse;   // the grid's coarsest level
     int tail;     // its first level of k_bmg_tail
     int t0, t1;   // its smoothing strips (level 0)
-    int ch, cw;   // dims at the next level (0 if none)
-    i64 coff;     // first cell at the next level
 };
 
 // Cells [c0, c1) of a grid in the packed fields.
@@ -84,16 +80,8 @@ struct BatchMg {
 };
 
 // Device view of one level of the batch.
-struct BLv {
+struct BLv : MarchView {
     const BLevel* info;
-    const float* wx;
-    const float* wy;
-    const float* invd;
-    const float* f;
-    const uint8_t* flags;  // level 0
-    const float* ec;       // next level's correction (prolongation)
-    float* fc;             // next level's right-hand side (restriction)
-    float dt;
     int level;
 };
 
@@ -114,212 +102,6 @@ template <bool L0> struct BCell {
             wyl = v.wy[c];
             wyh = y + 1 < h ? v.wy[c + w] : 0.f;
             inv = v.invd[c];
-        }
-    }
-};
-
-enum { BP_PLAIN = 0, BP_SELF = 1, BP_PROLONG = 2 };
-
-// s + weight * neighbour over a cell's open faces (x-, x+, y-, y+).
-__device__ __forceinline__ float nb_sum(float s, float wl, float wr, float wu, float wd, float nl, float nr, float nu,
-                                        float nd) {
-    if (wl != 0.f) s = fmaf(wl, nl, s);
-    if (wr != 0.f) s = fmaf(wr, nr, s);
-    if (wu != 0.f) s = fmaf(wu, nu, s);
-    if (wd != 0.f) s = fmaf(wd, nd, s);
-    return s;
-}
-
-// What a lane holds of a row: e and f of its two cells, and their flags
-// (level 0) or weights and 1 / diagonal (coarser levels).
-template <bool L0> struct BRow {
-    float2 e, f;
-    Flag2 raw;  // as loaded; fl: both
-    unsigned fl;
-    float2 wx, wy, inv;
-    float wr;   // the second cell's x+ weight, from the next lane
-    float ec;   // as loaded: the correction to prolong
-};
-
-// One red-black pair over a strip: the first colour of row y (from the old
-// values of the rows around it), then the second colour of row y - 1 (from
-// the new ones), which finishes that row; with REST the residual of row y - 2
-// follows and is summed to the next level, with RZ the finished row's z.r and
-// sum(z).  C1: the parity of x + y of the first colour.  FA: the first
-// colour in this row is the lane's first cell.
-template <bool L0, int MODE, int C1, bool RZ, bool REST, bool VEC> struct March {
-    const BLv& v;
-    const BLevel& L;
-    const float* __restrict__ ein;
-    float* __restrict__ eout;
-    int lane, x, y0, y1;
-    bool va, vb, own, ownb;
-    float tab;  // lane f: 1 / diagonal of a cell with face-open bits f (level 0)
-    i64 at;     // index of the lane's first cell in the next row to fetch
-    int next;   // that row
-    int stop;   // the last row needed
-    BRow<L0> r[5];  // rows y - 3 .. y + 1
-    float rsum = 0.f;
-    Acc<float> acc, zs;
-
-    __device__ __forceinline__ March(const BLv& v_, const BLevel& L_, const Strip& S, const float* ein_, float* eout_)
-        : v(v_), L(L_), ein(ein_), eout(eout_) {
-        lane = threadIdx.x & 31;
-        x = S.x0 + 2 * lane;
-        y0 = S.y0;
-        y1 = S.y1;
-        va = x < L.w;
-        vb = x + 1 < L.w;
-        const int lo = S.x0 ? S.x0 + 4 : 0, hi = S.x0 + 64 >= L.w ? L.w : S.x0 + 60;
-        own = x >= lo && x < hi;
-        ownb = own && vb;
-        const int n = __popc(lane & 15);
-        tab = L0 && n ? __frcp_rn((float)n * v.dt) : 0.f;
-    }
-
-    // Row `next` (zeros outside the grid, so that no weight points there).
-    __device__ __forceinline__ BRow<L0> fetch() {
-        BRow<L0> q;
-        q.e = q.f = q.wx = q.wy = q.inv = make_float2(0.f, 0.f);
-        q.fl = q.raw.a = q.raw.b = 0;
-        q.wr = q.ec = 0.f;
-        if (next >= 0 && next <= stop) {  // uniform per warp
-            q.f = ld2<VEC>(v.f + at, va, vb);
-            if (L0) {
-                q.raw.template load<VEC>(v.flags + at, va, vb);
-            } else {
-                q.wx = ld2<VEC>(v.wx + at, va, vb);
-                q.wy = ld2<VEC>(v.wy + at, va, vb);
-                q.inv = ld2<VEC>(v.invd + at, va, vb);
-            }
-            if (MODE != BP_SELF) q.e = ld2<VEC>(ein + at, va, vb);
-            if (MODE == BP_PROLONG && va) q.ec = v.ec[L.coff + (i64)(next >> 1) * L.cw + (x >> 1)];
-        }
-        ++next;
-        at += L.w;
-        return q;
-    }
-
-    __device__ __forceinline__ void push(const BRow<L0>& q) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) r[k] = r[k + 1];
-        r[4] = q;
-        if (MODE == BP_PROLONG) {
-            r[4].e.x += q.ec;
-            r[4].e.y += q.ec;
-        }
-        if (L0) {
-            r[4].fl = q.raw.template both<VEC>();
-        } else {
-            const float n = __shfl_down_sync(0xffffffffu, q.wx.x, 1);
-            r[4].wr = lane < 31 ? n : 0.f;
-        }
-    }
-
-    // Weights of the first (A) or second cell of row k.
-    template <bool A> __device__ __forceinline__ void weights(int k, float& wl, float& wr, float& wu, float& wd) const {
-        if (L0) {
-            const unsigned f = A ? r[k].fl : r[k].fl >> 8;
-            wl = (f & XLO) ? v.dt : 0.f;
-            wr = (f & XHI) ? v.dt : 0.f;
-            wu = (f & YLO) ? v.dt : 0.f;
-            wd = (f & YHI) ? v.dt : 0.f;
-        } else {
-            wl = A ? r[k].wx.x : r[k].wx.y;
-            wr = A ? r[k].wx.y : r[k].wr;
-            wu = A ? r[k].wy.x : r[k].wy.y;
-            wd = A ? r[k + 1].wy.x : r[k + 1].wy.y;
-        }
-    }
-    template <bool A> __device__ __forceinline__ float inv(int k) const {
-        if (L0) return __shfl_sync(0xffffffffu, tab, A ? r[k].fl : r[k].fl >> 8);
-        return A ? r[k].inv.x : r[k].inv.y;
-    }
-    // The four neighbours' values.
-    template <bool A> __device__ __forceinline__ void around(int k, float& nl, float& nr, float& nu, float& nd) const {
-        if (A) {
-            nl = __shfl_up_sync(0xffffffffu, r[k].e.y, 1);
-            nr = r[k].e.y;
-        } else {
-            nl = r[k].e.x;
-            nr = __shfl_down_sync(0xffffffffu, r[k].e.x, 1);
-        }
-        nu = A ? r[k - 1].e.x : r[k - 1].e.y;
-        nd = A ? r[k + 1].e.x : r[k + 1].e.y;
-    }
-    template <bool A> __device__ __forceinline__ float updated(int k) const {
-        float wl, wr, wu, wd, nl, nr, nu, nd;
-        weights<A>(k, wl, wr, wu, wd);
-        around<A>(k, nl, nr, nu, nd);
-        return nb_sum(A ? r[k].f.x : r[k].f.y, wl, wr, wu, wd, nl, nr, nu, nd) * inv<A>(k);
-    }
-    template <bool A> __device__ __forceinline__ float residual(int k) const {
-        float wl, wr, wu, wd, nl, nr, nu, nd;
-        weights<A>(k, wl, wr, wu, wd);
-        around<A>(k, nl, nr, nu, nd);
-        const float c = A ? r[k].e.x : r[k].e.y;
-        return (A ? r[k].f.x : r[k].f.y) - nb_sum(0.f, wl, wr, wu, wd, c - nl, c - nr, c - nu, c - nd);
-    }
-
-    template <bool FA> __device__ __forceinline__ void step(int y) {
-        float n;
-        if (MODE == BP_SELF) {
-            const float i = inv<FA>(3), f = FA ? r[3].f.x : r[3].f.y;
-            n = i != 0.f ? f * i : 0.f;
-        } else {
-            n = updated<FA>(3);
-        }
-        (FA ? r[3].e.x : r[3].e.y) = n;
-        const float m = updated<FA>(2);  // (the colours swap cells from row to row)
-        (FA ? r[2].e.x : r[2].e.y) = m;
-        if (y - 1 >= y0 && y - 1 < y1) {  // uniform per warp
-            st2<VEC>(eout + (at - 5 * (i64)L.w), r[2].e, own, ownb);  // (fetched: rows up to y + 3)
-            if (RZ) {
-                if (own) {
-                    acc.add(r[2].e.x * r[2].f.x);
-                    zs.add(r[2].e.x);
-                }
-                if (ownb) {
-                    acc.add(r[2].e.y * r[2].f.y);
-                    zs.add(r[2].e.y);
-                }
-            }
-        }
-        if (REST && y - 2 >= y0) {
-            const float a = residual<true>(1), b = residual<false>(1);
-            if ((y & 1) == 0) rsum = a + b;
-            else {
-                rsum += a;
-                rsum += b;
-                const int Y = (y - 2) >> 1;
-                if (Y < L.ch && 2 * Y < y1 && own) v.fc[L.coff + (i64)Y * L.cw + (x >> 1)] = rsum;
-            }
-        }
-    }
-
-    __device__ __forceinline__ void run() {
-        int y = y0 - (REST ? 2 : 1);
-        const int last = y0 + ((y1 - y0 + 1) & ~1) + (REST ? 1 : 0);
-        constexpr bool FA = REST ? C1 == 0 : C1 == 1;
-        next = y - 1;
-        stop = min(L.h - 1, last + 1);
-        at = L.off + (i64)next * L.w + x;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            r[k].e = r[k].f = r[k].wx = r[k].wy = r[k].inv = make_float2(0.f, 0.f);
-            r[k].fl = r[k].raw.a = r[k].raw.b = 0;
-            r[k].wr = r[k].ec = 0.f;
-        }
-        push(fetch());
-        push(fetch());
-        BRow<L0> q0 = fetch(), q1 = fetch();  // two rows ahead
-        for (; y < last; y += 2) {
-            push(q0);
-            q0 = fetch();
-            step<FA>(y);
-            push(q1);
-            q1 = fetch();
-            step<!FA>(y + 1);
         }
     }
 };
@@ -714,15 +496,39 @@ __global__ void __launch_bounds__(kMarchThreads, 7)
     }
 }
 
-// x += alpha p, r -= alpha Ap, max|r| and sum(r), one warp per chunk of a
-// grid's cells, four at a time where the fields' 16-byte groups allow it; 24
-// bytes per cell.  71 us for 21 M cells (76 at the copy rate, part of it in
+// A warp's walk over its chunk of a grid's cells, four at a time where the
+// fields' 16-byte groups allow it (vec), the cells around them one by one:
+// four(c) and single(c).
+template <class F4, class F1>
+__device__ __forceinline__ void walk_chunk(const Chunk& C, int vec, F4&& four, F1&& single) {
+    const int lane = threadIdx.x & 31;
+    const i64 g0 = vec ? (C.c0 + 3) / 4 * 4 : C.c1, g1 = vec ? C.c1 / 4 * 4 : C.c1;
+    if (g0 < g1) {
+        for (i64 c = g0 + 4 * lane; c < g1; c += 128) four(c);
+        if (C.c0 + lane < g0) single(C.c0 + lane);
+        if (g1 + lane < C.c1) single(g1 + lane);
+    } else {
+        for (i64 c = C.c0 + lane; c < C.c1; c += 32) single(c);
+    }
+}
+__device__ __forceinline__ float abs_or_inf(float v) { return isfinite(v) ? fabsf(v) : __int_as_float(0x7f800000); }
+__device__ __forceinline__ void chunk_partials(float rm, const Acc<float>& sum, double* __restrict__ out) {
+    for (int o = 16; o > 0; o >>= 1) rm = fmaxf(rm, __shfl_xor_sync(0xffffffffu, rm, o));
+    const F2 t = f2_warp(f2_of(sum));
+    if ((threadIdx.x & 31) == 0) {
+        out[0] = (double)rm;
+        out[1] = (double)t.hi + (double)t.lo;
+    }
+}
+
+// x += alpha p, r -= alpha Ap, max|r| and sum(r) (for the lazy projection);
+// 24 bytes per cell.  71 us for 21 M cells (76 at the copy rate, part of it in
 // L2), 181 with a block per tile.
 __global__ void __launch_bounds__(256)
     k_bmg_update(const Chunk* __restrict__ chunks, int n, const BState* __restrict__ st, float* __restrict__ x,
                  float* __restrict__ r, const float* p0, const float* p1, const float* __restrict__ ap, int vec,
                  double* __restrict__ partials) {
-    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (i >= n) return;
     const Chunk C = chunks[i];
     const BState& S = st[C.grid];
@@ -734,19 +540,12 @@ __global__ void __launch_bounds__(256)
     auto one = [&](float& xv, float& rv, float pv, float av) {
         xv = fmaf(al, pv, xv);
         rv = fmaf(nal, av, rv);
-        rm = fmaxf(rm, isfinite(rv) ? fabsf(rv) : __int_as_float(0x7f800000));
-        sum.add(rv);  // for the lazy projection
+        rm = fmaxf(rm, abs_or_inf(rv));
+        sum.add(rv);
     };
-    auto single = [&](i64 c) {
-        float xv = x[c], rv = r[c];
-        one(xv, rv, p[c], ap[c]);
-        x[c] = xv;
-        r[c] = rv;
-    };
-    // the whole groups of four between c0 and c1, the cells around them one by one
-    const i64 g0 = vec ? (C.c0 + 3) / 4 * 4 : C.c1, g1 = vec ? C.c1 / 4 * 4 : C.c1;
-    if (g0 < g1) {
-        for (i64 c = g0 + 4 * lane; c < g1; c += 128) {
+    walk_chunk(
+        C, vec,
+        [&](i64 c) {
             float4 xv = *reinterpret_cast<const float4*>(x + c), rv = *reinterpret_cast<const float4*>(r + c);
             const float4 pv = *reinterpret_cast<const float4*>(p + c), av = *reinterpret_cast<const float4*>(ap + c);
             one(xv.x, rv.x, pv.x, av.x);
@@ -755,18 +554,47 @@ __global__ void __launch_bounds__(256)
             one(xv.w, rv.w, pv.w, av.w);
             *reinterpret_cast<float4*>(x + c) = xv;
             *reinterpret_cast<float4*>(r + c) = rv;
-        }
-        if (C.c0 + lane < g0) single(C.c0 + lane);
-        if (g1 + lane < C.c1) single(g1 + lane);
-    } else {
-        for (i64 c = C.c0 + lane; c < C.c1; c += 32) single(c);
-    }
-    for (int o = 16; o > 0; o >>= 1) rm = fmaxf(rm, __shfl_xor_sync(0xffffffffu, rm, o));
-    const F2 t = f2_warp(f2_of(sum));
-    if (lane == 0) {
-        partials[2 * (i64)i] = (double)rm;
-        partials[2 * (i64)i + 1] = (double)t.hi + (double)t.lo;
-    }
+        },
+        [&](i64 c) {
+            float xv = x[c], rv = r[c];
+            one(xv, rv, p[c], ap[c]);
+            x[c] = xv;
+            r[c] = rv;
+        });
+    chunk_partials(rm, sum, partials + 2 * (i64)i);
+}
+
+// x = 0, r = b, max|b| and sum(b).
+__global__ void __launch_bounds__(256)
+    k_bmg_init(const Chunk* __restrict__ chunks, int n, float* __restrict__ x, float* __restrict__ r,
+               const float* __restrict__ b, int vec, double* __restrict__ partials) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const Chunk C = chunks[i];
+    float bm = 0.f;
+    Acc<float> sum;
+    auto one = [&](float bv) {
+        bm = fmaxf(bm, abs_or_inf(bv));
+        sum.add(bv);
+    };
+    walk_chunk(
+        C, vec,
+        [&](i64 c) {
+            const float4 bv = *reinterpret_cast<const float4*>(b + c);
+            one(bv.x);
+            one(bv.y);
+            one(bv.z);
+            one(bv.w);
+            *reinterpret_cast<float4*>(x + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<float4*>(r + c) = bv;
+        },
+        [&](i64 c) {
+            const float bv = b[c];
+            one(bv);
+            x[c] = 0.f;
+            r[c] = bv;
+        });
+    chunk_partials(bm, sum, partials + 2 * (i64)i);
 }
 
 // Coarse face weights of level l+1 from level l (tiles over level l+1).
@@ -963,14 +791,7 @@ static int bmg_build(pg_batch* B, float dt) {
             for (int g = 0; g < n; ++g) {
                 BLevel& L = info[l][g];
                 const int t0 = (int)st.size();
-                if (all || l < L.tail) {
-                    const int per = (L.h + rows - 1) / rows, rc = ((L.h + per - 1) / per + 1) & ~1;
-                    for (int y0 = 0; y0 < L.h; y0 += rc)
-                        for (int x0 = 0;; x0 += step) {
-                            st.push_back(Strip{g, y0, std::min(y0 + rc, L.h), x0});
-                            if (x0 + 64 >= L.w) break;
-                        }
-                }
+                if (all || l < L.tail) march_strips(g, L.h, L.w, step, rows, st);
                 L.t0 = t0;
                 L.t1 = (int)st.size();
             }
@@ -1068,8 +889,6 @@ static int bmg_build(pg_batch* B, float dt) {
     return PG_OK;
 }
 
-static int march_blocks(int n) { return (n + kMarchThreads / 32 - 1) / (kMarchThreads / 32); }
-
 template <bool L0, int MODE, int C1, bool RZ, bool REST>
 static void bpair(pg_batch* B, cudaStream_t s, int l, const float* ein, float* eout) {
     BatchMg& M = *B->mg;
@@ -1155,6 +974,13 @@ void bmg_update(pg_batch* B, cudaStream_t s, float* x) {
     PG_LAUNCH(KK_CG_UPDATE, s,
               k_bmg_update<<<(M.nchunk + 7) / 8, 256, 0, s>>>(M.chunks, M.nchunk, B->state, x, B->r, B->p0, B->p1, B->ap,
                                                               vec, M.partials));
+}
+
+void bmg_init(pg_batch* B, cudaStream_t s, float* x) {
+    BatchMg& M = *B->mg;
+    const int vec = ((uintptr_t)x & 15) == 0;
+    PG_LAUNCH(KK_CG_INIT, s,
+              k_bmg_init<<<(M.nchunk + 7) / 8, 256, 0, s>>>(M.chunks, M.nchunk, x, B->r, B->b, vec, M.partials));
 }
 
 const double* bmg_partials(const pg_batch* B) { return B->mg->partials; }

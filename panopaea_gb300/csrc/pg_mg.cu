@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "pg_solve.cuh"
+#include "pg_march2d.cuh"
 #include "pg_tma.cuh"
 
 namespace pg {
@@ -73,6 +74,11 @@ struct MgHierarchy {
     size_t ct_smem = 0;
     void* ct_mem = nullptr;  // its packed weights
     double nfluid = 0;  // cells with an open face (the lazy projection's count)
+    // 2D levels above the tail: pairs by k_mg_march, between e (level 0: z) and
+    // a twin
+    Strip* strips[kMaxLevels] = {};
+    int nstrips[kMaxLevels] = {};
+    float* twin[kMaxLevels] = {};
     // fine level of 3D grids: fused red-black pairs (k_mg_pair) ping-pong
     // between z and e0b; tensor maps of the flags and of the vectors met
     bool pairs = false;
@@ -276,6 +282,56 @@ __global__ void __launch_bounds__(kMgThreads)
     if (!last_block(&st->counter[3])) return;
     double rz, zsum;
     reduce_partials2<kMgThreads>(partials, partials + kMaxBlocks, gridDim.x, sm, rz, zsum);
+    if (threadIdx.x == 0) {
+        st->counter[3] = 0;
+        cg_finish_rz(st, rz, zsum);
+    }
+}
+
+// A smoothing pair of a 2D level by marching warps (pg_march2d.cuh), from ein to
+// eout, with the restriction of what it leaves (REST) or z.r and sum(z), as
+// k_mg_smooth finishes them (RZ).
+//
+// Both half-sweeps from one read of the level, half the launches, and the
+// restriction's: at 1000 x 1200 a level-0 pair takes 7 to 11 us with all that
+// where half-sweeps took 7 to 8.5 each, 17 with z.r, and the restriction 7; the
+// levels below 7 to 8.6 a pair, 4.6 a half-sweep and 5 a restriction.  The
+// step: 1.114 -> 1.013 ms; of 501 x 733 0.936 -> 0.852.
+template <bool L0, int MODE, int C1, bool RZ, bool REST>
+__global__ void __launch_bounds__(kMarchThreads)
+    k_mg_march(MarchView v, MarchLevel L, const float* __restrict__ ein, float* __restrict__ eout,
+               const Strip* __restrict__ strips, int n, int vec, CgState* st, double* partials) {
+    grid_dep();
+    if (st->done) return;
+    __shared__ double sm[RZ ? 2 * kMarchThreads : 1];
+    double s = 0.0, s2 = 0.0;
+    for (int i = blockIdx.x * (kMarchThreads / 32) + (threadIdx.x >> 5); i < n; i += gridDim.x * (kMarchThreads / 32)) {
+        const Strip S = strips[i];
+        if (vec) {
+            March<L0, MODE, C1, RZ, REST, true> m(v, L, S, ein, eout);
+            m.run();
+            if (RZ) {
+                s += m.acc.value();
+                s2 += m.zs.value();
+            }
+        } else {
+            March<L0, MODE, C1, RZ, REST, false> m(v, L, S, ein, eout);
+            m.run();
+            if (RZ) {
+                s += m.acc.value();
+                s2 += m.zs.value();
+            }
+        }
+    }
+    if (!RZ) return;
+    block_sum2<kMarchThreads>(s, s2, sm);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = s;
+        partials[kMaxBlocks + blockIdx.x] = s2;
+    }
+    if (!last_block(&st->counter[3])) return;
+    double rz, zsum;
+    reduce_partials2<kMarchThreads>(partials, partials + kMaxBlocks, gridDim.x, sm, rz, zsum);
     if (threadIdx.x == 0) {
         st->counter[3] = 0;
         cg_finish_rz(st, rz, zsum);
@@ -1639,6 +1695,10 @@ void release_mg(Extras* ex) {
         cudaFree(ex->mg->mem);
         cudaFree(ex->mg->e0b);
         cudaFree(ex->mg->ct_mem);
+        for (int l = 0; l < kMaxLevels; ++l) {
+            cudaFree(ex->mg->strips[l]);
+            cudaFree(ex->mg->twin[l]);
+        }
         cudaFree(ex->mg->cinv);
         delete ex->mg;
         ex->mg = nullptr;
@@ -1742,6 +1802,26 @@ static int coarsest_pinv(pg_grid* g, MgHierarchy* H) {
 }
 
 // (Re)build the hierarchy for the grid's current mask and dt.
+// The strips and twins of the 2D levels above the tail: chunks of 32 rows, of
+// fewer where those would leave SMs idle.
+static int march_setup(pg_grid* g, MgHierarchy* H) {
+    const int top = H->ct_ranks > 0 ? H->ct_lt : std::min(H->tail, H->nlev - 1);
+    for (int l = 0; l < top; ++l) {
+        const Dims& D = H->lv[l].D;
+        std::vector<Strip> st;
+        for (int rows = 32; rows >= 4; rows /= 2) {
+            st.clear();
+            march_strips(0, (int)D.h, (int)D.w, 56, rows, st);
+            if ((i64)st.size() >= (i64)g->num_sms * 16) break;
+        }
+        PG_CUDA(cudaMalloc(&H->strips[l], sizeof(Strip) * st.size()));
+        PG_CUDA(cudaMalloc(&H->twin[l], sizeof(float) * (size_t)D.nc()));
+        PG_CUDA(cudaMemcpy(H->strips[l], st.data(), sizeof(Strip) * st.size(), cudaMemcpyHostToDevice));
+        H->nstrips[l] = (int)st.size();
+    }
+    return PG_OK;
+}
+
 static int ensure_mg(pg_grid* g, double dt, MgHierarchy** out) {
     Extras* ex = extras_of(g);
     if (ex->mg && ex->mg->dt == dt && ex->mg->mask_version == g->mask_version) {
@@ -1834,6 +1914,10 @@ static int ensure_mg(pg_grid* g, double dt, MgHierarchy** out) {
         if (prc) return prc;
     }
     ctail_setup(H);
+    if (g->dims.nd == 2) {
+        const int mrc = march_setup(g, H);
+        if (mrc) return mrc;
+    }
     // coarse operators
     cudaStream_t s = g->stream;
     for (int l = 0; l + 1 < nl; ++l) {
@@ -2238,6 +2322,43 @@ static int vcycle_projected(pg_grid* g, const MgHierarchy& H, float* r, float* z
     return rc;
 }
 
+template <bool L0, int MODE, int C1, bool RZ, bool REST>
+static void march_t(pg_grid* g, const MgHierarchy& H, int l, const float* f, const float* ein, float* eout) {
+    const LV lv = view(H, l);
+    const MgLevel& C = H.lv[l + 1];
+    const MarchView v{lv.wx, lv.wy, lv.invd, f, lv.flags, C.e, C.f, lv.dt};
+    const MarchLevel L{lv.h, lv.w, 0, (int)C.D.h, (int)C.D.w, 0};
+    const int vec = lv.w % 2 == 0 && !(((uintptr_t)f | (uintptr_t)ein | (uintptr_t)eout) & 7);
+    const int nb = std::min(march_blocks(H.nstrips[l]), kMaxBlocks);
+    PG_LAUNCH(l == 0 ? KK_MG_SMOOTH : KK_MG_SMOOTH_C, g->stream,
+              launch_dep(g->dims.nc(), k_mg_march<L0, MODE, C1, RZ, REST>, nb, kMarchThreads, 0, g->stream, v, L, ein, eout,
+                         (const Strip*)H.strips[l], H.nstrips[l], vec, g->ws.state, g->ws.partials));
+}
+
+// The pairs of a marched level before (down, the last one restricting) or after
+// the coarser levels; e and its twin are written in turn, the last pair of
+// all leaves the result in e.
+template <bool L0>
+static void march_level(pg_grid* g, const MgHierarchy& H, int l, float* e, const float* f, int ns, bool down) {
+    float *to = H.twin[l], *other = e;
+    if (down) {
+        if (ns == 1) march_t<L0, BP_SELF, 0, false, true>(g, H, l, f, nullptr, to);
+        else march_t<L0, BP_SELF, 0, false, false>(g, H, l, f, nullptr, to);
+        for (int k = 1; k < ns; ++k, std::swap(to, other)) {
+            if (k == ns - 1) march_t<L0, BP_PLAIN, 0, false, true>(g, H, l, f, to, other);
+            else march_t<L0, BP_PLAIN, 0, false, false>(g, H, l, f, to, other);
+        }
+        return;
+    }
+    if (ns & 1) std::swap(to, other);  // (the pairs before ended in `other`)
+    if (ns == 1) march_t<L0, BP_PROLONG, 1, L0, false>(g, H, l, f, other, to);
+    else march_t<L0, BP_PROLONG, 1, false, false>(g, H, l, f, other, to);
+    for (int k = 1; k < ns; ++k, std::swap(to, other)) {
+        if (k == ns - 1) march_t<L0, BP_PLAIN, 1, L0, false>(g, H, l, f, to, other);
+        else march_t<L0, BP_PLAIN, 1, false, false>(g, H, l, f, to, other);
+    }
+}
+
 // l0 = 1: only the coarse part, from level 1's f (already restricted) to
 // its correction e.
 static int vcycle(pg_grid* g, const MgHierarchy& H, const float* r, float* z, int nsmooth, int l0) {
@@ -2275,6 +2396,11 @@ static int vcycle(pg_grid* g, const MgHierarchy& H, const float* r, float* z, in
     for (int l = l0; l < top; ++l) {
         float* e = E(l);
         const float* f = F(l);
+        if (H.nstrips[l]) {
+            if (l == 0) march_level<true>(g, H, l, e, f, nsmooth, true);
+            else march_level<false>(g, H, l, e, f, nsmooth, true);
+            continue;
+        }
         if (l == 0 && pairs) {
             pair(g, H, P, PR_SELF, 0, false, nullptr, pout[0]);
             for (int k = 1; k < nsmooth; ++k) pair(g, H, P, PR_PLAIN, 0, false, pout[(k - 1) & 1], pout[k & 1]);
@@ -2326,6 +2452,11 @@ static int vcycle(pg_grid* g, const MgHierarchy& H, const float* r, float* z, in
         float* e = E(l);
         const float* f = F(l);
         const float* ec = H.lv[l + 1].e;
+        if (H.nstrips[l]) {
+            if (l == 0) march_level<true>(g, H, l, e, f, nsmooth, false);
+            else march_level<false>(g, H, l, e, f, nsmooth, false);
+            continue;
+        }
         if (l == 0 && pairs) {
             for (int k = nsmooth; k < 2 * nsmooth; ++k)
                 pair(g, H, P, k == nsmooth ? PR_PROLONG : PR_PLAIN, 1, k == 2 * nsmooth - 1, pout[(k - 1) & 1],
