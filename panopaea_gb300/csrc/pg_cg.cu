@@ -458,7 +458,7 @@ __device__ __forceinline__ void df_axpy(float& xh, float& xl, float alpha, float
 // set, iteration 0 reads r = b0 and x = xl = 0 without loading them (the
 // init then writes neither): the same values, 16 bytes per cell fewer.
 template <bool DFX>
-__global__ void __launch_bounds__(kCgThreads)
+__global__ void __launch_bounds__(kCgThreads, DFX ? 4 : 5)
     k_cg_update4(float4* __restrict__ x, float4* __restrict__ r, const float4* p0, const float4* p1,
                  const float4* __restrict__ ap, i64 n4, CgState* st, double* partials, float4* __restrict__ xl,
                  const float4* __restrict__ b0, LoopCond loop) {
@@ -474,27 +474,38 @@ __global__ void __launch_bounds__(kCgThreads)
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float rm = 0.f, rs = 0.f;  // rs: sum(r) for the lazy projection (feeds a small correction term)
     int bad = 0;
-    auto one = [&](i64 c) {
-        const float4 xv = first ? zero4 : x[c], pv = p[c], rv = rin[c], av = ap[c];
-        float4 xo, ro;
+    // A thread's two vectors are loaded before either is used: the compiler,
+    // left to order them, had fewer in flight at 512^3 (629 -> 677 us).
+    struct In {
+        float4 x, p, r, a, lo;
+    };
+    auto load = [&](i64 c) {
+        In v;
+        v.p = p[c];
+        v.r = rin[c];
+        v.a = ap[c];
+        v.x = first ? zero4 : x[c];
+        if (DFX) v.lo = first ? zero4 : xl[c];
+        return v;
+    };
+    auto finish = [&](i64 c, In& v) {
+        float4 xo = v.x, ro;
         if (DFX) {
-            float4 lo = first ? zero4 : xl[c];
-            xo = xv;
-            df_axpy(xo.x, lo.x, alpha, pv.x);
-            df_axpy(xo.y, lo.y, alpha, pv.y);
-            df_axpy(xo.z, lo.z, alpha, pv.z);
-            df_axpy(xo.w, lo.w, alpha, pv.w);
-            xl[c] = lo;
+            df_axpy(xo.x, v.lo.x, alpha, v.p.x);
+            df_axpy(xo.y, v.lo.y, alpha, v.p.y);
+            df_axpy(xo.z, v.lo.z, alpha, v.p.z);
+            df_axpy(xo.w, v.lo.w, alpha, v.p.w);
+            xl[c] = v.lo;
         } else {
-            xo.x = xv.x + alpha * pv.x;
-            xo.y = xv.y + alpha * pv.y;
-            xo.z = xv.z + alpha * pv.z;
-            xo.w = xv.w + alpha * pv.w;
+            xo.x = v.x.x + alpha * v.p.x;
+            xo.y = v.x.y + alpha * v.p.y;
+            xo.z = v.x.z + alpha * v.p.z;
+            xo.w = v.x.w + alpha * v.p.w;
         }
-        ro.x = rv.x + nalpha * av.x;
-        ro.y = rv.y + nalpha * av.y;
-        ro.z = rv.z + nalpha * av.z;
-        ro.w = rv.w + nalpha * av.w;
+        ro.x = v.r.x + nalpha * v.a.x;
+        ro.y = v.r.y + nalpha * v.a.y;
+        ro.z = v.r.z + nalpha * v.a.z;
+        ro.w = v.r.w + nalpha * v.a.w;
         x[c] = xo;
         r[c] = ro;
         rm = fmaxf(fmaxf(fmaxf(rm, fabsf(ro.x)), fmaxf(fabsf(ro.y), fabsf(ro.z))), fabsf(ro.w));
@@ -504,10 +515,14 @@ __global__ void __launch_bounds__(kCgThreads)
     const i64 stride = (i64)gridDim.x * blockDim.x;
     i64 c = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     for (; c + stride < n4; c += 2 * stride) {
-        one(c);
-        one(c + stride);
+        In v0 = load(c), v1 = load(c + stride);
+        finish(c, v0);
+        finish(c + stride, v1);
     }
-    if (c < n4) one(c);
+    if (c < n4) {
+        In v = load(c);
+        finish(c, v);
+    }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&st->nan_seen, 1);
     double rsb = (double)rs;
     block_max0_sum<kCgThreads>(rm, rsb, sm);
