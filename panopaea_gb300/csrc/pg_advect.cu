@@ -7,14 +7,13 @@
 // Rust code.  3D is an extension: trilinear (math/interp.rs:23-36) with the
 // per-axis rules of the 2D code.
 //
-// The 3D float kernels are bound by instruction issue and the latency of two
-// rounds of loads, not by memory (8 to 17 loads and three rounded positions
-// per sample), so their common case has its own form, with the same results: floors by adding 2^23 rounded down
-// (positions below 2^22), addresses by adding strides, velocities that the
+// The 3D MAC kernel is bound by instruction issue and the latency of two rounds
+// of loads, not by memory (17 loads and three rounded positions per sample), so
+// its common case has its own form in float, with the same results: positions
+// below 2^22 in magnitude, addresses by adding strides, velocities that the
 // three faces of an index share loaded once.  Samples with a position beyond
-// that, or not finite, and the faces on the y and z boundary take the
-// general form.
-#include <algorithm>
+// that, or not finite, and the faces on the y and z boundary take the general
+// form.
 
 #include "pg_ops2d.cuh"
 
@@ -36,29 +35,12 @@ __global__ void k_advect_2d(T* __restrict__ dst, const T* __restrict__ q, const 
     }
 }
 
-// floor of v in [0, 2^22]: v + 2^23 rounded down holds it in the mantissa.
-constexpr float kFloorMagic = 8388608.f;
+// floor of v in [0, 2^22].  (Adding 2^23 rounded down instead of the two
+// conversions was 3% slower at 192^3 and 256^3, and 1.5% faster at 512^3.)
 constexpr float kFloorLimit = 4194304.f;
 __device__ __forceinline__ float floor_f(float v, int& i) {
-    const float r = __fadd_rd(v, kFloorMagic);
-    i = __float_as_int(r) - __float_as_int(kFloorMagic);
-    return sub_rn(r, kFloorMagic);
-}
-
-// cell_coord; SMALL: n <= 2^22 (float).
-template <bool SMALL, class T, class I>
-__device__ __forceinline__ void cell_at(T pos, I n, T hi, I& i0, T& frac) {
-    if constexpr (SMALL) {
-        const float p = fmin(fmax(sub_rn(pos, 0.5f), 0.f), hi);
-        float f = floor_f(p, i0);
-        if (i0 > n - 2) {
-            i0 = n - 2;
-            f = sub_rn(f, 1.f);  // (p <= n - 1)
-        }
-        frac = sub_rn(p, f);
-    } else {
-        cell_coord(pos, n, hi, i0, frac);
-    }
+    i = (int)v;
+    return (float)i;
 }
 
 // Where the scalar of cell (z, y, x) is back-traced to: the first of the 8
@@ -67,7 +49,7 @@ template <class T, class I> struct CellTrace {
     I at;
     T s, t, u;
 };
-template <bool SMALL, class T, class I>
+template <class T, class I>
 __device__ __forceinline__ CellTrace<T, I> cell_trace(const T* __restrict__ vel, I i, I d, I h, I w, I offy, I offx, T ndt,
                                                       T hix, T hiy, T hiz, FastDiv fw, FastDiv fh,
                                                       CellTrace<T, I>* forward = nullptr) {
@@ -84,9 +66,9 @@ __device__ __forceinline__ CellTrace<T, I> cell_trace(const T* __restrict__ vel,
     auto trace = [&](T step) {
         CellTrace<T, I> c;
         I ix, iy, iz;
-        cell_at<SMALL>(back(cx, step, vcx), w, hix, ix, c.s);
-        cell_at<SMALL>(back(cy, step, vcy), h, hiy, iy, c.t);
-        cell_at<SMALL>(back(cz, step, vcz), d, hiz, iz, c.u);
+        cell_coord(back(cx, step, vcx), w, hix, ix, c.s);
+        cell_coord(back(cy, step, vcy), h, hiy, iy, c.t);
+        cell_coord(back(cz, step, vcz), d, hiz, iz, c.u);
         c.at = (iz * h + iy) * w + ix;
         return c;
     };
@@ -115,13 +97,13 @@ template <class T> __device__ __forceinline__ T trilerp(const T (&c)[8], T s, T 
 }
 
 // advect, 3D extension
-template <bool SMALL, class T, class I>
+template <class T, class I>
 __global__ void k_advect_3d(T* __restrict__ dst, const T* __restrict__ q, const T* __restrict__ vel, Dims D, T ndt,
                             T hix, T hiy, T hiz, FastDiv fw, FastDiv fh) {
     const I d = (I)D.d, h = (I)D.h, w = (I)D.w, hw = h * w;
     const I offy = (I)D.offy(), offx = (I)D.offx();
     GRID_STRIDE(i, d * hw) {
-        const CellTrace<T, I> k = cell_trace<SMALL>(vel, i, d, h, w, offy, offx, ndt, hix, hiy, hiz, fw, fh);
+        const CellTrace<T, I> k = cell_trace<T, I>(vel, i, d, h, w, offy, offx, ndt, hix, hiy, hiz, fw, fh);
         T c[8];
         corners(q, k.at, w, hw, c);
         dst[i] = trilerp(c, k.s, k.t, k.u);
@@ -324,9 +306,6 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 && sizeof(I) == 4 ? k
     }
 }
 
-// Positions inside the grid are in floor_f's range.
-static bool small_sides(const Dims& D) { return std::max(D.d, std::max(D.h, D.w)) <= (i64)kFloorLimit; }
-
 template <class T> int launch_advect(const pg_grid* g, T* dst, const T* src, double dt, const T* vel) {
     const Dims& D = g->dims;
     if (D.h < 2 || D.w < 2 || (D.nd == 3 && D.d < 2))
@@ -338,20 +317,16 @@ template <class T> int launch_advect(const pg_grid* g, T* dst, const T* src, dou
     if (D.nf() < ((i64)1 << 31)) {
         if (D.nd == 2)
             PG_LAUNCH(KK_ADVECT, s, k_advect_2d<T, int><<<nb, kThreads, 0, s>>>(dst, src, vel, (int)D.h, (int)D.w, ndt, hix, hiy));
-        else if (sizeof(T) == 4 && small_sides(D))
-            PG_LAUNCH(KK_ADVECT, s,
-                      k_advect_3d<sizeof(T) == 4, T, int><<<nb, kThreads, 0, s>>>(
-                          dst, src, vel, D, ndt, hix, hiy, hiz, fast_div((unsigned)D.w), fast_div((unsigned)D.h)));
         else
             PG_LAUNCH(KK_ADVECT, s,
-                      k_advect_3d<false, T, int><<<nb, kThreads, 0, s>>>(dst, src, vel, D, ndt, hix, hiy, hiz,
-                                                                         fast_div((unsigned)D.w), fast_div((unsigned)D.h)));
+                      k_advect_3d<T, int><<<nb, kThreads, 0, s>>>(dst, src, vel, D, ndt, hix, hiy, hiz,
+                                                                  fast_div((unsigned)D.w), fast_div((unsigned)D.h)));
     } else {
         if (D.nd == 2)
             PG_LAUNCH(KK_ADVECT, s, k_advect_2d<T, i64><<<nb, kThreads, 0, s>>>(dst, src, vel, D.h, D.w, ndt, hix, hiy));
         else
             PG_LAUNCH(KK_ADVECT, s,
-                      k_advect_3d<false, T, i64><<<nb, kThreads, 0, s>>>(dst, src, vel, D, ndt, hix, hiy, hiz, FastDiv{},
+                      k_advect_3d<T, i64><<<nb, kThreads, 0, s>>>(dst, src, vel, D, ndt, hix, hiy, hiz, FastDiv{},
                                                                   FastDiv{}));
     }
     PG_CHECK_LAUNCH();
@@ -429,7 +404,7 @@ __global__ void k_maccormack(T* __restrict__ dst, const T* __restrict__ q, const
 // and BFECC's last pass reads its values where the limiter reads q's.  The
 // passes one by one (q2 written and read, the velocities averaged and traced
 // again) took 41 + 50 us for MacCormack at 192^3, where it takes 64 now.
-template <bool SMALL, class T>
+template <class T>
 __global__ void k_maccormack_3d(T* __restrict__ dst, const T* __restrict__ q, const T* __restrict__ q1,
                                 const T* __restrict__ vel, Dims D, T ndt, T hix, T hiy, T hiz, FastDiv fw, FastDiv fh) {
     typedef int I;
@@ -437,7 +412,7 @@ __global__ void k_maccormack_3d(T* __restrict__ dst, const T* __restrict__ q, co
     GRID_STRIDE(i, d * hw) {
         CellTrace<T, I> f;
         const CellTrace<T, I> k =
-            cell_trace<SMALL>(vel, i, d, h, w, (I)D.offy(), (I)D.offx(), ndt, hix, hiy, hiz, fw, fh, &f);
+            cell_trace<T, I>(vel, i, d, h, w, (I)D.offy(), (I)D.offx(), ndt, hix, hiy, hiz, fw, fh, &f);
         T c[8], e[8];
         corners(q1, f.at, w, hw, c);
         corners(q, k.at, w, hw, e);
@@ -451,13 +426,13 @@ __global__ void k_maccormack_3d(T* __restrict__ dst, const T* __restrict__ q, co
 }
 
 // qt = q + 0.5 (q - A(q1, -dt))
-template <bool SMALL, class T>
+template <class T>
 __global__ void k_bfecc_pre_3d(T* __restrict__ qt, const T* __restrict__ q, const T* __restrict__ q1,
                                const T* __restrict__ vel, Dims D, T dt, T hix, T hiy, T hiz, FastDiv fw, FastDiv fh) {
     typedef int I;
     const I d = (I)D.d, h = (I)D.h, w = (I)D.w, hw = h * w;
     GRID_STRIDE(i, d * hw) {
-        const CellTrace<T, I> k = cell_trace<SMALL>(vel, i, d, h, w, (I)D.offy(), (I)D.offx(), dt, hix, hiy, hiz, fw, fh);
+        const CellTrace<T, I> k = cell_trace<T, I>(vel, i, d, h, w, (I)D.offy(), (I)D.offx(), dt, hix, hiy, hiz, fw, fh);
         T c[8];
         corners(q1, k.at, w, hw, c);
         qt[i] = add_rn(q[i], mul_rn(T(0.5), sub_rn(q[i], trilerp(c, k.s, k.t, k.u))));
@@ -465,14 +440,14 @@ __global__ void k_bfecc_pre_3d(T* __restrict__ qt, const T* __restrict__ q, cons
 }
 
 // A(qt, dt), limited.
-template <bool SMALL, class T>
+template <class T>
 __global__ void k_bfecc_last_3d(T* __restrict__ dst, const T* __restrict__ qt, const T* __restrict__ q,
                                 const T* __restrict__ q1, const T* __restrict__ vel, Dims D, T ndt, T hix, T hiy, T hiz,
                                 FastDiv fw, FastDiv fh) {
     typedef int I;
     const I d = (I)D.d, h = (I)D.h, w = (I)D.w, hw = h * w;
     GRID_STRIDE(i, d * hw) {
-        const CellTrace<T, I> k = cell_trace<SMALL>(vel, i, d, h, w, (I)D.offy(), (I)D.offx(), ndt, hix, hiy, hiz, fw, fh);
+        const CellTrace<T, I> k = cell_trace<T, I>(vel, i, d, h, w, (I)D.offy(), (I)D.offx(), ndt, hix, hiy, hiz, fw, fh);
         T c[8], e[8];
         corners(qt, k.at, w, hw, c);
         corners(q, k.at, w, hw, e);
@@ -500,7 +475,7 @@ __global__ void k_bfecc_limit(T* __restrict__ dst, const T* __restrict__ q, cons
     }
 }
 
-template <bool SMALL, class T>
+template <class T>
 static int advect2_3d(const pg_grid* g, T* dst, const T* src, double dt, const T* vel, int scheme, const T* t1, T* t2) {
     const Dims& D = g->dims;
     const T ndt = -(T)dt;
@@ -510,12 +485,12 @@ static int advect2_3d(const pg_grid* g, T* dst, const T* src, double dt, const T
     cudaStream_t s = g->stream;
     if (scheme == 1) {
         PG_LAUNCH(KK_ADVECT, s,
-                  k_maccormack_3d<SMALL, T><<<nb, kThreads, 0, s>>>(dst, src, t1, vel, D, ndt, hix, hiy, hiz, fw, fh));
+                  k_maccormack_3d<T><<<nb, kThreads, 0, s>>>(dst, src, t1, vel, D, ndt, hix, hiy, hiz, fw, fh));
     } else {
         PG_LAUNCH(KK_ADVECT, s,
-                  k_bfecc_pre_3d<SMALL, T><<<nb, kThreads, 0, s>>>(t2, src, t1, vel, D, -ndt, hix, hiy, hiz, fw, fh));
+                  k_bfecc_pre_3d<T><<<nb, kThreads, 0, s>>>(t2, src, t1, vel, D, -ndt, hix, hiy, hiz, fw, fh));
         PG_LAUNCH(KK_ADVECT, s,
-                  k_bfecc_last_3d<SMALL, T><<<nb, kThreads, 0, s>>>(dst, t2, src, t1, vel, D, ndt, hix, hiy, hiz, fw, fh));
+                  k_bfecc_last_3d<T><<<nb, kThreads, 0, s>>>(dst, t2, src, t1, vel, D, ndt, hix, hiy, hiz, fw, fh));
     }
     PG_CHECK_LAUNCH();
     return PG_OK;
@@ -529,8 +504,7 @@ int launch_advect2(const pg_grid* g, T* dst, const T* src, double dt, const T* v
     if ((rc = launch_advect<T>(g, t1, src, dt, vel))) return rc;    // q1 = A(q, dt)
     if (D.nf() >= ((i64)1 << 31)) return bad_arg("second-order advection: grid too large for 32-bit indexing");
     if (D.nd == 3)
-        return sizeof(T) == 4 && small_sides(D) ? advect2_3d<sizeof(T) == 4, T>(g, dst, src, dt, vel, scheme, t1, t2)
-                                                : advect2_3d<false, T>(g, dst, src, dt, vel, scheme, t1, t2);
+        return advect2_3d<T>(g, dst, src, dt, vel, scheme, t1, t2);
     if ((rc = launch_advect<T>(g, t2, t1, -dt, vel))) return rc;    // q2 = A(q1, -dt)
     const T ndt = -(T)dt;
     const T hix = (T)((double)D.w - 1.00001), hiy = (T)((double)D.h - 1.00001);
