@@ -118,6 +118,46 @@ struct CgHead {
     }
 };
 
+// Maximum over the warp of values that are not negative and no NaN: their
+// bit patterns order as integers do, off the FP64 pipe.
+__device__ __forceinline__ float warp_max0(float v) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+__device__ __forceinline__ double warp_max0(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)__double2loint(v) : 0u);
+    return __hiloint2double((int)mh, (int)ml);
+}
+__device__ __forceinline__ float max0(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double max0(double a, double b) {  // a, b >= 0, no NaN
+    return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
+template <int NT, class T> __device__ __forceinline__ T block_max0(T v, double* buf) {
+    T* const m = (T*)buf;
+    v = warp_max0(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) m[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return threadIdx.x < 32 ? warp_max0(threadIdx.x < NT / 32 ? m[threadIdx.x] : T(0)) : T(0);
+}
+// block_max0 and block_sum at once, by two warps; buf: NT + 32 doubles.
+template <int NT, class T> __device__ __forceinline__ void block_max0_sum(T& m, double& s, double* buf) {
+    T* const mb = (T*)(buf + NT);
+    m = warp_max0(m);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) mb[threadIdx.x >> 5] = m;
+    buf[threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) s = fold32<NT>(buf);
+    if (threadIdx.x >= 32 && threadIdx.x < 64) {
+        m = warp_max0(threadIdx.x < 32 + NT / 32 ? mb[threadIdx.x - 32] : T(0));
+        if (threadIdx.x == 32) mb[0] = m;
+    }
+    __syncthreads();
+    m = mb[0];
+}
+
 // Device side: fold a freshly reduced z.r into the CG state.  Right after
 // init (iter == 0) it is sigma; afterwards beta = z.r / sigma (pcg.rs:67-68).
 // With the lazy projection on (nfluid > 0) z stands for z - m on the fluid
