@@ -5,7 +5,7 @@
 //
 // A block owns a kSX x kSY column tile and walks a chunk of z planes.  TMA
 // stages every plane of the source vector and p_old (one-cell halo) and of
-// the face flags (tile and halo) into a kSStages-deep shared-memory ring; for
+// the face flags (tile and halo) into a ring of shared-memory stages; for
 // plane q+1 the block computes p_new = z + beta p_old on the tile and its
 // one-cell ring into a 4-slot plane ring (and stores the tile's values), then
 // A p_new of plane q from the slots of planes q-1, q and q+1.  A staged plane
@@ -27,7 +27,6 @@ namespace {
 
 constexpr int kSX = 64, kSWarps = 8, kSRows = 2, kSY = kSWarps * kSRows;
 constexpr int kSThreads = 32 * kSWarps;
-constexpr int kSStages = 7;
 constexpr int kSVw = kSX + 8, kSVh = kSY + 2;  // z / p_old boxes from (x0 - 4, y0 - 1)
 constexpr int kSGw = kSX + 32, kSGh = kSY + 2;  // flags box from (x0 - 16, y0 - 1)
 constexpr int kSVBytes = kSVw * kSVh * 4;
@@ -37,8 +36,15 @@ constexpr int kSPOff = kSVPad, kSGOff = 2 * kSVPad;
 constexpr int kSStageBytes = kSGOff + ((kSGBytes + 127) / 128) * 128;
 constexpr int kSSw = kSX + 2, kSSh = kSY + 2;  // p_new of one plane (tile + ring)
 constexpr int kSSlotBytes = kSSw * kSSh * 4;
-constexpr int kSBarOff = kSStages * kSStageBytes + 4 * kSSlotBytes;
-constexpr size_t kSSmem = 128 + kSBarOff + kSStages * 8;
+// Planes in the ring, and the blocks per SM that they leave room for.  In the
+// multigrid solve more warps are worth more than planes in flight: 72 -> 69 us
+// at 256^3 and 634 -> 589 at 512^3 against 7 planes and two blocks, which plain
+// and Jacobi CG keep, and with them the order of their sums.
+template <int PM> struct SpmvCfg {
+    static constexpr int kStages = PM == PM_ZBUF ? 4 : 7, kBlocks = PM == PM_ZBUF ? 3 : 2;
+    static constexpr int kBarOff = kStages * kSStageBytes + 4 * kSSlotBytes;
+    static constexpr size_t kSmem = 128 + kBarOff + kStages * 8;
+};
 constexpr unsigned kSTx = 2 * kSVBytes + kSGBytes;
 static_assert(kSStageBytes % 128 == 0, "TMA boxes must stay 128-byte aligned");
 
@@ -52,14 +58,15 @@ struct SpmvArgs {
 };
 
 template <int PM>
-__global__ void __launch_bounds__(kSThreads, 2)
+__global__ void __launch_bounds__(kSThreads, SpmvCfg<PM>::kBlocks)
     k_cg_spmv3p(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUtensorMap pmap0,
                 const __grid_constant__ CUtensorMap pmap1, const __grid_constant__ CUtensorMap gmap, SpmvArgs a,
                 CgState* st, double* partials) {
+    constexpr int kSStages = SpmvCfg<PM>::kStages;
     extern __shared__ unsigned char spmv_smem_raw[];
     unsigned char* const base = spmv_smem_raw + ((128u - (smem_u32(spmv_smem_raw) & 127u)) & 127u);
     float(*const S)[kSSh][kSSw] = (float(*)[kSSh][kSSw])(base + kSStages * kSStageBytes);
-    uint64_t* const bars = (uint64_t*)(base + kSBarOff);
+    uint64_t* const bars = (uint64_t*)(base + SpmvCfg<PM>::kBarOff);
     const int tid = threadIdx.x, lane = tid & 31, ty = tid >> 5;
     // Jacobi: 1 / (n dt) for n open faces, computed as in zval (0 for n = 0)
     __shared__ float inv_diag[8];
@@ -449,10 +456,10 @@ template <int PM> static int spmv_cap(int num_sms) {
     static int cap = -1;
     if (cap < 0) {
         cap = 0;
-        if (cudaFuncSetAttribute(k_cg_spmv3p<PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSSmem) ==
+        if (cudaFuncSetAttribute(k_cg_spmv3p<PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SpmvCfg<PM>::kSmem) ==
             cudaSuccess) {
             int bps = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cg_spmv3p<PM>, kSThreads, kSSmem) ==
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cg_spmv3p<PM>, kSThreads, SpmvCfg<PM>::kSmem) ==
                 cudaSuccess)
                 cap = std::min(bps * num_sms, kMaxBlocks);
         }
@@ -491,11 +498,11 @@ bool spmv_tma_launch(cudaStream_t s, int num_sms, int pm, const float* zb, float
     a.tiles_y = (a.h + kSY - 1) / kSY;
     const int nb = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, cap, pm == PM_ZBUF ? kZMinPlanesMg : kZMinPlanes);
     if (pm == PM_ZBUF)
-        launch_dep(D.nc(), k_cg_spmv3p<PM_ZBUF>, nb, kSThreads, kSSmem, s, zm, pm0, pm1, gm, a, st, partials);
+        launch_dep(D.nc(), k_cg_spmv3p<PM_ZBUF>, nb, kSThreads, SpmvCfg<PM_ZBUF>::kSmem, s, zm, pm0, pm1, gm, a, st, partials);
     else if (pm == PM_JACOBI)
-        launch_dep(D.nc(), k_cg_spmv3p<PM_JACOBI>, nb, kSThreads, kSSmem, s, zm, pm0, pm1, gm, a, st, partials);
+        launch_dep(D.nc(), k_cg_spmv3p<PM_JACOBI>, nb, kSThreads, SpmvCfg<PM_JACOBI>::kSmem, s, zm, pm0, pm1, gm, a, st, partials);
     else
-        launch_dep(D.nc(), k_cg_spmv3p<PM_NONE>, nb, kSThreads, kSSmem, s, zm, pm0, pm1, gm, a, st, partials);
+        launch_dep(D.nc(), k_cg_spmv3p<PM_NONE>, nb, kSThreads, SpmvCfg<PM_NONE>::kSmem, s, zm, pm0, pm1, gm, a, st, partials);
     return true;
 }
 
