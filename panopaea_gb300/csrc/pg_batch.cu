@@ -107,10 +107,12 @@ __global__ void k_b_rhs(float* __restrict__ b, const float* __restrict__ vel, co
             if (interior) return !(f & bit);
             return fsolid != nullptr && fsolid[idx] != 0;
         };
-        const float top = masked(iyl, y > 0, YLO) ? 0.f : -vel[iyl];
-        const float bottom = masked(iyh, y < G.h - 1, YHI) ? 0.f : -vel[iyh];
-        const float ux_lo = masked(ixl, x > 0, XLO) ? 0.f : vel[ixl];
-        const float ux_hi = masked(ixh, x < G.w - 1, XHI) ? 0.f : vel[ixh];
+        // (every face is loaded, masked or not, so that no load waits for the flags)
+        const float vyl = vel[iyl], vyh = vel[iyh], vxl = vel[ixl], vxh = vel[ixh];
+        const float top = masked(iyl, y > 0, YLO) ? 0.f : -vyl;
+        const float bottom = masked(iyh, y < G.h - 1, YHI) ? 0.f : -vyh;
+        const float ux_lo = masked(ixl, x > 0, XLO) ? 0.f : vxl;
+        const float ux_hi = masked(ixh, x < G.w - 1, XHI) ? 0.f : vxh;
         b[c] = -add_rn(sub_rn(add_rn(-bottom, top), ux_lo), ux_hi);
     }
 }
@@ -126,26 +128,26 @@ __global__ void k_b_project(float* __restrict__ vel, const float* __restrict__ p
         const i64 n0 = (i64)(G.h + 1) * G.w;
         const float* pp = p + G.coff;
         const uint8_t* fl = flags + G.coff;
-        if (y < G.h && x <= G.w) {  // x face
-            const i64 i = G.foff + n0 + (i64)y * (G.w + 1) + x;
-            if (x == 0 || x == G.w) {
-                vel[i] = 0.f;
-            } else {
-                const i64 c = (i64)y * G.w + x;
-                const float e = sub_rn(pp[c - 1], pp[c]);
-                vel[i] = (zero_solid && !(fl[c] & XLO)) ? 0.f : add_rn(vel[i], mul_rn(dt, e));
-            }
+        // everything is loaded before anything is stored
+        const bool hx = y < G.h && x <= G.w, hy = y <= G.h && x < G.w;
+        const bool in_x = hx && x > 0 && x < G.w, in_y = hy && y > 0 && y < G.h;
+        const i64 ix = G.foff + n0 + (i64)y * (G.w + 1) + x, iy = G.foff + (i64)y * G.w + x, c = (i64)y * G.w + x;
+        unsigned f = 0;
+        float pc = 0.f, px = 0.f, py = 0.f, vx = 0.f, vy = 0.f;
+        if (in_x || in_y) {
+            f = fl[c];
+            pc = pp[c];
         }
-        if (y <= G.h && x < G.w) {  // y face
-            const i64 i = G.foff + (i64)y * G.w + x;
-            if (y == 0 || y == G.h) {
-                vel[i] = 0.f;
-            } else {
-                const i64 c = (i64)y * G.w + x;
-                const float e = -sub_rn(pp[c], pp[c - G.w]);
-                vel[i] = (zero_solid && !(fl[c] & YLO)) ? 0.f : add_rn(vel[i], mul_rn(dt, e));
-            }
+        if (in_x) {
+            px = pp[c - 1];
+            vx = vel[ix];
         }
+        if (in_y) {
+            py = pp[c - G.w];
+            vy = vel[iy];
+        }
+        if (hx) vel[ix] = in_x && !(zero_solid && !(f & XLO)) ? add_rn(vx, mul_rn(dt, sub_rn(px, pc))) : 0.f;
+        if (hy) vel[iy] = in_y && !(zero_solid && !(f & YLO)) ? add_rn(vy, mul_rn(dt, -sub_rn(pc, py))) : 0.f;
     }
 }
 
