@@ -364,16 +364,23 @@ constexpr int kPStages = 6;              // plane ring; loads run kPStages - 3 p
 constexpr int kPEw = kPX + 8, kPEh = kPY + 4;    // ein box from (x0 - 4, y0 - 2)
 constexpr int kPFw = kPX + 8, kPFh = kPY + 2;    // f box from (x0 - 4, y0 - 1)
 constexpr int kPGw = kPX + 32, kPGh = kPY + 2;   // flags box from (x0 - 16, y0 - 1)
-constexpr int kPEBytes = kPEw * kPEh * 4;        // 3456
-constexpr int kPFBytes = kPFw * kPFh * 4;        // 2880
-constexpr int kPGBytes = kPGw * kPGh;            // 960
+constexpr int kPEBytes = kPEw * kPEh * 4;        // 5760
+constexpr int kPFBytes = kPFw * kPFh * 4;        // 5184
+constexpr int kPGBytes = kPGw * kPGh;            // 1728
 constexpr int kPCw = kPX / 2 + 8, kPCh = kPY / 2 + 2;  // coarse-correction box from (x0/2 - 4, y0/2 - 1)
-constexpr int kPCBytes = kPCw * kPCh * 4;        // 960
+constexpr int kPCBytes = kPCw * kPCh * 4;        // 1600
 constexpr int kPFOff = kPEBytes;                 // every box starts on 128 bytes
 constexpr int kPGOff = kPFOff + ((kPFBytes + 127) / 128) * 128;
 constexpr int kPCOff = kPGOff + ((kPGBytes + 127) / 128) * 128;
-constexpr int kPSw = kPX + 2, kPSh = kPY + 2;    // new c1 values of one plane (tile + ring)
-constexpr int kPSlotBytes = kPSw * kPSh * 4;
+// New c1 values of one plane (tile + ring), without the c2 cells between
+// them: cell xl of a row is entry (xl + 1) / 2, so that a warp's accesses are
+// to consecutive words (two-way bank conflicts before) and the cell's own c1
+// value is one of its x neighbours.  256^3: plain pair 64 -> 60.6 us, with
+// z.r 75 -> 69, noise step 3.80 -> 3.73 ms.  A third block per SM (five
+// stages) changed nothing for the plain pairs; one 512-thread block on 64 x 32
+// tiles (fewer halos, wider barriers) made the step 3.83 ms.
+constexpr int kPSw = kPX / 2 + 1, kPSh = kPY + 2;
+constexpr int kPSlotBytes = ((kPSw * kPSh * 4 + 15) / 16) * 16;
 
 enum { PR_SELF = 0 /* c1 = f * invd (e = 0 before) */, PR_PLAIN = 1, PR_PROLONG = 2 /* ein + ec[parent] */ };
 
@@ -411,7 +418,9 @@ __global__ void __launch_bounds__(kPThreads, kPMinBlocks)
     // 128-byte aligned by an offset (pointer arithmetic keeps every access
     // below in the shared window: LDS/STS, not generic loads)
     unsigned char* const base = pair_smem_raw + ((128u - (smem_u32(pair_smem_raw) & 127u)) & 127u);
-    float(*const S1)[kPSh][kPSw] = (float(*)[kPSh][kPSw])(base + kStages * kStageBytes);
+    auto S1 = [&](int plane, int yl, int k) -> float& {
+        return ((float*)(base + kStages * kStageBytes + (plane & 3) * kPSlotBytes))[(yl + 1) * kPSw + k];
+    };
     uint64_t* const bars = (uint64_t*)(base + Cfg::kBarOff);
     const int tid = threadIdx.x, lane = tid & 31, ty = tid >> 5;
     const float dt = a.dt;
@@ -512,17 +521,17 @@ __global__ void __launch_bounds__(kPThreads, kPMinBlocks)
 #pragma unroll
             for (int r = 0; r < kPRows; ++r) {
                 const int yl = ty + r * kPWarps;
-                const int xl = 2 * lane + ((a.c1 + y0 + yl + p) & 1);
-                S1[p & 3][yl + 1][xl + 1] = c1_cell(yl, xl);
+                const int odd = (a.c1 + y0 + yl + p) & 1;
+                S1(p, yl, lane + odd) = c1_cell(yl, 2 * lane + odd);
             }
             if (tid < 64) {  // ring rows y0 - 1 and y0 + kPY
                 const int yl = tid < 32 ? -1 : kPY;
-                const int xl = 2 * lane + ((a.c1 + y0 + yl + p) & 1);
-                S1[p & 3][yl + 1][xl + 1] = c1_cell(yl, xl);
+                const int odd = (a.c1 + y0 + yl + p) & 1;
+                S1(p, yl, lane + odd) = c1_cell(yl, 2 * lane + odd);
             } else if (tid < 64 + 2 * kPY) {  // ring columns x0 - 1 and x0 + kPX
                 const int k = tid - 64;
                 const int xl = k < kPY ? -1 : kPX, yl = k < kPY ? k : k - kPY;
-                if (((x0 + xl + y0 + yl + p) & 1) == a.c1) S1[p & 3][yl + 1][xl + 1] = c1_cell(yl, xl);
+                if (((x0 + xl + y0 + yl + p) & 1) == a.c1) S1(p, yl, (xl + 1) >> 1) = c1_cell(yl, xl);
             }
             // the next step's plane p + 2 must have landed
             if (seq + i + 3 < seq + n) wait(seq + i + 3);
@@ -537,13 +546,13 @@ __global__ void __launch_bounds__(kPThreads, kPMinBlocks)
 #pragma unroll
                 for (int r = 0; r < kPRows; ++r) {
                     const int yl = ty + r * kPWarps, gy = y0 + yl;
-                    const int xl2 = 2 * lane + ((a.c1 + 1 + gy + q) & 1), xl1 = xl2 ^ 1;
-                    const float e1 = S1[q & 3][yl + 1][xl1 + 1];
+                    const int odd = (a.c1 + 1 + gy + q) & 1, k = lane + odd;
+                    const int xl2 = 2 * lane + odd, xl1 = xl2 ^ 1;
+                    const float exl = S1(q, yl, lane), exh = S1(q, yl, lane + 1);
+                    const float e1 = odd ? exl : exh;
                     const float fv = Fv(Pm, yl + 1, xl2 + 4);
-                    const float e2 =
-                        gs(Gv(Pm, yl + 1, xl2 + 16), fv, S1[q & 3][yl + 1][xl2], S1[q & 3][yl + 1][xl2 + 2],
-                           S1[q & 3][yl][xl2 + 1], S1[q & 3][yl + 2][xl2 + 1], S1[(q - 1) & 3][yl + 1][xl2 + 1],
-                           S1[(q + 1) & 3][yl + 1][xl2 + 1]);
+                    const float e2 = gs(Gv(Pm, yl + 1, xl2 + 16), fv, exl, exh, S1(q, yl - 1, k), S1(q, yl + 1, k),
+                                        S1(q - 1, yl, k), S1(q + 1, yl, k));
                     const int x = x0 + 2 * lane;
                     if (gy < h && x < w) {
                         const float2 v = (xl1 & 1) ? make_float2(e2, e1) : make_float2(e1, e2);
