@@ -359,8 +359,7 @@ constexpr int kPX = 64;
 constexpr int kPWarps = 8, kPRows = 2;  // warps per block, tile rows per thread
 constexpr int kPY = kPWarps * kPRows;
 constexpr int kPThreads = 32 * kPWarps;  // one (c1, c2) x-pair per thread, row and plane
-constexpr int kPMinBlocks = 2;           // resident blocks per SM the registers are sized for
-constexpr int kPStages = 6;              // plane ring; loads run kPStages - 3 planes ahead
+constexpr int kPStages = 5;              // plane ring; loads run kPStages - 3 planes ahead
 constexpr int kPEw = kPX + 8, kPEh = kPY + 4;    // ein box from (x0 - 4, y0 - 2)
 constexpr int kPFw = kPX + 8, kPFh = kPY + 2;    // f box from (x0 - 4, y0 - 1)
 constexpr int kPGw = kPX + 32, kPGh = kPY + 2;   // flags box from (x0 - 16, y0 - 1)
@@ -376,20 +375,20 @@ constexpr int kPCOff = kPGOff + ((kPGBytes + 127) / 128) * 128;
 // them: cell xl of a row is entry (xl + 1) / 2, so that a warp's accesses are
 // to consecutive words (two-way bank conflicts before) and the cell's own c1
 // value is one of its x neighbours.  256^3: plain pair 64 -> 60.6 us, with
-// z.r 75 -> 69, noise step 3.80 -> 3.73 ms.  A third block per SM (five
-// stages) changed nothing for the plain pairs; one 512-thread block on 64 x 32
-// tiles (fewer halos, wider barriers) made the step 3.83 ms.
+// z.r 75 -> 69, noise step 3.80 -> 3.73 ms.  One 512-thread block
+// per SM on 64 x 32 tiles (fewer halos, wider barriers) made the step 3.83 ms.
 constexpr int kPSw = kPX / 2 + 1, kPSh = kPY + 2;
 constexpr int kPSlotBytes = ((kPSw * kPSh * 4 + 15) / 16) * 16;
 
 enum { PR_SELF = 0 /* c1 = f * invd (e = 0 before) */, PR_PLAIN = 1, PR_PROLONG = 2 /* ein + ec[parent] */ };
 
 // Shared-memory layout per first-sweep mode: the prolonging pair also
-// stages the coarse correction's parent plane and runs one stage fewer
-// (kPMinBlocks blocks stay resident per SM).
+// stages the coarse correction's parent plane
+// (two blocks stay resident per SM; three of the other modes).
 template <int M1> struct PairCfg {
     static constexpr bool kCoarse = M1 == PR_PROLONG;
-    static constexpr int kStages = kCoarse ? 5 : kPStages;
+    static constexpr int kStages = kPStages;
+    static constexpr int kMinBlocks = kCoarse ? 2 : 3;  // resident blocks per SM the registers are sized for
     static constexpr int kStageBytes = kPCOff + (kCoarse ? ((kPCBytes + 127) / 128) * 128 : 0);
     static constexpr int kBarOff = kStages * kStageBytes + 4 * kPSlotBytes;
     static constexpr size_t kSmem = 128 + kBarOff + kStages * 8;
@@ -407,7 +406,7 @@ struct PairArgs {
 };
 
 template <int M1, bool RZ>
-__global__ void __launch_bounds__(kPThreads, kPMinBlocks)
+__global__ void __launch_bounds__(kPThreads, PairCfg<M1>::kMinBlocks)
     k_mg_pair(const __grid_constant__ CUtensorMap emap, const __grid_constant__ CUtensorMap fmap,
               const __grid_constant__ CUtensorMap gmap, const __grid_constant__ CUtensorMap cmap, PairArgs a,
               CgState* st, double* partials) {
@@ -2047,9 +2046,21 @@ static bool pair_plan(const MgHierarchy& H, const float* r, const float* z, Pair
     a.tiles_x = (a.w + kPX - 1) / kPX;
     a.tiles_y = (a.h + kPY - 1) / kPY;
     a.l2keep = H.l2keep;
-    // every resident block, each with an equal share of the plane-tiles
-    P->nb_plain = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, H.pair_cap_plain, kZMinPlanesMg);
-    P->nb_prolong = zwalk_blocks(a.tiles_x * a.tiles_y, a.d, H.pair_cap, kZMinPlanesMg);
+    // Every resident block, each with an equal share of the plane-tiles; the
+    // same number of blocks for every column of tiles where that leaves less
+    // than 1/32 of them out: neighbouring columns are then walked in step and
+    // meet their halos in L2 (256^3, 448 blocks: 165 MB read from DRAM by a
+    // plain pair for 237, 52.9 us for 60.6; noise step 3.73 -> 3.68 ms; 256
+    // blocks of 304 read 158 MB but take 63.8).  At 512^3 256 of 456 blocks
+    // would be whole: all 456 run, out of step, 1.02x its step before; 304 of
+    // them took 5% longer.
+    const int cols = a.tiles_x * a.tiles_y;
+    auto blocks = [&](int cap) {
+        const int nb = zwalk_blocks(cols, a.d, cap, kZMinPlanesMg), whole = nb / cols * cols;
+        return nb - whole <= nb / 32 ? whole : nb;
+    };
+    P->nb_prolong = blocks(H.pair_cap);
+    P->nb_plain = blocks(H.pair_cap_plain);
     return true;
 }
 
