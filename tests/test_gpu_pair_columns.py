@@ -7,6 +7,6 @@ import test_gpu_mg as mg
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dims", [(40, 16, 64), (9, 33, 208), (150, 72, 160), (8, 368, 1600)])
+@pytest.mark.parametrize("dims", [(40, 16, 64), (9, 33, 208), (150, 72, 160), (64, 176, 320)])
 def test_pairs_by_columns(pg, oracle, dims, monkeypatch):
     mg.test_fused_pairs_equal_half_sweeps(pg, oracle, dims, 1, monkeypatch)
