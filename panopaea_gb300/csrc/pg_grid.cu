@@ -16,6 +16,7 @@ int cuda_fail(cudaError_t e, const char* what) {
     char buf[512];
     snprintf(buf, sizeof buf, "%s: %s (%s)", what, cudaGetErrorString(e), cudaGetErrorName(e));
     set_error(buf);
+    cudaGetLastError();  // reported here: the next call's launch check must not find it again
     if (e == cudaErrorMemoryAllocation) return PG_OUT_OF_MEMORY;
     if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return PG_NO_DEVICE;
     return PG_CUDA_ERROR;

@@ -1753,8 +1753,7 @@ int pg_unet_create(int64_t d, int64_t h, int64_t w, pg_unet** out) {
     cudaError_t e = cudaMalloc(&net->arena, total);
     if (e != cudaSuccess) {
         delete net;
-        set_error("pg_unet_create: cudaMalloc failed");
-        return e == cudaErrorMemoryAllocation ? PG_OUT_OF_MEMORY : PG_CUDA_ERROR;
+        return cuda_fail(e, "pg_unet_create: cudaMalloc");
     }
     char* base = (char*)net->arena;
     for (auto& p : parts) {

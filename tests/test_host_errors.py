@@ -1,0 +1,40 @@
+"""A CUDA error that one call has returned is not returned again by the next
+(the runtime keeps it until it is asked for).  On the CPU, with the runtime's
+calls faked (tests/host_cuda.py)."""
+import pytest
+
+from host_cuda import host_cuda  # noqa: F401
+
+SCRIPT = r"""
+dims = (64, 80)
+g, x, b = grid(dims), cells(dims), cells(dims)
+result = []
+for precond, refine in ((0, 0), (1, 0), (2, 0), (2, 3)):
+    p, st = solver(precond=precond, refine=refine), N.PcgStats()
+    solve = lambda: lib.pg_solve_pressure_f32(g, C.byref(p), x, b, 0.5, C.byref(st))
+    fake.fake_fail_allocation(0)
+    first = solve()
+    fake.fake_fail_allocation(-1)
+    result.append((precond, refine, first, solve()))
+    h = grid(dims)  # (the next setting allocates again)
+    lib.pg_grid_destroy(g)
+    g = h
+
+# a network: its arena, then a call that checks its launches
+net, params = C.c_void_p(), cells((int(lib.pg_unet_num_params()),))
+fake.fake_fail_allocation(0)
+first = lib.pg_unet_create(16, 16, 16, C.byref(net))
+fake.fake_fail_allocation(-1)
+assert lib.pg_unet_create(16, 16, 16, C.byref(net)) == 0
+g = grid((16, 16, 16))
+x, b = cells((16, 16, 16)), cells((16, 16, 16))
+result.append(("unet", 0, first, lib.pg_unet_set_params(net, params, 1.0) or lib.pg_unet_forward_f32(net, g, b, 0.5, x)))
+"""
+
+
+def test_a_failed_allocation_is_reported_once(host_cuda):  # noqa: F811
+    rows = host_cuda(SCRIPT)
+    failed = [r for r in rows if r[2] == 7]
+    assert len(failed) >= 4 and failed[-1][0] == "unet", rows
+    for precond, refine, _, again in failed:
+        assert again == 0, (precond, refine, again)
