@@ -1809,7 +1809,6 @@ static int coarsest_pinv(pg_grid* g, MgHierarchy* H) {
     return PG_OK;
 }
 
-// (Re)build the hierarchy for the grid's current mask and dt.
 // The strips and twins of the 2D levels above the tail: chunks of 32 rows, of
 // fewer where those would leave SMs idle.
 static int march_setup(pg_grid* g, MgHierarchy* H) {
@@ -1830,13 +1829,9 @@ static int march_setup(pg_grid* g, MgHierarchy* H) {
     return PG_OK;
 }
 
-static int ensure_mg(pg_grid* g, double dt, MgHierarchy** out) {
-    Extras* ex = extras_of(g);
-    if (ex->mg && ex->mg->dt == dt && ex->mg->mask_version == g->mask_version) {
-        *out = ex->mg;
-        return PG_OK;
-    }
-    release_mg(ex);
+// The hierarchy of the grid's current mask and dt as ex->mg; on an error what
+// there is of it.
+static int build_mg(pg_grid* g, Extras* ex, double dt) {
     if (g->dims.nc() >= (i64)1 << 31) return bad_arg("PG_PRECOND_MG: grid too large for 32-bit level indexing");
     MgHierarchy* H = new MgHierarchy();
     H->id = next_hierarchy_id();
@@ -1961,8 +1956,22 @@ static int ensure_mg(pg_grid* g, double dt, MgHierarchy** out) {
         }
     }
     PG_CHECK_LAUNCH();
-    if (const int crc = coarsest_pinv(g, H)) return crc;
-    *out = H;
+    return coarsest_pinv(g, H);
+}
+
+// (Re)build the hierarchy for the grid's current mask and dt.  One whose build
+// failed is not kept: its key would match the next solve's.
+static int ensure_mg(pg_grid* g, double dt, MgHierarchy** out) {
+    Extras* ex = extras_of(g);
+    if (!ex->mg || ex->mg->dt != dt || ex->mg->mask_version != g->mask_version) {
+        release_mg(ex);
+        const int rc = build_mg(g, ex, dt);
+        if (rc) {
+            release_mg(ex);
+            return rc;
+        }
+    }
+    *out = ex->mg;
     return PG_OK;
 }
 
