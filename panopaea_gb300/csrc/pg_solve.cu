@@ -66,6 +66,7 @@ int Extras::buffer(int slot, size_t bytes, void** out) {
 
 Extras::~Extras() {
     for (int i = 0; i < kSlots; ++i) cudaFree(buf_[i]);
+    cudaFree(small);
     release_mg(this);
 }
 

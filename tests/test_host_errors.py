@@ -1,6 +1,7 @@
-"""A CUDA error that one call has returned is not returned again by the next
-(the runtime keeps it until it is asked for).  On the CPU, with the runtime's
-calls faked (tests/host_cuda.py)."""
+"""What the host code does with errors and memory, on the CPU with the runtime's
+calls faked (tests/host_cuda.py): a CUDA error that one call has returned is
+not returned again by the next (the runtime keeps it until it is asked for),
+and a destroyed grid leaves no device memory behind."""
 import pytest
 
 from host_cuda import host_cuda  # noqa: F401
@@ -38,3 +39,21 @@ def test_a_failed_allocation_is_reported_once(host_cuda):  # noqa: F811
     assert len(failed) >= 4 and failed[-1][0] == "unet", rows
     for precond, refine, _, again in failed:
         assert again == 0, (precond, refine, again)
+
+
+LEAK = r"""
+result = []
+for dims in ((64, 80), (32, 32, 32)):
+    for precond, refine in ((0, 0), (1, 2), (2, 0), (2, 3)):
+        live = fake.fake_live()
+        g, x, b = grid(dims), cells(dims), cells(dims)
+        p, st = solver(precond=precond, refine=refine), N.PcgStats()
+        rc = lib.pg_solve_pressure_f32(g, C.byref(p), x, b, 0.5, C.byref(st))
+        lib.pg_grid_destroy(g)
+        result.append((dims, precond, refine, rc, fake.fake_live() - live))
+"""
+
+
+def test_a_destroyed_grid_leaves_no_memory(host_cuda):  # noqa: F811
+    for dims, precond, refine, rc, left in host_cuda(LEAK):
+        assert rc == 0 and left == 0, (dims, precond, refine, rc, left)
