@@ -22,12 +22,13 @@
 // there move alpha by an FP32 ulp now and then, and 100 iterations on the
 // residual by 5e-6 of its norm, no closer to the exact one.)
 //
-// Measured, plain CG per iteration, the loop of two kernels against this:
-// 128^2 17.8 / 8.2 us, 384^2 24.2 / 13.5, 550 x 560 36.6 / 18.4, 64^3 34.8 /
-// 23.7.  Of the 8.2 us each exchange is about 3 (FP64 folds and a division at
-// 60 to 100 cycles per dependent operation, the trip through L2, fences).
-// Above kCoopMaxCells cells per thread the loop is at its memory traffic and
-// stays.
+// Measured, plain CG (Jacobi) per iteration, the loop of two kernels against
+// this: 128^2 13.9 / 8.0 us (17.2 / 8.2), 384^2 21.4 / 13.3 (37.0 / 14.1), 550 x
+// 560 32.2 / 18.3 (56.3 / 19.8), 64^3 39.9 / 23.6 (65.7 / 25.7).  Of the 8.0 us
+// each exchange is about 3 (FP64 folds and a division at 60 to 100 cycles per
+// dependent operation, the trip through L2, fences).  Above kCoopMaxCells
+// cells per thread the loop is at its memory traffic and stays, and so it does
+// where rows or planes are large beside a block's cells (coop_pays).
 #include <algorithm>
 #include <cstdlib>
 
@@ -72,12 +73,11 @@ __device__ __forceinline__ void coop_st2(unsigned long long* p, unsigned long lo
     asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
 }
 
-// z = M^-1 r at a cell with face-open bits f (as zof).
-template <int PM> __device__ __forceinline__ double coop_z(double rv, unsigned f, double dt) {
-    if (PM == PM_JACOBI) {
-        const int k = __popc(f);
-        return k ? rv * __drcp_rn((double)k * dt) : 0.0;
-    }
+// z = M^-1 r at a cell with face-open bits f (as zof).  inv_diag[k]: 1 / (k dt),
+// formed once per block: an FP64 reciprocal for every cell and halo cell took
+// half of a Jacobi iteration (64^3 41.5 us, 26.0 with the table).
+template <int PM> __device__ __forceinline__ double coop_z(double rv, unsigned f, const double* inv_diag) {
+    if (PM == PM_JACOBI) return f ? rv * inv_diag[__popc(f)] : 0.0;
     return rv;
 }
 
@@ -87,6 +87,7 @@ struct CoopShared {
     double sum, max;
     double scale;  // alpha or beta for the block
     int stop, bad;
+    double inv_diag[8];  // Jacobi
 };
 
 // Sum and, with MAX, maximum (>= 0) of every thread of the grid, the number of
@@ -184,6 +185,10 @@ __global__ void __launch_bounds__(kCoopMaxThreads) k_cg_coop(CoopArgs a) {
     unsigned number = 0;
     double sig = 0.0, bm = 0.0;
     bool bad = false;
+    if (PM == PM_JACOBI) {
+        if (tid < 8) sh.inv_diag[tid] = tid ? __drcp_rn((double)tid * a.dt) : 0.0;
+        __syncthreads();
+    }
 #pragma unroll
     for (int j = 0; j < K; ++j) {
         x[j] = p[j] = ap[j] = r[j] = 0.0;
@@ -196,7 +201,7 @@ __global__ void __launch_bounds__(kCoopMaxThreads) k_cg_coop(CoopArgs a) {
         a.r[base + l] = bv;
         bm = fmax(bm, fabs(bv));
         bad |= !isfinite(bv);
-        sig += coop_z<PM>(bv, f[j], a.dt) * bv;
+        sig += coop_z<PM>(bv, f[j], sh.inv_diag) * bv;
     }
     double sigma = 0.0, thr = 0.0, bmax = 0.0, rmax = 0.0, pap = 0.0, alpha = 0.0, beta = 0.0;  // thread 0
     int status = PG_NOT_CONVERGED;
@@ -226,14 +231,14 @@ __global__ void __launch_bounds__(kCoopMaxThreads) k_cg_coop(CoopArgs a) {
         for (int k = tid; k < 2 * a.H; k += nt) {
             const int c = k < a.H ? base - a.H + k : base + cnt + (k - a.H);
             if (c < 0 || c >= a.n) continue;
-            const double z = coop_z<PM>(__ldcg(a.r + c), PM == PM_JACOBI ? a.flags[c] : 0u, a.dt);
+            const double z = coop_z<PM>(__ldcg(a.r + c), PM == PM_JACOBI ? a.flags[c] : 0u, sh.inv_diag);
             S[c - base + a.H] = first ? z : z + bt * __ldcg(p_old + c);
         }
 #pragma unroll
         for (int j = 0; j < K; ++j) {
             const int l = j * nt + tid;
             if (l >= cnt) continue;
-            const double z = coop_z<PM>(r[j], f[j], a.dt);
+            const double z = coop_z<PM>(r[j], f[j], sh.inv_diag);
             p[j] = first ? z : z + bt * p[j];
             S[l + a.H] = p[j];
             p_new[base + l] = p[j];
@@ -287,7 +292,7 @@ __global__ void __launch_bounds__(kCoopMaxThreads) k_cg_coop(CoopArgs a) {
             a.r[base + l] = rv;
             rm = fmax(rm, fabs(rv));
             bad |= !isfinite(rv);
-            rz += coop_z<PM>(rv, f[j], a.dt) * rv;
+            rz += coop_z<PM>(rv, f[j], sh.inv_diag) * rv;
         }
         live = coop_exchange<true, true>(sh, a.slots, ++number, rz, rm, bad, [&] {
 #pragma unroll
@@ -361,6 +366,21 @@ int coop_launch(cudaStream_t s, int blocks, int threads, size_t smem, CoopArgs& 
     return e == cudaSuccess ? PG_OK : cuda_fail(e, "cooperative CG launch");
 }
 
+// Whether an iteration with C cells per block and rows (planes) of H cells is
+// faster here than in the loop.  A block computes p of its 2 H halo cells from
+// global memory, 0.27 us per 512 of them, which the loop does not.  An
+// iteration of the loop is at its launch latency on small grids, 14 us in 2D
+// (and from 30 K cells on grows, 1 us per 15 K), 20 in 3D up to about 120 K
+// cells (C of 800) and 33 beyond, so the halo may be as large as what that
+// leaves.  Measured, plain CG per iteration, the loop / this: 10 x 3000 14.3 /
+// 13.3, 5 x 5000 14.5 / 15.5, 20 x 6000 20.1 / 19.0, 18 x 9000 23.3 / 24.1, 25 x
+// 10000 29.9 / 27.8; 16 x 80 x 80 20.5 / 19.7, 8 x 100 x 100 20.3 / 23.6, 12 x 90
+// x 90 20.2 / 21.5, 12 x 100 x 100 33.4 / 24.9.  (Jacobi gains more everywhere.)
+bool coop_pays(int nd, i64 C, i64 H) {
+    if (nd == 2) return 2 * H <= 6000 + 9 * C;
+    return C >= 800 || H <= 6400;
+}
+
 bool coop_enabled() {
     const char* env = getenv("PG_CG_COOP");
     return !(env && env[0] == '0');
@@ -376,8 +396,8 @@ int set_stage_wait_polls_coop(unsigned polls) {
 size_t cg_coop_bytes() { return 2 * kCoopMaxBlocks * sizeof(CoopSlot); }
 
 // The whole solve in one cooperative launch where it applies (*done): grids
-// whose cells fit the registers of one block per SM and whose rows (planes)
-// around a block's cells fit its shared memory.  PG_CG_COOP=0 keeps the
+// whose cells fit the registers of one block per SM, whose rows (planes) around
+// a block's cells fit its shared memory and cost less than the loop's launches.  PG_CG_COOP=0 keeps the
 // two-kernel loop (a diagnostic switch); so does profiling, which times those
 // kernels one by one.
 int cg_coop_run(pg_grid* g, const CgConfig& cfg, const CgBuffers<double>& buf, int pm, bool* done) {
@@ -392,10 +412,14 @@ int cg_coop_run(pg_grid* g, const CgConfig& cfg, const CgBuffers<double>& buf, i
     int K = 1;
     while (K < kCoopMaxCells && C > (i64)K * kCoopMaxThreads) K *= 2;
     if (C > (i64)K * kCoopMaxThreads) return PG_OK;
-    // (at least a thread per polled block)
-    const int threads = (int)std::min<i64>(kCoopMaxThreads, std::max<i64>(160, ((C + K - 1) / K + 31) / 32 * 32));
     const i64 H = D.nd == 3 ? D.h * D.w : D.w;
     if (H > (i64)1 << 24 || (size_t)(C + 2 * H) * sizeof(double) > (size_t)kCoopSmemMax) return PG_OK;
+    if (!coop_pays(D.nd, C, H)) return PG_OK;
+    // threads: one per polled block, all of the block's cells, an eighth of its
+    // halo (4 x 64 x 64, 8192 halo cells: 160 threads 21.5 us, 512 13.1)
+    auto warps = [](i64 v) { return (v + 31) / 32 * 32; };
+    const int threads =
+        (int)std::min<i64>(kCoopMaxThreads, std::max({(i64)160, warps((C + K - 1) / K), warps((2 * H + 7) / 8)}));
     const size_t smem = (size_t)(C + 2 * H) * sizeof(double);
     CoopArgs a;
     a.x = buf.x;
