@@ -1652,7 +1652,8 @@ struct LearnedHook : ZHook {
     double dt = 1.0;
     const float* ap = nullptr;
     void bind(const void* p) override { ap = (const float*)p; }
-    uintptr_t key() const override { return (uintptr_t)net ^ (uintptr_t)0x9e3779b97f4a7c15ull; }
+    // (the convolutions' path too: each reads weights of its own layout)
+    uintptr_t key() const override { return (uintptr_t)net ^ (uintptr_t)(0x9e3779b97f4a7c14ull | tc_enabled()); }
     int apply(pg_grid* g, const void* rv, void* zv) override {
         const float* r = (const float*)rv;
         float* z = (float*)zv;
