@@ -33,6 +33,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -1192,7 +1193,13 @@ __global__ void k_adam(float* __restrict__ p, float* __restrict__ g, float* __re
 using namespace pg;
 using namespace pg::unet;
 
+static uint64_t next_net_id() {
+    static std::atomic<uint64_t> n{0};
+    return ++n;
+}
+
 struct pg_unet {
+    uint64_t id = next_net_id();  // never given out again
     int device = 0, num_sms = 0;
     int ld[3], lh[3], lw[3];
     i64 lv[3];
@@ -1652,8 +1659,10 @@ struct LearnedHook : ZHook {
     double dt = 1.0;
     const float* ap = nullptr;
     void bind(const void* p) override { ap = (const float*)p; }
-    // (the convolutions' path too: each reads weights of its own layout)
-    uintptr_t key() const override { return (uintptr_t)net ^ (uintptr_t)(0x9e3779b97f4a7c14ull | tc_enabled()); }
+    // The network by a number of its own (another may come to lie at its
+    // address), and the convolutions' path: each reads weights of its own layout.
+    // (The top bit: a multigrid hierarchy's number never has it.)
+    uintptr_t key() const override { return (uintptr_t)1 << 63 | (uintptr_t)net->id << 1 | (uintptr_t)tc_enabled(); }
     int apply(pg_grid* g, const void* rv, void* zv) override {
         const float* r = (const float*)rv;
         float* z = (float*)zv;

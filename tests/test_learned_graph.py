@@ -38,3 +38,22 @@ def test_the_convolution_switch_is_part_of_the_key(host_cuda):  # noqa: F811
         assert rc == 0
         # ten layers for the first application and ten in the loop
         assert (tensor, warp) == ((20, 0) if tc == "1" else (0, 20)), (tc, tensor, warp)
+
+
+REPLACED = PRE + r"""
+result = []
+for _ in range(8):
+    net = network()
+    first = net.value
+    before = fake.fake_captures()
+    solve(net), solve(net)
+    result.append((first, fake.fake_captures() - before))
+    lib.pg_unet_destroy(net)
+"""
+
+
+def test_a_network_at_the_address_of_another_gets_its_own_loop(host_cuda):  # noqa: F811
+    """The loop holds the network's buffers; those of a destroyed one are freed."""
+    rows = host_cuda(REPLACED)
+    assert len({at for at, _ in rows}) < len(rows)  # an address came back
+    assert [n for _, n in rows] == [1] * len(rows), rows
