@@ -5,6 +5,8 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -206,6 +208,60 @@ int cuda_fail(cudaError_t e, const char* what);
     } while (0)
 
 #define PG_CHECK_LAUNCH() PG_CUDA(cudaGetLastError())
+
+// What holds for a kernel on one device (its shared-memory opt-in, the blocks
+// that fit an SM), found out once for each by one thread; a failure is not
+// kept.
+template <class V> class PerDevice {
+    std::mutex m_;
+    std::map<int, V> known_;
+
+public:
+    // find(V*) -> cudaError_t, on the current device
+    template <class F> cudaError_t get(F&& find, V* out) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        std::lock_guard<std::mutex> lk(m_);
+        auto it = known_.find(dev);
+        if (it == known_.end()) {
+            V v{};
+            if ((e = find(&v)) != cudaSuccess) return e;
+            it = known_.emplace(dev, v).first;
+        }
+        *out = it->second;
+        return cudaSuccess;
+    }
+};
+
+// Kernel's opt-in to `smem` bytes of dynamic shared memory.
+template <auto Kernel> inline int opt_in(int smem) {
+    static PerDevice<bool> opted;
+    bool ok;
+    PG_CUDA(opted.get(
+        [&](bool* v) {
+            *v = true;
+            return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        },
+        &ok));
+    return PG_OK;
+}
+
+// A kernel's opt-in to `smem` bytes of dynamic shared memory and the blocks
+// of `threads` that are then resident on an SM; 0 where that fails (callers
+// take another path).
+template <class K> inline int resident_blocks(PerDevice<int>& known, K kernel, int threads, size_t smem) {
+    int n = 0;
+    const cudaError_t e = known.get(
+        [&](int* v) {
+            const cudaError_t a = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(v, kernel, threads, smem);
+        },
+        &n);
+    if (e == cudaSuccess) return n;
+    cudaGetLastError();
+    return 0;
+}
 
 inline int bad_arg(const char* msg) {
     set_error(msg);

@@ -738,19 +738,8 @@ __global__ void __launch_bounds__(kQThreads)
 }
 
 static int restrict_cap(const pg_grid* g) {
-    static int cap = -1;
-    if (cap < 0) {
-        cap = 0;
-        if (cudaFuncSetAttribute(k_mg_restrict3p, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQSmem) ==
-            cudaSuccess) {
-            int bps = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_mg_restrict3p, kQThreads, kQSmem) ==
-                cudaSuccess)
-                cap = std::min(bps * g->num_sms, kMaxBlocks);
-        }
-        cudaGetLastError();
-    }
-    return cap;
+    static PerDevice<int> known;
+    return std::min(resident_blocks(known, k_mg_restrict3p, kQThreads, kQSmem) * g->num_sms, kMaxBlocks);
 }
 
 // Child residual f - A e of cell (z, y, x) of level v, with every neighbour
@@ -2150,11 +2139,7 @@ static TailArgs tail_args(const MgHierarchy& H, int nsmooth) {
 static int launch_tail(pg_grid* g, const MgHierarchy& H, int nsmooth) {
     const TailArgs A = tail_args(H, nsmooth);
     const size_t smem = tail_smem(H);
-    static bool attr = false;
-    if (!attr) {
-        PG_CUDA(cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemMax));
-        attr = true;
-    }
+    if (const int rc = opt_in<k_mg_tail>(kTailSmemMax)) return rc;
     if (smem > (size_t)kTailSmemMax) return bad_arg("PG_PRECOND_MG: multigrid tail does not fit in shared memory");
     PG_LAUNCH(KK_MG_COARSE, g->stream, k_mg_tail<<<1, kTailThreads, smem, g->stream>>>(A, g->ws.state));
     return PG_OK;

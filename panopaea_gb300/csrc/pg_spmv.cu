@@ -453,19 +453,8 @@ bool cached_map(const void* p, int elem, const Dims& D, int bx, int by, CUtensor
 }
 
 template <int PM> static int spmv_cap(int num_sms) {
-    static int cap = -1;
-    if (cap < 0) {
-        cap = 0;
-        if (cudaFuncSetAttribute(k_cg_spmv3p<PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SpmvCfg<PM>::kSmem) ==
-            cudaSuccess) {
-            int bps = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cg_spmv3p<PM>, kSThreads, SpmvCfg<PM>::kSmem) ==
-                cudaSuccess)
-                cap = std::min(bps * num_sms, kMaxBlocks);
-        }
-        cudaGetLastError();
-    }
-    return cap;
+    static PerDevice<int> known;
+    return std::min(resident_blocks(known, k_cg_spmv3p<PM>, kSThreads, SpmvCfg<PM>::kSmem) * num_sms, kMaxBlocks);
 }
 
 }  // namespace
@@ -509,17 +498,8 @@ bool spmv_tma_launch(cudaStream_t s, int num_sms, int pm, const float* zb, float
 bool residual_df_tma_launch(cudaStream_t s, int num_sms, const float* b, const float* xh, const float* xl,
                             const uint8_t* flags, const Dims& D, float dt, float* r, double* partials,
                             unsigned int* counter, double* out, CgState* st) {
-    static int cap = -1;
-    if (cap < 0) {
-        cap = 0;
-        if (cudaFuncSetAttribute(k_residual_df3p, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem) ==
-            cudaSuccess) {
-            int bps = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_residual_df3p, kRThreads, kRSmem) == cudaSuccess)
-                cap = std::min(bps * num_sms, kMaxBlocks);
-        }
-        cudaGetLastError();
-    }
+    static PerDevice<int> known;
+    const int cap = std::min(resident_blocks(known, k_residual_df3p, kRThreads, kRSmem) * num_sms, kMaxBlocks);
     if (cap <= 0 || D.nd != 3 || D.w % 16 != 0 || D.nc() >= ((i64)1 << 31) || ((uintptr_t)r & 7)) return false;
     CUtensorMap hm, lm, bm, gm;
     if (!cached_map(xh, 4, D, kRVw, kRVh, &hm) || !cached_map(xl, 4, D, kRVw, kRVh, &lm) ||

@@ -1268,11 +1268,7 @@ int conv_t(const pg_unet* net, int lvl, const bf16* in, const uint2* w, bf16* ou
     constexpr int MT = COUT <= 32 ? 4 : (COUT <= 64 ? 2 : 1);
     const ConvGeom G = conv_geom(net->ld[lvl], net->lh[lvl], net->lw[lvl], MT);
     const size_t smem = (size_t)G.BX * G.BY * (G.TZ + 2) * kRowBytes;
-    static bool attr_set = false;
-    if (!attr_set) {
-        PG_CUDA(cudaFuncSetAttribute(k_conv<CIN, COUT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-        attr_set = true;
-    }
+    if (const int rc = opt_in<k_conv<CIN, COUT, MT>>(96 * 1024)) return rc;
     if (smem > 96 * 1024) return bad_arg("pg_unet: conv tile does not fit in shared memory");
     const int nb = G.tiles_x * G.tiles_y * ceil_div(G.D, G.TZ);
     PG_LAUNCH(KK_UNET_CONV, net->stream, k_conv<CIN, COUT, MT><<<nb, kConvThreads, smem, net->stream>>>(in, w, out, gate, G, epi));
@@ -1291,22 +1287,21 @@ int conv_tc_z(const pg_unet* net, int lvl, const bf16* in, const bf16* up, const
     struct Shape {
         size_t smem = Cf::kSmem + 256;
         int per_sm = 0;
-        cudaError_t e;
-    };
-    static const Shape shape = [&] {
-        Shape r;
-        const int maxb = 512 / Cf::kCols;
-        if ((r.e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)) ||
-            (r.e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_sm, kernel, tc::kThreads, r.smem)))
-            return r;
-        if (r.per_sm > maxb) {
-            r.smem = std::max(r.smem, (size_t)(228 * 1024 / (maxb + 1) - 1024 + 128));
-            r.e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_sm, kernel, tc::kThreads, r.smem);
-        }
-        if (!r.e && r.per_sm > maxb) r.per_sm = 0;
-        return r;
-    }();
-    PG_CUDA(shape.e);
+    } shape;
+    static PerDevice<Shape> known;
+    PG_CUDA(known.get(
+        [&](Shape* r) {
+            const int maxb = 512 / Cf::kCols;
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r->per_sm, kernel, tc::kThreads, r->smem);
+            if (!e && r->per_sm > maxb) {
+                r->smem = std::max(r->smem, (size_t)(228 * 1024 / (maxb + 1) - 1024 + 128));
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r->per_sm, kernel, tc::kThreads, r->smem);
+            }
+            if (r->per_sm > maxb) r->per_sm = 0;
+            return e;
+        },
+        &shape));
     if (shape.per_sm < 1) return bad_arg("pg_unet: tensor-core conv does not fit an SM");
     tc::Geom G;
     G.D = net->ld[lvl];
@@ -1391,11 +1386,7 @@ int wg_ctas(const pg_unet* net, int k) {
 }
 
 template <int CO> int wgrad_t(pg_unet* net, int k, const bf16* X, const bf16* up, const bf16* dZ) {
-    static bool attr_set = false;
-    if (!attr_set) {
-        PG_CUDA(cudaFuncSetAttribute(k_wgrad<CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * wg_stage(CO)));
-        attr_set = true;
-    }
+    if (const int rc = opt_in<k_wgrad<CO>>(2 * wg_stage(CO))) return rc;
     const int lvl = kLevel[k], S = wg_ctas(net, k);
     WgGeom G;
     G.D = net->ld[lvl];
