@@ -307,30 +307,54 @@ struct PassShape {
     bool along_x;
 };
 
-// Pairs per thread: four share more products (bior 2.2: 11 operations a pair,
-// 14 alone), worth it once the passes are bound by them; one where a block
-// leaves the chip idle and the serial FP64 chain of a thread is what a pass
-// waits for.  Measured, two analysis and two synthesis passes, one pair
-// against four: 256^2 bior 2.4 37 / 43 us, bior 2.2 37 / 34; 1024^2 111 / 117
-// and 76 / 76; 2048^2 385 / 363 and 248 / 226.
-inline int pass_pairs(const PassShape& s, int num_sms) {
-    return s.lines * (s.len / 2) >= (i64)num_sms * 128 * 4 ? 4 : 1;
+// The blocks (256 threads) of a pass with P pairs per thread.
+struct PassGrid {
+    int glog = 2, segs = 0;  // along x: log2 of the lanes per row, segments per row
+    i64 x, y = 1;
+    PassGrid(const PassShape& s, int P) {
+        const i64 groups = (s.len / 2 + P - 1) / P;
+        if (s.along_x) {
+            while (glog < 5 && (1 << glog) < groups) ++glog;
+            segs = (int)((groups + (1 << glog) - 1) >> glog);
+            const int per = 32 >> glog;
+            x = ((s.lines + per - 1) / per * segs + 7) / 8;
+        } else {
+            x = (s.lines + 31) / 32;
+            y = (groups + 7) / 8;
+        }
+    }
+};
+
+// Pairs per thread, four or one.  Four share products (bior 2.2: 11 FP64
+// operations a pair, 14 alone): kFourGain, in percent, is what that gives with
+// every SM busy (4096^2).  Against it stands that blocks of four times the work
+// fill the SMs less evenly -- a pass takes as long as the SM with the most
+// blocks, FP64 units being its bound -- and that a thread's FP64 chain is
+// longer, which shows while an SM has few blocks.  Measured, one / four pairs,
+// two analysis and two synthesis passes, us: 384^2 bior 2.2 15.6 / 23.2; 512^2
+// (one block per SM) haar 11.5 / 13.1, bior 2.2 24.5 / 23.6; 640^2 (two, on a
+// third of the SMs) haar 14.2 / 17.7, bior 2.2 33.2 / 38.5; 1024^2 haar 24.0 /
+// 28.1, bior 2.2 67.6 / 69.1, bior 2.4 104 / 110; 2048^2 haar 73 / 76, bior 2.2
+// 241 / 218, bior 2.4 377 / 357; 4096^2 haar 278 / 273, bior 2.2 938 / 816.
+constexpr int kFourGain[5] = {102, 106, 115, 110, 103};  // by PG_WAVELET_*
+inline int pass_pairs(int wavelet, const PassShape& s, int num_sms) {
+    auto blocks = [&](int pairs) {  // on the SM that gets most
+        const PassGrid g(s, pairs);
+        return (g.x * g.y + num_sms - 1) / num_sms;
+    };
+    const i64 four = blocks(4);
+    return 4 * four * 102 <= blocks(1) * kFourGain[wavelet] && (four >= 4 || kFourGain[wavelet] >= 110) ? 4 : 1;
 }
 
 template <int W, int P> inline void pass_launch(cudaStream_t st, bool down, const double* src, double* dst, const PassShape& s) {
-    const int half = (int)(s.len / 2), groups = (half + P - 1) / P;
+    const PassGrid g(s, P);
+    const dim3 nb((unsigned)g.x, (unsigned)g.y);
     if (s.along_x) {
-        int glog = 2;
-        while (glog < 5 && (1 << glog) < groups) ++glog;
-        const int segs = (groups + (1 << glog) - 1) >> glog, per = 32 >> glog;
-        const i64 items = (s.lines + per - 1) / per * segs;
-        const unsigned nb = (unsigned)((items + 7) / 8);
         if (down)
-            k_wdown_x<W, P><<<nb, 256, 0, st>>>(src, dst, (int)s.lines, (int)s.len, s.stride, glog, segs);
+            k_wdown_x<W, P><<<nb, 256, 0, st>>>(src, dst, (int)s.lines, (int)s.len, s.stride, g.glog, g.segs);
         else
-            k_wup_x<W, P><<<nb, 256, 0, st>>>(src, dst, (int)s.lines, (int)s.len, s.stride, glog, segs);
+            k_wup_x<W, P><<<nb, 256, 0, st>>>(src, dst, (int)s.lines, (int)s.len, s.stride, g.glog, g.segs);
     } else {
-        const dim3 nb((unsigned)((s.lines + 31) / 32), (unsigned)((groups + 7) / 8));
         if (down)
             k_wdown_y<W, P><<<nb, 256, 0, st>>>(src, dst, (int)s.len, (int)s.lines, s.stride);
         else
@@ -344,7 +368,7 @@ inline bool pass_run(cudaStream_t st, int num_sms, int wavelet, bool down, const
     if (wavelet < 0 || wavelet > 4 || s.len < 2 * kFilters[wavelet].n || s.len > most || s.lines > most) return false;
     if (!s.along_x && (s.len / 2 + 7) / 8 > 65535) return false;  // grid.y
     if (s.along_x && s.lines * ((s.len + 7) / 8) > most) return false;
-    const bool four = pass_pairs(s, num_sms) == 4;
+    const bool four = pass_pairs(wavelet, s, num_sms) == 4;
 #define PG_WPASS(W)                                              \
     case W:                                                      \
         if (four)                                                \
