@@ -1546,7 +1546,8 @@ int backward(pg_unet* net) {
     return PG_OK;
 }
 
-constexpr int kHeadBlocks = 608;  // (training: its FP64 sums are the bound, so every SM gets as many)
+// Blocks of the training form: its FP64 sums are the bound, so every SM gets as many.
+int head_blocks(const pg_unet* net) { return 4 * net->num_sms; }
 
 // out = A in on the network's stream (A = dt * the grid's masked Laplacian).
 int apply_a(pg_unet* net, const pg_grid* g, float* out, const float* in, double dt) {
@@ -1562,7 +1563,7 @@ int head(pg_unet* net, const pg_grid* g, double dt, float* p_out, const float* p
     const i64 V0 = net->lv[0];
     const float c2 = 2.0f / (float)V0;
     cudaStream_t s = net->stream;
-    const int nb = (int)std::min<i64>(kHeadBlocks, std::max<i64>(1, (V0 + kHeadThreads - 1) / kHeadThreads));
+    const int nb = (int)std::min<i64>(head_blocks(net), std::max<i64>(1, (V0 + kHeadThreads - 1) / kHeadThreads));
     const int nw = blocks_for(net, V0, kHeadThreads);  // without sums
     const float* wh = net->params + param_offset(kL);
     const float* ae = nullptr;
@@ -1746,7 +1747,7 @@ int pg_unet_create(int64_t d, int64_t h, int64_t w, pg_unet** out) {
     add((void**)&net->r, 4 * V0);
     add((void**)&net->ad, 4 * V0);
     add((void**)&net->scal, 32);
-    add((void**)&net->red, 8 * std::max(kRedBlocks, kHeadBlocks * 17));
+    add((void**)&net->red, 8 * std::max(2 * kRedBlocks, head_blocks(net) * 17));
     add((void**)&net->loss, 8);
     for (int k = 0; k < kL; ++k) add((void**)&net->wpart[k], 4 * (size_t)wg_ctas(net, k) * 27 * kCin[k] * kCout[k]);
     size_t total = 0;

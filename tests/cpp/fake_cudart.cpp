@@ -34,7 +34,7 @@ std::set<std::pair<int, const void*>> opted_in;  // (device, kernel) with more t
 std::vector<Launch> log_;
 std::map<cudaStream_t, Graph*> capturing;
 std::map<void*, size_t> live;
-int device = 0, resident = 2;
+int device = 0, resident = 2, sms = 152;
 long allocations = 0, alloc_fails_at = -1, attr_fails_at = -1, captures = 0;
 thread_local cudaError_t last = cudaSuccess;
 thread_local struct {
@@ -67,6 +67,7 @@ extern "C" {
 
 // What the tests set and read.
 void fake_set_device(int d) { device = d; }
+void fake_set_sms(int n) { sms = n; }
 void fake_set_resident(int n) { resident = n; }                     // blocks per SM, shared memory allowing
 void fake_fail_allocation(long n) { alloc_fails_at = n < 0 ? -1 : allocations + n; }  // the n-th from now on (0: the next)
 void fake_fail_attribute(long n) { attr_fails_at = n; }
@@ -175,7 +176,7 @@ cudaError_t cudaGetDevice(int* d) {
     return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
-    *v = a == cudaDevAttrMultiProcessorCount ? 152 : 0;
+    *v = a == cudaDevAttrMultiProcessorCount ? sms : 0;
     return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize(void) { return cudaSuccess; }

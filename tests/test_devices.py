@@ -71,3 +71,22 @@ for k in range(60):
 def test_a_failed_query_is_not_kept(host_cuda):  # noqa: F811
     for k, rc, same in host_cuda(FAILURES):
         assert not any(rc) and same, (k, rc)
+
+
+HEAD = r"""
+V = (48, 48, 48)
+result = []
+for sms in (152, 100):
+    fake.fake_set_sms(sms)
+    g, net, loss = grid(V), C.c_void_p(), C.c_double()
+    assert lib.pg_unet_create(*V, C.byref(net)) == 0
+    log()
+    rc = lib.pg_unet_accumulate_f32(net, g, cells(V), cells(V), 0.5, C.byref(loss))
+    result.append((sms, rc, [n for k, n, _ in log() if "6k_head" in k]))
+"""
+
+
+def test_the_loss_runs_on_every_sm(host_cuda):  # noqa: F811
+    """The last launch, the one with the FP64 sums, has as many blocks for every SM."""
+    for sms, rc, blocks in host_cuda(HEAD):
+        assert rc == 0 and blocks[-1] == min(4 * sms, 48**3 // 256), (sms, blocks)
