@@ -1205,6 +1205,7 @@ struct pg_unet {
     i64 lv[3];
     cudaStream_t stream = nullptr;
     void* arena = nullptr;
+    void* cat = nullptr;  // C0 and C1: the mma.sync path's
     float* params = nullptr;
     float* grads = nullptr;
     float* adam_m = nullptr;
@@ -1483,6 +1484,12 @@ int forward(pg_unet* net, const pg_grid* g, const float* b, double dt) {
     int rc;
     const bool cat = !tc_enabled();
     if ((rc = prep_weights(net))) return rc;
+    if (cat && !net->cat) {
+        const size_t n0 = 48 * (size_t)net->lv[0], n1 = 96 * (size_t)net->lv[1];
+        PG_CUDA(cudaMalloc(&net->cat, sizeof(bf16) * (n0 + n1)));
+        net->C0 = (bf16*)net->cat;
+        net->C1 = net->C0 + n0;
+    }
     const i64 V0 = net->lv[0];
     cudaStream_t s = net->stream;
     PG_LAUNCH(KK_UNET_MISC, s, k_sumsq<<<kRedBlocks, kRedThreads, 0, s>>>(b, V0, net->red));
@@ -1731,8 +1738,6 @@ int pg_unet_create(int64_t d, int64_t h, int64_t w, pg_unet** out) {
     for (int k = 0; k < kL; ++k) add((void**)&net->Y[k], 2 * (size_t)net->lv[kLevel[k]] * kCout[k]);
     add((void**)&net->P0, 2 * V1 * 16);
     add((void**)&net->P1, 2 * V2 * 32);
-    add((void**)&net->C1, 2 * V1 * 96);
-    add((void**)&net->C0, 2 * V0 * 48);
     add((void**)&net->G0a, 2 * V0 * 16);
     add((void**)&net->G0b, 2 * V0 * 16);
     add((void**)&net->dC0, 2 * V0 * 48);
@@ -1769,6 +1774,7 @@ int pg_unet_create(int64_t d, int64_t h, int64_t w, pg_unet** out) {
 
 int pg_unet_destroy(pg_unet* net) {
     if (!net) return PG_OK;
+    cudaFree(net->cat);
     if (net->arena) cudaFree(net->arena);
     delete net;
     return PG_OK;

@@ -73,6 +73,11 @@ void fake_fail_allocation(long n) { alloc_fails_at = n < 0 ? -1 : allocations + 
 void fake_fail_attribute(long n) { attr_fails_at = n; }
 long fake_allocations(void) { return allocations; }
 long fake_live(void) { return (long)live.size(); }
+long fake_live_bytes(void) {
+    long n = 0;
+    for (auto& a : live) n += (long)a.second;
+    return n;
+}
 long fake_captures(void) { return captures; }
 void fake_log_clear(void) { log_.clear(); }
 int fake_log_size(void) { return (int)log_.size(); }

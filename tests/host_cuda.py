@@ -24,7 +24,7 @@ lib = N.load(build_if_missing=False)
 fake = C.CDLL(%(fake)r)
 for f in ("fake_fail_allocation", "fake_fail_attribute"):
     getattr(fake, f).argtypes = [C.c_long]
-for f in ("fake_allocations", "fake_live", "fake_captures"):
+for f in ("fake_allocations", "fake_live", "fake_live_bytes", "fake_captures"):
     getattr(fake, f).restype = C.c_long
 fake.fake_log_name.restype = C.c_char_p
 

@@ -1,7 +1,8 @@
 """What the host code does with errors and memory, on the CPU with the runtime's
 calls faked (tests/host_cuda.py): a CUDA error that one call has returned is
 not returned again by the next (the runtime keeps it until it is asked for),
-and a destroyed grid leaves no device memory behind."""
+a destroyed grid leaves no device memory behind, and a network has none for
+a path it does not take."""
 import pytest
 
 from host_cuda import host_cuda  # noqa: F401
@@ -57,3 +58,32 @@ for dims in ((64, 80), (32, 32, 32)):
 def test_a_destroyed_grid_leaves_no_memory(host_cuda):  # noqa: F811
     for dims, precond, refine, rc, left in host_cuda(LEAK):
         assert rc == 0 and left == 0, (dims, precond, refine, rc, left)
+
+
+NETWORK = r"""
+V = (32, 32, 32)
+g = grid(V)
+solve_st, loss = N.PcgStats(), C.c_double()
+empty = fake.fake_live_bytes()
+net = C.c_void_p()
+assert lib.pg_unet_create(*V, C.byref(net)) == 0
+created = fake.fake_live_bytes()
+rc, grown = [], []
+for tc in ("1", "0", "0", "1"):
+    os.environ["PG_UNET_TC"] = tc
+    rc.append(lib.pg_unet_accumulate_f32(net, g, cells(V), cells(V), 0.5, C.byref(loss)))
+    rc.append(lib.pg_solve_pressure_learned_f32(g, C.byref(solver(refine=0)), net, cells(V), cells(V), 0.5, C.byref(solve_st)))
+    grown.append(fake.fake_live_bytes() - created)
+lib.pg_unet_destroy(net)
+lib.pg_grid_destroy(g)
+result = [rc, grown, fake.fake_live_bytes()]
+"""
+
+
+def test_the_concatenations_are_allocated_where_they_are_written(host_cuda):  # noqa: F811
+    rc, grown, left = host_cuda(NETWORK)
+    assert not any(rc) and left == 0, (rc, left)
+    solver_only, with_cat = grown[0], grown[1]
+    cells = 32**3
+    assert with_cat - solver_only == 2 * (48 * cells + 96 * cells // 8), grown
+    assert grown[1:] == [with_cat] * 3
