@@ -3,9 +3,9 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
-#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -211,10 +211,11 @@ int cuda_fail(cudaError_t e, const char* what);
 
 // What holds for a kernel on one device (its shared-memory opt-in, the blocks
 // that fit an SM), found out once for each by one thread; a failure is not
-// kept.
+// kept.  Asked at every launch, so what is known is read without a lock.
 template <class V> class PerDevice {
+    static constexpr int kDevices = 64;
     std::mutex m_;
-    std::map<int, V> known_;
+    std::atomic<const V*> known_[kDevices] = {};
 
 public:
     // find(V*) -> cudaError_t, on the current device
@@ -222,14 +223,19 @@ public:
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
-        std::lock_guard<std::mutex> lk(m_);
-        auto it = known_.find(dev);
-        if (it == known_.end()) {
-            V v{};
-            if ((e = find(&v)) != cudaSuccess) return e;
-            it = known_.emplace(dev, v).first;
+        if (dev >= kDevices) return find(out);
+        const V* v = known_[dev].load(std::memory_order_acquire);
+        if (!v) {
+            std::lock_guard<std::mutex> lk(m_);
+            v = known_[dev].load(std::memory_order_relaxed);
+            if (!v) {
+                V found{};
+                if ((e = find(&found)) != cudaSuccess) return e;
+                v = new V(found);  // (kept for the process)
+                known_[dev].store(v, std::memory_order_release);
+            }
         }
-        *out = it->second;
+        *out = *v;
         return cudaSuccess;
     }
 };
