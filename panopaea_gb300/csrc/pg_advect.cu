@@ -403,7 +403,7 @@ __global__ void k_maccormack(T* __restrict__ dst, const T* __restrict__ q, const
 // traced forward (step -ndt) and q traced back leave from the same velocity,
 // and BFECC's last pass reads its values where the limiter reads q's.  The
 // passes one by one (q2 written and read, the velocities averaged and traced
-// again) took 41 + 50 us for MacCormack at 192^3, where it takes 64 now.
+// again) took 41 + 50 us for MacCormack at 192^3, where it takes 61 now.
 template <class T>
 __global__ void k_maccormack_3d(T* __restrict__ dst, const T* __restrict__ q, const T* __restrict__ q1,
                                 const T* __restrict__ vel, Dims D, T ndt, T hix, T hiy, T hiz, FastDiv fw, FastDiv fh) {

@@ -32,7 +32,7 @@ constexpr int kBmgMaxLevels = 16;
 constexpr int kBmgCoarseMax = 2048;
 constexpr int kRtX = 32, kRtY = 8;  // setup tile: 32 x 8 coarse cells
 // Cells (of all its levels together, 20 bytes each) that a block keeps in
-// shared memory, two blocks per SM: 64 x 64 and the levels below it are 5456.
+// shared memory, two blocks per SM: 64 x 64 and the levels below it are 5440.
 constexpr int kBmgTailCells = 5600;
 constexpr int kBmgTailThreads = 512;
 constexpr int kUpdateCells = 2048;  // cells per warp of the CG update

@@ -1177,7 +1177,6 @@ struct CtLevel {
 
 struct CtArgs {
     int lt, ls, nl, nsmooth, ranks;
-    int nd;
     int zero4;          // float4s of shared memory that start as zeros (e and f of every level)
     int toff;           // residual terms of one slab
     int coff, cP;       // the first local level's e around the rank's own planes; one colour of it
@@ -2154,7 +2153,6 @@ static size_t ctail_layout(const MgHierarchy& H, int lt, int ls, int R, CtArgs* 
     A->lt = lt;
     A->ls = ls;
     A->nl = H.nlev;
-    A->nd = H.D0.nd;
     A->dt = (float)H.dt;
     A->ranks = R;
     // planes per rank: doubled from the last distributed level on

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const bf16* __restrict__ 
 // ---------------------------------------------------------------------------
 // The same convolution on the fifth-generation tensor cores: tcgen05.mma
 // (kind::f16, BF16 operands, FP32 accumulators in tensor memory), issued by
-// one thread, operands described in shared memory.
+// the elected lane of a warp of its own, operands described in shared memory.
 //
 // GEMM per tile: M = 128 output voxels (an 8 x 16 x-y tile of one z plane),
 // N = C_out, K = 27 taps x C_in; TZ consecutive z planes per tile, each with
