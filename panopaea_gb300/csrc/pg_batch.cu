@@ -496,8 +496,10 @@ template <int PM> static int b_graph(pg_batch* B, float dt, float* x, int nsmoot
     if (err == cudaSuccess) {
         b_iter<PM>(B, cs, dt, x, nsmooth);
         k_b_cond<<<1, 1, 0, cs>>>(B->active, h);
+        const cudaError_t launched = cudaGetLastError();  // (the body would lack a kernel)
         cudaGraph_t g2 = nullptr;
         err = cudaStreamEndCapture(cs, &g2);
+        if (err == cudaSuccess) err = launched;
     }
     prof_capture_end();
     cudaStreamDestroy(cs);

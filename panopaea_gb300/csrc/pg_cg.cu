@@ -712,7 +712,7 @@ static void update_launch(cudaStream_t s, int nb, T* x, T* r, const T* p0, const
 }
 
 template <class T, int PM>
-static void launch_iter(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook* hook, LoopCond loop = {}) {
+static int launch_iter(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook* hook, LoopCond loop = {}) {
     const Dims& D = g->dims;
     cudaStream_t s = g->stream;
     PG_LAUNCH(KK_CG_SPMV, s,
@@ -742,7 +742,7 @@ static void launch_iter(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook
         PG_LAUNCH(KK_CG_UPDATE, s,
                   launch_dep(n, k_cg_update<T, PM>, nb, kCgThreads, 0, s, buf.x, buf.r, buf.p[0], buf.p[1], buf.ap, g->flags, n,
                              dt, g->ws.state, g->ws.partials, loop));
-    if (PM == PM_ZBUF) hook->apply(g, buf.r, buf.z);
+    return PM == PM_ZBUF ? hook->apply(g, buf.r, buf.z) : PG_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -815,18 +815,24 @@ static int get_graph(pg_grid* g, const CgBuffers<T>& buf, T dt, int nb, ZHook* h
     g->stream = cs;
     const int64_t before = prof_capture_begin();
     cudaError_t err = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    int rc = PG_OK;
     if (err == cudaSuccess) {
-        for (int k = 0; k < kBodyIters<PM>; ++k) launch_iter<T, PM>(g, buf, dt, nb, hook, LoopCond{h, 1});
+        for (int k = 0; k < kBodyIters<PM> && !rc; ++k) rc = launch_iter<T, PM>(g, buf, dt, nb, hook, LoopCond{h, 1});
+        // a launch that failed: the body lacks its kernel (without the update
+        // the loop would not end)
+        const cudaError_t launched = cudaGetLastError();
         cudaGraph_t captured = nullptr;
         err = cudaStreamEndCapture(cs, &captured);
+        if (err == cudaSuccess) err = launched;
     }
     E.body_kernels = (int)(prof_capture_end() - before) / kBodyIters<PM>;
     g->stream = saved;
     cudaStreamDestroy(cs);
-    if (err != cudaSuccess) {
+    if (rc || err != cudaSuccess) {
         cudaGraphDestroy(E.graph);
         E = CgGraph();
-        return cuda_fail(err, "CG graph capture");
+        if (rc) cudaGetLastError();
+        return rc ? rc : cuda_fail(err, "CG graph capture");
     }
     PG_CUDA(cudaGraphInstantiate(&E.exec, E.graph, 0));
     std::copy(key, key + 9, E.key);
@@ -881,7 +887,8 @@ static int run_loop(pg_grid* g, const CgConfig& cfg, const CgBuffers<T>& buf, ZH
     bool done = G != nullptr;
     while (!done && launched < cfg.max_iter) {
         const i64 todo = std::min<i64>(chunk, cfg.max_iter - launched);
-        for (i64 k = 0; k < todo; ++k) launch_iter<T, PM>(g, buf, dt, nb, hook);
+        for (i64 k = 0; k < todo; ++k)
+            if ((rc = launch_iter<T, PM>(g, buf, dt, nb, hook))) return rc;
         PG_CHECK_LAUNCH();
         launched += todo;
         PG_CUDA(cudaMemcpyAsync(ws.state_host + slot, ws.state, sizeof(CgState), cudaMemcpyDeviceToHost, s));

@@ -35,7 +35,7 @@ std::vector<Launch> log_;
 std::map<cudaStream_t, Graph*> capturing;
 std::map<void*, size_t> live;
 int device = 0, resident = 2, sms = 152;
-long allocations = 0, alloc_fails_at = -1, attr_fails_at = -1, captures = 0;
+long allocations = 0, alloc_fails_at = -1, attr_fails_at = -1, launch_fails_at = -1, captures = 0;
 thread_local cudaError_t last = cudaSuccess;
 thread_local struct {
     dim3 grid, block;
@@ -50,6 +50,7 @@ cudaError_t ret(cudaError_t e) {
 cudaError_t note(const void* f, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
     Lock lk(mu);
     if (smem > 48 * 1024 && !opted_in.count({device, f})) return ret(cudaErrorInvalidValue);
+    if (launch_fails_at >= 0 && launch_fails_at-- == 0) return ret(cudaErrorLaunchOutOfResources);
     const Launch l{names[f], grid, block, smem};
     auto c = capturing.find(s);
     (c == capturing.end() ? log_ : c->second->launches).push_back(l);
@@ -71,6 +72,7 @@ void fake_set_sms(int n) { sms = n; }
 void fake_set_resident(int n) { resident = n; }                     // blocks per SM, shared memory allowing
 void fake_fail_allocation(long n) { alloc_fails_at = n < 0 ? -1 : allocations + n; }  // the n-th from now on (0: the next)
 void fake_fail_attribute(long n) { attr_fails_at = n; }
+void fake_fail_launch(long n) { launch_fails_at = n; }  // (a failed one within a capture ends it)
 long fake_allocations(void) { return allocations; }
 long fake_live(void) { return (long)live.size(); }
 long fake_live_bytes(void) {

@@ -22,7 +22,7 @@ sys.modules["panopaea_gb300"] = pkg
 from panopaea_gb300 import _native as N
 lib = N.load(build_if_missing=False)
 fake = C.CDLL(%(fake)r)
-for f in ("fake_fail_allocation", "fake_fail_attribute"):
+for f in ("fake_fail_allocation", "fake_fail_attribute", "fake_fail_launch"):
     getattr(fake, f).argtypes = [C.c_long]
 for f in ("fake_allocations", "fake_live", "fake_live_bytes", "fake_captures"):
     getattr(fake, f).restype = C.c_long
