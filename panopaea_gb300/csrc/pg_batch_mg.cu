@@ -678,7 +678,7 @@ __global__ void k_bmg_rz_finalize(const BLevel* __restrict__ info0, BState* __re
 // host side
 
 static uint64_t next_bmg_id() {
-    static uint64_t n = 0;
+    static std::atomic<uint64_t> n{0};
     return ++n;
 }
 

@@ -104,7 +104,7 @@ struct MgHierarchy {
 };
 
 static uint64_t next_hierarchy_id() {
-    static uint64_t n = 0;
+    static std::atomic<uint64_t> n{0};
     return ++n;
 }
 
